@@ -41,8 +41,8 @@ REFERENCE = os.environ.get("GI_REFERENCE_DIR", "/root/reference")
 
 
 def reference_dir() -> str | None:
-    """The reference checkout, or None where it is absent."""
-    return REFERENCE if os.path.isdir(REFERENCE) else None
+    """The reference checkout, or None where it is absent (or an empty folder)."""
+    return REFERENCE if os.path.isdir(os.path.join(REFERENCE, "Code")) else None
 
 # (source, first line, last line, expected text at first kernel/struct line, output)
 CUTS = [
@@ -74,7 +74,7 @@ HOST_CUTS = [
 
 
 def extract() -> bool:
-    if not os.path.isdir(REFERENCE):
+    if reference_dir() is None:
         return False
     os.makedirs(OUT, exist_ok=True)
     for rel, a, b, expect, out in CUTS + HOST_CUTS:
