@@ -291,6 +291,9 @@ struct gi_ctx {
     int diag_blocks1 = 0, diag_blocks2 = 0;
     double *pot_buf = nullptr;
     size_t pot_cap = 0;
+    void *work = nullptr;     // workspace of the synchronous calls (gi_internal_ctx_workspace)
+    void *work_pinned = nullptr;
+    size_t work_cap = 0;
     int occ[4][9];  // resident one-sided force CTAs per SM: [accum][i-bodies per thread]
 };
 
@@ -348,6 +351,8 @@ static void ctx_free(gi_ctx *c)
     cudaFree(c->diag_work);
     cudaFreeHost(c->diag_host);
     cudaFree(c->pot_buf);
+    cudaFree(c->work);
+    cudaFreeHost(c->work_pinned);
 }
 
 extern "C" int gi_ctx_create(gi_ctx **out, int device)
@@ -1592,6 +1597,23 @@ extern "C" int gi_graph_destroy(gi_graph *gr)
 int gi_internal_fail(int status, const char *msg) { return fail(status, "%s", msg); }
 
 int gi_internal_ctx_device(gi_ctx *c) { return c ? c->device : -1; }
+
+int gi_internal_ctx_workspace(gi_ctx *c, size_t bytes, void **dev, void **pinned)
+{
+    DeviceGuard g(c->device);
+    if (!c->work_pinned)
+        GI_CUDA(cudaMallocHost(&c->work_pinned, kPinnedBytes), "cudaMallocHost workspace");
+    if (bytes > c->work_cap) {
+        cudaFree(c->work);
+        c->work = nullptr;
+        c->work_cap = 0;
+        GI_CUDA(cudaMalloc(&c->work, bytes), "cudaMalloc workspace");
+        c->work_cap = bytes;
+    }
+    *dev = c->work;
+    *pinned = c->work_pinned;
+    return GI_OK;
+}
 
 int gi_internal_ctx_cluster_tries(gi_ctx *c)
 {

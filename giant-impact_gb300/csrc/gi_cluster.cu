@@ -7,26 +7,37 @@
 // started it, which is its smallest index.  Those groups are exactly the
 // connected components of the "touching" graph, so here:
 //
-//   1. grid: cell = touch * (1 + 2^-10), computed in double, so two touching
-//      bodies are always in the same or adjacent cells; cells hashed into
-//      M = 2^k >= 2N buckets, counting sort (as the contact pass does);
-//   2. union: one thread per body i visits the 27 neighbour buckets and, for
-//      every j > i that touches i (the reference's FP32 test, evaluated with
-//      the same roundings), links the two trees.  Links always hang the root
-//      with the larger index under the one with the smaller index (one
-//      atomicCAS on a root), so a tree's root is its smallest member: the
-//      reference's group number;
+//   1. cells: cubes of side touch (1 - 2^-10) / sqrt(3), so the bodies of one
+//      cell all touch each other; each occupied cell takes a slot of an
+//      open-addressing table (exact cell coordinates, never shared by two
+//      cells) and its bodies are listed together;
+//   2. union: a body starts under its cell's smallest index, so a cell costs
+//      one tree and no pair tests.  Touching bodies lie at most two cells
+//      apart on an axis: one warp per cell looks up the neighbour cells, skips
+//      those already in its tree and tests body pairs (the reference's FP32
+//      test, evaluated with the same roundings) until one touches, which
+//      links the two trees.  The 13 forward adjacent cells come first, the 49
+//      further ones in a second launch, when most are in the same tree.  Links
+//      always hang the root with the larger index under the one with the
+//      smaller index (one atomicCAS on a root), so a tree's root is its
+//      smallest member: the reference's group number;
 //   3. flatten: group[i] = root of i (found without writes, so that no
-//      thread overwrites a final root); sizes by atomicAdd;
+//      thread overwrites a final root); sizes by atomicAdd, one per warp and
+//      group;
 //   4. pick: Earth = largest group, smallest name on a tie (the reference's
 //      first strict maximum); Moon = largest of the others; both by a 64-bit
 //      atomicMax of (size << 32 | ~name);
 //   5. tag: scope byte (1 Earth, 2 Moon) and the origin counts.
+// What bounds it is latency: a handful of short launches over data in L2.
+// A remnant's cells hold hundreds of bodies, each within touch of tens of
+// thousands: testing every pair, one thread per body, took 52 ms for 66,000
+// such bodies (55.0 ms for the whole end-of-impact analysis, now 0.55 ms).
 // Every loop is bounded: a failed link moves to a strictly smaller index, so
 // a link takes at most N tries; the kernels still stop after a set number
 // (gi_options.cluster_tries, 2^22 by default) and raise an error flag that
 // the host turns into GI_ERR_TIMEOUT.
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
@@ -35,15 +46,20 @@
 
 namespace gi {
 
-__device__ __forceinline__ int cluster_cell(float x, double inv_cell)
+// Cell coordinate along one axis.  Two bodies of one cell differ by at most
+// a cell side (up to 2^-23 of it: the double product errs by 2^-53 of at most
+// 1e9), so their FP32 distance is below touch.  Coordinates beyond 1e9 cells
+// and NaN have no cell: such bodies are "loose" and tested one by one.
+__device__ __forceinline__ bool cluster_cell(float4 p, double inv_cell, int3 &c)
 {
-    double f = floor((double)x * inv_cell);
-    if (!(f >= -1.0e9)) f = -1.0e9;  // also NaN
-    if (f > 1.0e9) f = 1.0e9;
-    return (int)f;
+    const double x = floor((double)p.x * inv_cell), y = floor((double)p.y * inv_cell),
+                 z = floor((double)p.z * inv_cell);
+    if (!(fabs(x) < 1.0e9 && fabs(y) < 1.0e9 && fabs(z) < 1.0e9)) return false;
+    c = make_int3((int)x, (int)y, (int)z);
+    return true;
 }
 
-__device__ __forceinline__ unsigned int cluster_bucket(int cx, int cy, int cz, unsigned int mask)
+__device__ __forceinline__ unsigned int cluster_hash(int cx, int cy, int cz, unsigned int mask)
 {
     unsigned int h = (unsigned int)cx * 2246822519u;
     h ^= (unsigned int)cy * 3266489917u;
@@ -54,28 +70,105 @@ __device__ __forceinline__ unsigned int cluster_bucket(int cx, int cy, int cz, u
     return h & mask;
 }
 
+// One slot of the cell table.  All words start at ~0.
+struct CellTable {
+    int *rep;              // a body of the cell, -1 = free
+    unsigned int *leader;  // the cell's smallest body index
+    unsigned int *count;   // bodies - 1; then the next place of its list
+    int4 *cell;            // coordinates and cell number
+};
+
+// Occupied cell k: first place in the list, bodies, slot, smallest body.
+struct CellInfo {
+    unsigned int beg, cnt;
+    int slot, leader;
+};
+
+// Counters of a call, zero at its start.
+struct ClusterCounters {
+    unsigned int cells, loose, placed;
+};
+
+// Every body to its cell's slot (linear probing; the table has at least two
+// slots per body).
 __global__ void __launch_bounds__(256)
-cluster_keys(const float4 *__restrict__ pos, int n, double inv_cell, unsigned int mask,
-             unsigned int *__restrict__ keys, unsigned int *__restrict__ hist,
-             int *__restrict__ parent)
+cluster_insert(const float4 *__restrict__ pos, int n, double inv_cell, unsigned int mask,
+               CellTable tab, CellInfo *__restrict__ info, int *__restrict__ slot_of,
+               int *__restrict__ loose, ClusterCounters *ctr)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 p = pos[i];
-        const unsigned int b = cluster_bucket(cluster_cell(p.x, inv_cell), cluster_cell(p.y, inv_cell),
-                                              cluster_cell(p.z, inv_cell), mask);
-        keys[i] = b;
-        parent[i] = i;
-        atomicAdd(&hist[b], 1u);
+        int3 c;
+        if (!cluster_cell(pos[i], inv_cell, c)) {
+            slot_of[i] = -1;
+            loose[atomicAdd(&ctr->loose, 1u)] = i;
+            continue;
+        }
+        unsigned int s = cluster_hash(c.x, c.y, c.z, mask);
+        for (unsigned int t = 0; t <= mask; ++t, s = (s + 1u) & mask) {
+            int cur = __ldcg(&tab.rep[s]);
+            if (cur < 0) {
+                cur = atomicCAS(&tab.rep[s], -1, i);
+                if (cur < 0) {
+                    const unsigned int k = atomicAdd(&ctr->cells, 1u);
+                    tab.cell[s] = make_int4(c.x, c.y, c.z, (int)k);
+                    info[k].slot = (int)s;
+                    break;
+                }
+            }
+            int3 d = c;
+            cluster_cell(pos[cur], inv_cell, d);  // rep bodies have a cell
+            if (d.x == c.x && d.y == c.y && d.z == c.z) break;
+        }
+        slot_of[i] = (int)s;
+        atomicMin(&tab.leader[s], (unsigned int)i);
+        atomicAdd(&tab.count[s], 1u);
     }
 }
 
+// A range of the body list for every occupied cell, in any order.
 __global__ void __launch_bounds__(256)
-cluster_scatter(int n, const unsigned int *__restrict__ keys, unsigned int *__restrict__ cursor,
-                int *__restrict__ sorted)
+cluster_ranges(CellTable tab, CellInfo *__restrict__ info, ClusterCounters *ctr)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned int cells = ctr->cells;
+    const unsigned int stride = gridDim.x * blockDim.x;
+    for (unsigned int k0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; k0 < cells; k0 += stride) {
+        const unsigned int k = k0 + lane;
+        int s = 0;
+        unsigned int cnt = 0;
+        if (k < cells) {
+            s = info[k].slot;
+            cnt = tab.count[s] + 1u;
+        }
+        unsigned int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        unsigned int base = 0;
+        if (lane == 31) base = atomicAdd(&ctr->placed, incl);
+        base = __shfl_sync(0xffffffffu, base, 31);
+        if (k < cells) {
+            info[k].beg = base + incl - cnt;
+            info[k].cnt = cnt;
+            info[k].leader = (int)tab.leader[s];
+            tab.count[s] = base + incl - cnt;
+        }
+    }
+}
+
+// The bodies listed cell by cell, each under its cell's smallest index.
+__global__ void __launch_bounds__(256)
+cluster_scatter(const float4 *__restrict__ pos, int n, CellTable tab,
+                const int *__restrict__ slot_of, float4 *__restrict__ list,
+                int *__restrict__ parent)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const unsigned int slot = atomicAdd(&cursor[keys[i]], 1u);
-        sorted[slot] = i;
+        const int s = slot_of[i];
+        parent[i] = s < 0 ? i : (int)tab.leader[s];
+        if (s < 0) continue;
+        list[atomicAdd(&tab.count[s], 1u)] = pos[i];
     }
 }
 
@@ -128,47 +221,160 @@ __device__ __forceinline__ bool touching(float4 a, float4 b, float touch)
     return __fsqrt_rn(r2) < touch;
 }
 
-__global__ void __launch_bounds__(256)
-cluster_union(const float4 *__restrict__ pos, int n, const unsigned int *__restrict__ cursor,
-              const int *__restrict__ sorted, unsigned int mask, double inv_cell, float touch,
-              int tries, int *parent, int *__restrict__ err)
+// touching() of the closest points of two boxes, in its roundings: each axis
+// difference, square, sum and root is monotone, so a false result proves that
+// no pair of their bodies touches.
+__device__ __forceinline__ bool boxes_touch(float3 alo, float3 ahi, float3 blo, float3 bhi,
+                                            float touch)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 pi = pos[i];
-    const int cx = cluster_cell(pi.x, inv_cell), cy = cluster_cell(pi.y, inv_cell),
-              cz = cluster_cell(pi.z, inv_cell);
-    unsigned int seen[27];
-    int nseen = 0;
-    for (int o = 0; o < 27; ++o) {
-        const unsigned int b =
-            cluster_bucket(cx + o % 3 - 1, cy + (o / 3) % 3 - 1, cz + o / 9 - 1, mask);
-        bool dup = false;
-        for (int q = 0; q < nseen; ++q) dup |= seen[q] == b;
-        if (dup) continue;
-        seen[nseen++] = b;
-        const unsigned int beg = b ? cursor[b - 1] : 0u, end = cursor[b];
-        for (unsigned int s = beg; s < end; ++s) {
-            const int j = sorted[s];
-            if (j <= i) continue;
-            if (!touching(pi, pos[j], touch)) continue;
-            if (!link(parent, i, j, tries)) atomicExch(err, 1);
+    const float gx = fmaxf(fmaxf(__fsub_rn(blo.x, ahi.x), __fsub_rn(alo.x, bhi.x)), 0.0f);
+    const float gy = fmaxf(fmaxf(__fsub_rn(blo.y, ahi.y), __fsub_rn(alo.y, bhi.y)), 0.0f);
+    const float gz = fmaxf(fmaxf(__fsub_rn(blo.z, ahi.z), __fsub_rn(alo.z, bhi.z)), 0.0f);
+    return touching(make_float4(gx, gy, gz, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f), touch);
+}
+
+// Whether any body of cell a touches one of cell b, by one warp: 32 bodies of
+// a at a time, one per lane, against b's in turn; lanes whose body cannot
+// reach b's box sit out.
+__device__ __forceinline__ bool cells_touch_warp(const float4 *__restrict__ list, CellInfo a,
+                                                 CellInfo b, float touch, int lane)
+{
+    const float kInf = __int_as_float(0x7f800000);
+    float3 lo = make_float3(kInf, kInf, kInf), hi = make_float3(-kInf, -kInf, -kInf);
+    for (unsigned int u = lane; u < b.cnt; u += 32) {
+        const float4 q = list[b.beg + u];
+        lo = make_float3(fminf(lo.x, q.x), fminf(lo.y, q.y), fminf(lo.z, q.z));
+        hi = make_float3(fmaxf(hi.x, q.x), fmaxf(hi.y, q.y), fmaxf(hi.z, q.z));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
+        lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
+        lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
+        hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
+        hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
+        hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
+    }
+    for (unsigned int u = 0; u < a.cnt; u += 32) {
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+        bool in = u + lane < a.cnt;
+        if (in) {
+            p = list[a.beg + u + lane];
+            const float3 q = make_float3(p.x, p.y, p.z);
+            in = boxes_touch(q, q, lo, hi, touch);
+        }
+        if (!__any_sync(0xffffffffu, in)) continue;
+        for (unsigned int v = 0; v < b.cnt; v += 4) {
+            bool hit = false;
+#pragma unroll
+            for (unsigned int w = 0; w < 4; ++w)  // the last body again past the end
+                hit |= touching(p, list[b.beg + min(v + w, b.cnt - 1u)], touch);
+            if (__any_sync(0xffffffffu, hit && in)) return true;
+        }
+    }
+    return false;
+}
+
+// Pair tests a lane makes by itself; larger cell pairs go to the whole warp.
+constexpr unsigned int kLanePairs = 64;
+
+// One warp per occupied cell.  FAR = false: its 13 forward neighbours that
+// share a face, edge or corner; FAR = true: the 49 forward cells beyond them,
+// two a lane.
+template <bool FAR>
+__global__ void __launch_bounds__(128)
+cluster_link(const float4 *__restrict__ list, CellTable tab, const CellInfo *__restrict__ info,
+             unsigned int mask, float touch, int tries, int *parent,
+             const ClusterCounters *__restrict__ ctr, int *__restrict__ err)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned int cells = ctr->cells, nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (unsigned int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < cells; k += nwarps) {
+        const CellInfo a = info[k];
+        const int4 c = tab.cell[a.slot];
+        for (int round = 0; round < (FAR ? 2 : 1); ++round) {
+            // forward half of the 3^3 or 5^3 block around the cell
+            constexpr int kSide = FAR ? 5 : 3, kHalf = kSide / 2;
+            const int o = kSide * kSide * kSide / 2 + 1 + round * 32 + lane;
+            const int ox = o % kSide - kHalf, oy = o / kSide % kSide - kHalf,
+                      oz = o / (kSide * kSide) - kHalf;
+            bool look = o < kSide * kSide * kSide;
+            if (FAR) look = look && (abs(ox) == 2 || abs(oy) == 2 || abs(oz) == 2);
+            CellInfo b{0u, 0u, 0, 0};
+            if (look) {
+                unsigned int s = cluster_hash(c.x + ox, c.y + oy, c.z + oz, mask);
+                for (unsigned int t = 0; t <= mask; ++t, s = (s + 1u) & mask) {
+                    if (__ldg(&tab.rep[s]) < 0) break;
+                    const int4 d = __ldg(&tab.cell[s]);
+                    if (d.x == c.x + ox && d.y == c.y + oy && d.z == c.z + oz) {
+                        b = info[d.w];
+                        break;
+                    }
+                }
+            }
+            bool open = b.cnt > 0u && find_root(parent, a.leader) != find_root(parent, b.leader);
+            bool hit = false;
+            if (open && (unsigned long long)a.cnt * b.cnt <= kLanePairs) {
+                for (unsigned int u = 0; u < a.cnt && !hit; ++u) {
+                    const float4 p = list[a.beg + u];
+                    for (unsigned int v = 0; v < b.cnt && !hit; ++v)
+                        hit = touching(p, list[b.beg + v], touch);
+                }
+                open = false;
+            }
+            for (unsigned int todo = __ballot_sync(0xffffffffu, open); todo; todo &= todo - 1u) {
+                const int src = __ffs(todo) - 1;
+                CellInfo q;
+                q.beg = __shfl_sync(0xffffffffu, b.beg, src);
+                q.cnt = __shfl_sync(0xffffffffu, b.cnt, src);
+                const bool swap = a.cnt < q.cnt;  // the larger cell's bodies on the lanes
+                const bool any = cells_touch_warp(list, swap ? q : a, swap ? a : q, touch, lane);
+                if (lane == src) hit = any;
+            }
+            // the lanes link together: their attempts on one root collide and
+            // are tried again on the root that won
+            if (hit && !link(parent, a.leader, b.leader, tries)) atomicExch(err, 1);
         }
     }
 }
 
+// Bodies without a cell (beyond 1e9 cells, or not finite): one warp each
+// against every body.
+__global__ void __launch_bounds__(128)
+cluster_link_loose(const float4 *__restrict__ pos, int n, const int *__restrict__ loose,
+                   float touch, int tries, int *parent, const ClusterCounters *__restrict__ ctr,
+                   int *__restrict__ err)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned int total = ctr->loose, nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (unsigned int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < total; w += nwarps) {
+        const int i = loose[w];
+        const float4 p = pos[i];
+        for (int j = lane; j < n; j += 32)
+            if (j != i && touching(p, pos[j], touch) && !link(parent, i, j, tries))
+                atomicExch(err, 1);
+    }
+}
+
+// sizes start at -1 (the ~0 fill); one atomic per warp and group.
 __global__ void __launch_bounds__(256)
 cluster_flatten(int *parent, int n, int *__restrict__ size, int *__restrict__ ngroups)
 {
+    const int lane = threadIdx.x & 31;
     int roots = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int r = find_root_ro(parent, i);
-        __stcg(&parent[i], r);
-        atomicAdd(&size[r], 1);
-        roots += r == i;
+    for (int i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; i0 < n; i0 += gridDim.x * blockDim.x) {
+        const int i = i0 + lane;
+        int r = -1;
+        if (i < n) {
+            r = find_root_ro(parent, i);
+            __stcg(&parent[i], r);
+            roots += r == i;
+        }
+        const unsigned int same = __match_any_sync(0xffffffffu, r);
+        if (r >= 0 && lane == __ffs(same) - 1) atomicAdd(&size[r], __popc(same));
     }
     for (int o = 16; o > 0; o >>= 1) roots += __shfl_down_sync(0xffffffffu, roots, o);
-    if ((threadIdx.x & 31) == 0 && roots) atomicAdd(ngroups, roots);
+    if (lane == 0 && roots) atomicAdd(ngroups, roots);
 }
 
 __device__ __forceinline__ unsigned long long group_key(int size, int name)
@@ -189,7 +395,7 @@ cluster_pick(const int *__restrict__ group, const int *__restrict__ size, int n,
     const int skip = exclude_key ? key_name(*exclude_key) : -1;
     unsigned long long k = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        if (group[i] == i && i != skip) k = max(k, group_key(size[i], i));
+        if (group[i] == i && i != skip) k = max(k, group_key(size[i] + 1, i));
     for (int o = 16; o > 0; o >>= 1) k = max(k, __shfl_down_sync(0xffffffffu, k, o));
     if ((threadIdx.x & 31) == 0 && k) atomicMax(best, k);
 }
@@ -227,6 +433,8 @@ struct ClusterResult {
     int counts[8];
     int ngroups;
     int err;
+    gi::ClusterCounters ctr;
+    int pad;
 };
 
 int cuda_status(cudaError_t e, const char *what)
@@ -266,38 +474,48 @@ extern "C" int gi_find_earth_moon(gi_ctx *ctx, const float *pos, int n, float to
     unsigned int m = 1024;
     while (m < 2u * (unsigned int)n && m < (1u << 30)) m <<= 1;
     if (m > 1024u * 8192u) return gi_internal_fail(GI_ERR_BAD_SIZE, "gi_find_earth_moon: n too large");
-    // one allocation: parent, size, keys, sorted (n each), cursor (m),
-    // scan sums (8192), result
-    const size_t words = 4 * (size_t)n + m + 8192;
-    const size_t bytes = words * 4 + sizeof(ClusterResult) + 16;
-    unsigned char *buf = nullptr;
-    cudaError_t e = cudaMallocAsync(&buf, bytes, s);
-    if (e != cudaSuccess) return cuda_status(e, "cudaMallocAsync");
-    int *parent = reinterpret_cast<int *>(buf);
-    int *size = parent + n;
-    unsigned int *keys = reinterpret_cast<unsigned int *>(size + n);
-    int *sorted = reinterpret_cast<int *>(keys + n);
-    unsigned int *cursor = reinterpret_cast<unsigned int *>(sorted + n);
-    unsigned int *sums = cursor + m;
-    size_t roff = (words * 4 + 15) & ~(size_t)15;
-    ClusterResult *res = reinterpret_cast<ClusterResult *>(buf + roff);
-    ClusterResult host{};
-    const double inv_cell = 1.0 / ((double)touch * (1.0 + 1.0 / 1024.0));
-    const int blocks = (n + 255) / 256;
-    const int gridded = std::min(blocks, 4096);
+    // One block of the context's workspace: the result, the cell
+    // coordinates, the body list and the cell list (16-byte words), then the
+    // words that start at ~0 (rep, leader, count, size), then the rest.
+    const size_t M = m, N = (size_t)n;
+    const size_t head = (sizeof(ClusterResult) + 15) & ~(size_t)15;
+    const size_t bytes = head + 16 * (M + 2 * N) + 4 * (3 * M + N) + 4 * 3 * N;
+    void *work = nullptr, *pinned = nullptr;
+    if (int st = gi_internal_ctx_workspace(ctx, bytes, &work, &pinned)) return st;
+    unsigned char *buf = static_cast<unsigned char *>(work);
+    ClusterResult *res = reinterpret_cast<ClusterResult *>(buf);
+    gi::CellTable tab;
+    tab.cell = reinterpret_cast<int4 *>(buf + head);
+    float4 *list = reinterpret_cast<float4 *>(tab.cell + M);
+    gi::CellInfo *info = reinterpret_cast<gi::CellInfo *>(list + N);
+    tab.rep = reinterpret_cast<int *>(info + N);
+    tab.leader = reinterpret_cast<unsigned int *>(tab.rep + M);
+    tab.count = tab.leader + M;
+    int *size = reinterpret_cast<int *>(tab.count + M);
+    int *parent = size + N, *slot_of = parent + N, *loose = slot_of + N;
+    ClusterResult &host = *static_cast<ClusterResult *>(pinned);
+    // Where the squares of the touch test leave FP32's normal range, cells
+    // would not decide as the test does: no body gets one then.
+    const bool plain = touch > 1.0e-17f && touch < 1.0e18f;
+    const double inv_cell = plain ? std::sqrt(3.0) / ((double)touch * (1.0 - 1.0 / 1024.0)) : HUGE_VAL;
+    const float4 *P = reinterpret_cast<const float4 *>(pos);
+    const int tries = gi_internal_ctx_cluster_tries(ctx);
+    const int gridded = std::min((n + 255) / 256, 4096);
+    const int warps = std::min((n + 3) / 4, 16384);  // blocks of four warps, one cell each
+    cudaError_t e;
     do {
-        if ((e = cudaMemsetAsync(size, 0, (size_t)n * 4, s)) != cudaSuccess) break;
-        if ((e = cudaMemsetAsync(cursor, 0, (size_t)m * 4, s)) != cudaSuccess) break;
         if ((e = cudaMemsetAsync(res, 0, sizeof(ClusterResult), s)) != cudaSuccess) break;
-        gi::cluster_keys<<<gridded, 256, 0, s>>>(reinterpret_cast<const float4 *>(pos), n, inv_cell,
-                                                 m - 1, keys, cursor, parent);
-        if ((e = gi_bucket_scan(cursor, m, sums, s)) != cudaSuccess) break;
-        gi::cluster_scatter<<<gridded, 256, 0, s>>>(n, keys, cursor, sorted);
-        // cursor[b] is now the end of bucket b
-        gi::cluster_union<<<blocks, 256, 0, s>>>(reinterpret_cast<const float4 *>(pos), n, cursor,
-                                                 sorted, m - 1, inv_cell, touch,
-                                                 gi_internal_ctx_cluster_tries(ctx), parent,
-                                                 &res->err);
+        if ((e = cudaMemsetAsync(tab.rep, 0xff, 4 * (3 * M + N), s)) != cudaSuccess) break;
+        gi::cluster_insert<<<gridded, 256, 0, s>>>(P, n, inv_cell, m - 1, tab, info, slot_of, loose,
+                                                   &res->ctr);
+        gi::cluster_ranges<<<gridded, 256, 0, s>>>(tab, info, &res->ctr);
+        gi::cluster_scatter<<<gridded, 256, 0, s>>>(P, n, tab, slot_of, list, parent);
+        gi::cluster_link<false><<<warps, 128, 0, s>>>(list, tab, info, m - 1, touch, tries, parent,
+                                                      &res->ctr, &res->err);
+        gi::cluster_link<true><<<warps, 128, 0, s>>>(list, tab, info, m - 1, touch, tries, parent,
+                                                     &res->ctr, &res->err);
+        gi::cluster_link_loose<<<std::min(warps, 1024), 128, 0, s>>>(P, n, loose, touch, tries, parent,
+                                                                     &res->ctr, &res->err);
         gi::cluster_flatten<<<gridded, 256, 0, s>>>(parent, n, size, &res->ngroups);
         gi::cluster_pick<<<gridded, 256, 0, s>>>(parent, size, n, nullptr, &res->keys[0]);
         gi::cluster_pick<<<gridded, 256, 0, s>>>(parent, size, n, &res->keys[0], &res->keys[1]);
@@ -307,9 +525,8 @@ extern "C" int gi_find_earth_moon(gi_ctx *ctx, const float *pos, int n, float to
         if ((e = cudaMemcpyAsync(&host, res, sizeof host, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
             break;
     } while (false);
-    const cudaError_t ef = cudaFreeAsync(buf, s);
-    if (e == cudaSuccess) e = ef;
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    const cudaError_t es = cudaStreamSynchronize(s);  // the workspace is idle again
+    if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) return cuda_status(e, "gi_find_earth_moon");
     if (host.err) return gi_internal_fail(GI_ERR_TIMEOUT, "gi_find_earth_moon: a link did not settle");
     auto name = [](unsigned long long k) { return k ? (int)(~(unsigned int)(k & 0xffffffffull)) : -1; };
@@ -414,10 +631,11 @@ extern "C" int gi_find_disk(gi_ctx *ctx, const float *pos, const float *vel, con
         int counts[3];
         int pad;
     };
-    Res *res = nullptr;
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&res), sizeof(Res), s);
-    if (e != cudaSuccess) return cuda_status(e, "cudaMallocAsync");
-    Res host{};
+    void *work = nullptr, *pinned = nullptr;
+    if (int st = gi_internal_ctx_workspace(ctx, sizeof(Res), &work, &pinned)) return st;
+    Res *res = static_cast<Res *>(work);
+    Res &host = *static_cast<Res *>(pinned);
+    cudaError_t e;
     const int blocks = std::min((run->n + 255) / 256, 4096);
     const float4 *P = reinterpret_cast<const float4 *>(pos);
     do {
@@ -432,9 +650,8 @@ extern "C" int gi_find_disk(gi_ctx *ctx, const float *pos, const float *vel, con
         if ((e = cudaMemcpyAsync(&host, res, sizeof host, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
             break;
     } while (false);
-    const cudaError_t ef = cudaFreeAsync(res, s);
-    if (e == cudaSuccess) e = ef;
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    const cudaError_t es = cudaStreamSynchronize(s);  // the workspace is idle again
+    if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) return cuda_status(e, "gi_find_disk");
     double r = 0.0;
     std::memcpy(&r, &host.rmax, sizeof r);

@@ -210,8 +210,11 @@ long long gi_internal_pair_run(RunDev &d, int n, int pcl, const PairDev &p, long
 int gi_internal_pair_default_pcl(int n);
 // Device ordinal of a context (-1 for NULL).
 int gi_internal_ctx_device(gi_ctx *ctx);
+// The context's workspace of at least `bytes` device bytes (16-byte aligned)
+// and a pinned page of kPinnedBytes, for calls that wait for the GPU before
+// they return: it is idle between calls, whatever stream they run on.  Kept
+// until the context is destroyed; grown, never shared between contexts.
+constexpr size_t kPinnedBytes = 4096;
+int gi_internal_ctx_workspace(gi_ctx *ctx, size_t bytes, void **dev, void **pinned);
 // Attempts one union-find link of gi_find_earth_moon may make (gi_options).
 int gi_internal_ctx_cluster_tries(gi_ctx *ctx);
-// gi_grid.cu: exclusive scan of m <= 1024 * 8192 counters in place; sums
-// holds 8192 words of scratch.
-cudaError_t gi_bucket_scan(unsigned int *a, unsigned int m, unsigned int *sums, cudaStream_t s);

@@ -74,6 +74,32 @@ def test_groups_repeat_on_percolating_gas(gi, orc, torch_cuda):
     ctx.close()
 
 
+@pytest.mark.parametrize("touch", [1.5, 0.3, 40.0, 1e-18, 1e19])
+def test_groups_by_cells_match_reference_loop(gi, orc, torch_cuda, touch):
+    """What the cells of the grouping must not change: crowded cells whose
+    bodies touch across a corner or just miss, clumps two cells apart, bodies
+    beyond the cells' range (some on one spot) and not finite, and touch
+    distances whose square leaves FP32's normal range."""
+    rng = np.random.default_rng(11)
+    parts = [_gas(12, 300, 14.0)[:, :3] - 7.0]
+    for k, (m, gap) in enumerate([(150, 1.49), (150, 1.52), (40, 1.4999), (90, 2.9)]):
+        at = np.array([40.0 * (k + 1), -3.0, 0.9])
+        step = np.array([1.0, 1.0, 1.0]) / np.sqrt(3.0) * gap
+        for c in (at, at + step):
+            parts.append(c + rng.uniform(-0.004, 0.004, size=(m, 3)))
+    far = rng.choice([1.0e9, 2.5e9, -3.0e12], size=(40, 3))
+    odd = np.array([[np.nan, 0, 0], [np.inf, 1, 1], [-np.inf, 1, 1], [np.inf, 1, 1], [0.1, 0.2, np.nan]])
+    p = np.concatenate(parts + [far, odd])
+    pos = np.zeros((len(p), 4), np.float32)
+    pos[:, :3] = p[rng.permutation(len(p))]
+    n = len(pos)
+    bounds = [n // 5, 2 * n // 5, 3 * n // 5]
+    ctx = gi.Context(0)
+    em, g, sc = _groups(gi, torch_cuda, ctx, pos, bounds, touch)
+    _check_against(em, g, sc, orc.groups_ref(pos, touch), orc, bounds)
+    ctx.close()
+
+
 def _gas(seed, n, box):
     rng = np.random.default_rng(seed)
     pos = np.zeros((n, 4), np.float32)
