@@ -255,17 +255,12 @@ struct StreamScratch {
     long long *delta = nullptr;         // contact corrections, 3 per body
     size_t delta_cap = 0;               // bodies
     double *fsum = nullptr;  // far-field sums, 3 per body: FP64 (one-sided GI_EPI_SUM launches)
-                             // or int64 fixed point (paired far field)
+                             // or int64 fixed point (paired far field); behind them the
+                             // contact pass's counters (kCtrWords), cleared with them
     // The contact pass runs on `aux`, beside the far field on the caller's
     // stream: forked after the previous step, joined before the epilogue.
     cudaStream_t aux = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    // Paired far field, side-by-side path: the far field on `far` (middle
-    // priority), the grid build and tiled contacts on `aux` (highest), the
-    // warp contact kernel on `aux_lo` (lowest), so that its blocks run in
-    // the room the far field's CTAs leave rather than in their place.
-    cudaStream_t far = nullptr, aux_lo = nullptr;
-    cudaEvent_t ev_far = nullptr, ev_lo = nullptr, ev_grid = nullptr;
 };
 
 struct gi_ctx {
@@ -336,12 +331,7 @@ static void ctx_free(gi_ctx *c)
         cudaFree(x.fsum);
         if (x.ev_fork) cudaEventDestroy(x.ev_fork);
         if (x.ev_join) cudaEventDestroy(x.ev_join);
-        if (x.ev_far) cudaEventDestroy(x.ev_far);
-        if (x.ev_lo) cudaEventDestroy(x.ev_lo);
-        if (x.ev_grid) cudaEventDestroy(x.ev_grid);
         if (x.aux) cudaStreamDestroy(x.aux);
-        if (x.far) cudaStreamDestroy(x.far);
-        if (x.aux_lo) cudaStreamDestroy(x.aux_lo);
     }
     c->scratch.clear();
     cudaFree(c->mirror_pos);
@@ -583,6 +573,8 @@ static void pair_far_unit(int n, const PairDev &p, RunDev &d)
     d.far_inv = (float)std::ldexp(1.0, -E);
 }
 
+constexpr int kPairSplitN = 32768;  // runs below it cut an item's chunks between warps
+
 // Stride of a run's item permutation: coprime with the item count, about
 // the items of one i-block, so that consecutive CTAs hold different i-blocks.
 static int pair_stride(long long items, int nblocks)
@@ -597,6 +589,26 @@ static int pair_stride(long long items, int nblocks)
     return (int)p;
 }
 
+// How the warps share an item of a run of n bodies: log2 of the rows a lane
+// holds and of the warps per item.  The i-block's rows go to 32 << ipl each;
+// below kPairSplitN the item's chunks are cut too, so that a lone short run
+// has enough warps for the 608 schedulers.  Measured, the kernel alone in
+// back-to-back launches (us; rows a lane / chunks a warp):
+//   n = 1,500: 2/1 6.2, 4/1 8.2, 8/1 10.3, 8/4 30.8
+//   n = 4,500: 2/1 14.4, 4/1 14.0, 8/1 16.4, 8/4 30.8
+//   n = 8,192: 4/1 26.7, 8/1 26.6, 8/2 28.7, 8/4 32.2
+//   n = 16,000: 4/2 79.9, 8/1 76.8, 8/2 77.1, 8/4 87.5
+//   n = 24,000: 4/4 165, 8/1 159, 8/2 156.6, 8/4 164
+// A short warp pays the staging and the i-side atomics for fewer pairs, which
+// costs a batch of such runs 2 to 8 %, so the cut is no finer than a lone run
+// needs.
+static void pair_shape(int n, int pcl, int *ipl, int *tpi)
+{
+    *ipl = n <= 3072 ? 1 : n <= 6144 ? 2 : 3;
+    const int cut = n < 12288 ? 2 : n < kPairSplitN ? 1 : 0;
+    *tpi = gi::kPairRowsLog2 - 5 - *ipl + std::min(cut, pcl);
+}
+
 long long gi_internal_pair_run(RunDev &d, int n, int pcl, const PairDev &p, long long item_start)
 {
     d.ipt = gi::kPairIpl;
@@ -609,7 +621,8 @@ long long gi_internal_pair_run(RunDev &d, int n, int pcl, const PairDev &p, long
     const long long ri = pair_items(n, pcl);
     d.pitems = (int)std::min(ri, 0x7fffffffLL);
     d.pstride = pair_stride(ri, d.pnb);
-    return ri;
+    pair_shape(n, pcl, &d.pipl, &d.ptpi);
+    return ri << d.ptpi;
 }
 
 extern "C" int gi_debug_pair_plan(gi_ctx *c, int n, int pcl_in, long long out[6])
@@ -627,7 +640,7 @@ extern "C" int gi_debug_pair_plan(gi_ctx *c, int n, int pcl_in, long long out[6]
     out[0] = d.pcl;
     out[1] = d.pnc;
     out[2] = d.pnb;
-    out[3] = items;
+    out[3] = items >> d.ptpi;
     out[4] = d.pstride;
     out[5] = d.pk0;
     return GI_OK;
@@ -671,6 +684,7 @@ static int make_pair_plan(const gi_ctx *c, const gi_run *runs, int nruns,
         if (items > 0x7fffffffLL) return fail(GI_ERR_BAD_SIZE, "too many work items");
         t.nitems = (int)items;
         for (size_t m = 0; m < pd.size(); ++m) t.params[m] = pd[m];
+        gi_grid_runs(t);
         plan.tables.push_back(t);
         plan.ipt.push_back(gi::kPairIpl);
         plan.bodies.push_back(nb);
@@ -734,6 +748,7 @@ static int make_plan(const gi_ctx *c, const gi_run *runs, int nruns,
         if (items > 0x7fffffffLL) return fail(GI_ERR_BAD_SIZE, "too many work items");
         t.nitems = (int)items;
         for (size_t m = 0; m < pd.size(); ++m) t.params[m] = pd[m];
+        gi_grid_runs(t);
         plan.tables.push_back(t);
         plan.ipt.push_back(p);
         plan.bodies.push_back(nb);
@@ -773,13 +788,6 @@ static int ensure_scratch(gi_ctx *c, const Plan &plan, cudaStream_t s, StreamScr
                 "cudaStreamCreateWithPriority");
         GI_CUDA(cudaEventCreateWithFlags(&x.ev_fork, cudaEventDisableTiming), "cudaEventCreate");
         GI_CUDA(cudaEventCreateWithFlags(&x.ev_join, cudaEventDisableTiming), "cudaEventCreate");
-        GI_CUDA(cudaStreamCreateWithPriority(&x.far, cudaStreamNonBlocking, (lo + hi) / 2),
-                "cudaStreamCreateWithPriority");
-        GI_CUDA(cudaStreamCreateWithPriority(&x.aux_lo, cudaStreamNonBlocking, lo),
-                "cudaStreamCreateWithPriority");
-        GI_CUDA(cudaEventCreateWithFlags(&x.ev_far, cudaEventDisableTiming), "cudaEventCreate");
-        GI_CUDA(cudaEventCreateWithFlags(&x.ev_lo, cudaEventDisableTiming), "cudaEventCreate");
-        GI_CUDA(cudaEventCreateWithFlags(&x.ev_grid, cudaEventDisableTiming), "cudaEventCreate");
     }
     if (grow_t || !x.counters) {
         cudaFree(x.counters);
@@ -814,7 +822,9 @@ static int ensure_scratch(gi_ctx *c, const Plan &plan, cudaStream_t s, StreamScr
         x.fsum = nullptr;
         x.delta_cap = 0;
         GI_CUDA(cudaMalloc(&x.delta, (size_t)plan.max_end * 3 * sizeof(long long)), "cudaMalloc delta");
-        GI_CUDA(cudaMalloc(&x.fsum, (size_t)plan.max_end * 3 * sizeof(double)), "cudaMalloc fsum");
+        GI_CUDA(cudaMalloc(&x.fsum, (size_t)plan.max_end * 3 * sizeof(double) +
+                                        gi::kCtrWords * sizeof(unsigned int)),
+                "cudaMalloc fsum");
         x.delta_cap = plan.max_end;
     }
     return GI_OK;
@@ -840,6 +850,10 @@ static int convert_params(const gi_pair_params *params, int nparams, std::vector
 // uniform balls (default tuning): the side-by-side pass takes 33 % off at
 // n = 8,192, 5 % at 49,152, 2 % at 98,304, and adds 5 % at 131,072.
 constexpr long long kOverlapMaxPairs = 1LL << 34;
+// Paired far field: tables of fewer pairs run everything on the caller's
+// stream, their far field being shorter than the events between streams and
+// the waiting for room cost.
+constexpr long long kBesideMinPairs = 400000000LL;
 // Far-field CTAs per SM while the contact pass runs beside it.  Measured on
 // the 66,000-body impact (ms per fused step, settled / collision phase):
 // 3 CTAs 1.72 / 2.60, 4: 1.68 / 2.57, 6: 1.68 / 2.59, 8: 1.67 / 2.54; the
@@ -851,10 +865,10 @@ constexpr int kSideBySideCtas = 8;
 // far field are independent until the epilogue, so for tables of fewer than
 // kOverlapMaxPairs pairs they run side by side, forked from the caller's
 // stream with events and joined before the epilogue:
-//   - paired far field (the default): the far field on the scratch's
-//     middle-priority stream, the grid build and the tiled contacts on the
-//     highest-priority one, the warp contacts on the lowest (their small
-//     blocks fill the registers the far field's CTAs leave free);
+//   - paired far field (the default): the far field on the caller's stream,
+//     the grid and the contacts on one of the highest priority, the row
+//     contacts of large tables on another (their one-warp blocks fit in the
+//     registers the far field's CTAs leave free);
 //   - one-sided modes: the contact pass on the aux stream, the far field on
 //     the caller's stream with kSideBySideCtas resident CTAs per SM (at that
 //     size it runs as fast as at full occupancy and leaves room on every SM
@@ -880,41 +894,40 @@ static int run_force_plan(gi_ctx *c, const StreamScratch *x, const Plan &plan, i
         a.delta = x->delta;
         a.fsum = x->fsum;
         a.fsum_fx = nullptr;
+        a.fsum_plane = 0;
         int maxn = 0;
         long long pairs = 0;
         for (int r = 0; r < tab.nruns; ++r) {
             maxn = std::max(maxn, tab.runs[r].n);
             pairs += (long long)tab.runs[r].n * tab.runs[r].n;
         }
+        unsigned int *const ctr =
+            reinterpret_cast<unsigned int *>(x->fsum + 3 * (size_t)plan.max_end);
+        const GridWork gw(x->grid_work, plan.bodies[t], plan.max_end);
         if (plan.paired) {
-            // The far-field sums start at zero; captured with the launches
-            // when the stream is capturing.
+            // The far-field sums and the contact pass's counters start at
+            // zero; captured with the launches when the stream is capturing.
             a.fsum_fx = reinterpret_cast<long long *>(x->fsum);
-            GI_CUDA(cudaMemsetAsync(a.fsum_fx, 0, (size_t)plan.max_end * 3 * sizeof(long long), s),
+            a.fsum_plane = (size_t)plan.max_end;
+            GI_CUDA(cudaMemsetAsync(a.fsum_fx, 0, (size_t)plan.max_end * 3 * sizeof(long long) +
+                                                      gi::kCtrWords * sizeof(unsigned int), s),
                     "cudaMemsetAsync far-field sums");
-            if (pairs >= kOverlapMaxPairs) {
-                GI_CUDA(gi_launch_contacts(pos, vel, tab, plan.bodies[t], plan.max_end,
-                                           x->grid_work, x->delta, c->sm_count, s),
-                        "contact pass");
-                GI_CUDA(gi_launch_pair_force(a, tab, s), "paired force kernel launch");
-            } else {
-                // The far field is launched first: it is the long kernel, and
-                // a synchronous caller would otherwise wait for the contact
-                // pass's dozen launches before it starts.
+            const bool beside = pairs >= kBesideMinPairs && pairs < kOverlapMaxPairs;
+            const cudaStream_t q = beside ? x->aux : s;
+            if (beside) {
                 GI_CUDA(cudaEventRecord(x->ev_fork, s), "cudaEventRecord");
-                GI_CUDA(cudaStreamWaitEvent(x->far, x->ev_fork, 0), "cudaStreamWaitEvent");
                 GI_CUDA(cudaStreamWaitEvent(x->aux, x->ev_fork, 0), "cudaStreamWaitEvent");
-                GI_CUDA(gi_launch_pair_force(a, tab, x->far), "paired force kernel launch");
-                GI_CUDA(cudaEventRecord(x->ev_far, x->far), "cudaEventRecord");
-                GI_CUDA(gi_launch_contacts(pos, vel, tab, plan.bodies[t], plan.max_end,
-                                           x->grid_work, x->delta, c->sm_count, x->aux,
-                                           x->aux_lo, x->ev_grid),
-                        "contact pass");
+            }
+            // the grid goes first, while the GPU has room for its clusters
+            GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count, true, q), "cell grid");
+            if (!beside)
+                GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, s), "tiled contacts");
+            GI_CUDA(gi_launch_pair_force(a, tab, gw, x->delta, !beside, s), "paired force kernel launch");
+            if (beside) {
+                GI_CUDA(gi_launch_rows(pos, vel, tab, gw, x->delta, q), "row contacts");
+                GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, q), "tiled contacts");
                 GI_CUDA(cudaEventRecord(x->ev_join, x->aux), "cudaEventRecord");
-                GI_CUDA(cudaEventRecord(x->ev_lo, x->aux_lo), "cudaEventRecord");
-                GI_CUDA(cudaStreamWaitEvent(s, x->ev_far, 0), "cudaStreamWaitEvent");
                 GI_CUDA(cudaStreamWaitEvent(s, x->ev_join, 0), "cudaStreamWaitEvent");
-                GI_CUDA(cudaStreamWaitEvent(s, x->ev_lo, 0), "cudaStreamWaitEvent");
             }
             GI_CUDA(gi_launch_pair_finish(epi, a, tab, maxn, c->sm_count, s), "epilogue launch");
             continue;
@@ -926,19 +939,24 @@ static int run_force_plan(gi_ctx *c, const StreamScratch *x, const Plan &plan, i
         // there).  Captured with the launch when the stream is capturing.
         GI_CUDA(cudaMemsetAsync(x->counters, 0, (2 + plan.ticks[t]) * sizeof(unsigned int), s),
                 "cudaMemsetAsync counters");
-        if (pairs >= kOverlapMaxPairs) {
-            GI_CUDA(gi_launch_contacts(pos, vel, tab, plan.bodies[t], plan.max_end, x->grid_work,
-                                       x->delta, c->sm_count, s),
-                    "contact pass");
+        GI_CUDA(cudaMemsetAsync(ctr, 0, gi::kCtrWords * sizeof(unsigned int), s),
+                "cudaMemsetAsync counters");
+        const bool beside = pairs < kOverlapMaxPairs;
+        const cudaStream_t q = beside ? x->aux : s;
+        if (beside) {
+            GI_CUDA(cudaEventRecord(x->ev_fork, s), "cudaEventRecord");
+            GI_CUDA(cudaStreamWaitEvent(x->aux, x->ev_fork, 0), "cudaStreamWaitEvent");
+        }
+        // Beside the persistent far field the grid is built by small blocks: a
+        // cluster's CTAs would keep the far field's off their SMs for good.
+        GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count, !beside, q), "cell grid");
+        GI_CUDA(gi_launch_rows(pos, vel, tab, gw, x->delta, q), "row contacts");
+        GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, q), "tiled contacts");
+        if (!beside) {
             GI_CUDA(gi_launch_force(p, c->opt.accum, epi, a, tab, c->sm_count * occ, s),
                     "force kernel launch");
             continue;
         }
-        GI_CUDA(cudaEventRecord(x->ev_fork, s), "cudaEventRecord");
-        GI_CUDA(cudaStreamWaitEvent(x->aux, x->ev_fork, 0), "cudaStreamWaitEvent");
-        GI_CUDA(gi_launch_contacts(pos, vel, tab, plan.bodies[t], plan.max_end, x->grid_work,
-                                   x->delta, c->sm_count, x->aux),
-                "contact pass");
         GI_CUDA(cudaEventRecord(x->ev_join, x->aux), "cudaEventRecord");
         GI_CUDA(gi_launch_force(p, c->opt.accum, GI_EPI_SUM, a, tab,
                                 c->sm_count * std::min(occ, kSideBySideCtas), s),

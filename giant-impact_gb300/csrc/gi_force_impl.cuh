@@ -360,6 +360,11 @@ cudaError_t launch_force_ipt(int acc, int epi, const ForceArgs &a, const LaunchT
     dim3 g(grid), block(GI_NT);
 #define GI_CASE(A, E)                                                    \
     if (acc == A && epi == E) {                                          \
+        /* the contact kernels share its SMs (GI_EPI_SUM) */             \
+        static std::atomic<int> known[64];                               \
+        const cudaError_t e = gi_full_carveout(                          \
+            reinterpret_cast<const void *>(force_kernel<IPT, A, E>), known); \
+        if (e != cudaSuccess) return e;                                  \
         force_kernel<IPT, A, E><<<g, block, 0, s>>>(a, tab);             \
         return cudaGetLastError();                                       \
     }

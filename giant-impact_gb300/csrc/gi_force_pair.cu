@@ -10,21 +10,29 @@
 // cuts the pair arithmetic on the FMA pipe, the unit that bounds the far
 // field, from 22 to 14 lane operations per pair.
 //
-// Work decomposition.  An i-block is 1024 consecutive bodies of one run, one
-// CTA of 4 warps, 8 bodies per lane held in registers.  A j-chunk is 64
-// consecutive bodies of the run, two per lane (slots l and l + 32).  A work
-// item is (run, i-block a, a range of `cpi` chunks); block a takes the
-// chunks from its own first body onwards, so every pair i < j is covered
-// exactly once:
-//   - a chunk wholly after a warp's 256 rows: every pair, unmasked;
-//   - a chunk inside the warp's rows (the diagonal): only i < j;
+// Work decomposition.  An i-block is 1024 consecutive bodies of one run; a
+// j-chunk is 64 consecutive bodies of the run, two per lane (slots l and
+// l + 32).  A work item is (run, i-block a, a range of `cpi` chunks); block a
+// takes the chunks from its own first body onwards, so every pair i < j is
+// covered exactly once.  An item is taken by independent warps, each a CTA of
+// its own: a warp holds 32 ipl of the block's rows in registers (ipl = 8: four
+// warps an item) and takes cpt of the item's chunks:
+//   - a chunk wholly after the warp's rows: every pair, unmasked;
+//   - a chunk inside the warp's rows (the diagonal): only i < j, and no row
+//     whose pairs of the chunk are all masked;
 //   - a chunk wholly before the warp's rows: skipped (the warp that owns
 //     those bodies meets this warp's bodies as its j).
+// One-warp CTAs: no barrier, no warp waits for the item's longest one, and
+// the hardware hands out the next task per warp.  At N = 66,000 the kernel
+// alone takes 1.012 ms; CTAs of an item's four warps, their j-sums merged in
+// shared memory, took 1.070.
+// ipl and cpt depend on n alone (pair_shape in gi_api.cu): short runs have too
+// few items for the GPU's 608 warp schedulers, so theirs are cut finer.
 // Items are numbered block-major; block a has ceil((C - 16 a) / cpi) of them
 // (C = chunks of the run; cpi divides 16, so this is k0 - a 16 / cpi and the
-// items before block a are an arithmetic series, decoded by bisection).  CTA
-// t of a run takes item (t * stride) mod items, the stride coprime with the
-// item count and about one i-block's items long: CTAs resident together then
+// items before block a are an arithmetic series, decoded by bisection).  Item
+// slot t of a run is item (t * stride) mod items, the stride coprime with the
+// item count and about one i-block's items long: warps resident together then
 // hold different i-blocks, so their i-side atomics do not queue on the same
 // addresses.
 //
@@ -39,7 +47,14 @@
 // i-body and step, all packed: 3 FADD2 (dp), FMUL2 + 2 FFMA2 (r2), 2 FMNMX,
 // 2 MUFU.RSQ, 2 FMUL2 (r^-3), 3 FFMA2 (i-sums), 3 FFMA2 (j-sums): 14
 // FMA-pipe lane operations per pair, with no per-step fold of the j-sums
-// (each half is one j's).
+// (each half is one j's).  What bounds the loop is the register file: an FFMA2
+// with three distinct operands issues every 3.2 to 5.3 cycles rather than 2,
+// and the six sums are of that kind, so a step of 64 pairs takes 36 cycles a
+// scheduler where the FMA pipe alone would take 28.  Scalar instructions for
+// any group of the operations were slower (1.05 to 1.20 ms at N = 66,000,
+// against 1.012): they need more issue slots and registers than they save.
+// The step loop is not unrolled: 8 rows are enough independent work (1.012
+// against 1.042 ms unrolled twice).
 //
 // Masses (gm = sqrt(G) m, so G m_i m_j = gm_i gm_j).  The i-sums gather
 // dp r^-3 over a chunk and are scaled by the chunk's gm_j when folded;
@@ -51,21 +66,21 @@
 // gm_j and negated.
 //
 // Accumulation and determinism.  Chunk sums are FP32 (32 terms a half per
-// i-body, 256 a half per j-body and warp); a chunk's two halves are folded
-// into the i-body's running FP32 sum in shared memory (at most 16 chunks an
-// item).  Everything beyond that is 64-bit fixed point with a power-of-two
-// unit chosen per run so that no sum of a body's pair terms can overflow it
-// (|F| <= n gm_max^2 < 2^62 units): the j-sums of a CTA are added in shared
-// memory, then both sides into one int64 triple per body in global memory.
+// i-body, 32 ipl a half per j-body and warp); a chunk's two halves are folded
+// into the i-body's running FP32 sum in shared memory (at most 16 chunks).
+// Everything beyond that is 64-bit fixed point with a power-of-two unit chosen
+// per run so that no sum of a body's pair terms can overflow it (|F| <=
+// n gm_max^2 < 2^62 units), added to one int64 per body and component in
+// global memory (a plane per component: a warp's atomics are contiguous).
 // Integer addition is associative, so the result does not depend on which
-// CTA finished first: it depends only on the run's bodies, n and cpi.
+// warp finished first: it depends only on the run's bodies, n and cpi.
 // pair_finish_kernel converts the sums, adds the contact corrections and
 // stores the force or steps the bodies with the arithmetic of the one-sided
 // kernel's epilogue.
 #include <algorithm>
 #include <atomic>
 
-#include "gi_force_impl.cuh"
+#include "gi_contact.cuh"
 
 namespace gi {
 
@@ -83,18 +98,17 @@ __device__ __forceinline__ long long pair_items_before(long long a, long long k0
 //   IMIX: the warp's rows straddle the Fe/Si boundary; w takes the per-row
 //         gm_i.  Every other warp has one i mass, applied after the sums.
 // ax[k] (per component) gathers row k's terms, one half per j of the lane.
-template <bool EDGE, bool IMIX>
+template <int IPL, bool EDGE, bool IMIX>
 __device__ __forceinline__ void pair_chunk(const float4 *__restrict__ cxy,
                                            const float4 *__restrict__ czg, const int lane,
-                                           const int di, const float2 (&nx)[kPairIpl],
-                                           const float2 (&ny)[kPairIpl],
-                                           const float2 (&nz)[kPairIpl],
-                                           const float2 (&gi)[kPairIpl], float2 (&ax)[kPairIpl],
-                                           float2 (&ay)[kPairIpl], float2 (&az)[kPairIpl],
-                                           float2 &bx, float2 &by, float2 &bz)
+                                           const int di, const float (&nx)[IPL],
+                                           const float (&ny)[IPL], const float (&nz)[IPL],
+                                           const float (&gi)[IPL], float2 (&ax)[IPL],
+                                           float2 (&ay)[IPL], float2 (&az)[IPL], float2 &bx,
+                                           float2 &by, float2 &bz)
 {
     bx = by = bz = make_float2(0.0f, 0.0f);
-#pragma unroll 2
+#pragma unroll 1
     for (int s = 0; s < 32; ++s) {
         const int jl = (lane + s) & 31;
         const float4 q = cxy[jl];
@@ -102,17 +116,20 @@ __device__ __forceinline__ void pair_chunk(const float4 *__restrict__ cxy,
         const float2 X = make_float2(q.x, q.y), Y = make_float2(q.z, q.w),
                      Z = make_float2(g.x, g.y);
 #pragma unroll
-        for (int k = 0; k < kPairIpl; ++k) {
-            const float2 dx = __fadd2_rn(X, nx[k]);
-            const float2 dy = __fadd2_rn(Y, ny[k]);
-            const float2 dz = __fadd2_rn(Z, nz[k]);
+        for (int k = 0; k < IPL; ++k) {
+            // rows from here on have no j > i in the chunk
+            if (EDGE && di + 32 * k >= kPairChunk) break;
+            const float2 dx = __fadd2_rn(X, make_float2(nx[k], nx[k]));
+            const float2 dy = __fadd2_rn(Y, make_float2(ny[k], ny[k]));
+            const float2 dz = __fadd2_rn(Z, make_float2(nz[k], nz[k]));
             // fma(dz, dz, fma(dx, dx, dy*dy)) per lane, as the reference
             float2 r2 = __fmul2_rn(dy, dy);
             r2 = __ffma2_rn(dx, dx, r2);
             r2 = __ffma2_rn(dz, dz, r2);
             const float2 ri = make_float2(rsqrt_mufu(fmaxf(r2.x, 1.0f)),
                                           rsqrt_mufu(fmaxf(r2.y, 1.0f)));
-            float2 w = IMIX ? __fmul2_rn(__fmul2_rn(ri, ri), __fmul2_rn(ri, gi[k]))
+            float2 w = IMIX ? __fmul2_rn(__fmul2_rn(ri, ri),
+                                         __fmul2_rn(ri, make_float2(gi[k], gi[k])))
                             : __fmul2_rn(__fmul2_rn(ri, ri), ri);
             float2 wi = w;
             if (EDGE) {
@@ -122,10 +139,10 @@ __device__ __forceinline__ void pair_chunk(const float4 *__restrict__ cxy,
                 wi = __fmul2_rn(w, make_float2(g.z, g.w));
             }
             ax[k] = __ffma2_rn(wi, dx, ax[k]);
-            ay[k] = __ffma2_rn(wi, dy, ay[k]);
-            az[k] = __ffma2_rn(wi, dz, az[k]);
             bx = __ffma2_rn(w, dx, bx);
+            ay[k] = __ffma2_rn(wi, dy, ay[k]);
             by = __ffma2_rn(w, dy, by);
+            az[k] = __ffma2_rn(wi, dz, az[k]);
             bz = __ffma2_rn(w, dz, bz);
         }
         // the j-sums move to the lane that meets these j next
@@ -138,132 +155,35 @@ __device__ __forceinline__ void pair_chunk(const float4 *__restrict__ cxy,
     }
 }
 
-// One warp over the item's chunks.  Row r's running i-sum (si[d * 1024 + r],
-// shared memory) gathers sum_chunks gm_j sum_j w dp; each chunk's j-sums go,
-// times -gm_j and scale_j, into the CTA's fixed-point j-sums.
-template <bool IMIX>
-__device__ __forceinline__ void pair_warp(const float4 *__restrict__ cxy,
-                                          const float4 *__restrict__ czg,
-                                          unsigned long long *__restrict__ sj,
-                                          float *__restrict__ si, const int c0, const int nch,
-                                          const int wi0, const int warp, const int lane,
-                                          const int nfe, const PairDev &P, const float scale_j,
-                                          const float2 (&nx)[kPairIpl],
-                                          const float2 (&ny)[kPairIpl],
-                                          const float2 (&nz)[kPairIpl],
-                                          const float2 (&gi)[kPairIpl])
+// Shared memory of one warp: the staged chunks and its rows' running sums.
+struct PairSmem {
+    float4 cxy[kPairStage * 32];  // (x_a, x_b, y_a, y_b)
+    float4 czg[kPairStage * 32];  // (z_a, z_b, gm_a, gm_b)
+    float si[3][kPairWarpRows];
+};
+
+__device__ __forceinline__ void add_fx(long long *p, float v)
 {
-#pragma unroll 1
-    for (int c = 0; c < nch; ++c) {
-        const int jc0 = (c0 + c) * kPairChunk;  // relative to the run
-        if (jc0 + kPairChunk <= wi0) continue;  // before this warp's rows
-        const bool diag = jc0 < wi0 + kPairWarpRows;
-        const bool straddle = jc0 < nfe && nfe < jc0 + kPairChunk;
-        float2 ax[kPairIpl], ay[kPairIpl], az[kPairIpl];
-#pragma unroll
-        for (int k = 0; k < kPairIpl; ++k) ax[k] = ay[k] = az[k] = make_float2(0.0f, 0.0f);
-        float2 bx, by, bz;
-        float gc;  // the chunk's gm_j, applied at the fold (1 for EDGE chunks)
-        if (diag || straddle) {
-            pair_chunk<true, IMIX>(cxy + c * 32, czg + c * 32, lane, wi0 - jc0, nx, ny, nz, gi,
-                                   ax, ay, az, bx, by, bz);
-            gc = 1.0f;
-        } else {
-            pair_chunk<false, IMIX>(cxy + c * 32, czg + c * 32, lane, 0, nx, ny, nz, gi, ax, ay,
-                                    az, bx, by, bz);
-            gc = jc0 < nfe ? P.gm_fe : P.gm_si;
-        }
-        // j side: lane l holds j = jc0 + l (.x) and jc0 + 32 + l (.y); the
-        // force on j is -gm_j times its sum
-        const float4 g = czg[c * 32 + lane];
-        const float ga = -g.z * scale_j, gb = -g.w * scale_j;
-        unsigned long long *da = sj + (size_t)(c * kPairChunk + lane) * 3;
-        unsigned long long *db = sj + (size_t)(c * kPairChunk + 32 + lane) * 3;
-        atomicAdd(da + 0, (unsigned long long)__float2ll_rn(ga * bx.x));
-        atomicAdd(da + 1, (unsigned long long)__float2ll_rn(ga * by.x));
-        atomicAdd(da + 2, (unsigned long long)__float2ll_rn(ga * bz.x));
-        atomicAdd(db + 0, (unsigned long long)__float2ll_rn(gb * bx.y));
-        atomicAdd(db + 1, (unsigned long long)__float2ll_rn(gb * by.y));
-        atomicAdd(db + 2, (unsigned long long)__float2ll_rn(gb * bz.y));
-        // i side: the two halves, scaled by the chunk's gm_j, into the
-        // running sums (each thread owns its rows: no atomics)
-#pragma unroll
-        for (int k = 0; k < kPairIpl; ++k) {
-            const int r = warp * kPairWarpRows + k * 32 + lane;
-            si[r] = __fmaf_rn(ax[k].x + ax[k].y, gc, si[r]);
-            si[kPairRows + r] = __fmaf_rn(ay[k].x + ay[k].y, gc, si[kPairRows + r]);
-            si[2 * kPairRows + r] = __fmaf_rn(az[k].x + az[k].y, gc, si[2 * kPairRows + r]);
-        }
-    }
+    atomicAdd(reinterpret_cast<unsigned long long *>(p), (unsigned long long)__float2ll_rn(v));
 }
 
-// Shared memory of one work item of 2^pcl chunks.
-__host__ __device__ constexpr size_t pair_smem_bytes(int pcl)
+// One warp: rows wi0 .. wi0 + 32 IPL, chunks c0 .. c1 (relative to the run).
+// Row r's running i-sum (sm.si[.][r]) gathers sum_chunks gm_j sum_j w dp; each
+// chunk's j-sums go, times -gm_j and scale_j, into the global sums.
+template <int IPL, bool IMIX>
+__device__ __forceinline__ void pair_rows(PairSmem &sm, const ForceArgs &a, const RunDev &R,
+                                          const PairDev &P, const int c0, const int c1,
+                                          const int wi0, const int lane, const float scale_j,
+                                          const float scale_i)
 {
-    return (size_t)(1 << pcl) * 32 * (2 * sizeof(float4)) +
-           (size_t)(1 << pcl) * kPairChunk * 3 * sizeof(unsigned long long) +
-           3 * (size_t)kPairRows * sizeof(float);
-}
-
-// 152 registers (no spills): 3 CTAs per SM use 58,368 of the 65,536, and a
-// 64-thread block of the contact pass fits beside them on every SM.
-__global__ void __maxnreg__(152)
-pair_force_kernel(const ForceArgs a, const __grid_constant__ LaunchTable tab)
-{
-    extern __shared__ float4 pair_smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int item = blockIdx.x;
-    const RunDev &R = tab.runs[find_run(tab, item)];
-    const PairDev &P = tab.params[R.param];
-    const int cpi = 1 << R.pcl;
-    float4 *cxy = pair_smem;                  // cpi * 32: (x_a, x_b, y_a, y_b)
-    float4 *czg = pair_smem + cpi * 32;       // cpi * 32: (z_a, z_b, gm_a, gm_b)
-    unsigned long long *sj =
-        reinterpret_cast<unsigned long long *>(pair_smem + 2 * cpi * 32);  // cpi * 64 * 3
-    float *si = reinterpret_cast<float *>(sj + (size_t)cpi * kPairChunk * 3);  // 3 * 1024
-
-    // ---- decode (i-block a, item k of the block).  Consecutive CTAs take
-    // items a stride apart, so the CTAs running at once work on different
-    // i-blocks and their sums land on different addresses.
-    const long long t = ((long long)(item - R.item_start) * R.pstride) % R.pitems;
-    const long long k0 = R.pk0, q = kPairBlockChunks >> R.pcl;
-    int lo = 0, hi = R.pnb - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (pair_items_before(mid, k0, q) <= t) lo = mid;
-        else hi = mid - 1;
-    }
-    const int blk = lo;
-    const int c0 = blk * kPairBlockChunks + (int)(t - pair_items_before(blk, k0, q)) * cpi;
-    const int nch = min(cpi, R.pnc - c0);
+    constexpr int kRows = 32 * IPL;
     const int rbeg = R.offset, n = R.n, nfe = R.nfe;
-
-    // ---- stage the j-range, clear the j-sums and the running i-sums
-    for (int u = threadIdx.x; u < nch * 32; u += blockDim.x) {
-        const int ja = (c0 + (u >> 5)) * kPairChunk + (u & 31), jb = ja + 32;  // relative to the run
-        float4 pa = make_float4(GI_FAR_J, GI_FAR_J, GI_FAR_J, 0.0f), pb = pa;
-        float ga = 0.0f, gb = 0.0f;
-        if (ja < n) {
-            pa = __ldg(&a.pos[rbeg + ja]);
-            ga = ja < nfe ? P.gm_fe : P.gm_si;
-        }
-        if (jb < n) {
-            pb = __ldg(&a.pos[rbeg + jb]);
-            gb = jb < nfe ? P.gm_fe : P.gm_si;
-        }
-        cxy[u] = make_float4(pa.x, pb.x, pa.y, pb.y);
-        czg[u] = make_float4(pa.z, pb.z, ga, gb);
-    }
-    for (int u = threadIdx.x; u < nch * kPairChunk * 3; u += blockDim.x) sj[u] = 0ull;
-    for (int u = threadIdx.x; u < 3 * kPairRows; u += blockDim.x) si[u] = 0.0f;
-
-    // ---- this lane's 8 i-bodies: rows wi0 + k 32 + lane, k = 0..7, each
-    // duplicated in both halves of its registers.  Rows beyond the run sit
-    // at GI_FAR_I, where r^-3 underflows to zero.
-    const int wi0 = blk * kPairRows + warp * kPairWarpRows;  // relative to the run
-    float2 nx[kPairIpl], ny[kPairIpl], nz[kPairIpl], gi[kPairIpl];
+    long long *const out = a.fsum_fx + rbeg;
+    const size_t plane = a.fsum_plane;
+    // this lane's rows; beyond the run at GI_FAR_I, where r^-3 underflows to 0
+    float nx[IPL], ny[IPL], nz[IPL], gi[IPL];
 #pragma unroll
-    for (int k = 0; k < kPairIpl; ++k) {
+    for (int k = 0; k < IPL; ++k) {
         const int i = wi0 + k * 32 + lane;
         float4 p = make_float4(GI_FAR_I, GI_FAR_I, GI_FAR_I, 0.0f);
         float g = 0.0f;
@@ -271,44 +191,156 @@ pair_force_kernel(const ForceArgs a, const __grid_constant__ LaunchTable tab)
             p = __ldg(&a.pos[rbeg + i]);
             g = i < nfe ? P.gm_fe : P.gm_si;
         }
-        nx[k] = make_float2(-p.x, -p.x);
-        ny[k] = make_float2(-p.y, -p.y);
-        nz[k] = make_float2(-p.z, -p.z);
-        gi[k] = make_float2(g, g);
+        nx[k] = -p.x;
+        ny[k] = -p.y;
+        nz[k] = -p.z;
+        gi[k] = g;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) sm.si[d][k * 32 + lane] = 0.0f;
     }
+#pragma unroll 1
+    for (int cb = c0; cb < c1; cb += kPairStage) {
+        const int ce = min(cb + kPairStage, c1);
+        __syncwarp();  // the previous chunks are consumed
+        for (int c = cb; c < ce; ++c) {
+            const int ja = c * kPairChunk + lane, jb = ja + 32;
+            float4 pa = make_float4(GI_FAR_J, GI_FAR_J, GI_FAR_J, 0.0f), pb = pa;
+            float ga = 0.0f, gb = 0.0f;
+            if (ja < n) {
+                pa = __ldg(&a.pos[rbeg + ja]);
+                ga = ja < nfe ? P.gm_fe : P.gm_si;
+            }
+            if (jb < n) {
+                pb = __ldg(&a.pos[rbeg + jb]);
+                gb = jb < nfe ? P.gm_fe : P.gm_si;
+            }
+            sm.cxy[(c - cb) * 32 + lane] = make_float4(pa.x, pb.x, pa.y, pb.y);
+            sm.czg[(c - cb) * 32 + lane] = make_float4(pa.z, pb.z, ga, gb);
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int c = cb; c < ce; ++c) {
+            const float4 *cxy = sm.cxy + (c - cb) * 32, *czg = sm.czg + (c - cb) * 32;
+            const int jc0 = c * kPairChunk;
+            const bool diag = jc0 < wi0 + kRows;
+            const bool straddle = jc0 < nfe && nfe < jc0 + kPairChunk;
+            float2 ax[IPL], ay[IPL], az[IPL];
+#pragma unroll
+            for (int k = 0; k < IPL; ++k) ax[k] = ay[k] = az[k] = make_float2(0.0f, 0.0f);
+            float2 bx, by, bz;
+            float gc;  // the chunk's gm_j, applied at the fold (1 for EDGE chunks)
+            if (diag || straddle) {
+                pair_chunk<IPL, true, IMIX>(cxy, czg, lane, wi0 - jc0, nx, ny, nz, gi, ax, ay, az,
+                                            bx, by, bz);
+                gc = 1.0f;
+            } else {
+                pair_chunk<IPL, false, IMIX>(cxy, czg, lane, 0, nx, ny, nz, gi, ax, ay, az, bx, by,
+                                             bz);
+                gc = jc0 < nfe ? P.gm_fe : P.gm_si;
+            }
+            // j side: lane l holds j = jc0 + l (.x) and jc0 + 32 + l (.y);
+            // the force on j is -gm_j times its sum
+            const float4 g = czg[lane];
+            const float ga = -g.z * scale_j, gb = -g.w * scale_j;
+            const int ja = jc0 + lane, jb = ja + 32;
+            if (ja < n) {
+                add_fx(out + ja, ga * bx.x);
+                add_fx(out + plane + ja, ga * by.x);
+                add_fx(out + 2 * plane + ja, ga * bz.x);
+            }
+            if (jb < n) {
+                add_fx(out + jb, gb * bx.y);
+                add_fx(out + plane + jb, gb * by.y);
+                add_fx(out + 2 * plane + jb, gb * bz.y);
+            }
+            // i side: the two halves, scaled by the chunk's gm_j, into the
+            // running sums (each lane owns its rows)
+#pragma unroll
+            for (int k = 0; k < IPL; ++k) {
+                const int r = k * 32 + lane;
+                sm.si[0][r] = __fmaf_rn(ax[k].x + ax[k].y, gc, sm.si[0][r]);
+                sm.si[1][r] = __fmaf_rn(ay[k].x + ay[k].y, gc, sm.si[1][r]);
+                sm.si[2][r] = __fmaf_rn(az[k].x + az[k].y, gc, sm.si[2][r]);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < IPL; ++k) {
+        const int r = k * 32 + lane, i = wi0 + r;
+        if (i >= n) break;
+        add_fx(out + i, sm.si[0][r] * scale_i);
+        add_fx(out + plane + i, sm.si[1][r] * scale_i);
+        add_fx(out + 2 * plane + i, sm.si[2][r] * scale_i);
+    }
+}
+
+template <int IPL>
+__device__ __forceinline__ void pair_task(PairSmem &sm, const ForceArgs &a, const RunDev &R,
+                                          const PairDev &P, const int c0, const int c1,
+                                          const int wi0, const int lane)
+{
     // A warp whose rows are all of one class takes its gm_i out of the pair
     // loop: it scales the j-sums and the finished i-sums instead.
-    const bool imix = wi0 < nfe && nfe < wi0 + kPairWarpRows;
-    const float gmw = imix ? 1.0f : (wi0 < nfe ? P.gm_fe : P.gm_si);
-    const float inv = R.far_inv, scale_i = inv * gmw;
-    __syncthreads();
+    const float inv = R.far_inv;
+    if (wi0 < R.nfe && R.nfe < wi0 + 32 * IPL) {
+        pair_rows<IPL, true>(sm, a, R, P, c0, c1, wi0, lane, inv, inv);
+    } else {
+        const float scale = inv * (wi0 < R.nfe ? P.gm_fe : P.gm_si);
+        pair_rows<IPL, false>(sm, a, R, P, c0, c1, wi0, lane, scale, scale);
+    }
+}
 
-    if (imix)
-        pair_warp<true>(cxy, czg, sj, si, c0, nch, wi0, warp, lane, nfe, P, inv, nx, ny, nz, gi);
+__device__ __forceinline__ void pair_item(PairSmem &sm, const ForceArgs &a, const LaunchTable &tab,
+                                          int cta, int lane)
+{
+    const RunDev &R = tab.runs[find_run(tab, cta)];
+    const PairDev &P = tab.params[R.param];
+    // ---- decode: item slot, rows and chunks of the item; then (i-block, item
+    // of the block)
+    const int local = cta - R.item_start;
+    const int slot = local >> R.ptpi, part = local & ((1 << R.ptpi) - 1);
+    const int rlog = kPairRowsLog2 - 5 - R.pipl;  // log2 of the row groups of an i-block
+    const long long t = ((long long)slot * R.pstride) % R.pitems;
+    const long long k0 = R.pk0, q = kPairBlockChunks >> R.pcl;
+    int lo = 0, hi = R.pnb - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (pair_items_before(mid, k0, q) <= t) lo = mid;
+        else hi = mid - 1;
+    }
+    const int wi0 = lo * kPairRows + ((part & ((1 << rlog) - 1)) << (5 + R.pipl));
+    const int cpt = 1 << (R.pcl - (R.ptpi - rlog));  // chunks of this warp
+    const int cb = lo * kPairBlockChunks + ((int)(t - pair_items_before(lo, k0, q)) << R.pcl) +
+                   (part >> rlog) * cpt;
+    const int c0 = max(cb, wi0 / kPairChunk), c1 = min(cb + cpt, R.pnc);
+    if (c0 >= c1) return;  // wholly before the rows, or no rows
+    if (R.pipl == 3) pair_task<8>(sm, a, R, P, c0, c1, wi0, lane);
+    else if (R.pipl == 2) pair_task<4>(sm, a, R, P, c0, c1, wi0, lane);
+    else pair_task<2>(sm, a, R, P, c0, c1, wi0, lane);
+}
+
+// The far field and, of small tables, the contact pass's row path
+// (gi_contact.cuh) in one launch of one-warp CTAs: the first `rows` CTAs take
+// rows, the others far-field tasks.  The two are independent until the
+// epilogue, and the row path, which waits on memory, runs in the far field's
+// issue gaps.  One launch on one stream: each event between streams costs 2 to
+// 5 us, a step of a few thousand bodies 20 to 50.
+// 162 registers (no spills): 12 CTAs per SM.  ptxas's allocation moves the
+// loop by 5 %: held to 160 it takes 1.073 ms at N = 66,000 (262,144: 16.8),
+// at 162 1.012 (15.25), at 168 1.037, with the sums in another order 1.032.
+__global__ void __maxnreg__(168)
+pair_force_kernel(const ForceArgs a, const GridView g, long long *__restrict__ delta, int rows,
+                  const __grid_constant__ LaunchTable tab)
+{
+    __shared__ union Smem {
+        PairSmem pair;
+        RowSmem row;
+        __device__ Smem() {}
+    } sm;
+    if ((int)blockIdx.x < rows)
+        contact_rows(sm.row, a.pos, a.vel, g, delta, tab, blockIdx.x);
     else
-        pair_warp<false>(cxy, czg, sj, si, c0, nch, wi0, warp, lane, nfe, P, scale_i, nx, ny, nz,
-                         gi);
-
-    // ---- i side into the global fixed-point sums
-    unsigned long long *out = reinterpret_cast<unsigned long long *>(a.fsum_fx);
-#pragma unroll
-    for (int k = 0; k < kPairIpl; ++k) {
-        const int i = wi0 + k * 32 + lane;
-        if (i >= n) continue;
-        const int r = warp * kPairWarpRows + k * 32 + lane;
-        unsigned long long *o = out + 3 * (size_t)(rbeg + i);
-        atomicAdd(o + 0, (unsigned long long)__float2ll_rn(si[r] * scale_i));
-        atomicAdd(o + 1, (unsigned long long)__float2ll_rn(si[kPairRows + r] * scale_i));
-        atomicAdd(o + 2, (unsigned long long)__float2ll_rn(si[2 * kPairRows + r] * scale_i));
-    }
-    // ---- j side of the whole CTA
-    __syncthreads();
-    unsigned long long *oj = out + 3 * ((size_t)rbeg + (size_t)c0 * kPairChunk);
-    const int nj = min(nch * kPairChunk, n - c0 * kPairChunk);
-    for (int u = threadIdx.x; u < nj * 3; u += blockDim.x) {
-        const unsigned long long v = sj[u];
-        if (v) atomicAdd(oj + u, v);
-    }
+        pair_item(sm.pair, a, tab, blockIdx.x - rows, threadIdx.x);
 }
 
 // The epilogue: F = fixed-point far field + contact correction, rounded once
@@ -323,9 +355,10 @@ __global__ void __launch_bounds__(256) pair_finish_kernel(const ForceArgs a,
     const double far_unit = R.far_unit;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < R.n; k += gridDim.x * blockDim.x) {
         const int i = R.offset + k;
-        const long long *q = a.fsum_fx + 3 * (size_t)i;
-        const double fd[3] = {(double)__ldcg(q) * far_unit, (double)__ldcg(q + 1) * far_unit,
-                              (double)__ldcg(q + 2) * far_unit};
+        const long long *q = a.fsum_fx + i;
+        const double fd[3] = {(double)__ldcg(q) * far_unit,
+                              (double)__ldcg(q + a.fsum_plane) * far_unit,
+                              (double)__ldcg(q + 2 * a.fsum_plane) * far_unit};
         finish_body<EPI>(a, R, unit, i, fd);
     }
 }
@@ -334,27 +367,15 @@ __global__ void __launch_bounds__(256) pair_finish_kernel(const ForceArgs a,
 
 using namespace gi;
 
-cudaError_t gi_launch_pair_force(const ForceArgs &a, const LaunchTable &tab, cudaStream_t s)
+cudaError_t gi_launch_pair_force(const ForceArgs &a, const LaunchTable &tab, const GridWork &g,
+                                 long long *delta, bool with_rows, cudaStream_t s)
 {
     if (tab.nitems <= 0) return cudaSuccess;
-    int pcl = 0;
-    for (int r = 0; r < tab.nruns; ++r) pcl = std::max(pcl, tab.runs[r].pcl);
-    const size_t smem = pair_smem_bytes(pcl);
-    // Items of more than 8 chunks take more than the 48 KB of shared memory
-    // a kernel gets by default: raise its limit once per device (the first
-    // such launch on a device comes before any capture, which cannot grow
-    // scratch either).
-    static std::atomic<int> raised[64];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    static std::atomic<int> known[64];
+    cudaError_t e = gi_full_carveout(reinterpret_cast<const void *>(pair_force_kernel), known);
     if (e != cudaSuccess) return e;
-    if (smem > (48u << 10) && dev >= 0 && dev < 64 && !raised[dev].load()) {
-        e = cudaFuncSetAttribute(pair_force_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)pair_smem_bytes(4));
-        if (e != cudaSuccess) return e;
-        raised[dev].store(1);
-    }
-    pair_force_kernel<<<tab.nitems, kPairWarps * 32, smem, s>>>(a, tab);
+    const int rows = with_rows ? tab.rows : 0;
+    pair_force_kernel<<<rows + tab.nitems, 32, 0, s>>>(a, g.view(), delta, rows, tab);
     return cudaGetLastError();
 }
 

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/gi_api.h"
 
 // Threads per CTA of the one-sided force kernel (gi_force_impl.cuh); also
@@ -44,7 +46,7 @@ struct PairDev {
 
 struct RunDev {
     int offset, n, nfe, param;
-    int item_start;   // first work item of this run
+    int item_start;   // first work item of this run (paired: first CTA)
     int nsplit;       // j-chunks per i-block
     int jchunk;       // bodies per big chunk (GI_NT * 2^lg)
     int nib;          // i-blocks
@@ -60,9 +62,15 @@ struct RunDev {
     int pnb;          // i-blocks of the run, ceil(n / kPairRows)
     int pk0;          // work items of i-block 0, ceil(pnc / 2^pcl)
     int pitems;       // work items of the run
-    int pstride;      // CTA t of the run takes item (t * pstride) mod pitems (coprime)
+    int pstride;      // item slot t of the run is item (t * pstride) mod pitems (coprime)
+    int pipl;         // log2 of the rows a lane holds: 32 << pipl rows a warp
+    int ptpi;         // log2 of the warps (CTAs) that share an item
     float far_inv;    // 1 / far_unit: scale of a far-field sum into fixed point
     double far_unit;  // fixed-point unit of the far-field sums (a power of two)
+    // cell grid of the contact pass (gi_grid_runs)
+    int glog;         // log2 of the run's buckets; 0: no grid, every body is a candidate
+    int gbase, gslot; // its first bucket and first slot
+    int row_start;    // its first row-path CTA
 };
 
 struct LaunchTable {
@@ -70,6 +78,8 @@ struct LaunchTable {
     int nitems;
     int sep_test;
     int dense_min;  // contact pass: bucket size from which the tiled kernel takes it
+    int rows;       // row-path CTAs of all runs
+    int gridn;      // bodies of the largest run with a grid (0: none)
     RunDev runs[GI_MAX_RUNS];
     PairDev params[GI_MAX_PARAMS];
 };
@@ -85,7 +95,8 @@ struct ForceArgs {
     unsigned int *queue;  // [0] next work item, [1] CTAs finished (zero between launches)
     const long long *delta;  // contact corrections, 3 per body, fixed point (gi_grid.cu)
     double *fsum;            // GI_EPI_SUM: far-field sums, 3 per body
-    long long *fsum_fx;      // GI_ACC_PAIRED: far-field sums, 3 per body, fixed point
+    long long *fsum_fx;      // GI_ACC_PAIRED: far-field sums, fixed point, one plane per
+    size_t fsum_plane;       // component, fsum_plane bodies apart
 };
 
 // Launchers (gi_force_ipt*.cu).  Return cudaError_t of the launch.
@@ -105,24 +116,28 @@ cudaError_t gi_launch_finish(int epi, const ForceArgs &a, const LaunchTable &tab
 // gi_force_pair.cu: the far field with each unordered pair evaluated once.
 // Its shape is fixed here, where the planner reads it.
 namespace gi {
-constexpr int kPairWarps = 4;                             // warps per CTA
-constexpr int kPairIpl = 8;                               // i-bodies per lane
-constexpr int kPairWarpRows = 32 * kPairIpl;              // 256 rows per warp
-constexpr int kPairRows = kPairWarps * kPairWarpRows;     // 1024: the i-block
+constexpr int kPairIpl = 8;                               // i-bodies per lane, at most
+constexpr int kPairWarpRows = 32 * kPairIpl;              // 256 rows per warp, at most
+constexpr int kPairRowsLog2 = 10;
+constexpr int kPairRows = 1 << kPairRowsLog2;             // 1024: the i-block
 constexpr int kPairChunk = 64;                            // j-chunk: two bodies per lane
 constexpr int kPairBlockChunks = kPairRows / kPairChunk;  // 16
 constexpr int kPairMaxCpi = 16;                           // j-chunks per work item, at most
+constexpr int kPairStage = 8;                             // chunks staged at a time (8 KB)
 static_assert(kPairMaxCpi <= kPairBlockChunks && kPairBlockChunks % kPairMaxCpi == 0,
               "chunks per item must divide the chunks of an i-block");
 }  // namespace gi
 // Far-field sums of every body of the table's runs into a.fsum_fx (which
-// must be zero on entry); then the epilogue, as gi_launch_finish.
-cudaError_t gi_launch_pair_force(const ForceArgs &a, const LaunchTable &tab, cudaStream_t s);
+// must be zero on entry), and with_rows the row path's corrections into delta
+// (the grid must be built); then the epilogue, as gi_launch_finish.
+struct GridWork;
+cudaError_t gi_launch_pair_force(const ForceArgs &a, const LaunchTable &tab, const GridWork &g,
+                                 long long *delta, bool with_rows, cudaStream_t s);
 cudaError_t gi_launch_pair_finish(int epi, const ForceArgs &a, const LaunchTable &tab, int maxn,
                                   int nsm, cudaStream_t s);
 
 // gi_grid.cu: contact corrections of every body of the table's runs into
-// delta (3 x int64 per body) through a hashed cell grid.  Its scratch layout
+// delta (3 x int64 per body) through a cell grid.  Its scratch layout
 // is computed here, as constexpr functions, so that gi_noalloc.cu can check
 // at compile time that its static array holds the largest run it accepts.
 namespace gi {
@@ -131,9 +146,13 @@ namespace gi {
 constexpr unsigned int kDenseFloor = 32;
 // Cost classes of the tiled path's work items (128-body tiles staged - 1).
 constexpr unsigned int kItemClasses = 16;
-// Tiled-path counters: items, tiled buckets, queue head, one spare, then a
-// count and a fill cursor per cost class.
+// Tiled-path counters: items, tiled buckets, queue head, candidate buckets,
+// then a count and a fill cursor per cost class.
 constexpr int kCtrWords = 4 + 2 * (int)kItemClasses;
+// Runs of at most this many bodies take no grid.
+constexpr int kDirectMax = 4096;
+// Bodies of a row-path CTA (one warp), of a run with a grid and without.
+constexpr int kRowBodies = 8, kDirectBodies = 2;
 }  // namespace gi
 
 // Buckets of the grid for `bodies` bodies: a power of two >= 2 * bodies.
@@ -154,28 +173,83 @@ constexpr size_t gi_dense_item_capacity(long long bodies)
 }
 constexpr size_t gi_dense_bucket_capacity(long long bodies)
 {
-    return (size_t)bodies / gi::kDenseFloor + 1;
+    return (size_t)bodies / gi::kDenseFloor + GI_MAX_RUNS;  // each run rounds up
 }
 
-// Words of grid scratch: slot-ordered positions and velocities (float4, 8
-// words per slot); keys (indexed by global body index) and sorted (by slot):
-// max_end words each; cursor and bucket state: one word per bucket each;
-// block sums: 8192; the tiled path's counters and up to 3 words to align the
-// items to 16 bytes; items as listed and as ordered (4 words each); tiled
-// buckets.
+// Words of grid scratch: the slots' positions and velocities, and a second,
+// sub-cell ordered copy of the tiled buckets' (16 words per body); items as
+// listed and as ordered (4 words each); candidate and tiled buckets (2 words
+// each); bucket starts (one word per bucket and one more) and states; block
+// sums: 9216; keys and ranks of the grid-wide build (indexed by global body).
 constexpr size_t gi_grid_words(long long max_end, long long bodies)
 {
-    return 8 * (size_t)bodies + 2 * (size_t)max_end + 2 * (size_t)gi_grid_buckets(bodies) + 8192 +
-           gi::kCtrWords + 3 + 8 * gi_dense_item_capacity(bodies) +
-           gi_dense_bucket_capacity(bodies);
+    return 16 * (size_t)bodies + 8 * gi_dense_item_capacity(bodies) +
+           4 * gi_dense_bucket_capacity(bodies) + 2 * (size_t)gi_grid_buckets(bodies) + 1 + 9216 +
+           2 * (size_t)max_end;
 }
-// With s_warp and ev_grid given, the warp-per-body kernel runs on s_warp
-// after the grid is built (ev_grid is recorded on s and waited on by
-// s_warp); the caller then joins s_warp as well as s.
-cudaError_t gi_launch_contacts(const float4 *pos, const float4 *vel, const LaunchTable &tab,
-                               long long bodies, int max_end, unsigned int *work,
-                               long long *delta, int nsm, cudaStream_t s,
-                               cudaStream_t s_warp = nullptr, cudaEvent_t ev_grid = nullptr);
+// What the row path reads of it.
+struct GridView {
+    const float4 *spos, *svel;
+    const unsigned int *start;
+};
+// The scratch of one table's contact pass, carved from `work` (16-byte
+// aligned): 16-byte words first, then single words (see gi_grid_words).
+struct GridWork {
+    float4 *spos, *svel, *dpos, *dvel;
+    uint4 *raw, *items;
+    uint2 *cand, *tiled;
+    unsigned int *start, *state, *sums, *keys, *ranks;
+    size_t icap, bcap;
+    unsigned int buckets;
+    GridWork(unsigned int *work, long long bodies, int max_end)
+    {
+        buckets = gi_grid_buckets(bodies);
+        icap = gi_dense_item_capacity(bodies);
+        bcap = gi_dense_bucket_capacity(bodies);
+        spos = reinterpret_cast<float4 *>(work);
+        svel = spos + bodies;
+        dpos = svel + bodies;
+        dvel = dpos + bodies;
+        raw = reinterpret_cast<uint4 *>(dvel + bodies);
+        items = raw + icap;
+        cand = reinterpret_cast<uint2 *>(items + icap);
+        tiled = cand + bcap;
+        start = reinterpret_cast<unsigned int *>(tiled + bcap);
+        state = start + buckets + 1;
+        sums = state + buckets;
+        keys = sums + 9216;
+        ranks = keys + max_end;
+    }
+    GridView view() const { return GridView{spos, svel, start}; }
+};
+// Sets the grid and row fields of the table and its runs.
+void gi_grid_runs(LaunchTable &tab);
+// The contact pass, in this order: the grid (with the tiled path's work
+// items); the row path, here or in gi_launch_pair_force; the tiled path.
+// delta receives every body's correction.  ctr: gi::kCtrWords words, zero on
+// entry of the first.  clusters: build the grids of runs below 131,072 bodies
+// with one thread-block cluster each (see grid_cluster_kernel).
+cudaError_t gi_launch_grid(const float4 *pos, const float4 *vel, const LaunchTable &tab,
+                           const GridWork &g, long long *delta, unsigned int *ctr, int nsm,
+                           bool clusters, cudaStream_t s);
+cudaError_t gi_launch_rows(const float4 *pos, const float4 *vel, const LaunchTable &tab,
+                           const GridWork &g, long long *delta, cudaStream_t s);
+cudaError_t gi_launch_tiles(const LaunchTable &tab, const GridWork &g, long long *delta,
+                            unsigned int *ctr, int nsm, cudaStream_t s);
+
+// Asks once per device (known: its flags) for the largest shared-memory
+// carveout of a kernel.  Kernels that are to share an SM need the same one: an
+// SM changes its carveout only when it is empty.
+inline cudaError_t gi_full_carveout(const void *kernel, std::atomic<int> (&known)[64])
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || (dev >= 0 && dev < 64 && known[dev].load())) return e;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess && dev >= 0 && dev < 64) known[dev].store(1);
+    return e;
+}
 
 // gi_aux.cu
 cudaError_t gi_launch_move(float4 *pos, float4 *vel, const float4 *force,
@@ -203,8 +277,8 @@ int gi_internal_collision_pairdev(const gi_force_collision_consts *c, PairDev *d
 // Device scratch bytes one run of n bodies needs in `ctx` (admission estimate).
 long long gi_internal_scratch_bytes(gi_ctx *ctx, int n);
 // The paired far field's decomposition of one run of n bodies with 2^pcl
-// j-chunks per work item, its items numbered from item_start: fills the
-// run's pcl ... far_inv and item_start, returns its work items.
+// j-chunks per work item, its CTAs numbered from item_start: fills the run's
+// pcl ... far_inv and item_start, returns its CTAs.
 long long gi_internal_pair_run(RunDev &d, int n, int pcl, const PairDev &p, long long item_start);
 // log2 of the j-chunks per item of a run of n bodies without a tuning table.
 int gi_internal_pair_default_pcl(int n);

@@ -14,7 +14,7 @@
 // For them, gi_forces_collision_noalloc computes the same forces, bit for bit
 // (the same kernels with the same default decomposition), with all of its
 // scratch in one statically allocated device array, g_noalloc_scratch, of
-// GI_NOALLOC_BYTES (8 MiB; the largest run takes 4.3 MiB of it).  Every GPU that loads the library holds that
+// GI_NOALLOC_BYTES (8 MiB; the largest run takes 5.6 MiB of it).  Every GPU that loads the library holds that
 // array until the process exits.  The array limits a call to
 // GI_NOALLOC_MAX_BODIES (32,768) bodies; larger calls are refused.
 //
@@ -48,7 +48,9 @@ namespace {
 constexpr size_t kMaxBodies = GI_NOALLOC_MAX_BODIES;
 constexpr size_t kTriple = 3 * sizeof(long long);  // one int64 triple per body
 constexpr size_t kSumOff = 0;                         // far-field sums (paired kernel)
-constexpr size_t kDeltaOff = kSumOff + kTriple * kMaxBodies;  // contact corrections
+constexpr size_t kCtrRoom = 256;  // the contact pass's counters, behind the sums
+static_assert(gi::kCtrWords * sizeof(unsigned int) <= kCtrRoom, "the counters must fit");
+constexpr size_t kDeltaOff = kSumOff + kTriple * kMaxBodies + kCtrRoom;  // contact corrections
 constexpr size_t kGridOff = kDeltaOff + kTriple * kMaxBodies;  // the cell grid
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -159,6 +161,7 @@ extern "C" int gi_forces_collision_noalloc(const float *pos, const float *vel, f
                                                  tab.params[0], 0);
     tab.nruns = 1;
     tab.nitems = (int)items;
+    gi_grid_runs(tab);
     tab.sep_test = GI_SEP_REF_INT;
     tab.dense_min = 256;
 
@@ -178,12 +181,17 @@ extern "C" int gi_forces_collision_noalloc(const float *pos, const float *vel, f
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return gi_internal_fail(GI_ERR_CUDA, "device query failed");
     cudaStream_t s = (cudaStream_t)stream;
-    // The far-field sums must start at zero; the array keeps whatever the
-    // previous call left, so clear them in stream order.
-    if (cudaMemsetAsync(sums, 0, kTriple * (size_t)n, s) != cudaSuccess)
+    // The far-field sums and the contact pass's counters must start at zero;
+    // the array keeps whatever the previous call left, so clear them in stream
+    // order.
+    unsigned int *ctr = reinterpret_cast<unsigned int *>(sums + 3 * (size_t)n);
+    if (cudaMemsetAsync(sums, 0, kTriple * (size_t)n + gi::kCtrWords * sizeof(unsigned int), s) !=
+        cudaSuccess)
         return gi_internal_fail(GI_ERR_CUDA, "clearing the static scratch sums failed");
-    if (gi_launch_contacts(reinterpret_cast<const float4 *>(pos), reinterpret_cast<const float4 *>(vel),
-                           tab, n, n, grid, delta, nsm, s) != cudaSuccess)
+    const float4 *p4 = reinterpret_cast<const float4 *>(pos), *v4 = reinterpret_cast<const float4 *>(vel);
+    const GridWork g(grid, n, n);
+    if (gi_launch_grid(p4, v4, tab, g, delta, ctr, nsm, true, s) != cudaSuccess ||
+        gi_launch_tiles(tab, g, delta, ctr, nsm, s) != cudaSuccess)
         return gi_internal_fail(GI_ERR_CUDA, "contact pass launch failed");
     ForceArgs a;
     std::memset(&a, 0, sizeof a);
@@ -192,7 +200,8 @@ extern "C" int gi_forces_collision_noalloc(const float *pos, const float *vel, f
     a.force = reinterpret_cast<float4 *>(force);
     a.delta = delta;
     a.fsum_fx = sums;
-    if (gi_launch_pair_force(a, tab, s) != cudaSuccess)
+    a.fsum_plane = (size_t)n;
+    if (gi_launch_pair_force(a, tab, g, delta, true, s) != cudaSuccess)
         return gi_internal_fail(GI_ERR_CUDA, "force kernel launch failed");
     if (gi_launch_pair_finish(GI_EPI_FORCE, a, tab, n, nsm, s) != cudaSuccess)
         return gi_internal_fail(GI_ERR_CUDA, "epilogue launch failed");

@@ -1,0 +1,68 @@
+"""The contact pass's grid builds (none, one cluster per run, grid-wide) and
+the far field's splits of short runs, at the run sizes where the library
+changes from one to the next: a run's forces are the same bits alone and
+beside a run that takes the grid-wide build, and match the FP64 oracle."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+FORCE_TOL = 1e-5
+
+
+def _dev(torch, a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def _aliased(seed, n):
+    """Bodies whose cells meet on the torus of buckets: a crowded clump, copies
+    of its cells whole torus widths away (16 to 256 cells, each axis), singles
+    strewn over the aliases, and bodies at the cells' range limits."""
+    rng = np.random.default_rng(seed)
+    pos = np.zeros((n, 4), np.float32)
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    x = d * 2.2 * rng.uniform(size=(n, 1)) ** 0.6
+    part = rng.uniform(size=n)
+    far = part > 0.6
+    shift = rng.choice([-256, -64, -32, -16, 0, 16, 32, 64, 128], size=(n, 3))
+    x[far] += shift[far]
+    gas = part > 0.8  # sparse elsewhere, so that the oracle's sums stay plain
+    x[gas] = rng.uniform(-60, 60, size=(gas.sum(), 3))
+    pos[:, :3] = x
+    pos[:3, :3] = [[3e9, 0, 0], [-3e9, 1, 1], [3e9, 0.25, 0.25]]
+    vel = np.zeros((n, 4), np.float32)
+    vel[:, :3] = rng.normal(scale=1.5, size=(n, 3))
+    return pos, vel
+
+
+@pytest.mark.parametrize("n", [1, 9, 3072, 3073, 4096, 4097, 6145, 12287, 12288, 32768, 65535, 65536,
+                               131071])
+def test_sizes_at_path_limits(gi, orc, torch_cuda, n):
+    import gi_workloads as wl
+    torch = torch_cuda
+    p = wl.params(gi)
+    ctx = gi.Context(0)
+    pos, vel = _aliased(n, n) if n > 16 else (np.zeros((n, 4), np.float32), np.zeros((n, 4), np.float32))
+    pos[:, :3] += np.arange(n)[:, None] * np.float32(1e-3) if n <= 16 else 0
+    nfe = n // 7
+    big, bvel, bfe = gi.ic_uniform_ball(5, 131072, 60.0)
+    run = wl.run_desc(gi, 0, n, nfe)
+    dp, dv = _dev(torch, np.concatenate([pos, big])), _dev(torch, np.concatenate([vel, bvel]))
+    alone, both = torch.zeros_like(dp), torch.zeros_like(dp)
+    ctx.forces(dp.data_ptr(), dv.data_ptr(), alone.data_ptr(), [run], p)
+    ctx.forces(dp.data_ptr(), dv.data_ptr(), both.data_ptr(), [run, wl.run_desc(gi, n, 131072, bfe)], p)
+    torch.cuda.synchronize()
+    assert torch.equal(alone[:n], both[:n])
+    idx = np.unique(np.linspace(0, n - 1, 96).astype(np.int32))
+    f64, _ = orc.forces_fp64(pos, vel, [run], p, idx=idx)
+    got = alone.cpu().numpy()[idx, :3]
+    if n > 1:
+        assert rel_l2(got, f64) < FORCE_TOL
+    else:
+        assert not got.any()
+    ctx.close()
