@@ -1135,7 +1135,7 @@ def run_ours(a):
             "fp32_tflops": conventional, "e2e": e2e, "roofline": roof, "cpu_baseline": cpu,
             "ref_gpu": refgpu, "accuracy": accuracy, "collision_phase": collision,
             "hbm": hbm, "large_n": large, "sweep": sweep,
-            "serve": serve, "clocks": clk, "gpu_launches": 14 * a.steps,
+            "serve": serve, "clocks": clk, "gpu_launches": 5 * a.steps,
             "wall_s_timed_region": t_wall, "state_finite": state_ok,
             "step_ms_min_max": [min(step_ms), max(step_ms)],
         }

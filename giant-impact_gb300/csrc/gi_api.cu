@@ -850,10 +850,12 @@ static int convert_params(const gi_pair_params *params, int nparams, std::vector
 // uniform balls (default tuning): the side-by-side pass takes 33 % off at
 // n = 8,192, 5 % at 49,152, 2 % at 98,304, and adds 5 % at 131,072.
 constexpr long long kOverlapMaxPairs = 1LL << 34;
-// Paired far field: tables of fewer pairs run everything on the caller's
-// stream, their far field being shorter than the events between streams and
-// the waiting for room cost.
-constexpr long long kBesideMinPairs = 400000000LL;
+// Paired far field: tables of fewer pairs (n = 7,000) run everything on the
+// caller's stream, their far field being shorter than what the events between
+// streams and the waiting for room cost.  Measured, us a step (settled bodies,
+// side by side / one stream): n = 4,500 49 / 48, 6,000 53 / 52, 8,000 61 / 63,
+// 11,000 66 / 82, 20,000 141 / 165, 66,000 1,062 / 1,098.
+constexpr long long kBesideMinPairs = 50000000LL;
 // Far-field CTAs per SM while the contact pass runs beside it.  Measured on
 // the 66,000-body impact (ms per fused step, settled / collision phase):
 // 3 CTAs 1.72 / 2.60, 4: 1.68 / 2.57, 6: 1.68 / 2.59, 8: 1.67 / 2.54; the

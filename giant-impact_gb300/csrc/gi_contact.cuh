@@ -315,7 +315,7 @@ __device__ __forceinline__ unsigned int bucket_tiled(const Torus &T, const unsig
 // What bounds it is the issue rate: at 66,000 settled bodies (about 150
 // candidates and 18 contacts a body) one warp per body, with its own 27
 // bucket look-ups, a candidate search over them and half-empty evaluations,
-// took 70 us alone, this path @@ROW@@.
+// took 70 us alone, this path 31.
 constexpr int kRowStage = 128;  // candidates staged at a time
 constexpr int kRowList = 512;   // hits listed: 16 per lane before they are drained
 constexpr int kRowLaw = 4;      // hits of a lane evaluated at a time
