@@ -284,8 +284,6 @@ struct gi_ctx {
     double *diag_work = nullptr;
     double *diag_host = nullptr;  // pinned: the result's read-back
     int diag_blocks1 = 0, diag_blocks2 = 0;
-    double *pot_buf = nullptr;
-    size_t pot_cap = 0;
     void *work = nullptr;     // workspace of the synchronous calls (gi_internal_ctx_workspace)
     void *work_pinned = nullptr;
     size_t work_cap = 0;
@@ -340,7 +338,6 @@ static void ctx_free(gi_ctx *c)
     cudaFree(c->mirror2_vel);
     cudaFree(c->diag_work);
     cudaFreeHost(c->diag_host);
-    cudaFree(c->pot_buf);
     cudaFree(c->work);
     cudaFreeHost(c->work_pinned);
 }
@@ -602,14 +599,15 @@ static int pair_stride(long long items, int nblocks)
 // A short warp pays the staging and the i-side atomics for fewer pairs, which
 // costs a batch of such runs 2 to 8 %, so the cut is no finer than a lone run
 // needs.
-static void pair_shape(int n, int pcl, int *ipl, int *tpi)
+static void pair_shape(int n, int pcl, int want, int *ipl, int *tpi)
 {
-    *ipl = n <= 3072 ? 1 : n <= 6144 ? 2 : 3;
-    const int cut = n < 12288 ? 2 : n < kPairSplitN ? 1 : 0;
+    *ipl = want ? want : n <= 3072 ? 1 : n <= 6144 ? 2 : 3;
+    const int cut = want ? 0 : n < 12288 ? 2 : n < kPairSplitN ? 1 : 0;
     *tpi = gi::kPairRowsLog2 - 5 - *ipl + std::min(cut, pcl);
 }
 
-long long gi_internal_pair_run(RunDev &d, int n, int pcl, const PairDev &p, long long item_start)
+long long gi_internal_pair_run(RunDev &d, int n, int pcl, const PairDev &p, long long item_start,
+                               int ipl)
 {
     d.ipt = gi::kPairIpl;
     d.pcl = pcl;
@@ -621,7 +619,7 @@ long long gi_internal_pair_run(RunDev &d, int n, int pcl, const PairDev &p, long
     const long long ri = pair_items(n, pcl);
     d.pitems = (int)std::min(ri, 0x7fffffffLL);
     d.pstride = pair_stride(ri, d.pnb);
-    pair_shape(n, pcl, &d.pipl, &d.ptpi);
+    pair_shape(n, pcl, ipl, &d.pipl, &d.ptpi);
     return ri << d.ptpi;
 }
 
@@ -1336,6 +1334,12 @@ extern "C" int gi_diag_fp64(gi_ctx *c, const float *pos, const float *vel,
     return GI_OK;
 }
 
+// Runs up to this size take every ordered pair (potential_tile): their sums of
+// 128 are too few for the rounding of other ones to average out to 1e-9 (7e-10
+// at 10,000 bodies, 2e-10 from 13,000 on), and a call takes 110 us at 8,000
+// either way (before: 550).
+constexpr int kPotentialOneSided = 12288;
+
 extern "C" int gi_potential_fp64(gi_ctx *c, const float *pos, const gi_run *runs, int nruns,
                                  const gi_pair_params *params, int nparams, double *out,
                                  void *stream)
@@ -1349,47 +1353,44 @@ extern "C" int gi_potential_fp64(gi_ctx *c, const float *pos, const gi_run *runs
     if ((st = check_body_ptr(pos, "pos"))) return st;
     DeviceGuard g(c->device);
     cudaStream_t s = (cudaStream_t)stream;
-    std::vector<double> host;
     for (int r0 = 0; r0 < nruns; r0 += GI_MAX_RUNS) {
         LaunchTable t;
         std::memset(&t, 0, sizeof t);
-        std::vector<int> idx;
-        int blocks = 0;
+        int idx[GI_MAX_RUNS];
+        long long ctas = 0;
         for (int r = r0; r < std::min(nruns, r0 + GI_MAX_RUNS); ++r) {
             if (runs[r].n <= 0) continue;
+            idx[t.nruns] = r;
             RunDev &d = t.runs[t.nruns++];
             d.offset = runs[r].offset;
             d.n = runs[r].n;
             d.nfe = runs[r].nfe;
             d.param = runs[r].params;
-            d.item_start = blocks;
-            blocks += (runs[r].n + GI_NT - 1) / GI_NT;
-            idx.push_back(r);
+            if (d.n <= kPotentialOneSided) {
+                d.item_start = (int)std::min(ctas, 0x7fffffffLL);
+                d.pitems = ((d.n + 31) / 32) * ((d.n + 127) / 128);
+                ctas += d.pitems;
+                continue;
+            }
+            // the far field's items, all rows eight to a lane
+            ctas += gi_internal_pair_run(d, d.n, gi_internal_pair_default_pcl(d.n), pd[d.param], ctas, 3);
         }
         if (!t.nruns) continue;
-        t.nitems = blocks;
+        if (ctas > 0x7fffffffLL) return fail(GI_ERR_BAD_SIZE, "too many work items");
+        t.nitems = (int)ctas;
         for (size_t m = 0; m < pd.size(); ++m) t.params[m] = pd[m];
-        if ((size_t)blocks > c->pot_cap) {
-            GI_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
-            cudaFree(c->pot_buf);
-            c->pot_buf = nullptr;
-            c->pot_cap = 0;
-            GI_CUDA(cudaMalloc(&c->pot_buf, (size_t)blocks * sizeof(double)), "cudaMalloc potential");
-            c->pot_cap = blocks;
-        }
-        GI_CUDA(gi_launch_potential((const float4 *)pos, t, c->pot_buf, blocks, s), "potential launch");
-        host.resize(blocks);
-        GI_CUDA(cudaMemcpyAsync(host.data(), c->pot_buf, (size_t)blocks * sizeof(double),
-                                cudaMemcpyDeviceToHost, s),
-                "D2H potential");
-        GI_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
-        for (int k = 0; k < t.nruns; ++k) {
-            const int b0 = t.runs[k].item_start;
-            const int b1 = (k + 1 < t.nruns) ? t.runs[k + 1].item_start : blocks;
-            double u = 0.0;
-            for (int b = b0; b < b1; ++b) u += host[b];
-            out[idx[k]] = u;
-        }
+        void *work = nullptr, *pinned = nullptr;
+        const size_t head = GI_MAX_RUNS * sizeof(double);
+        if ((st = gi_internal_ctx_workspace(c, head + (size_t)ctas * sizeof(double), &work, &pinned)))
+            return st;
+        double *res = static_cast<double *>(work), *host = static_cast<double *>(pinned);
+        cudaError_t e = gi_launch_potential((const float4 *)pos, t, res + GI_MAX_RUNS, res, s);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(host, res, t.nruns * sizeof(double), cudaMemcpyDeviceToHost, s);
+        const cudaError_t es = cudaStreamSynchronize(s);  // the workspace is idle again
+        if (e == cudaSuccess) e = es;
+        if (e != cudaSuccess) return cuda_fail(e, "potential");
+        for (int k = 0; k < t.nruns; ++k) out[idx[k]] = host[k];
     }
     return GI_OK;
 }

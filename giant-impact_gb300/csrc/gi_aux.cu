@@ -1,5 +1,5 @@
 // gi_aux.cu -- the memory-bound kernels around the force pass: kick-drift,
-// FP64 diagnostic reductions, the pair potential, and the FFMA throughput
+// FP64 diagnostic reductions, and the FFMA throughput
 // microbenchmark that gives the force kernel its roofline denominator.
 #include <algorithm>
 
@@ -346,77 +346,6 @@ diag_pass2(const float4 *__restrict__ pos, const float4 *__restrict__ vel,
     out[7] = s[0]; out[8] = s[1]; out[9] = s[2];
 }
 
-// -------------------------------------------------------------- potential --
-// Per i-block of 128 bodies, sum over every j of the run of U(r_ij):
-// far pairs -gm_i gm_j / r (FP32, rsqrt refined by one Newton step), contact
-// pairs the full-K polynomial; 128-term tiles folded in FP64.  One double
-// per block (already halved), summed by the host in block order.
-__global__ void __launch_bounds__(GI_NT)
-potential_kernel(const float4 *__restrict__ pos, const __grid_constant__ LaunchTable tab,
-                 double *__restrict__ per_block)
-{
-    __shared__ float4 sP[GI_NT];
-    __shared__ double sRed[GI_NT / 32];
-    const int tid = threadIdx.x;
-    // Locate the run: runs[r].item_start is the first block of run r.
-    int lo = 0, hi = tab.nruns - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (tab.runs[mid].item_start <= (int)blockIdx.x) lo = mid;
-        else hi = mid - 1;
-    }
-    const RunDev &R = tab.runs[lo];
-    const PairDev &P = tab.params[R.param];
-    const int rbeg = R.offset, rend = R.offset + R.n, sw = R.offset + R.nfe;
-    const int i = rbeg + (blockIdx.x - R.item_start) * GI_NT + tid;
-    const bool valid = i < rend;
-    float xi = GI_FAR_I, yi = GI_FAR_I, zi = GI_FAR_I;
-    if (valid) { const float4 p = pos[i]; xi = p.x; yi = p.y; zi = p.z; }
-    const bool ife = i < sw;
-    double acc = 0.0;
-    for (int jt = rbeg; jt < rend; jt += GI_NT) {
-        const int j = jt + tid;
-        float4 pj;
-        if (j < rend) { pj = pos[j]; pj.w = (j < sw) ? P.gm_fe : P.gm_si; }
-        else pj = make_float4(GI_FAR_J, GI_FAR_J, GI_FAR_J, 0.0f);
-        __syncthreads();
-        sP[tid] = pj;
-        __syncthreads();
-        float far = 0.0f, near = 0.0f;
-#pragma unroll 4
-        for (int jj = 0; jj < GI_NT; ++jj) {
-            const float4 q = sP[jj];
-            const float dx = q.x - xi, dy = q.y - yi, dz = q.z - zi;
-            const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
-            const bool c = r2 < 1.0f;
-            // Contact pairs (and the self pair, r2 == 0) are taken out of the
-            // far sum; rr keeps rsqrt finite for them.
-            const float rr = c ? 1.0f : r2;
-            float ri = rsqrtf(rr);
-            ri = ri * __fmaf_rn(-0.5f * rr, ri * ri, 1.5f);  // one Newton-Raphson step
-            far = __fmaf_rn(c ? 0.0f : q.w, ri, far);
-            if (c && (jt + jj) != i && valid) {
-                const int test = ife + ((jt + jj) < sw);
-                const float G = P.G[test], K = P.K[test];
-                const float r = __fsqrt_rn(r2);
-                const float u = -G + G * (r - 1.0f) - K * (r - r * r * r * (1.0f / 3.0f) - 2.0f / 3.0f);
-                near += u;
-            }
-        }
-        const float gmi = ife ? P.gm_fe : P.gm_si;
-        acc += -(double)gmi * (double)far + (double)near;
-    }
-    if (!valid) acc = 0.0;
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if ((tid & 31) == 0) sRed[tid >> 5] = acc;
-    __syncthreads();
-    if (tid == 0) {
-        double t = 0.0;
-        for (int w = 0; w < GI_NT / 32; ++w) t += sRed[w];
-        per_block[blockIdx.x] = 0.5 * t;
-    }
-}
-
 // ------------------------------------------------------------ FFMA peak --
 // Eight independent FMA chains per thread; 2 flops per FMA.
 __global__ void __launch_bounds__(256) ffma_peak_kernel(float *sink, int iters)
@@ -486,14 +415,6 @@ cudaError_t gi_launch_diag(const float4 *pos, const float4 *vel,
     gi::diag_pass2<<<nblocks2, 256, 0, s>>>(pos, vel, label, scope, run.offset, run.n, run.nfe,
                                             fe_blocks(nblocks2), mass_fe, mass_si, out_dev, work,
                                             ticket + 1);
-    return cudaGetLastError();
-}
-
-cudaError_t gi_launch_potential(const float4 *pos, const LaunchTable &tab,
-                                double *per_block, int nblocks, cudaStream_t s)
-{
-    if (nblocks <= 0) return cudaSuccess;
-    gi::potential_kernel<<<nblocks, GI_NT, 0, s>>>(pos, tab, per_block);
     return cudaGetLastError();
 }
 

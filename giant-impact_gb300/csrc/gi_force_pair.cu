@@ -162,6 +162,25 @@ struct PairSmem {
     float si[3][kPairWarpRows];
 };
 
+// Chunk c of the run (its bodies from pos on) into place `at`.
+__device__ __forceinline__ void pair_stage(PairSmem &sm, const float4 *__restrict__ pos,
+                                           const RunDev &R, const PairDev &P, int c, int at, int lane)
+{
+    const int ja = c * kPairChunk + lane, jb = ja + 32;
+    float4 pa = make_float4(GI_FAR_J, GI_FAR_J, GI_FAR_J, 0.0f), pb = pa;
+    float ga = 0.0f, gb = 0.0f;
+    if (ja < R.n) {
+        pa = __ldg(&pos[ja]);
+        ga = ja < R.nfe ? P.gm_fe : P.gm_si;
+    }
+    if (jb < R.n) {
+        pb = __ldg(&pos[jb]);
+        gb = jb < R.nfe ? P.gm_fe : P.gm_si;
+    }
+    sm.cxy[at * 32 + lane] = make_float4(pa.x, pb.x, pa.y, pb.y);
+    sm.czg[at * 32 + lane] = make_float4(pa.z, pb.z, ga, gb);
+}
+
 __device__ __forceinline__ void add_fx(long long *p, float v)
 {
     atomicAdd(reinterpret_cast<unsigned long long *>(p), (unsigned long long)__float2ll_rn(v));
@@ -202,21 +221,7 @@ __device__ __forceinline__ void pair_rows(PairSmem &sm, const ForceArgs &a, cons
     for (int cb = c0; cb < c1; cb += kPairStage) {
         const int ce = min(cb + kPairStage, c1);
         __syncwarp();  // the previous chunks are consumed
-        for (int c = cb; c < ce; ++c) {
-            const int ja = c * kPairChunk + lane, jb = ja + 32;
-            float4 pa = make_float4(GI_FAR_J, GI_FAR_J, GI_FAR_J, 0.0f), pb = pa;
-            float ga = 0.0f, gb = 0.0f;
-            if (ja < n) {
-                pa = __ldg(&a.pos[rbeg + ja]);
-                ga = ja < nfe ? P.gm_fe : P.gm_si;
-            }
-            if (jb < n) {
-                pb = __ldg(&a.pos[rbeg + jb]);
-                gb = jb < nfe ? P.gm_fe : P.gm_si;
-            }
-            sm.cxy[(c - cb) * 32 + lane] = make_float4(pa.x, pb.x, pa.y, pb.y);
-            sm.czg[(c - cb) * 32 + lane] = make_float4(pa.z, pb.z, ga, gb);
-        }
+        for (int c = cb; c < ce; ++c) pair_stage(sm, a.pos + rbeg, R, P, c, c - cb, lane);
         __syncwarp();
 #pragma unroll 1
         for (int c = cb; c < ce; ++c) {
@@ -290,13 +295,11 @@ __device__ __forceinline__ void pair_task(PairSmem &sm, const ForceArgs &a, cons
     }
 }
 
-__device__ __forceinline__ void pair_item(PairSmem &sm, const ForceArgs &a, const LaunchTable &tab,
-                                          int cta, int lane)
+// CTA `cta` of run R: its first row wi0 and its chunks [c0, c1) (none when
+// they are all before the rows, or there are no rows).
+__device__ __forceinline__ void pair_decode(const RunDev &R, int cta, int &wi0, int &c0, int &c1)
 {
-    const RunDev &R = tab.runs[find_run(tab, cta)];
-    const PairDev &P = tab.params[R.param];
-    // ---- decode: item slot, rows and chunks of the item; then (i-block, item
-    // of the block)
+    // item slot, rows and chunks of the item; then (i-block, item of the block)
     const int local = cta - R.item_start;
     const int slot = local >> R.ptpi, part = local & ((1 << R.ptpi) - 1);
     const int rlog = kPairRowsLog2 - 5 - R.pipl;  // log2 of the row groups of an i-block
@@ -308,12 +311,22 @@ __device__ __forceinline__ void pair_item(PairSmem &sm, const ForceArgs &a, cons
         if (pair_items_before(mid, k0, q) <= t) lo = mid;
         else hi = mid - 1;
     }
-    const int wi0 = lo * kPairRows + ((part & ((1 << rlog) - 1)) << (5 + R.pipl));
+    wi0 = lo * kPairRows + ((part & ((1 << rlog) - 1)) << (5 + R.pipl));
     const int cpt = 1 << (R.pcl - (R.ptpi - rlog));  // chunks of this warp
     const int cb = lo * kPairBlockChunks + ((int)(t - pair_items_before(lo, k0, q)) << R.pcl) +
                    (part >> rlog) * cpt;
-    const int c0 = max(cb, wi0 / kPairChunk), c1 = min(cb + cpt, R.pnc);
-    if (c0 >= c1) return;  // wholly before the rows, or no rows
+    c0 = max(cb, wi0 / kPairChunk);
+    c1 = min(cb + cpt, R.pnc);
+}
+
+__device__ __forceinline__ void pair_item(PairSmem &sm, const ForceArgs &a, const LaunchTable &tab,
+                                          int cta, int lane)
+{
+    const RunDev &R = tab.runs[find_run(tab, cta)];
+    const PairDev &P = tab.params[R.param];
+    int wi0, c0, c1;
+    pair_decode(R, cta, wi0, c0, c1);
+    if (c0 >= c1) return;
     if (R.pipl == 3) pair_task<8>(sm, a, R, P, c0, c1, wi0, lane);
     else if (R.pipl == 2) pair_task<4>(sm, a, R, P, c0, c1, wi0, lane);
     else pair_task<2>(sm, a, R, P, c0, c1, wi0, lane);
@@ -341,6 +354,276 @@ pair_force_kernel(const ForceArgs a, const GridView g, long long *__restrict__ d
         contact_rows(sm.row, a.pos, a.vel, g, delta, tab, blockIdx.x);
     else
         pair_item(sm.pair, a, tab, blockIdx.x - rows, threadIdx.x);
+}
+
+// ------------------------------------------------------------- potential --
+// U(r) of every unordered pair once (gi_potential_fp64), over the far field's
+// work items: the same warps, rows and chunks.  No per-body sums, so the
+// chunk's bodies are broadcast from shared memory, two in the halves of a
+// packed register, against the lane's 8 rows.  Per pair the one-sided form's
+// arithmetic: r2 as in the far field, rsqrt of max(r2, 1) refined by one
+// Newton step, rounded, and added with j's mass to the row's FP32 sum of 128
+// bodies, which is folded in FP64 with i's mass.  (That product's rounding is
+// not even for every mass: 2.6e-8 of the sum for sqrt(G) m = 0.4 and none for
+// 1, so the rounding points stay where a sum over ordered pairs has them: 128
+// bodies a sum, and of the pairs of two classes half weighted with either
+// mass.)  Pairs
+// with r2 < 1 are left out of the sum and get the full-K polynomial: a lane
+// that met one looks its step's pairs over.  Chunks on the diagonal take every
+// pair by itself.
+//
+// 12 packed operations, 6 selects and 2 MUFU a step of 64 pairs, 9 of the
+// packed ones with two distinct operands at most, so the register file holds
+// it less than the far field.  A call on 66,000 bodies takes 1.04 to
+// 1.18 ms (every ordered pair, unpacked, in blocks of 128: 5.3).
+
+__device__ __forceinline__ float max_nan(float a, float b)  // NaN if a is
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+__device__ __forceinline__ float rsqrt_refined(float rr)
+{
+    const float ri = rsqrt_mufu(rr);
+    return ri * __fmaf_rn(-0.5f * rr, ri * ri, 1.5f);
+}
+
+// hi + lo += x, hi's rounding kept in lo (TwoSum).
+__device__ __forceinline__ void add_exact(float &hi, float &lo, float x)
+{
+    const float s = __fadd_rn(hi, x), b = __fsub_rn(s, hi);
+    lo += __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b));
+    hi = s;
+}
+
+// The contact potential of one pair, r2 < 1.
+__device__ __forceinline__ float contact_potential(float G, float K, float r2)
+{
+    const float r = __fsqrt_rn(r2);
+    return -G + G * (r - 1.0f) - K * (r - r * r * r * (1.0f / 3.0f) - 2.0f / 3.0f);
+}
+
+// A chunk wholly after the rows: far[k] gathers row k's pairs, weighted with
+// j's mass, or with i's (SWAP); returns the contact potentials.  jfe: Fe
+// bodies of the chunk (its first ones); i0: the lane's first row.
+template <bool SWAP>
+__device__ __forceinline__ float potential_chunk(const float4 *__restrict__ cxy,
+                                                 const float4 *__restrict__ czg, const PairDev &P,
+                                                 int jfe, int i0, int nfe,
+                                                 const float (&nx)[kPairIpl],
+                                                 const float (&ny)[kPairIpl],
+                                                 const float (&nz)[kPairIpl],
+                                                 float2 (&far)[kPairIpl])
+{
+    float near = 0.0f;
+#pragma unroll 1
+    for (int s = 0; s < 32; ++s) {
+        const float4 q = cxy[s], g = czg[s];
+        const float2 X = make_float2(q.x, q.y), Y = make_float2(q.z, q.w), Z = make_float2(g.x, g.y);
+        bool close = false;
+#pragma unroll
+        for (int k = 0; k < kPairIpl; ++k) {
+            const float2 dx = __fadd2_rn(X, make_float2(nx[k], nx[k]));
+            const float2 dy = __fadd2_rn(Y, make_float2(ny[k], ny[k]));
+            const float2 dz = __fadd2_rn(Z, make_float2(nz[k], nz[k]));
+            float2 r2 = __fmul2_rn(dy, dy);
+            r2 = __ffma2_rn(dx, dx, r2);
+            r2 = __ffma2_rn(dz, dz, r2);
+            const bool cx = r2.x < 1.0f, cy = r2.y < 1.0f;  // not in the far sum
+            close |= cx | cy;
+            const float gk = i0 + k * 32 < nfe ? P.gm_fe : P.gm_si;
+            const float2 gm = make_float2(cx ? 0.0f : SWAP ? gk : g.z, cy ? 0.0f : SWAP ? gk : g.w);
+            const float2 rr = make_float2(max_nan(r2.x, 1.0f), max_nan(r2.y, 1.0f));
+            const float2 ri = make_float2(rsqrt_mufu(rr.x), rsqrt_mufu(rr.y));
+            const float2 h = __fmul2_rn(rr, make_float2(-0.5f, -0.5f));
+            const float2 t = __ffma2_rn(h, __fmul2_rn(ri, ri), make_float2(1.5f, 1.5f));
+            far[k] = __ffma2_rn(gm, __fmul2_rn(ri, t), far[k]);
+        }
+        if (close) {
+#pragma unroll
+            for (int k = 0; k < kPairIpl; ++k) {
+                const float2 dx = __fadd2_rn(X, make_float2(nx[k], nx[k]));
+                const float2 dy = __fadd2_rn(Y, make_float2(ny[k], ny[k]));
+                const float2 dz = __fadd2_rn(Z, make_float2(nz[k], nz[k]));
+                float2 r2 = __fmul2_rn(dy, dy);
+                r2 = __ffma2_rn(dx, dx, r2);
+                r2 = __ffma2_rn(dz, dz, r2);
+                const int ic = i0 + k * 32 < nfe;
+                if (r2.x < 1.0f)
+                    near += contact_potential(P.G[ic + (s < jfe)], P.K[ic + (s < jfe)], r2.x);
+                if (r2.y < 1.0f)
+                    near += contact_potential(P.G[ic + (s + 32 < jfe)], P.K[ic + (s + 32 < jfe)], r2.y);
+            }
+        }
+    }
+    return near;
+}
+
+// Short runs (pipl 0): every ordered pair, a lane's body against a tile of 128;
+// a run of 2,000 bodies has too few sums of 128 for their rounding to average
+// out, so its sums are the same ones whatever the decomposition.
+__device__ __forceinline__ double potential_tile(PairSmem &sm, const float4 *__restrict__ run,
+                                                 const RunDev &R, const PairDev &P, int local,
+                                                 int lane)
+{
+    float4 *const tile = sm.cxy;  // x, y, z, gm
+    const int tiles = (R.n + 127) / 128, i = local / tiles * 32 + lane, jt = local % tiles * 128;
+    const bool ife = i < R.nfe;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        const int j = jt + 32 * v + lane;
+        float4 p = make_float4(GI_FAR_J, GI_FAR_J, GI_FAR_J, 0.0f);
+        if (j < R.n) {
+            p = __ldg(&run[j]);
+            p.w = j < R.nfe ? P.gm_fe : P.gm_si;
+        }
+        tile[32 * v + lane] = p;
+    }
+    float4 p = make_float4(GI_FAR_I, GI_FAR_I, GI_FAR_I, 0.0f);
+    if (i < R.n) p = __ldg(&run[i]);
+    __syncwarp();
+    float far = 0.0f, near = 0.0f;
+#pragma unroll 4
+    for (int s = 0; s < 128; ++s) {
+        const float4 q = tile[s];
+        const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+        const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+        const bool c = r2 < 1.0f;  // contact pairs and the body itself: not in the far sum
+        far = __fmaf_rn(c ? 0.0f : q.w, rsqrt_refined(c ? 1.0f : r2), far);
+        if (c && jt + s != i && i < R.n) {
+            const int cls = ife + (jt + s < R.nfe);
+            near += contact_potential(P.G[cls], P.K[cls], r2);
+        }
+    }
+    const double u = -(double)(ife ? P.gm_fe : P.gm_si) * (double)far + (double)near;
+    return i < R.n ? 0.5 * u : 0.0;
+}
+
+// One potential per CTA into per_cta (0 for an empty one).
+__global__ void __launch_bounds__(32)
+potential_kernel(const float4 *__restrict__ pos, const __grid_constant__ LaunchTable tab,
+                 double *__restrict__ per_cta)
+{
+    __shared__ PairSmem sm;
+    constexpr int IPL = kPairIpl;
+    const int lane = threadIdx.x;
+    const RunDev &R = tab.runs[find_run(tab, blockIdx.x)];
+    const PairDev &P = tab.params[R.param];
+    const float4 *const run = pos + R.offset;
+    if (R.pipl == 0) {
+        double u = potential_tile(sm, run, R, P, blockIdx.x - R.item_start, lane);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) u += __shfl_down_sync(0xffffffffu, u, o);
+        if (lane == 0) per_cta[blockIdx.x] = u;
+        return;
+    }
+    int wi0, c0, c1;
+    pair_decode(R, blockIdx.x, wi0, c0, c1);
+    double acc = 0.0;
+    const int n = R.n, nfe = R.nfe;
+    const bool imix = wi0 < nfe && nfe < wi0 + 32 * IPL;
+    float nx[IPL], ny[IPL], nz[IPL];
+#pragma unroll
+    for (int k = 0; k < IPL; ++k) {
+        const int i = wi0 + k * 32 + lane;
+        float4 p = make_float4(GI_FAR_I, GI_FAR_I, GI_FAR_I, 0.0f);
+        if (c0 < c1 && i < n) p = __ldg(&run[i]);
+        nx[k] = -p.x;
+        ny[k] = -p.y;
+        nz[k] = -p.z;
+    }
+    const auto class_of = [&](int k) { return (int)(wi0 + k * 32 + lane < nfe); };
+    float2 far[IPL];  // per row, one sum per half: 128 bodies each, then folded
+#pragma unroll
+    for (int k = 0; k < IPL; ++k) far[k] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+    for (int cb = c0; cb < c1; cb += kPairStage) {
+        const int ce = min(cb + kPairStage, c1);
+        __syncwarp();
+        for (int c = cb; c < ce; ++c) pair_stage(sm, run, R, P, c, c - cb, lane);
+        __syncwarp();
+#pragma unroll 1
+        for (int c = cb; c < ce; ++c) {
+            const float4 *cxy = sm.cxy + (c - cb) * 32, *czg = sm.czg + (c - cb) * 32;
+            const int jc0 = c * kPairChunk;
+            // in every other group of four chunks the pairs' roots are weighted
+            // with i's mass, and j's is applied at the fold
+            const int g0 = jc0 & ~255;  // the group's first body
+            const bool swap = (jc0 & 256) && !(g0 < nfe && nfe < g0 + 256) && jc0 >= wi0 + 32 * IPL;
+            float near = 0.0f;
+                if (jc0 < wi0 + 32 * IPL) {  // diagonal: each pair by itself
+#pragma unroll 1
+                for (int s = 0; s < kPairChunk; ++s) {
+                    const int j = jc0 + s;
+                    if (j >= n) break;
+                    const float4 q = cxy[s & 31], g = czg[s & 31];
+                    const float X = s < 32 ? q.x : q.y, Y = s < 32 ? q.z : q.w,
+                                Z = s < 32 ? g.x : g.y, gmj = s < 32 ? g.z : g.w;
+#pragma unroll
+                    for (int k = 0; k < IPL; ++k) {
+                        const int i = wi0 + k * 32 + lane;
+                        if (i >= j) continue;  // each pair once; no rows past the run
+                        const float dx = X + nx[k], dy = Y + ny[k], dz = Z + nz[k];
+                        const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+                        const int cls = (i < nfe) + (j < nfe);
+                        if (r2 < 1.0f) near += contact_potential(P.G[cls], P.K[cls], r2);
+                        else far[k].x = __fmaf_rn(gmj, rsqrt_refined(r2), far[k].x);
+                    }
+                }
+            } else if (swap) {
+                near = potential_chunk<true>(cxy, czg, P, nfe - jc0, wi0 + lane, nfe, nx, ny, nz, far);
+            } else {
+                near = potential_chunk<false>(cxy, czg, P, nfe - jc0, wi0 + lane, nfe, nx, ny, nz, far);
+            }
+            acc += (double)near;
+            const bool diag = jc0 < wi0 + 32 * IPL;
+            if (((c - c0) & (diag ? 1 : 3)) == (diag ? 1 : 3) || c + 1 == c1) {
+                // 128 bodies a sum: the rows' sums without rounding (hi + lo);
+                // each with its own mass where that differs
+                float hi = 0.0f, lo = 0.0f;
+#pragma unroll
+                for (int k = 0; k < IPL; ++k) {
+                    if (imix && !swap) {
+                        acc -= (double)(class_of(k) ? P.gm_fe : P.gm_si) *
+                               ((double)far[k].x + (double)far[k].y);
+                    } else {
+                        add_exact(hi, lo, far[k].x);
+                        add_exact(hi, lo, far[k].y);
+                    }
+                    far[k] = make_float2(0.0f, 0.0f);
+                }
+                const bool fe = swap ? g0 < nfe : wi0 < nfe;
+                acc -= (double)(fe ? P.gm_fe : P.gm_si) * ((double)hi + (double)lo);
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (lane == 0) per_cta[blockIdx.x] = acc;
+}
+
+// Each run's CTAs summed in a fixed order: thread t takes CTAs t, t + 1024,
+// ..., then a fixed shuffle tree and the 32 warps in order.
+__global__ void __launch_bounds__(1024)
+potential_sum_kernel(const __grid_constant__ LaunchTable tab, const double *__restrict__ per_cta,
+                     double *__restrict__ out)
+{
+    __shared__ double sh[32];
+    const RunDev &R = tab.runs[blockIdx.x];
+    const int end = R.item_start + (R.pitems << R.ptpi);
+    double v = 0.0;
+    for (int k = R.item_start + threadIdx.x; k < end; k += 1024) v += per_cta[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < 32; ++w) t += sh[w];
+        out[blockIdx.x] = t;
+    }
 }
 
 // The epilogue: F = fixed-point far field + contact correction, rounded once
@@ -388,5 +671,14 @@ cudaError_t gi_launch_pair_finish(int epi, const ForceArgs &a, const LaunchTable
     if (epi == GI_EPI_FORCE) pair_finish_kernel<GI_EPI_FORCE><<<grid, 256, 0, s>>>(a, tab);
     else if (epi == GI_EPI_STEP) pair_finish_kernel<GI_EPI_STEP><<<grid, 256, 0, s>>>(a, tab);
     else return cudaErrorInvalidValue;
+    return cudaGetLastError();
+}
+
+cudaError_t gi_launch_potential(const float4 *pos, const LaunchTable &tab, double *per_cta,
+                                double *out, cudaStream_t s)
+{
+    if (tab.nitems <= 0) return cudaSuccess;
+    potential_kernel<<<tab.nitems, 32, 0, s>>>(pos, tab, per_cta);
+    potential_sum_kernel<<<tab.nruns, 1024, 0, s>>>(tab, per_cta, out);
     return cudaGetLastError();
 }

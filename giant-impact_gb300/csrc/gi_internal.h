@@ -133,6 +133,10 @@ static_assert(kPairMaxCpi <= kPairBlockChunks && kPairBlockChunks % kPairMaxCpi 
 struct GridWork;
 cudaError_t gi_launch_pair_force(const ForceArgs &a, const LaunchTable &tab, const GridWork &g,
                                  long long *delta, bool with_rows, cudaStream_t s);
+// Pair potentials of the table's runs (planned as for gi_launch_pair_force):
+// one double per CTA in per_cta, one per run in out, in table order.
+cudaError_t gi_launch_potential(const float4 *pos, const LaunchTable &tab, double *per_cta,
+                                double *out, cudaStream_t s);
 cudaError_t gi_launch_pair_finish(int epi, const ForceArgs &a, const LaunchTable &tab, int maxn,
                                   int nsm, cudaStream_t s);
 
@@ -264,9 +268,6 @@ cudaError_t gi_launch_diag(const float4 *pos, const float4 *vel,
                            const RunDev &run, float mass_fe, float mass_si, double *work,
                            int nblocks1, int nblocks2, double *out_dev, int *ticket,
                            cudaStream_t s);
-cudaError_t gi_launch_potential(const float4 *pos, const LaunchTable &tab,
-                                double *per_block, int nblocks_per_run,
-                                cudaStream_t s);
 cudaError_t gi_launch_ffma_peak(float *sink, int blocks, int iters, cudaStream_t s);
 
 // gi_api.cu helpers for the library's other translation units: record an
@@ -278,8 +279,10 @@ int gi_internal_collision_pairdev(const gi_force_collision_consts *c, PairDev *d
 long long gi_internal_scratch_bytes(gi_ctx *ctx, int n);
 // The paired far field's decomposition of one run of n bodies with 2^pcl
 // j-chunks per work item, its CTAs numbered from item_start: fills the run's
-// pcl ... far_inv and item_start, returns its CTAs.
-long long gi_internal_pair_run(RunDev &d, int n, int pcl, const PairDev &p, long long item_start);
+// pcl ... far_inv and item_start, returns its CTAs.  ipl: log2 of the rows a
+// lane holds (0: the far field's choice).
+long long gi_internal_pair_run(RunDev &d, int n, int pcl, const PairDev &p, long long item_start,
+                               int ipl = 0);
 // log2 of the j-chunks per item of a run of n bodies without a tuning table.
 int gi_internal_pair_default_pcl(int n);
 // Device ordinal of a context (-1 for NULL).

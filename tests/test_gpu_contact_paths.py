@@ -66,3 +66,26 @@ def test_sizes_at_path_limits(gi, orc, torch_cuda, n):
     else:
         assert not got.any()
     ctx.close()
+
+
+@pytest.mark.parametrize("n,nfe", [(1, 0), (33, 33), (129, 5), (3000, 0), (12288, 300), (12289, 700), (20011, 20011),
+                                   (33000, 1000)])
+def test_potential_sizes(gi, orc, torch_cuda, n, nfe):
+    """Pair potential at the sizes where its decomposition changes, with the
+    Fe boundary inside a lane group, a chunk, at 0 and at n: the FP64 oracle's
+    to the FP32 pair arithmetic (each term to about 1e-7), and the same bits
+    alone and in a batch."""
+    import gi_workloads as wl
+    torch = torch_cuda
+    p = wl.params(gi)
+    pos, vel, _ = gi.ic_uniform_ball(n, n, max(1.0, (n / 4.0) ** (1 / 3)))
+    other, ovel, ofe = gi.ic_uniform_ball(77, 15000, 30.0)
+    d = _dev(torch, np.concatenate([pos, other]))
+    ctx = gi.Context(0)
+    run, rest = wl.run_desc(gi, 0, n, nfe), wl.run_desc(gi, n, 15000, ofe)
+    alone = ctx.potential(d.data_ptr(), [run], p)[0]
+    both = ctx.potential(d.data_ptr(), [rest, run], p)
+    assert both[1] == alone and ctx.potential(d.data_ptr(), [rest], p)[0] == both[0]
+    want = orc.potential_fp64(pos, [run], p).sum() / 2.0
+    assert abs(alone - want) <= 2e-7 * abs(want)
+    ctx.close()
