@@ -279,11 +279,10 @@ struct gi_ctx {
     float4 *mirror_pos = nullptr, *mirror_vel = nullptr;
     float4 *mirror2_pos = nullptr, *mirror2_vel = nullptr;
     size_t mirror_cap = 0;
-    // 16 doubles per block of the larger diagnostics grid, 16 for the
-    // result, then the passes' two tickets
+    // 16 doubles per block of the diagnostics grid, then the ticket
     double *diag_work = nullptr;
-    double *diag_host = nullptr;  // pinned: the result's read-back
-    int diag_blocks1 = 0, diag_blocks2 = 0;
+    double *diag_host = nullptr;  // pinned: the kernel writes its result there
+    int diag_blocks = 0;
     void *work = nullptr;     // workspace of the synchronous calls (gi_internal_ctx_workspace)
     void *work_pinned = nullptr;
     size_t work_cap = 0;
@@ -303,8 +302,7 @@ static int ctx_init(gi_ctx *c, int device)
                     device, prop.major, prop.minor);
     c->sm_count = prop.multiProcessorCount;
     DeviceGuard g(device);
-    c->diag_blocks1 = gi_diag_blocks(1, c->sm_count);  // shared by the two material classes
-    c->diag_blocks2 = gi_diag_blocks(2, c->sm_count);
+    c->diag_blocks = gi_diag_blocks(c->sm_count);  // shared by the two material classes
     for (int acc : {GI_ACC_KAHAN, GI_ACC_FP32, GI_ACC_FP64})
         for (int p : {1, 2, 4, 8}) {
             const int o = std::min({gi_force_occupancy(p, acc, GI_EPI_FORCE),
@@ -1307,28 +1305,23 @@ extern "C" int gi_diag_fp64(gi_ctx *c, const float *pos, const float *vel,
     if ((st = check_body_ptr(pos, "pos")) || (st = check_body_ptr(vel, "vel"))) return st;
     DeviceGuard g(c->device);
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t nbmax = (size_t)std::max(c->diag_blocks1, c->diag_blocks2);
+    const size_t nb = (size_t)c->diag_blocks;
     if (!c->diag_work) {
-        GI_CUDA(cudaMalloc(&c->diag_work, (nbmax + 2) * 16 * sizeof(double)), "cudaMalloc diag");
+        GI_CUDA(cudaMalloc(&c->diag_work, (nb + 1) * 16 * sizeof(double)), "cudaMalloc diag");
     }
     if (!c->diag_host) {
         GI_CUDA(cudaMallocHost(&c->diag_host, 16 * sizeof(double)), "cudaMallocHost diag");
     }
-    double *out_dev = c->diag_work + nbmax * 16;
-    int *ticket = (int *)(c->diag_work + (nbmax + 1) * 16);
+    int *ticket = (int *)(c->diag_work + nb * 16);
     RunDev rd;
     std::memset(&rd, 0, sizeof rd);
     rd.offset = q.offset;
     rd.n = q.n;
     rd.nfe = q.nfe;
     GI_CUDA(gi_launch_diag((const float4 *)pos, (const float4 *)vel, label, scope, rd,
-                           params->MassFe, params->MassSi, c->diag_work, c->diag_blocks1,
-                           c->diag_blocks2, out_dev, ticket, s),
+                           params->MassFe, params->MassSi, c->diag_work, c->diag_blocks,
+                           c->diag_host, ticket, s),
             "diag launch");
-    // through pinned memory: a copy into the caller's pageable buffer would
-    // be staged by the driver
-    GI_CUDA(cudaMemcpyAsync(c->diag_host, out_dev, 15 * sizeof(double), cudaMemcpyDeviceToHost, s),
-            "D2H diag");
     GI_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
     std::memcpy(out, c->diag_host, 15 * sizeof(double));
     return GI_OK;

@@ -94,12 +94,13 @@ __device__ __forceinline__ void stream_bodies(const float4 *__restrict__ pos,
 
 // The sums of the diagnostics are kept per thread in float-float pairs on
 // the FP32 pipe: a value is hi + lo, about 48 significant bits.  TwoSum and
-// the FMA form of TwoProd are error-free, and every addition renormalises
-// the pair, so a thread's sum of n terms is exact to about n 2^-48 of the
-// terms' magnitudes.  This GPU issues FP64 at a small fraction of its FP32
-// rate: with the per-body work in FP64 the two passes ran at ~850 GB/s, with
-// it on the FP32 pipe they are bound by HBM.  FP64 remains for the block
-// partials and everything after them.
+// the FMA form of TwoProd are error-free, and every addition renormalises the
+// pair, so a thread's sum of n terms is exact to about n 2^-48 of the terms'
+// magnitudes.  (Gathering lo without that is 3 operations of 11 less and 10 to
+// 1,000 times further off in the sums that cancel.)  This GPU
+// issues FP64 at a small fraction of its FP32 rate: with the per-body work in
+// FP64 the sums ran at ~850 GB/s.  FP64 remains for the block partials and
+// everything after them.
 struct FF {
     float hi, lo;
 };
@@ -112,7 +113,7 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
 }
 
 // a += xh + xl, renormalised (|lo| <= ulp(hi) / 2).
-__device__ __forceinline__ void ff_add2(FF &a, float xh, float xl)
+__device__ __forceinline__ void ff_add(FF &a, float xh, float xl)
 {
     float s, e;
     two_sum(a.hi, xh, s, e);
@@ -121,23 +122,11 @@ __device__ __forceinline__ void ff_add2(FF &a, float xh, float xl)
     a.lo = __fsub_rn(e, __fsub_rn(a.hi, s));
 }
 
-__device__ __forceinline__ void ff_add(FF &a, float x) { ff_add2(a, x, 0.0f); }
-
-// a += x * y, the product taken exactly (p + e with e = fma(x, y, -p)).
-__device__ __forceinline__ void ff_add_prod(FF &a, float x, float y)
-{
-    const float p = __fmul_rn(x, y);
-    ff_add2(a, p, __fmaf_rn(x, y, -p));
-}
-
-// x - c for a float x and a double c given as ch + cl (ch = (float)c):
-// TwoSum of x and -ch is exact, cl is folded into the low part.
-__device__ __forceinline__ FF ff_sub_d(float x, float ch, float cl)
+// x - c for floats, exactly.
+__device__ __forceinline__ FF ff_diff(float x, float c)
 {
     FF r;
-    float e;
-    two_sum(x, -ch, r.hi, e);
-    r.lo = __fsub_rn(e, cl);
+    two_sum(x, -c, r.hi, r.lo);
     return r;
 }
 
@@ -154,196 +143,127 @@ __device__ __forceinline__ void ff_add_cross(FF &a, FF u, FF v, FF w, FF z)
     e2 = __fmaf_rn(w.hi, z.lo, __fmaf_rn(w.lo, z.hi, e2));
     float s, t;
     two_sum(p1, -p2, s, t);
-    ff_add2(a, s, __fadd_rn(t, __fsub_rn(e1, e2)));
+    ff_add(a, s, __fadd_rn(t, __fsub_rn(e1, e2)));
 }
 
-__device__ __forceinline__ double ff_value(const FF &a) { return (double)a.hi + (double)a.lo; }
+// The sums of a block's bodies, all of one material class.
+constexpr int kDiagSums = 10;    // x, v (3 each), v.v, r x w (3)
+constexpr int kDiagParts = 11;   // the same times the class mass, then the count
 
-// Sum of the lanes' pairs to lane 0 (float-float), NV of them.
-template <int NV>
-__device__ __forceinline__ void warp_ff_sum(FF (&v)[NV])
+// The whole diagnostic in one pass over the state (32 B per body): with r = x
+// - x0 and w = v - v0 taken from one body of the run (exact as float-float
+// pairs), the sums of m, m x, m v, m v.v and m r x w give the mass, the centre
+// of mass, the momenta, and the angular momentum about the centre of mass
+// relative to its velocity, L = sum m r x w - M rc x wc (impactBasicFunctions.h:
+// 507-652 in double; rc, wc the centre's r and w).  Taking x0 from the run
+// keeps that difference harmless wherever the system is and however it moves.
+// The call, read-back included, takes 108 us on 8.4M bodies and 25 us on 66,000;
+// a first pass for the centre, then a second over the same 32 B, took 144 and
+// 65.  What bounds it is the FP32 pipe beside HBM: 225 operations a body.
+//
+// Each block takes one material class, so the class mass multiplies the
+// block's sums once, in FP64: blocks [0, nbfe) the run's Fe bodies [0, nfe),
+// the others its Si bodies [nfe, n), each class in a grid-stride loop over its
+// own blocks.  Block b's partials are work[16 b ..]; the block that takes the
+// last ticket sums them in a fixed order (a warp per value: lane l takes
+// blocks l, l + 32, ..., then a fixed shuffle tree), so the result is
+// deterministic for a given grid.
+// out = [mass, com3, vcom3, L3, ke, p3, count].
+__global__ void __launch_bounds__(256)
+diag_kernel(const float4 *__restrict__ pos, const float4 *__restrict__ vel,
+            const unsigned char *__restrict__ label, int scope, int off, int n, int nfe, int nbfe,
+            double mfe, double msi, double *__restrict__ work, int *__restrict__ ticket,
+            double *__restrict__ out)
 {
+    const bool fe = (int)blockIdx.x < nbfe;
+    const int k0 = fe ? 0 : nfe, k1 = fe ? nfe : n;
+    const int b = fe ? (int)blockIdx.x : (int)blockIdx.x - nbfe;
+    const int nb = fe ? nbfe : (int)gridDim.x - nbfe;
+    const double m = fe ? mfe : msi;
+    // the run's first body; a component that is not finite counts as 0
+    float x0[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    if (n > 0) {
+        const float4 p = pos[off], u = vel[off];
+        const float c[6] = {p.x, p.y, p.z, u.x, u.y, u.z};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int c = 0; c < NV; ++c) {
-            const float h = __shfl_down_sync(0xffffffffu, v[c].hi, o);
-            const float l = __shfl_down_sync(0xffffffffu, v[c].lo, o);
-            ff_add2(v[c], h, l);
-        }
+        for (int d = 0; d < 6; ++d) x0[d] = fabsf(c[d]) <= 3.0e38f ? c[d] : 0.0f;
     }
-}
-
-// Lane 0 of each warp passes its values (FP64); the block's warps are
-// added in warp order and thread c < NV writes value c of the block to
-// dst.  Then each block takes a ticket: the block that takes the last one
-// returns true, after a fence, so every block's partials are visible to it.
-template <int NV>
-__device__ __forceinline__ bool block_store_last(const double (&v)[NV], double *dst,
-                                                 int *ticket)
-{
-    __shared__ double sh[NV][8];
+    FF v[kDiagSums];
+#pragma unroll
+    for (int c = 0; c < kDiagSums; ++c) v[c] = FF{0.0f, 0.0f};
+    int cnt = 0;
+    stream_bodies(pos, vel, label, scope, off, k0 + b * blockDim.x + threadIdx.x, k1,
+                  nb * blockDim.x, [&](float4 p, float4 u) {
+                      const FF r[3] = {ff_diff(p.x, x0[0]), ff_diff(p.y, x0[1]), ff_diff(p.z, x0[2])};
+                      const FF w[3] = {ff_diff(u.x, x0[3]), ff_diff(u.y, x0[4]), ff_diff(u.z, x0[5])};
+                      const float pp[3] = {p.x, p.y, p.z}, uu[3] = {u.x, u.y, u.z};
+#pragma unroll
+                      for (int d = 0; d < 3; ++d) {
+                          ff_add(v[d], pp[d], 0.0f);
+                          ff_add(v[3 + d], uu[d], 0.0f);
+                          const float q = __fmul_rn(uu[d], uu[d]);
+                          ff_add(v[6], q, __fmaf_rn(uu[d], uu[d], -q));
+                      }
+                      ff_add_cross(v[7], r[1], w[2], r[2], w[1]);
+                      ff_add_cross(v[8], r[2], w[0], r[0], w[2]);
+                      ff_add_cross(v[9], r[0], w[1], r[1], w[0]);
+                      ++cnt;
+                  });
+    // the warp's sums to lane 0, then the block's warps in order
+    __shared__ double part[kDiagParts][8];
     __shared__ int s_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
 #pragma unroll
-        for (int c = 0; c < NV; ++c) sh[c][warp] = v[c];
+    for (int c = 0; c < kDiagSums; ++c) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float h = __shfl_down_sync(0xffffffffu, v[c].hi, o);
+            const float l = __shfl_down_sync(0xffffffffu, v[c].lo, o);
+            ff_add(v[c], h, l);
+        }
+        if (lane == 0) part[c][warp] = (double)v[c].hi + (double)v[c].lo;
     }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) part[kDiagSums][warp] = (double)cnt;
     __syncthreads();
-    if (threadIdx.x < NV) {
+    if (threadIdx.x < kDiagParts) {
         double x = 0.0;
-        const int nw = blockDim.x >> 5;
-        for (int w = 0; w < nw; ++w) x += sh[threadIdx.x][w];
-        dst[threadIdx.x] = x;
+        for (int w = 0; w < 8; ++w) x += part[threadIdx.x][w];
+        work[16 * blockIdx.x + threadIdx.x] = threadIdx.x < kDiagSums ? m * x : x;
     }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
     __syncthreads();
-    if (s_last) __threadfence();
-    return s_last != 0;
-}
-
-// Both passes give each block one material class, so the class mass
-// multiplies the block's sums once, in FP64: blocks [0, nbfe) take the
-// run's Fe bodies [0, nfe), blocks [nbfe, gridDim.x) its Si bodies [nfe, n),
-// each class in a grid-stride loop over its own blocks (nbfe in proportion
-// to nfe).  Block b's partials are work[16 b ..].
-__device__ __forceinline__ void class_range(int nfe, int n, int nbfe, double mfe, double msi,
-                                            int &k0, int &k1, int &b, int &nb, double &m)
-{
-    const bool fe = (int)blockIdx.x < nbfe;
-    k0 = fe ? 0 : nfe;
-    k1 = fe ? nfe : n;
-    b = fe ? (int)blockIdx.x : (int)blockIdx.x - nbfe;
-    nb = fe ? nbfe : (int)gridDim.x - nbfe;
-    m = fe ? mfe : msi;
-}
-
-// The block partials summed in a fixed order, by the block that finished
-// last: thread t takes blocks t, t + 256, ... in order (read past L1), then
-// a fixed shuffle tree within each warp, then the 8 warps in order.  The
-// result is deterministic for a given grid; it is valid in thread 0.
-template <int NV>
-__device__ __forceinline__ void ordered_sums(const double *work, int nblocks, double (&res)[NV])
-{
-    __shared__ double sh[NV][8];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    double v[NV];
+    if (!s_last) return;
+    __threadfence();
+    __shared__ double sum[kDiagParts + 1];  // the last: Fe bodies
+    for (int c = warp; c < kDiagParts + 1; c += 8) {
+        const int end = c == kDiagParts ? nbfe : (int)gridDim.x;
+        double x = 0.0;
+        for (int q = lane; q < end; q += 32) x += __ldcg(work + 16 * q + min(c, kDiagSums));
 #pragma unroll
-    for (int c = 0; c < NV; ++c) v[c] = 0.0;
-    for (int b = t; b < nblocks; b += 256)
-#pragma unroll
-        for (int c = 0; c < NV; ++c) v[c] += __ldcg(work + 16 * b + c);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int c = 0; c < NV; ++c) v[c] += __shfl_down_sync(0xffffffffu, v[c], o);
-    if (lane == 0) {
-#pragma unroll
-        for (int c = 0; c < NV; ++c) sh[c][warp] = v[c];
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) sum[c] = x;
     }
     __syncthreads();
-    if (t == 0) {
-#pragma unroll
-        for (int c = 0; c < NV; ++c) {
-            double x = 0.0;
-            for (int w = 0; w < 8; ++w) x += sh[c][w];
-            res[c] = x;
-        }
-    }
-}
-
-// Pass 1: mass, sum m x, sum m v, kinetic energy, count (9 doubles / block);
-// its last block writes out = [mass, com3, vcom3, -, -, -, ke, p3, count].
-__global__ void __launch_bounds__(256)
-diag_pass1(const float4 *__restrict__ pos, const float4 *__restrict__ vel,
-           const unsigned char *__restrict__ label, int scope, int off, int n,
-           int nfe, int nbfe, double mfe, double msi, double *__restrict__ work,
-           int *__restrict__ ticket, double *__restrict__ out)
-{
-    int k0, k1, b, nb;
-    double m;
-    class_range(nfe, n, nbfe, mfe, msi, k0, k1, b, nb, m);
-    FF v[7];
-#pragma unroll
-    for (int c = 0; c < 7; ++c) v[c] = FF{0.0f, 0.0f};
-    int cnt = 0;
-    stream_bodies(pos, vel, label, scope, off, k0 + b * blockDim.x + threadIdx.x, k1,
-                  nb * blockDim.x, [&](float4 p, float4 u) {
-                      ff_add(v[0], p.x);
-                      ff_add(v[1], p.y);
-                      ff_add(v[2], p.z);
-                      ff_add(v[3], u.x);
-                      ff_add(v[4], u.y);
-                      ff_add(v[5], u.z);
-                      ff_add_prod(v[6], u.x, u.x);
-                      ff_add_prod(v[6], u.y, u.y);
-                      ff_add_prod(v[6], u.z, u.z);
-                      ++cnt;
-                  });
-    warp_ff_sum<7>(v);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-    const double d[9] = {m * cnt,
-                         m * ff_value(v[0]), m * ff_value(v[1]), m * ff_value(v[2]),
-                         m * ff_value(v[3]), m * ff_value(v[4]), m * ff_value(v[5]),
-                         0.5 * m * ff_value(v[6]), (double)cnt};
-    if (!block_store_last<9>(d, work + 16 * blockIdx.x, ticket)) return;
-    double s[9];
-    ordered_sums<9>(work, gridDim.x, s);
     if (threadIdx.x != 0) return;
-    const double M = s[0];
+    const double count = sum[kDiagSums], cfe = sum[kDiagParts];
+    const double M = mfe * cfe + msi * (count - cfe);
+    double rc[3], wc[3];
     out[0] = M;
-    for (int c = 0; c < 3; ++c) {
-        out[1 + c] = M > 0.0 ? s[1 + c] / M : 0.0;
-        out[4 + c] = M > 0.0 ? s[4 + c] / M : 0.0;
-        out[11 + c] = s[4 + c];
+    for (int d = 0; d < 3; ++d) {
+        out[1 + d] = M > 0.0 ? sum[d] / M : 0.0;
+        out[4 + d] = M > 0.0 ? sum[3 + d] / M : 0.0;
+        out[11 + d] = sum[3 + d];
+        rc[d] = M > 0.0 ? out[1 + d] - (double)x0[d] : 0.0;
+        wc[d] = M > 0.0 ? out[4 + d] - (double)x0[3 + d] : 0.0;
     }
-    out[10] = s[7];
-    out[14] = s[8];
-}
-
-// Pass 2: angular momentum about the com, relative to the com velocity
-// (impactBasicFunctions.h:507-652 in double): r = x - com and w = v - vcom
-// as float-float pairs, sum of r x w per class; its last block writes
-// out[7..9].
-__global__ void __launch_bounds__(256, 4)
-diag_pass2(const float4 *__restrict__ pos, const float4 *__restrict__ vel,
-           const unsigned char *__restrict__ label, int scope, int off, int n,
-           int nfe, int nbfe, double mfe, double msi, double *__restrict__ out,
-           double *__restrict__ work, int *__restrict__ ticket)
-{
-    int k0, k1, b, nb;
-    double m;
-    class_range(nfe, n, nbfe, mfe, msi, k0, k1, b, nb, m);
-    float ch[6], cl[6];  // com xyz, vcom xyz as float pairs
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-        const double x = out[1 + c];
-        ch[c] = (float)x;
-        cl[c] = (float)(x - (double)ch[c]);
-    }
-    FF L[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) L[c] = FF{0.0f, 0.0f};
-    stream_bodies(pos, vel, label, scope, off, k0 + b * blockDim.x + threadIdx.x, k1,
-                  nb * blockDim.x, [&](float4 p, float4 u) {
-                      const FF rx = ff_sub_d(p.x, ch[0], cl[0]), ry = ff_sub_d(p.y, ch[1], cl[1]),
-                               rz = ff_sub_d(p.z, ch[2], cl[2]);
-                      const FF wx = ff_sub_d(u.x, ch[3], cl[3]), wy = ff_sub_d(u.y, ch[4], cl[4]),
-                               wz = ff_sub_d(u.z, ch[5], cl[5]);
-                      ff_add_cross(L[0], ry, wz, rz, wy);
-                      ff_add_cross(L[1], rz, wx, rx, wz);
-                      ff_add_cross(L[2], rx, wy, ry, wx);
-                  });
-    warp_ff_sum<3>(L);
-    const double d[3] = {m * ff_value(L[0]), m * ff_value(L[1]), m * ff_value(L[2])};
-    if (!block_store_last<3>(d, work + 16 * blockIdx.x, ticket)) return;
-    double s[3];
-    ordered_sums<3>(work, gridDim.x, s);
-    if (threadIdx.x != 0) return;
-    out[7] = s[0]; out[8] = s[1]; out[9] = s[2];
+    out[7] = sum[7] - M * (rc[1] * wc[2] - rc[2] * wc[1]);
+    out[8] = sum[8] - M * (rc[2] * wc[0] - rc[0] * wc[2]);
+    out[9] = sum[9] - M * (rc[0] * wc[1] - rc[1] * wc[0]);
+    out[10] = 0.5 * sum[6];
+    out[14] = count;
 }
 
 // ------------------------------------------------------------ FFMA peak --
@@ -379,42 +299,34 @@ cudaError_t gi_launch_move(float4 *pos, float4 *vel, const float4 *force,
     return cudaGetLastError();
 }
 
-// One resident wave per pass: the grid-stride loops give every block the
-// same number of bodies, so a grid of exactly the resident blocks has no
-// partial last wave.
-int gi_diag_blocks(int pass, int sm_count)
+int gi_diag_blocks(int sm_count)
 {
     int per_sm = 0;
-    const cudaError_t e = pass == 1
-        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gi::diag_pass1, 256, 0)
-        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gi::diag_pass2, 256, 0);
-    if (e != cudaSuccess || per_sm < 1) per_sm = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gi::diag_kernel, 256, 0) != cudaSuccess ||
+        per_sm < 1)
+        per_sm = 1;
     return std::max(2, per_sm * sm_count);
 }
 
 cudaError_t gi_launch_diag(const float4 *pos, const float4 *vel,
                            const unsigned char *label, int scope,
                            const RunDev &run, float mass_fe, float mass_si, double *work,
-                           int nblocks1, int nblocks2, double *out_dev, int *ticket,
-                           cudaStream_t s)
+                           int max_blocks, double *out, int *ticket, cudaStream_t s)
 {
-    if (nblocks1 < 2 || nblocks2 < 2) return cudaErrorInvalidValue;
+    if (max_blocks < 2) return cudaErrorInvalidValue;
+    // One resident wave (the grid-stride loops give every block the same
+    // number of bodies, so there is no partial last wave), but no more blocks
+    // than two bodies a thread: a small run's time is the blocks' sums.
+    const int nblocks = std::max(2, std::min(max_blocks, (run.n + 511) / 512));
     // blocks for the Fe bodies in proportion to their number (at least one
     // when there are any), the rest for the Si bodies
-    const auto fe_blocks = [&](int nblocks) {
-        int nbfe = run.n > 0 ? (int)((long long)nblocks * run.nfe / run.n) : 0;
-        if (run.nfe > 0 && nbfe < 1) nbfe = 1;
-        if (nbfe > nblocks - 1) nbfe = nblocks - 1;
-        return nbfe;
-    };
-    cudaError_t e = cudaMemsetAsync(ticket, 0, 2 * sizeof(int), s);
+    int nbfe = run.n > 0 ? (int)((long long)nblocks * run.nfe / run.n) : 0;
+    if (run.nfe > 0 && nbfe < 1) nbfe = 1;
+    if (nbfe > nblocks - 1) nbfe = nblocks - 1;
+    cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof(int), s);
     if (e != cudaSuccess) return e;
-    gi::diag_pass1<<<nblocks1, 256, 0, s>>>(pos, vel, label, scope, run.offset, run.n, run.nfe,
-                                            fe_blocks(nblocks1), mass_fe, mass_si, work, ticket,
-                                            out_dev);
-    gi::diag_pass2<<<nblocks2, 256, 0, s>>>(pos, vel, label, scope, run.offset, run.n, run.nfe,
-                                            fe_blocks(nblocks2), mass_fe, mass_si, out_dev, work,
-                                            ticket + 1);
+    gi::diag_kernel<<<nblocks, 256, 0, s>>>(pos, vel, label, scope, run.offset, run.n, run.nfe, nbfe,
+                                            mass_fe, mass_si, work, ticket, out);
     return cudaGetLastError();
 }
 

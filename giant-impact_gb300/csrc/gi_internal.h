@@ -258,16 +258,14 @@ inline cudaError_t gi_full_carveout(const void *kernel, std::atomic<int> (&known
 // gi_aux.cu
 cudaError_t gi_launch_move(float4 *pos, float4 *vel, const float4 *force,
                            const LaunchTable &tab, cudaStream_t s);
-// The diagnostics' blocks for pass 1 or 2: the resident blocks of that pass
-// on sm_count SMs.
-int gi_diag_blocks(int pass, int sm_count);
-// Both passes of the FP64 diagnostics; work holds 16 doubles per block of
-// the larger grid, out_dev 15 doubles, ticket 2 ints (cleared here).
+// The FP64 diagnostics' resident blocks on sm_count SMs.
+int gi_diag_blocks(int sm_count);
+// work holds 16 doubles per block, out 15 doubles (device, or pinned host
+// memory), ticket an int (cleared here).
 cudaError_t gi_launch_diag(const float4 *pos, const float4 *vel,
                            const unsigned char *label, int scope,
                            const RunDev &run, float mass_fe, float mass_si, double *work,
-                           int nblocks1, int nblocks2, double *out_dev, int *ticket,
-                           cudaStream_t s);
+                           int max_blocks, double *out, int *ticket, cudaStream_t s);
 cudaError_t gi_launch_ffma_peak(float *sink, int blocks, int iters, cudaStream_t s);
 
 // gi_api.cu helpers for the library's other translation units: record an
