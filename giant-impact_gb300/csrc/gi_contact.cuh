@@ -143,18 +143,18 @@ __device__ __forceinline__ float contact_coef(const PairRow &w, int sep_test, fl
     return __fmaf_rn(mag, invr, w.far);
 }
 
-// contact_coef with j's velocity read (from shared memory) only for pairs
+// contact_coef with the velocities read (from shared memory) only for pairs
 // inside the shell band, where the separation test needs it.  Same
 // arithmetic, same result.
 __device__ __forceinline__ float contact_coef_at(const PairRow &w, int sep_test, float dx,
-                                                 float dy, float dz, float r2, float4 vi,
-                                                 const float4 *vj)
+                                                 float dy, float dz, float r2,
+                                                 const float4 *vi, const float4 *vj)
 {
     float K = w.K;
     if (!(r2 >= w.Tband)) {
-        const float4 v = *vj;
-        const float dvx = __fsub_rn(v.x, vi.x), dvy = __fsub_rn(v.y, vi.y),
-                    dvz = __fsub_rn(v.z, vi.z);
+        const float4 u = *vi, v = *vj;
+        const float dvx = __fsub_rn(v.x, u.x), dvy = __fsub_rn(v.y, u.y),
+                    dvz = __fsub_rn(v.z, u.z);
         const float dpdv = __fmaf_rn(dz, dvz, __fmaf_rn(dx, dvx, __fmul_rn(dy, dvy)));
         const bool sep = (sep_test == GI_SEP_SIGN) ? (dpdv > 0.0f) : (dpdv >= 1.0f);
         if (sep) K = (r2 >= w.Tmid) ? w.KRmid : w.KRin;

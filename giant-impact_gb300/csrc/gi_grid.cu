@@ -30,8 +30,8 @@
 // contacts per body) whose bodies all share one cell are sorted by sub-cell
 // and go through contact_tile_kernel: a work item is (bucket, neighbour
 // bucket, chunk of 128 of its bodies); its CTA stages the neighbour bucket in
-// shared memory 128 bodies at a time, each thread filters the tile into a hit
-// list and evaluates the law on the hits only, and a pair of two dense cells
+// shared memory 128 bodies at a time, evaluates the law on the hits only, or on
+// whole blocks of pairs that are mostly hits, and a pair of two dense cells
 // is evaluated once for both bodies.  The candidate sets, the pair law and
 // the fixed-point terms are the same on both paths and integer addition is
 // exact, so the corrections are bit-identical whichever path a body takes.
@@ -604,85 +604,153 @@ __device__ __forceinline__ float box_gap2(float3 ilo, float3 ihi, float3 jlo, fl
     return __fmaf_rn(gz, gz, __fmaf_rn(gx, gx, __fmul_rn(gy, gy)));
 }
 
-// Shared-memory position of staged slot k (0..127).  Lanes walking their
-// hit lists (ascending slots) from staggered starts read slots about 4
-// apart; this layout puts such slots in distinct banks, for the 16-byte
-// staged bodies and for the 4-byte j-side sums alike.
-__device__ __forceinline__ int swz(int k) { return ((k & 3) << 5) | (k >> 2); }
+// Whether most pairs of two boxes of bodies are likely contacts: the mean
+// square distance of evenly filled boxes is below kTileNear.
+constexpr float kTileNear = 0.9f;
+__device__ __forceinline__ bool box_near(float3 ilo, float3 ihi, float3 jlo, float3 jhi)
+{
+    const auto axis = [](float a0, float a1, float b0, float b1) {
+        const float d = (b0 + b1) - (a0 + a1), a = a1 - a0, b = b1 - b0;
+        return 0.25f * d * d + (a * a + b * b) * (1.0f / 12.0f);
+    };
+    return axis(ilo.x, ihi.x, jlo.x, jhi.x) + axis(ilo.y, ihi.y, jlo.y, jhi.y) +
+               axis(ilo.z, ihi.z, jlo.z, jhi.z) < kTileNear;
+}
 
-// The contact law on one thread's hits of a staged tile (slots my[0 .. nh)),
-// starting at the (lane / 32)-th part of the list so that lanes with alike
-// lists (neighbouring bodies) rarely hit one slot's shared sums at once.
-// PAIR: the pair's j-side term goes to the slot's shared sums too.  MIXED:
-// the tile holds Fe bodies, so the pair-class row is chosen per hit; a tile
-// of Si bodies alone (most of them: Fe is the small core) uses row_si.
+// The tiled path's shared memory.
+constexpr int kTileDense = 512;               // hits of 1,024 pairs: see tile_block
+constexpr int kTileQueue = kTileDense + 32;  // pairs a warp may have queued
+struct TileSmem {
+    float4 sp[128], sv[128];     // the staged bodies: x, y, z, body index (bits); velocity
+    float4 ip[128], iv[128];     // the chunk's bodies, the same
+    unsigned int js[6][128];     // sums of the staged bodies (pair items)
+    unsigned int is[6][128];     // queued pairs' sums of the chunk's bodies
+    float4 row[3][2];            // the law's constants per pair class (PairRow, Fe bodies of the pair)
+    float3 blo[4], bhi[4];       // box of each staged block of 32
+    int bcls[4];                 // its bodies: 0 Si, 1 Fe, 2 both
+    unsigned short queue[4][kTileQueue];  // per warp: lane of i | staged slot of j << 5
+    unsigned int w;              // the item to take next
+};
+
+__device__ __forceinline__ PairRow tile_row(const TileSmem &sm, int cls)
+{
+    const float4 a = sm.row[cls][0], b = sm.row[cls][1];
+    return PairRow{a.x, a.y, a.z, a.w, b.x, b.y, b.z};
+}
+
+// The 32 bodies of a warp against a staged block of 32, all pairs: in step r
+// lane l takes slot (l + r) mod 32, so that the lanes' loads and their
+// additions to the slots' shared sums never meet in a bank, and no list is
+// kept.  For a block with itself steps 1 to 16 cover each pair once (the
+// pair's terms are the same, with opposite signs, from either body).
 template <bool PAIR, bool MIXED>
-__device__ __forceinline__ void tile_hits(FixSum3 &acc, const unsigned char *my, int nh, int lane,
-                                          const float4 *sp, const float4 *sv,
-                                          unsigned int (*js)[128], long long *delta, float4 pi,
-                                          float4 vi, const PairRow &row_fe, const PairRow &row_si,
-                                          int sw, int sep_test, float inv_unit)
+__device__ __forceinline__ void tile_block(FixSum3 &acc, TileSmem &sm, int s, bool diag, int lane,
+                                           float4 pi, float4 vi, int ife, int cls, long long *delta,
+                                           int sw, int sep_test, float inv_unit)
 {
     const float2 npxy = make_float2(-pi.x, -pi.y);
-    int h = (lane * nh) >> 5;
-    for (int n = 0; n < nh; ++n) {
-        const int k = swz(my[h]);  // shared-memory position of the slot
-        h = h + 1 == nh ? 0 : h + 1;
-        const float4 pj = sp[k];
-        const int j = __float_as_int(pj.w);  // never i: b and nb differ, or k > t
+    PairRow row = tile_row(sm, MIXED ? 0 : ife + cls);
+    const int r1 = !diag ? 32 : lane < 16 ? 17 : 16;
+    for (int r = diag; r < r1; ++r) {
+        const int k = 32 * s + ((lane + r) & 31);
+        const float4 pj = sm.sp[k];
         const float2 dxy = __fadd2_rn(make_float2(pj.x, pj.y), npxy);
         const float dx = dxy.x, dy = dxy.y, dz = pj.z - pi.z;
         const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
-        const float c = contact_coef_at(MIXED ? select_row(j < sw, row_fe, row_si) : row_si,
-                                        sep_test, dx, dy, dz, r2, vi, &sv[k]) *
-                        inv_unit;
-        if (PAIR) fix_add3_pair(acc, js, k, delta + 3 * (size_t)j, c, dx, dy, dz, r2);
-        else fix_add3<false>(acc, c, dx, dy, dz, r2);
+        if (r2 < 1.0f) {
+            const int j = __float_as_int(pj.w);
+            if (MIXED) row = tile_row(sm, ife + (int)(j < sw));
+            const float c = contact_coef_at(row, sep_test, dx, dy, dz, r2, &vi, &sm.sv[k]) * inv_unit;
+            if (PAIR) fix_add3_pair(acc, sm.js, k, delta + 3 * (size_t)j, c, dx, dy, dz, r2);
+            else fix_add3<false>(acc, c, dx, dy, dz, r2);
+        }
     }
-    // at most 128 hits a tile: fold before kFixFold terms can be pending
-    if (acc.n >= kFixFold - 128u) fix_fold(acc);
+}
+
+// One queued pair per lane (all of them hits), n lanes.
+template <bool PAIR>
+__device__ __forceinline__ void tile_pair(TileSmem &sm, unsigned int e, bool on, int warp,
+                                          long long *delta, int sw, int sep_test, float inv_unit)
+{
+    if (!on) return;
+    const int t = 32 * warp + (int)(e & 31u), k = (int)(e >> 5);
+    const float4 pi = sm.ip[t], pj = sm.sp[k];
+    const int i = __float_as_int(pi.w), j = __float_as_int(pj.w);
+    const float2 dxy = __fadd2_rn(make_float2(pj.x, pj.y), make_float2(-pi.x, -pi.y));
+    const float dx = dxy.x, dy = dxy.y, dz = pj.z - pi.z;
+    const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+    const PairRow row = tile_row(sm, (int)(i < sw) + (int)(j < sw));
+    const float c = contact_coef_at(row, sep_test, dx, dy, dz, r2, &sm.iv[t], &sm.sv[k]) * inv_unit;
+    FixSum3 a;
+    fix_zero(a);
+    fix_add3<false>(a, c, dx, dy, dz, r2);
+    if (a.n) {
+        const unsigned int h[3] = {a.hx, a.hy, a.hz}, l[3] = {a.lx, a.ly, a.lz};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            atomicAdd(&sm.is[d][t], h[d] - __float_as_uint(kFixM));
+            atomicAdd(&sm.is[3 + d][t], l[d] - __float_as_uint(kFixC));
+            if (PAIR) {
+                atomicAdd(&sm.js[d][k], __float_as_uint(kFixM) - h[d]);
+                atomicAdd(&sm.js[3 + d][k], __float_as_uint(kFixC) - l[d]);
+            }
+        }
+    } else {  // out of the split's range: to the global sums
+        unsigned long long *di = reinterpret_cast<unsigned long long *>(delta + 3 * (size_t)i);
+        unsigned long long *dj = reinterpret_cast<unsigned long long *>(delta + 3 * (size_t)j);
+        const long long v[3] = {a.x, a.y, a.z};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            atomicAdd(di + d, (unsigned long long)v[d]);
+            if (PAIR) atomicAdd(dj + d, 0ull - (unsigned long long)v[d]);
+        }
+    }
 }
 
 // Items come from a queue, longest first.  For an item the CTA holds up to
-// 128 bodies of the bucket b (one per thread, all in one cell), stages the
-// neighbour bucket nb in shared memory 128 bodies at a time, and each
-// thread collects the tile slots within r2 < 1 of its body before
-// evaluating the contact law on those alone.  A warp skips each staged
-// block of 32 bodies whose bounding box is provably out of reach of its own
-// bodies' box.  When nb is tiled too, each pair is evaluated once for both
-// bodies: the item covers nb's tiles from the chunk's own slots on (all of
-// them when nb != b; within the chunk's own tile only slots above the
-// thread's), and the staged bodies' shared sums go into their corrections
-// with 64-bit global atomics once per tile.
-// 72 registers: 7 CTAs of 128 threads per SM, with no spills.
+// 128 bodies of the bucket b (one per thread, all in one cell) and stages the
+// neighbour bucket nb in shared memory 128 bodies at a time.  Each warp takes
+// the staged blocks of 32 in turn and skips a block whose bounding box is
+// provably out of reach of its own bodies' box.  Of the others it takes those
+// of which at least half the pairs are contacts as a whole (tile_block: a
+// crowded core's pairs mostly are); from the rest it filters the hits
+// (r2 < 1) into a queue of pairs and evaluates the law on full warps of
+// those, whose sums go through shared memory on both sides.  When nb is tiled
+// too, each pair is evaluated once for both bodies: the item covers nb's
+// tiles from the chunk's own slots on (all of them when nb != b; within the
+// chunk's own tile only slots above the thread's), and the staged bodies'
+// shared sums go into their corrections with 64-bit global atomics once per
+// tile.
+//
+// What bounds it is the issue rate.  One hit list per thread left 46 % of the
+// lanes idle (a block of few hits 78 %), and the lists' scattered additions
+// to shared memory took four passes each: 796 us alone on a 66,000-body
+// remnant (74M pairs), 585 this way.  Thresholds from 0.6 to 0.9 (kTileNear)
+// and 384 to 640 (kTileDense) are within 1 % of each other.
+// Staged slots past the end and threads past the chunk hold positions at
+// infinity, which no pair test passes.
 __global__ void __maxnreg__(72)
 contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ svel,
                     const float4 *__restrict__ dpos, const float4 *__restrict__ dvel,
                     long long *__restrict__ delta, const __grid_constant__ LaunchTable tab,
                     const uint4 *__restrict__ items, unsigned int *__restrict__ ctr)
 {
-    constexpr int kStride = 132;  // bytes per hit list row: rows start in distinct banks
-    __shared__ float4 sp[128];    // x, y, z, body index (bits)
-    __shared__ float4 sv[128];
-    __shared__ float3 blo[4], bhi[4];  // box of each staged block of 32
-    __shared__ unsigned int js[6][128];  // j-side sums of the staged slots (pair items)
-    __shared__ unsigned char hits[128 * kStride];
-    __shared__ unsigned int s_w;  // the item to take next
+    __shared__ TileSmem sm;
     const unsigned int total = ctr[kCtrItems];
     const int t = threadIdx.x;
-    const int tz = swz(t);  // where this thread stages its slot
     const int lane = t & 31, warp = t >> 5;
+    const unsigned int all = 0xffffffffu;
     const float kInf = __int_as_float(0x7f800000);
-    unsigned char *my = hits + t * kStride;
+    unsigned short *const queue = sm.queue[warp];
 #pragma unroll
-    for (int d = 0; d < 6; ++d) js[d][t] = 0u;
+    for (int d = 0; d < 6; ++d) sm.js[d][t] = sm.is[d][t] = 0u;
     // Thread 0 takes the next item from the queue when the current one
     // reaches its last tile: the atomic's latency hides behind that tile,
     // and the CTA still takes items close to the queue's longest-first order.
-    if (t == 0) s_w = atomicAdd(&ctr[kCtrHead], 1u);
+    if (t == 0) sm.w = atomicAdd(&ctr[kCtrHead], 1u);
     __syncthreads();
     for (;;) {
-        const unsigned int w = s_w;
+        const unsigned int w = sm.w;
         if (w >= total) break;
         const uint4 rec = items[w];
         unsigned int nw = 0u;  // thread 0: the next item
@@ -693,75 +761,131 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
         const RunDev &R = tab.runs[rec.w & 0xffu];
         const int sw = R.offset + R.nfe;
         const float inv_unit = tab.params[R.param].inv_unit;
-        const float4 pi = valid ? dpos[s0 + t] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 pi = valid ? dpos[s0 + t] : make_float4(kInf, kInf, kInf, __int_as_float(-1));
         const float4 vi = valid ? dvel[s0 + t] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const int i = valid ? __float_as_int(pi.w) : -1;
+        const int i = __float_as_int(pi.w), ife = i < sw;
         const float4 *npos = pair ? dpos : spos, *nvel = pair ? dvel : svel;
-        const PairRow row_fe = pair_row(tab.params[R.param], i < sw, true);
-        const PairRow row_si = pair_row(tab.params[R.param], i < sw, false);
+        sm.ip[t] = pi;  // read by its own warp alone
+        sm.iv[t] = vi;
+        if (t < 3) {
+            const PairRow q = pair_row(tab.params[R.param], t > 0, t > 1);
+            sm.row[t][0] = make_float4(q.G, q.K, q.Tband, q.Tmid);
+            sm.row[t][1] = make_float4(q.KRmid, q.KRin, q.far, 0.0f);
+        }
         float3 ilo = valid ? make_float3(pi.x, pi.y, pi.z) : make_float3(kInf, kInf, kInf);
         float3 ihi = valid ? make_float3(pi.x, pi.y, pi.z) : make_float3(-kInf, -kInf, -kInf);
         warp_box(ilo, ihi);
+        const bool full = (unsigned int)(32 * warp + 32) <= ni;
         FixSum3 acc;
         fix_zero(acc);
         for (unsigned int base = first; base < nend; base += 128u) {
             __syncthreads();  // the previous tile is consumed
-            if (pair && base != first) flush_slot(js, tz, __float_as_int(sp[tz].w), delta);
+            if (pair && base != first) flush_slot(sm.js, t, __float_as_int(sm.sp[t].w), delta);
             if (t == 0 && base + 128u >= nend) nw = atomicAdd(&ctr[kCtrHead], 1u);
             const unsigned int u = base + (unsigned int)t;
             float3 lo = make_float3(kInf, kInf, kInf), hi = make_float3(-kInf, -kInf, -kInf);
-            bool fe_slot = false;  // the staged body is of the run's Fe core
+            float4 q = make_float4(kInf, kInf, kInf, 0.0f);
             if (u < nend) {
-                const float4 q = npos[u];
-                fe_slot = __float_as_int(q.w) < sw;
-                sp[tz] = q;
-                sv[tz] = nvel[u];
+                q = npos[u];
+                sm.sv[t] = nvel[u];
                 lo = hi = make_float3(q.x, q.y, q.z);
             }
+            sm.sp[t] = q;
             warp_box(lo, hi);
+            const unsigned int in = __ballot_sync(all, u < nend);
+            const unsigned int fe = __ballot_sync(all, u < nend && __float_as_int(q.w) < sw);
             if (lane == 0) {
-                blo[warp] = lo;
-                bhi[warp] = hi;
+                sm.blo[warp] = lo;
+                sm.bhi[warp] = hi;
+                sm.bcls[warp] = fe == 0u ? 0 : fe == in ? 1 : 2;
             }
-            // does any staged body belong to the Fe core?
-            const int mixed = __syncthreads_or(fe_slot);
-            if (!valid) continue;
+            __syncthreads();
             const int cnt = (int)min(128u, nend - base);
-            const int kmin = (self && base == first) ? t + 1 : 0;  // own tile: each pair once
-            int nh = 0;
-            for (int s = 0; s < 4 && 32 * s < cnt; ++s) {
-                if (box_gap2(ilo, ihi, blo[s], bhi[s]) >= 1.0f) continue;  // the same for the warp
-                const int k1 = min(cnt, 32 * s + 32);
-                for (int k = 32 * s; k < k1; k += 4) {  // swz(k + c) = 32 c + k / 4
+            const bool own = self && base == first;  // own tile: each pair once
+            int qn = 0;                              // queued pairs, the same in the warp
+            bool queued = false;
+            const auto drain = [&] {
+                const int n = min(qn, 32);
+                qn -= n;
+                __syncwarp();  // the entries are written
+                const unsigned int e = lane < n ? queue[qn + lane] : 0u;
+                __syncwarp();  // and read, before their places are written again
+                if (pair) tile_pair<true>(sm, e, lane < n, warp, delta, sw, tab.sep_test, inv_unit);
+                else tile_pair<false>(sm, e, lane < n, warp, delta, sw, tab.sep_test, inv_unit);
+            };
+            for (int s = own ? warp : 0; 32 * s < cnt; ++s) {
+                const float3 jlo = sm.blo[s], jhi = sm.bhi[s];
+                if (box_gap2(ilo, ihi, jlo, jhi) >= 1.0f) continue;  // the same for the warp
+                const bool diag = own && s == warp;
+                bool dense = full && 32 * s + 32 <= cnt && box_near(ilo, ihi, jlo, jhi);
+                unsigned int m = 0u;
+                if (!dense) {
+                    for (int k = 0; k < 32 && 32 * s + k < cnt; k += 8) {
+                        unsigned int g = 0u;
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        if (k + c >= k1) break;
-                        const float4 pj = sp[32 * c + (k >> 2)];
-                        const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-                        const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
-                        if (r2 < 1.0f && k + c >= kmin) my[nh++] = (unsigned char)(k + c);
+                        for (int c = 0; c < 8; ++c) {
+                            const float4 pj = sm.sp[32 * s + k + c];
+                            const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+                            const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+                            if (r2 < 1.0f) g |= 1u << c;
+                        }
+                        m |= g << k;
                     }
+                    if (diag) m &= 0xfffffffeu << lane;
+                    const int hits = __reduce_add_sync(all, __popc(m));
+                    if (hits == 0) continue;
+                    dense = hits >= (diag ? kTileDense / 2 : kTileDense);
                 }
+                if (dense) {
+                    const int cls = sm.bcls[s];
+                    if (pair) {
+                        if (cls == 2)
+                            tile_block<true, true>(acc, sm, s, diag, lane, pi, vi, ife, cls, delta, sw,
+                                                   tab.sep_test, inv_unit);
+                        else
+                            tile_block<true, false>(acc, sm, s, diag, lane, pi, vi, ife, cls, delta, sw,
+                                                    tab.sep_test, inv_unit);
+                    } else {
+                        tile_block<false, true>(acc, sm, s, diag, lane, pi, vi, ife, cls, delta, sw,
+                                                tab.sep_test, inv_unit);
+                    }
+                    continue;
+                }
+                // Queue the hits, one of each lane at a time and from staggered
+                // slots: 32 queued pairs are then of many bodies on either side.
+                queued = true;
+                for (unsigned int rm = __funnelshift_r(m, m, lane);;) {
+                    const unsigned int some = __ballot_sync(all, rm != 0u);
+                    if (!some) break;
+                    if (rm) {
+                        const int b = __ffs(rm) - 1;
+                        queue[qn + __popc(some & ((1u << lane) - 1u))] =
+                            (unsigned short)(lane | (32 * s + ((b + lane) & 31)) << 5);
+                        rm &= rm - 1u;
+                    }
+                    qn += __popc(some);
+                }
+                while (qn >= 32) drain();
             }
-            if (pair) {
-                if (mixed)
-                    tile_hits<true, true>(acc, my, nh, lane, sp, sv, js, delta, pi, vi, row_fe,
-                                          row_si, sw, tab.sep_test, inv_unit);
-                else
-                    tile_hits<true, false>(acc, my, nh, lane, sp, sv, js, delta, pi, vi, row_fe,
-                                           row_si, sw, tab.sep_test, inv_unit);
-            } else {
-                if (mixed)
-                    tile_hits<false, true>(acc, my, nh, lane, sp, sv, js, delta, pi, vi, row_fe,
-                                           row_si, sw, tab.sep_test, inv_unit);
-                else
-                    tile_hits<false, false>(acc, my, nh, lane, sp, sv, js, delta, pi, vi, row_fe,
-                                            row_si, sw, tab.sep_test, inv_unit);
+            if (qn) drain();
+            if (acc.n >= kFixFold - 128u) fix_fold(acc);  // a tile adds at most 128 terms
+            if (queued) {
+                __syncwarp();
+                long long v[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    v[d] = (long long)(int)sm.is[d][t] * (1ll << 23) + (int)sm.is[3 + d][t];
+                    sm.is[d][t] = sm.is[3 + d][t] = 0u;
+                }
+                acc.x += v[0];
+                acc.y += v[1];
+                acc.z += v[2];
+                __syncwarp();
             }
         }
-        __syncthreads();  // the last tile's j-side sums are complete; s_w is read
-        if (pair) flush_slot(js, tz, __float_as_int(sp[tz].w), delta);
-        if (t == 0) s_w = nw;
+        __syncthreads();  // the last tile's j-side sums are complete; sm.w is read
+        if (pair) flush_slot(sm.js, t, __float_as_int(sm.sp[t].w), delta);
+        if (t == 0) sm.w = nw;
         __syncthreads();  // the next item's index is visible
         fix_fold(acc);
         const long long ax = acc.x, ay = acc.y, az = acc.z;

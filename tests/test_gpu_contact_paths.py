@@ -89,3 +89,38 @@ def test_potential_sizes(gi, orc, torch_cuda, n, nfe):
     want = orc.potential_fp64(pos, [run], p).sum() / 2.0
     assert abs(alone - want) <= 2e-7 * abs(want)
     ctx.close()
+
+
+@pytest.mark.parametrize("m", [31, 32, 33, 64, 95, 127, 128, 129, 160, 257, 700])
+@pytest.mark.parametrize("spread", [0.3, 0.99])
+def test_crowded_cell_sizes(gi, torch_cuda, m, spread):
+    """Neighbouring cells of m bodies each, at the sizes where the tiled path's
+    chunks, staged blocks and tiles end, packed (all pairs are contacts) or
+    over their cells (few are), bodies alone beside them and a coincident
+    pair: the same bits tiled and on the row path."""
+    import gi_workloads as wl
+    torch = torch_cuda
+    p = wl.params(gi)
+    rng = np.random.default_rng(1000 * m + int(100 * spread))
+    cells = np.array([(0, 0, 0), (1, 0, 0), (1, 1, 0), (-1, 0, 1), (0, -1, -1)], np.float64)
+    n = 5 * m + 4000
+    pos, vel = np.zeros((n, 4), np.float32), np.zeros((n, 4), np.float32)
+    x = rng.uniform(-9, 9, size=(n, 3))
+    for k, c in enumerate(cells):
+        x[k * m:(k + 1) * m] = c + rng.uniform(0, spread, size=(m, 3))
+    x[5 * m:5 * m + 40] = rng.uniform(-2, 3, size=(40, 3))
+    x[1] = x[0]
+    x = x[rng.permutation(n)]  # the Fe boundary falls inside the cells
+    pos[:, :3] = x
+    vel[:, :3] = rng.normal(scale=1.5, size=(n, 3))
+    run = wl.run_desc(gi, 0, n, n // 3)
+    dp, dv = _dev(torch, pos), _dev(torch, vel)
+    out = []
+    for dense_min in (32, 1 << 30):
+        ctx = gi.Context(0, dense_min=dense_min)
+        f = torch.zeros_like(dp)
+        ctx.forces(dp.data_ptr(), dv.data_ptr(), f.data_ptr(), [run], p)
+        torch.cuda.synchronize()
+        out.append(f)
+        ctx.close()
+    assert torch.equal(out[0], out[1])
