@@ -920,9 +920,9 @@ static int run_force_plan(gi_ctx *c, const StreamScratch *x, const Plan &plan, i
             GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count, true, q), "cell grid");
             if (!beside)
                 GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, s), "tiled contacts");
-            GI_CUDA(gi_launch_pair_force(a, tab, gw, x->delta, !beside, s), "paired force kernel launch");
+            GI_CUDA(gi_launch_pair_force(a, tab, gw, x->delta, ctr, !beside, s), "paired force kernel launch");
             if (beside) {
-                GI_CUDA(gi_launch_rows(pos, vel, tab, gw, x->delta, q), "row contacts");
+                GI_CUDA(gi_launch_rows(pos, vel, tab, gw, x->delta, ctr, q), "row contacts");
                 GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, q), "tiled contacts");
                 GI_CUDA(cudaEventRecord(x->ev_join, x->aux), "cudaEventRecord");
                 GI_CUDA(cudaStreamWaitEvent(s, x->ev_join, 0), "cudaStreamWaitEvent");
@@ -948,7 +948,7 @@ static int run_force_plan(gi_ctx *c, const StreamScratch *x, const Plan &plan, i
         // Beside the persistent far field the grid is built by small blocks: a
         // cluster's CTAs would keep the far field's off their SMs for good.
         GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count, !beside, q), "cell grid");
-        GI_CUDA(gi_launch_rows(pos, vel, tab, gw, x->delta, q), "row contacts");
+        GI_CUDA(gi_launch_rows(pos, vel, tab, gw, x->delta, ctr, q), "row contacts");
         GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, q), "tiled contacts");
         if (!beside) {
             GI_CUDA(gi_launch_force(p, c->opt.accum, epi, a, tab, c->sm_count * occ, s),

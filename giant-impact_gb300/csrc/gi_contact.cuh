@@ -58,10 +58,21 @@ __device__ __forceinline__ unsigned int bucket_size(const unsigned int *start, u
 
 // Counters of the tiled path, in one block of kCtrWords words that start at
 // zero: item count, tiled-bucket count, queue head, candidate buckets, then
-// the items per cost class and the fill of each class while ordering.
+// the items per cost class and the fill of each class while ordering,
+// then a bit per run: has candidate buckets.
 constexpr int kCtrItems = 0, kCtrTiled = 1, kCtrHead = 2, kCtrCand = 3, kCtrClass = 4,
-              kCtrFill = 4 + (int)kItemClasses;
-static_assert(kCtrFill + (int)kItemClasses == kCtrWords, "tiled-path counter block");
+              kCtrFill = kCtrClass + (int)kItemClasses, kCtrCrowds = kCtrFill + (int)kItemClasses;
+static_assert(kCtrCrowds + GI_MAX_RUNS / 32 == kCtrWords, "tiled-path counter block");
+
+__device__ __forceinline__ void set_crowds(unsigned int *ctr, unsigned int run)
+{
+    atomicOr(&ctr[kCtrCrowds + (run >> 5)], 1u << (run & 31u));
+}
+
+__device__ __forceinline__ bool has_crowds(const unsigned int *ctr, unsigned int run)
+{
+    return (__ldg(&ctr[kCtrCrowds + (run >> 5)]) >> (run & 31u)) & 1u;
+}
 
 // The bodies of a bucket that share its majority cell take the tiled path when
 // they are at least tab.dense_min (256 unless set), or at least a quarter of
@@ -266,7 +277,7 @@ __device__ __forceinline__ void fix_add3(FixSum3 &a, float c, float dx, float dy
 // dense_hi), by one warp: their number and their cell c, 0 for none.  They are
 // the bucket's majority cell; bodies of another cell that share the bucket
 // (the torus is at least 16 cells wide, so they are far away) stay on the row
-// path.  The same answer wherever it is asked.
+// path.
 __device__ __forceinline__ unsigned int bucket_tiled(const Torus &T, const unsigned int *start,
                                                      const float4 *spos, unsigned int b,
                                                      unsigned int dmin, int lane, int3 &c)
@@ -302,6 +313,17 @@ __device__ __forceinline__ unsigned int bucket_tiled(const Torus &T, const unsig
     return __any_sync(0xffffffffu, crowded) ? same : 0u;
 }
 
+// Whether bucket b's tiled bodies, if it has any, are those of cell c.  The
+// states are written for buckets of at least dense_lo bodies alone.
+__device__ __forceinline__ bool cell_tiled(const GridView &g, unsigned int b, int3 c,
+                                           unsigned int dmin)
+{
+    const unsigned int beg = __ldg(&g.start[b]);
+    if (__ldg(&g.start[b + 1]) - beg < dense_lo(dmin) || __ldg(&g.state[b]) == 0u) return false;
+    const int3 d = cell_of(__ldg(&g.dpos[beg]));
+    return c.x == d.x && c.y == d.y && c.z == d.z;
+}
+
 // The row path: one warp, a few consecutive bodies of a run.  Bodies that
 // share their candidates form a group; the warp's lanes are split evenly among
 // a group's bodies (1 to 8 of them, 32 to 4 lanes each), so a lone body gets
@@ -316,6 +338,13 @@ __device__ __forceinline__ unsigned int bucket_tiled(const Torus &T, const unsig
 // candidates and 18 contacts a body) one warp per body, with its own 27
 // bucket look-ups, a candidate search over them and half-empty evaluations,
 // took 70 us alone, this path 31.
+//
+// A tiled cell is no candidate here: its items give both sides of its pairs
+// with its neighbours, and add to the corrections beside this path.  The few
+// bodies around a remnant's core had thousands of such candidates, a warp
+// with the longest list lasting 130 us (4,500 bodies) to 330 us (66,000) after
+// the rest were done: a step of 20,000 remnant bodies took 531 us with them,
+// 391 without.
 constexpr int kRowStage = 128;  // candidates staged at a time
 constexpr int kRowList = 512;   // hits listed: 16 per lane before they are drained
 constexpr int kRowLaw = 4;      // hits of a lane evaluated at a time
@@ -375,13 +404,13 @@ struct RowBody {
 
 // One group: the lanes [k W, (k + 1) W) have body k of it, W = 1 << wlog.
 // [beg, beg + cnt): the lane's range of candidates (ranges without candidates
-// come last, or have the next one's excl).
+// come last, or have the next one's excl).  add: to delta, else stored there.
 template <bool DIRECT>
 __device__ __forceinline__ void row_group(RowSmem &sm, const float4 *__restrict__ cpos,
                                           const float4 *__restrict__ cvel,
                                           long long *__restrict__ delta, const LaunchTable &tab,
                                           const RunDev &R, const PairDev &P, const RowBody &B,
-                                          int wlog, unsigned int beg, unsigned int cnt, int lane)
+                                          int wlog, unsigned int beg, unsigned int cnt, bool add, int lane)
 {
     const int W = 1 << wlog, way = lane & (W - 1);
     const unsigned int mine = (wlog == 5 ? 0xffffffffu : (1u << W) - 1u) << (lane & ~(W - 1));
@@ -470,7 +499,12 @@ __device__ __forceinline__ void row_group(RowSmem &sm, const float4 *__restrict_
     for (int o = W / 2; o > 0; o >>= 1)
 #pragma unroll
         for (int d = 0; d < 3; ++d) a[d] += __shfl_xor_sync(0xffffffffu, a[d], o);
-    if (B.i >= 0 && way < 3) delta[3 * (size_t)B.i + way] = way == 0 ? a[0] : way == 1 ? a[1] : a[2];
+    if (B.i >= 0 && way < 3) {
+        long long *const d = &delta[3 * (size_t)B.i + way];
+        const long long v = way == 0 ? a[0] : way == 1 ? a[1] : a[2];
+        if (!add) *d = v;
+        else if (v) atomicAdd(reinterpret_cast<unsigned long long *>(d), (unsigned long long)v);
+    }
 }
 
 // Runs without a grid: kDirectBodies bodies from `first` on, every body of the
@@ -490,7 +524,7 @@ __device__ __forceinline__ void row_direct(RowSmem &sm, const float4 *__restrict
     B.pi = k < R.n ? __ldg(&pos[B.i]) : z;
     B.vi = k < R.n ? __ldg(&vel[B.i]) : z;
     row_group<true>(sm, pos + R.offset, vel + R.offset, delta, tab, R, tab.params[R.param], B, kWlog,
-                    0u, (unsigned int)R.n, lane);
+                    0u, (unsigned int)R.n, false, lane);
 }
 
 // Runs with a grid: kRowBodies (8) consecutive slots.  Slots run along x, so
@@ -499,8 +533,9 @@ __device__ __forceinline__ void row_direct(RowSmem &sm, const float4 *__restrict
 // side, each one contiguous range (two where the torus wraps).
 __device__ __forceinline__ void row_slots(RowSmem &sm, const GridView &g,
                                           long long *__restrict__ delta, const LaunchTable &tab,
-                                          const RunDev &R, int first, int lane)
+                                          const RunDev &R, unsigned int run, int first, int lane)
 {
+    const bool crowds = has_crowds(g.ctr, run);
     const PairDev &P = tab.params[R.param];
     const Torus T = torus_of(R);
     const unsigned int dmin = (unsigned int)tab.dense_min;
@@ -509,15 +544,7 @@ __device__ __forceinline__ void row_slots(RowSmem &sm, const GridView &g,
     const unsigned int slot = (unsigned int)(R.gslot + first + lane);
     const int3 c = valid ? cell_of(__ldg(&g.spos[slot])) : make_int3(0, 0, 0);
     const unsigned int key = bucket_of(T, c.x, c.y, c.z);
-    bool in = valid;
-    unsigned int ask = __ballot_sync(0xffffffffu, valid && bucket_size(g.start, key) >= dense_lo(dmin));
-    while (ask) {
-        const unsigned int b = __shfl_sync(0xffffffffu, key, __ffs(ask) - 1);
-        int3 m;
-        const bool tiled = bucket_tiled(T, g.start, g.spos, b, dmin, lane, m) != 0u;
-        if (valid && key == b) in = !(tiled && c.x == m.x && c.y == m.y && c.z == m.z);
-        ask &= ~__ballot_sync(0xffffffffu, valid && key == b);
-    }
+    const bool in = valid && !(crowds && cell_tiled(g, key, c, dmin));
     // a body joins the one before it where their x ranges meet; a group is a
     // chain of joined bodies
     const int bx = __shfl_up_sync(0xffffffffu, c.x, 1), by = __shfl_up_sync(0xffffffffu, c.y, 1),
@@ -528,12 +555,12 @@ __device__ __forceinline__ void row_slots(RowSmem &sm, const GridView &g,
                          c.x >= bx && c.x <= bx + 3);
     while (rest) {
         const int src = __ffs(rest) - 1;
-        const int n = __ffs(~(joined >> src >> 1));  // bodies of the group (8 at most)
-        rest &= ~(((1u << n) - 1u) << src);
+        int n = __ffs(~(joined >> src >> 1));  // bodies of the group (8 at most)
         const int xlo = __shfl_sync(0xffffffffu, c.x, src) - 1,
                   width = __shfl_sync(0xffffffffu, c.x, src + n - 1) + 2 - xlo,
                   gy = __shfl_sync(0xffffffffu, c.y, src), gz = __shfl_sync(0xffffffffu, c.z, src);
         unsigned int beg = 0u, end = 0u;
+        bool crowd = false;
         if (lane < 18) {  // the two pieces of each of the nine rows
             const int r = lane >> 1, side = T.xm + 1;
             const unsigned int base = row_of(T, gy + r % 3 - 1, gz + r / 3 - 1);
@@ -543,7 +570,26 @@ __device__ __forceinline__ void row_slots(RowSmem &sm, const GridView &g,
                 beg = __ldg(&g.start[base + lo]);
                 end = __ldg(&g.start[base + hi]);
             }
+            if (crowds && end - beg >= dense_lo(dmin))
+                for (int x = lo; x < hi; ++x)
+                    crowd |= bucket_size(g.start, base + x) >= dense_lo(dmin) && g.state[base + x];
         }
+        if (__any_sync(0xffffffffu, crowd)) {
+            // Next to a tiled bucket; a tiled neighbour cell's items give both
+            // sides of its pairs.  The first cell's bodies alone, its other
+            // neighbours one to a lane.
+            n = min(n, __ffs(~(__ballot_sync(0xffffffffu, in && c.x == xlo + 1) >> src)) - 1);
+            beg = end = 0u;
+            if (lane < 27) {
+                const int3 d = make_int3(xlo + lane % 3, gy + lane / 3 % 3 - 1, gz + lane / 9 - 1);
+                const unsigned int b = bucket_of(T, d.x, d.y, d.z);
+                if (!cell_tiled(g, b, d, dmin)) {
+                    beg = __ldg(&g.start[b]);
+                    end = __ldg(&g.start[b + 1]);
+                }
+            }
+        }
+        rest &= ~(((1u << n) - 1u) << src);
         // the lanes among the group's bodies
         const int wlog = n > 4 ? 2 : n > 2 ? 3 : n > 1 ? 4 : 5;
         const int k = lane >> wlog;
@@ -553,7 +599,7 @@ __device__ __forceinline__ void row_slots(RowSmem &sm, const GridView &g,
         B.pi = k < n ? __ldg(&g.spos[B.self]) : z;
         B.vi = k < n ? __ldg(&g.svel[B.self]) : z;
         B.i = k < n ? __float_as_int(B.pi.w) : -1;
-        row_group<false>(sm, g.spos, g.svel, delta, tab, R, P, B, wlog, beg, end - beg, lane);
+        row_group<false>(sm, g.spos, g.svel, delta, tab, R, P, B, wlog, beg, end - beg, crowds, lane);
     }
 }
 
@@ -571,7 +617,7 @@ __device__ __forceinline__ void contact_rows(RowSmem &sm, const float4 *__restri
     }
     const RunDev &R = tab.runs[lo];
     const int first = (w - R.row_start) * (R.glog ? kRowBodies : kDirectBodies);
-    if (R.glog) row_slots(sm, g, delta, tab, R, first, threadIdx.x);
+    if (R.glog) row_slots(sm, g, delta, tab, R, lo, first, threadIdx.x);
     else row_direct(sm, pos, vel, delta, tab, R, first, threadIdx.x);
 }
 

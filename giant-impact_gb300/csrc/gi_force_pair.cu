@@ -651,14 +651,15 @@ __global__ void __launch_bounds__(256) pair_finish_kernel(const ForceArgs a,
 using namespace gi;
 
 cudaError_t gi_launch_pair_force(const ForceArgs &a, const LaunchTable &tab, const GridWork &g,
-                                 long long *delta, bool with_rows, cudaStream_t s)
+                                 long long *delta, const unsigned int *ctr, bool with_rows,
+                                 cudaStream_t s)
 {
     if (tab.nitems <= 0) return cudaSuccess;
     static std::atomic<int> known[64];
     cudaError_t e = gi_full_carveout(reinterpret_cast<const void *>(pair_force_kernel), known);
     if (e != cudaSuccess) return e;
     const int rows = with_rows ? tab.rows : 0;
-    pair_force_kernel<<<rows + tab.nitems, 32, 0, s>>>(a, g.view(), delta, rows, tab);
+    pair_force_kernel<<<rows + tab.nitems, 32, 0, s>>>(a, g.view(ctr), delta, rows, tab);
     return cudaGetLastError();
 }
 

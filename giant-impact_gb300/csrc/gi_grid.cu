@@ -59,6 +59,15 @@ __device__ __forceinline__ void put_body(const float4 *__restrict__ pos,
     svel[slot] = __ldg(&vel[i]);
 }
 
+// Clears the corrections of a run with candidates for the tiled path (other
+// runs' are stored by the row path): thread t of nt.
+__device__ __forceinline__ void clear_delta(long long *__restrict__ delta, const RunDev &R, int t,
+                                            int nt)
+{
+    long long *const d = delta + 3 * (size_t)R.offset;
+    for (long long k = t; k < 3 * (long long)R.n; k += nt) d[k] = 0;
+}
+
 // Pair form of fix_add3 for an unordered pair evaluated once: adds
 // round(c d) to body i's sums and -round(c d), exactly the term body j's own
 // evaluation would give (dp and dv change sign exactly, c is symmetric, and
@@ -131,18 +140,17 @@ contact_row_kernel(const float4 *__restrict__ pos, const float4 *__restrict__ ve
     __shared__ RowSmem sm;
     contact_rows(sm, pos, vel, g, delta, tab, blockIdx.x);
 }
-
 // Work item of the tiled path, self-contained so that the tile kernel reads
 // it in one load, with no hop through the bucket bounds:
 //   x = first slot of the chunk of (up to) 128 bodies of bucket b,
 //   y = first slot of the neighbour bucket nb to stage (the chunk's own
 //       first slot when nb == b, else the start of nb),
 //   z = end of nb,
-//   w = run | cost class << 8 | pair << 12 | self << 13 | bodies of the
+//   w = run | cost class << 8 | tiled << 12 | self << 13 | bodies of the
 //       chunk << 16.
 // The cost class is the number of 128-body tiles the item stages, minus
-// one, capped at kItemClasses - 1; pair: nb is tiled too (each pair is
-// evaluated once for both bodies); self: nb == b.
+// one, capped at kItemClasses - 1; tiled: nb's tiled bodies (dpos), else all
+// of its bodies (spos); self: nb == b.
 // (kItemClasses lives in gi_internal.h.)
 
 // Sub-cell of a body inside its unit cell: 4 x 4 x 4 sub-cells of D/4,
@@ -159,15 +167,13 @@ __device__ __forceinline__ unsigned int subcell_of(float4 p)
 }
 
 // One warp, one candidate bucket b: how many of its bodies are tiled (state, 0
-// for none); clears their corrections (the tiled path adds into them) and
-// copies them to the front of the bucket's dpos / dvel, ordered by sub-cell
+// for none), and copies them to the front of the bucket's dpos / dvel, ordered by sub-cell
 // (counting sort in cnt[64]), so that the 32 bodies of a warp, and the 32 of a
 // staged block, sit close together.  The slots stay as they are for the row
 // path.  Order within a bucket is free: the contact sums are exact integer
 // sums.
 __device__ __forceinline__ bool dense_prep(const Torus &T, const GridWork &g, unsigned int b,
-                                           unsigned int dmin, long long *delta, unsigned int *cnt,
-                                           unsigned int lane)
+                                           unsigned int dmin, unsigned int *cnt, unsigned int lane)
 {
     int3 m;
     const unsigned int t = bucket_tiled(T, g.start, g.spos, b, dmin, (int)lane, m);
@@ -188,8 +194,6 @@ __device__ __forceinline__ bool dense_prep(const Torus &T, const GridWork &g, un
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
             if (u0 + 32u * v >= end || !main(p[v])) continue;
-            long long *d = delta + 3 * (size_t)__float_as_int(p[v].w);
-            d[0] = d[1] = d[2] = 0;
             atomicAdd(&cnt[subcell_of(p[v])], 1u);
         }
     }
@@ -226,13 +230,13 @@ __device__ __forceinline__ bool dense_prep(const Torus &T, const GridWork &g, un
 
 // One warp, one tiled bucket b of run `run`: an item per (chunk of 128 of its
 // tiled bodies, non-empty neighbour bucket nb).  Lanes 0..26 look up the 27
-// neighbour buckets at once.  A pair of tiled buckets is listed once, from the
-// lower bucket number (nb >= b): its item takes nb's tiled bodies and
-// evaluates each contact pair once for both bodies (nb's others are far away).
-// A bucket whose neighbour cell is not the tiled one gets its sums otherwise,
-// so its item adds to b's bodies only.  take(cls, n) is called by one lane per cost class for n items and
-// returns the place of the first (one counter update per class, not per item);
-// put(place, item) stores one.
+// neighbour buckets at once.  Items evaluate each contact pair once for both
+// bodies, so a pair of tiled buckets is listed once, from the lower bucket
+// number (nb >= b), with nb's tiled bodies (its others are far away); where
+// the neighbour cell is not nb's tiled one, the item takes all of nb, and the
+// row path passes over b.  take(cls, n) is called by one lane per cost class
+// for n items and returns the place of the first (one counter update per
+// class, not per item); put(place, item) stores one.
 template <class Take, class Put>
 __device__ __forceinline__ void dense_items(const Torus &T, const GridWork &g, unsigned int b,
                                             unsigned int run, unsigned int dmin, unsigned int lane,
@@ -400,9 +404,13 @@ grid_cluster_kernel(const float4 *__restrict__ pos, const float4 *__restrict__ v
     cluster.sync();  // the slots are written, the counts read
     const unsigned int ncand = c0->cand;
     const unsigned int gw = (unsigned int)(rank * 32 + warp), nw = (unsigned int)ctas * 32u;
+    if (ncand != 0u) {
+        clear_delta(delta, R, rank * 1024 + tid, ctas * 1024);
+        if (rank == 0 && tid == 0) set_crowds(ctr, blockIdx.y);
+    }
     for (unsigned int w = gw; w < ncand; w += nw) {
         const unsigned int b = cand[w].x;
-        if (!dense_prep(T, g, b, dmin, delta, cnt + 64 * warp, (unsigned int)lane)) continue;
+        if (!dense_prep(T, g, b, dmin, cnt + 64 * warp, (unsigned int)lane)) continue;
         if (lane == 0) tiled[atomicAdd(&c0->tiled, 1u)] = make_uint2(b, 0u);
     }
     cluster.sync();  // no CTA leaves before its counters are read
@@ -447,7 +455,10 @@ grid_keys(const float4 *__restrict__ pos, const __grid_constant__ LaunchTable ta
         const unsigned int r = atomicAdd(&g.start[b], 1u);  // counts until they are scanned
         g.keys[i] = b;
         g.ranks[i] = r;
-        if (r == dlo - 1u) g.cand[atomicAdd(&ctr[kCtrCand], 1u)] = make_uint2(b, blockIdx.y);
+        if (r == dlo - 1u) {
+            g.cand[atomicAdd(&ctr[kCtrCand], 1u)] = make_uint2(b, blockIdx.y);
+            set_crowds(ctr, blockIdx.y);
+        }
     }
 }
 
@@ -508,10 +519,13 @@ __global__ void __launch_bounds__(1024) scan_add(unsigned int *__restrict__ a, i
 
 __global__ void __launch_bounds__(256)
 grid_scatter(const float4 *__restrict__ pos, const float4 *__restrict__ vel,
-             const __grid_constant__ LaunchTable tab, const GridWork g)
+             const __grid_constant__ LaunchTable tab, const GridWork g,
+             long long *__restrict__ delta, const unsigned int *__restrict__ ctr)
 {
     const RunDev &R = tab.runs[blockIdx.y];
     if (R.glog == 0) return;
+    if (has_crowds(ctr, blockIdx.y))
+        clear_delta(delta, R, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < R.n; k += gridDim.x * blockDim.x) {
         const int i = R.offset + k;
         put_body(pos, vel, i, g.start[g.keys[i]] + g.ranks[i], g.spos, g.svel);
@@ -521,15 +535,14 @@ grid_scatter(const float4 *__restrict__ pos, const float4 *__restrict__ vel,
 // The crowded buckets of a grid-wide build, one warp per candidate, then one
 // per tiled bucket, then the items into cost-class order.
 __global__ void __launch_bounds__(64)
-dense_prep_kernel(const __grid_constant__ LaunchTable tab, const GridWork g, long long *delta,
-                  unsigned int *ctr)
+dense_prep_kernel(const __grid_constant__ LaunchTable tab, const GridWork g, unsigned int *ctr)
 {
     __shared__ unsigned int cnt[2][64];
     const unsigned int lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const unsigned int total = ctr[kCtrCand];
     for (unsigned int w = 2u * blockIdx.x + warp; w < total; w += 2u * gridDim.x) {
         const uint2 cb = g.cand[w];
-        if (dense_prep(torus_of(tab.runs[cb.y]), g, cb.x, (unsigned int)tab.dense_min, delta,
+        if (dense_prep(torus_of(tab.runs[cb.y]), g, cb.x, (unsigned int)tab.dense_min,
                        cnt[warp], lane) && lane == 0u)
             g.tiled[atomicAdd(&ctr[kCtrTiled], 1u)] = cb;
     }
@@ -623,7 +636,7 @@ constexpr int kTileQueue = kTileDense + 32;  // pairs a warp may have queued
 struct TileSmem {
     float4 sp[128], sv[128];     // the staged bodies: x, y, z, body index (bits); velocity
     float4 ip[128], iv[128];     // the chunk's bodies, the same
-    unsigned int js[6][128];     // sums of the staged bodies (pair items)
+    unsigned int js[6][128];     // sums of the staged bodies
     unsigned int is[6][128];     // queued pairs' sums of the chunk's bodies
     float4 row[3][2];            // the law's constants per pair class (PairRow, Fe bodies of the pair)
     float3 blo[4], bhi[4];       // box of each staged block of 32
@@ -643,7 +656,7 @@ __device__ __forceinline__ PairRow tile_row(const TileSmem &sm, int cls)
 // additions to the slots' shared sums never meet in a bank, and no list is
 // kept.  For a block with itself steps 1 to 16 cover each pair once (the
 // pair's terms are the same, with opposite signs, from either body).
-template <bool PAIR, bool MIXED>
+template <bool MIXED>
 __device__ __forceinline__ void tile_block(FixSum3 &acc, TileSmem &sm, int s, bool diag, int lane,
                                            float4 pi, float4 vi, int ife, int cls, long long *delta,
                                            int sw, int sep_test, float inv_unit)
@@ -661,14 +674,12 @@ __device__ __forceinline__ void tile_block(FixSum3 &acc, TileSmem &sm, int s, bo
             const int j = __float_as_int(pj.w);
             if (MIXED) row = tile_row(sm, ife + (int)(j < sw));
             const float c = contact_coef_at(row, sep_test, dx, dy, dz, r2, &vi, &sm.sv[k]) * inv_unit;
-            if (PAIR) fix_add3_pair(acc, sm.js, k, delta + 3 * (size_t)j, c, dx, dy, dz, r2);
-            else fix_add3<false>(acc, c, dx, dy, dz, r2);
+            fix_add3_pair(acc, sm.js, k, delta + 3 * (size_t)j, c, dx, dy, dz, r2);
         }
     }
 }
 
 // One queued pair per lane (all of them hits), n lanes.
-template <bool PAIR>
 __device__ __forceinline__ void tile_pair(TileSmem &sm, unsigned int e, bool on, int warp,
                                           long long *delta, int sw, int sep_test, float inv_unit)
 {
@@ -690,10 +701,8 @@ __device__ __forceinline__ void tile_pair(TileSmem &sm, unsigned int e, bool on,
         for (int d = 0; d < 3; ++d) {
             atomicAdd(&sm.is[d][t], h[d] - __float_as_uint(kFixM));
             atomicAdd(&sm.is[3 + d][t], l[d] - __float_as_uint(kFixC));
-            if (PAIR) {
-                atomicAdd(&sm.js[d][k], __float_as_uint(kFixM) - h[d]);
-                atomicAdd(&sm.js[3 + d][k], __float_as_uint(kFixC) - l[d]);
-            }
+            atomicAdd(&sm.js[d][k], __float_as_uint(kFixM) - h[d]);
+            atomicAdd(&sm.js[3 + d][k], __float_as_uint(kFixC) - l[d]);
         }
     } else {  // out of the split's range: to the global sums
         unsigned long long *di = reinterpret_cast<unsigned long long *>(delta + 3 * (size_t)i);
@@ -702,7 +711,7 @@ __device__ __forceinline__ void tile_pair(TileSmem &sm, unsigned int e, bool on,
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             atomicAdd(di + d, (unsigned long long)v[d]);
-            if (PAIR) atomicAdd(dj + d, 0ull - (unsigned long long)v[d]);
+            atomicAdd(dj + d, 0ull - (unsigned long long)v[d]);
         }
     }
 }
@@ -715,12 +724,11 @@ __device__ __forceinline__ void tile_pair(TileSmem &sm, unsigned int e, bool on,
 // of which at least half the pairs are contacts as a whole (tile_block: a
 // crowded core's pairs mostly are); from the rest it filters the hits
 // (r2 < 1) into a queue of pairs and evaluates the law on full warps of
-// those, whose sums go through shared memory on both sides.  When nb is tiled
-// too, each pair is evaluated once for both bodies: the item covers nb's
-// tiles from the chunk's own slots on (all of them when nb != b; within the
-// chunk's own tile only slots above the thread's), and the staged bodies'
-// shared sums go into their corrections with 64-bit global atomics once per
-// tile.
+// those, whose sums go through shared memory on both sides.  Each pair is
+// evaluated once for both bodies: a self item covers the tiles from the
+// chunk's own slots on (within the chunk's own tile only slots above the
+// thread's), and the staged bodies' shared sums go into their corrections
+// with 64-bit global atomics once per tile.
 //
 // What bounds it is the issue rate.  One hit list per thread left 46 % of the
 // lanes idle (a block of few hits 78 %), and the lists' scattered additions
@@ -756,7 +764,7 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
         unsigned int nw = 0u;  // thread 0: the next item
         const unsigned int s0 = rec.x, first = rec.y, nend = rec.z;
         const unsigned int ni = rec.w >> 16;
-        const bool pair = (rec.w >> 12) & 1u, self = (rec.w >> 13) & 1u;
+        const bool tiled = (rec.w >> 12) & 1u, self = (rec.w >> 13) & 1u;
         const bool valid = (unsigned int)t < ni;
         const RunDev &R = tab.runs[rec.w & 0xffu];
         const int sw = R.offset + R.nfe;
@@ -764,7 +772,7 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
         const float4 pi = valid ? dpos[s0 + t] : make_float4(kInf, kInf, kInf, __int_as_float(-1));
         const float4 vi = valid ? dvel[s0 + t] : make_float4(0.f, 0.f, 0.f, 0.f);
         const int i = __float_as_int(pi.w), ife = i < sw;
-        const float4 *npos = pair ? dpos : spos, *nvel = pair ? dvel : svel;
+        const float4 *npos = tiled ? dpos : spos, *nvel = tiled ? dvel : svel;
         sm.ip[t] = pi;  // read by its own warp alone
         sm.iv[t] = vi;
         if (t < 3) {
@@ -780,7 +788,7 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
         fix_zero(acc);
         for (unsigned int base = first; base < nend; base += 128u) {
             __syncthreads();  // the previous tile is consumed
-            if (pair && base != first) flush_slot(sm.js, t, __float_as_int(sm.sp[t].w), delta);
+            if (base != first) flush_slot(sm.js, t, __float_as_int(sm.sp[t].w), delta);
             if (t == 0 && base + 128u >= nend) nw = atomicAdd(&ctr[kCtrHead], 1u);
             const unsigned int u = base + (unsigned int)t;
             float3 lo = make_float3(kInf, kInf, kInf), hi = make_float3(-kInf, -kInf, -kInf);
@@ -810,8 +818,7 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
                 __syncwarp();  // the entries are written
                 const unsigned int e = lane < n ? queue[qn + lane] : 0u;
                 __syncwarp();  // and read, before their places are written again
-                if (pair) tile_pair<true>(sm, e, lane < n, warp, delta, sw, tab.sep_test, inv_unit);
-                else tile_pair<false>(sm, e, lane < n, warp, delta, sw, tab.sep_test, inv_unit);
+                tile_pair(sm, e, lane < n, warp, delta, sw, tab.sep_test, inv_unit);
             };
             for (int s = own ? warp : 0; 32 * s < cnt; ++s) {
                 const float3 jlo = sm.blo[s], jhi = sm.bhi[s];
@@ -838,17 +845,12 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
                 }
                 if (dense) {
                     const int cls = sm.bcls[s];
-                    if (pair) {
-                        if (cls == 2)
-                            tile_block<true, true>(acc, sm, s, diag, lane, pi, vi, ife, cls, delta, sw,
-                                                   tab.sep_test, inv_unit);
-                        else
-                            tile_block<true, false>(acc, sm, s, diag, lane, pi, vi, ife, cls, delta, sw,
-                                                    tab.sep_test, inv_unit);
-                    } else {
-                        tile_block<false, true>(acc, sm, s, diag, lane, pi, vi, ife, cls, delta, sw,
-                                                tab.sep_test, inv_unit);
-                    }
+                    if (cls == 2)
+                        tile_block<true>(acc, sm, s, diag, lane, pi, vi, ife, cls, delta, sw,
+                                         tab.sep_test, inv_unit);
+                    else
+                        tile_block<false>(acc, sm, s, diag, lane, pi, vi, ife, cls, delta, sw,
+                                          tab.sep_test, inv_unit);
                     continue;
                 }
                 // Queue the hits, one of each lane at a time and from staggered
@@ -884,7 +886,7 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
             }
         }
         __syncthreads();  // the last tile's j-side sums are complete; sm.w is read
-        if (pair) flush_slot(sm.js, t, __float_as_int(sm.sp[t].w), delta);
+        flush_slot(sm.js, t, __float_as_int(sm.sp[t].w), delta);
         if (t == 0) sm.w = nw;
         __syncthreads();  // the next item's index is visible
         fix_fold(acc);
@@ -989,9 +991,9 @@ cudaError_t gi_launch_grid(const float4 *pos, const float4 *vel, const LaunchTab
     gi::scan_blocks<<<sb, 1024, 0, s>>>(g.start, (int)m + 1, g.sums);
     gi::scan_sums<<<1, 1024, 0, s>>>(g.sums, sb);
     gi::scan_add<<<sb, 1024, 0, s>>>(g.start, (int)m + 1, g.sums);
-    gi::grid_scatter<<<gk, 256, 0, s>>>(pos, vel, tab, g);
+    gi::grid_scatter<<<gk, 256, 0, s>>>(pos, vel, tab, g, delta, ctr);
     const int gb = (int)std::min<size_t>((g.bcap + 1) / 2, 8 * (size_t)nsm);
-    gi::dense_prep_kernel<<<gb, 64, 0, s>>>(tab, g, delta, ctr);
+    gi::dense_prep_kernel<<<gb, 64, 0, s>>>(tab, g, ctr);
     gi::dense_items_kernel<<<gb, 64, 0, s>>>(tab, g, ctr);
     const int go = (int)std::min<size_t>((g.icap + 255) / 256, 4 * (size_t)nsm);
     gi::dense_order_kernel<<<go, 256, 0, s>>>(g.raw, ctr, g.items);
@@ -999,13 +1001,14 @@ cudaError_t gi_launch_grid(const float4 *pos, const float4 *vel, const LaunchTab
 }
 
 cudaError_t gi_launch_rows(const float4 *pos, const float4 *vel, const LaunchTable &tab,
-                           const GridWork &g, long long *delta, cudaStream_t s)
+                           const GridWork &g, long long *delta, const unsigned int *ctr,
+                           cudaStream_t s)
 {
     if (tab.rows == 0) return cudaSuccess;
     static std::atomic<int> known[64];
     const cudaError_t e = gi_full_carveout(reinterpret_cast<const void *>(gi::contact_row_kernel), known);
     if (e != cudaSuccess) return e;
-    gi::contact_row_kernel<<<tab.rows, 32, 0, s>>>(pos, vel, g.view(), delta, tab);
+    gi::contact_row_kernel<<<tab.rows, 32, 0, s>>>(pos, vel, g.view(ctr), delta, tab);
     return cudaGetLastError();
 }
 

@@ -132,7 +132,8 @@ static_assert(kPairMaxCpi <= kPairBlockChunks && kPairBlockChunks % kPairMaxCpi 
 // (the grid must be built); then the epilogue, as gi_launch_finish.
 struct GridWork;
 cudaError_t gi_launch_pair_force(const ForceArgs &a, const LaunchTable &tab, const GridWork &g,
-                                 long long *delta, bool with_rows, cudaStream_t s);
+                                 long long *delta, const unsigned int *ctr, bool with_rows,
+                                 cudaStream_t s);
 // Pair potentials of the table's runs (planned as for gi_launch_pair_force):
 // one double per CTA in per_cta, one per run in out, in table order.
 cudaError_t gi_launch_potential(const float4 *pos, const LaunchTable &tab, double *per_cta,
@@ -151,8 +152,8 @@ constexpr unsigned int kDenseFloor = 32;
 // Cost classes of the tiled path's work items (128-body tiles staged - 1).
 constexpr unsigned int kItemClasses = 16;
 // Tiled-path counters: items, tiled buckets, queue head, candidate buckets,
-// then a count and a fill cursor per cost class.
-constexpr int kCtrWords = 4 + 2 * (int)kItemClasses;
+// then a count and a fill cursor per cost class, then a bit per run.
+constexpr int kCtrWords = 4 + 2 * (int)kItemClasses + GI_MAX_RUNS / 32;
 // Runs of at most this many bodies take no grid.
 constexpr int kDirectMax = 4096;
 // Bodies of a row-path CTA (one warp), of a run with a grid and without.
@@ -193,8 +194,8 @@ constexpr size_t gi_grid_words(long long max_end, long long bodies)
 }
 // What the row path reads of it.
 struct GridView {
-    const float4 *spos, *svel;
-    const unsigned int *start;
+    const float4 *spos, *svel, *dpos;
+    const unsigned int *start, *state, *ctr;
 };
 // The scratch of one table's contact pass, carved from `work` (16-byte
 // aligned): 16-byte words first, then single words (see gi_grid_words).
@@ -224,12 +225,15 @@ struct GridWork {
         keys = sums + 9216;
         ranks = keys + max_end;
     }
-    GridView view() const { return GridView{spos, svel, start}; }
+    GridView view(const unsigned int *ctr) const
+    {
+        return GridView{spos, svel, dpos, start, state, ctr};
+    }
 };
 // Sets the grid and row fields of the table and its runs.
 void gi_grid_runs(LaunchTable &tab);
 // The contact pass, in this order: the grid (with the tiled path's work
-// items); the row path, here or in gi_launch_pair_force; the tiled path.
+// items); the row path, here or in gi_launch_pair_force, and the tiled path.
 // delta receives every body's correction.  ctr: gi::kCtrWords words, zero on
 // entry of the first.  clusters: build the grids of runs below 131,072 bodies
 // with one thread-block cluster each (see grid_cluster_kernel).
@@ -237,7 +241,8 @@ cudaError_t gi_launch_grid(const float4 *pos, const float4 *vel, const LaunchTab
                            const GridWork &g, long long *delta, unsigned int *ctr, int nsm,
                            bool clusters, cudaStream_t s);
 cudaError_t gi_launch_rows(const float4 *pos, const float4 *vel, const LaunchTable &tab,
-                           const GridWork &g, long long *delta, cudaStream_t s);
+                           const GridWork &g, long long *delta, const unsigned int *ctr,
+                           cudaStream_t s);
 cudaError_t gi_launch_tiles(const LaunchTable &tab, const GridWork &g, long long *delta,
                             unsigned int *ctr, int nsm, cudaStream_t s);
 

@@ -201,7 +201,7 @@ extern "C" int gi_forces_collision_noalloc(const float *pos, const float *vel, f
     a.delta = delta;
     a.fsum_fx = sums;
     a.fsum_plane = (size_t)n;
-    if (gi_launch_pair_force(a, tab, g, delta, true, s) != cudaSuccess)
+    if (gi_launch_pair_force(a, tab, g, delta, ctr, true, s) != cudaSuccess)
         return gi_internal_fail(GI_ERR_CUDA, "force kernel launch failed");
     if (gi_launch_pair_finish(GI_EPI_FORCE, a, tab, n, nsm, s) != cudaSuccess)
         return gi_internal_fail(GI_ERR_CUDA, "epilogue launch failed");
