@@ -633,16 +633,25 @@ __device__ __forceinline__ bool box_near(float3 ilo, float3 ihi, float3 jlo, flo
 // The tiled path's shared memory.
 constexpr int kTileDense = 512;               // hits of 1,024 pairs: see tile_block
 constexpr int kTileQueue = kTileDense + 32;  // pairs a warp may have queued
+// An item is handed out in up to 8 units of its blocks of 32 staged bodies, as
+// long as there are at most kTileUnits of them per CTA: a tile keeps a warp
+// busy for 30 us or more, and a small remnant has fewer items than the GPU has
+// room for.  us a step, whole items / units: 4,500 remnant bodies 211 / 108,
+// 9,000 291 / 168, 20,000 392 / 305, 40,000 758 / 749; 16 and 32 units per CTA
+// take 2 to 5 % more from 40,000 bodies on.
+constexpr unsigned int kTilePartsLog2 = 3, kTileUnits = 8;
 struct TileSmem {
     float4 sp[128], sv[128];     // the staged bodies: x, y, z, body index (bits); velocity
     float4 ip[128], iv[128];     // the chunk's bodies, the same
     unsigned int js[6][128];     // sums of the staged bodies
     unsigned int is[6][128];     // queued pairs' sums of the chunk's bodies
     float4 row[3][2];            // the law's constants per pair class (PairRow, Fe bodies of the pair)
-    float3 blo[4], bhi[4];       // box of each staged block of 32
+    float3 ilo[4], ihi[4];       // box of each warp's bodies
+    float3 blo[4], bhi[4];       // and of each staged block of 32
     int bcls[4];                 // its bodies: 0 Si, 1 Fe, 2 both
     unsigned short queue[4][kTileQueue];  // per warp: lane of i | staged slot of j << 5
-    unsigned int w;              // the item to take next
+    unsigned int units, plog;    // units in all; log2 of an item's
+    unsigned int w;              // the unit to take next
 };
 
 __device__ __forceinline__ PairRow tile_row(const TileSmem &sm, int cls)
@@ -658,9 +667,11 @@ __device__ __forceinline__ PairRow tile_row(const TileSmem &sm, int cls)
 // pair's terms are the same, with opposite signs, from either body).
 template <bool MIXED>
 __device__ __forceinline__ void tile_block(FixSum3 &acc, TileSmem &sm, int s, bool diag, int lane,
-                                           float4 pi, float4 vi, int ife, int cls, long long *delta,
-                                           int sw, int sep_test, float inv_unit)
+                                           float4 pi, int cls, long long *delta, int sw,
+                                           int sep_test, float inv_unit)
 {
+    const float4 vi = sm.iv[threadIdx.x];
+    const int ife = __float_as_int(pi.w) < sw;
     const float2 npxy = make_float2(-pi.x, -pi.y);
     PairRow row = tile_row(sm, MIXED ? 0 : ife + cls);
     const int r1 = !diag ? 32 : lane < 16 ? 17 : 16;
@@ -725,8 +736,8 @@ __device__ __forceinline__ void tile_pair(TileSmem &sm, unsigned int e, bool on,
 // crowded core's pairs mostly are); from the rest it filters the hits
 // (r2 < 1) into a queue of pairs and evaluates the law on full warps of
 // those, whose sums go through shared memory on both sides.  Each pair is
-// evaluated once for both bodies: a self item covers the tiles from the
-// chunk's own slots on (within the chunk's own tile only slots above the
+// evaluated once for both bodies: a self item covers the blocks from the
+// chunk's own slots on, a warp those from its own (there only slots above the
 // thread's), and the staged bodies' shared sums go into their corrections
 // with 64-bit global atomics once per tile.
 //
@@ -744,7 +755,6 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
                     const uint4 *__restrict__ items, unsigned int *__restrict__ ctr)
 {
     __shared__ TileSmem sm;
-    const unsigned int total = ctr[kCtrItems];
     const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
     const unsigned int all = 0xffffffffu;
@@ -752,29 +762,46 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
     unsigned short *const queue = sm.queue[warp];
 #pragma unroll
     for (int d = 0; d < 6; ++d) sm.js[d][t] = sm.is[d][t] = 0u;
-    // Thread 0 takes the next item from the queue when the current one
+    // Thread 0 takes the next unit from the queue when the current one
     // reaches its last tile: the atomic's latency hides behind that tile,
     // and the CTA still takes items close to the queue's longest-first order.
-    if (t == 0) sm.w = atomicAdd(&ctr[kCtrHead], 1u);
+    if (t == 0) {
+        sm.w = atomicAdd(&ctr[kCtrHead], 1u);
+        const unsigned int total = ctr[kCtrItems];
+        unsigned int plog = 0u;
+        while (plog < kTilePartsLog2 && total << (plog + 1u) <= kTileUnits * gridDim.x) ++plog;
+        sm.plog = plog;
+        sm.units = total << plog;
+    }
     __syncthreads();
     for (;;) {
-        const unsigned int w = sm.w;
-        if (w >= total) break;
-        const uint4 rec = items[w];
-        unsigned int nw = 0u;  // thread 0: the next item
-        const unsigned int s0 = rec.x, first = rec.y, nend = rec.z;
+        const unsigned int w = sm.w, plog = sm.plog;
+        if (w >= sm.units) break;
+        const uint4 rec = items[w >> plog];
+        unsigned int nw = 0u;  // thread 0: the next unit
+        const unsigned int s0 = rec.x;
+        // the unit's part of nb, in blocks of 32 from rec.y on
+        const unsigned int per = ((((rec.z - rec.y + 31u) / 32u) - 1u) >> plog) + 1u;
+        const unsigned int first = rec.y + 32u * per * (w & ((1u << plog) - 1u));
+        const unsigned int nend = min(rec.z, first + 32u * per);
+        if (first >= nend) {
+            __syncthreads();  // sm.w is read
+            if (t == 0) sm.w = atomicAdd(&ctr[kCtrHead], 1u);
+            __syncthreads();
+            continue;
+        }
         const unsigned int ni = rec.w >> 16;
-        const bool tiled = (rec.w >> 12) & 1u, self = (rec.w >> 13) & 1u;
+        const bool tiled = (rec.w >> 12) & 1u;
+        // block 0's place after the warp's own, where nb is b itself
+        int rel = (rec.w >> 13) & 1u ? (int)(first - rec.y) / 32 - warp : 1;
         const bool valid = (unsigned int)t < ni;
         const RunDev &R = tab.runs[rec.w & 0xffu];
         const int sw = R.offset + R.nfe;
         const float inv_unit = tab.params[R.param].inv_unit;
         const float4 pi = valid ? dpos[s0 + t] : make_float4(kInf, kInf, kInf, __int_as_float(-1));
-        const float4 vi = valid ? dvel[s0 + t] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const int i = __float_as_int(pi.w), ife = i < sw;
         const float4 *npos = tiled ? dpos : spos, *nvel = tiled ? dvel : svel;
         sm.ip[t] = pi;  // read by its own warp alone
-        sm.iv[t] = vi;
+        sm.iv[t] = valid ? dvel[s0 + t] : make_float4(0.f, 0.f, 0.f, 0.f);
         if (t < 3) {
             const PairRow q = pair_row(tab.params[R.param], t > 0, t > 1);
             sm.row[t][0] = make_float4(q.G, q.K, q.Tband, q.Tmid);
@@ -783,10 +810,14 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
         float3 ilo = valid ? make_float3(pi.x, pi.y, pi.z) : make_float3(kInf, kInf, kInf);
         float3 ihi = valid ? make_float3(pi.x, pi.y, pi.z) : make_float3(-kInf, -kInf, -kInf);
         warp_box(ilo, ihi);
+        if (lane == 0) {
+            sm.ilo[warp] = ilo;
+            sm.ihi[warp] = ihi;
+        }
         const bool full = (unsigned int)(32 * warp + 32) <= ni;
         FixSum3 acc;
         fix_zero(acc);
-        for (unsigned int base = first; base < nend; base += 128u) {
+        for (unsigned int base = first; base < nend; base += 128u, rel += 4) {
             __syncthreads();  // the previous tile is consumed
             if (base != first) flush_slot(sm.js, t, __float_as_int(sm.sp[t].w), delta);
             if (t == 0 && base + 128u >= nend) nw = atomicAdd(&ctr[kCtrHead], 1u);
@@ -809,7 +840,6 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
             }
             __syncthreads();
             const int cnt = (int)min(128u, nend - base);
-            const bool own = self && base == first;  // own tile: each pair once
             int qn = 0;                              // queued pairs, the same in the warp
             bool queued = false;
             const auto drain = [&] {
@@ -820,11 +850,11 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
                 __syncwarp();  // and read, before their places are written again
                 tile_pair(sm, e, lane < n, warp, delta, sw, tab.sep_test, inv_unit);
             };
-            for (int s = own ? warp : 0; 32 * s < cnt; ++s) {
-                const float3 jlo = sm.blo[s], jhi = sm.bhi[s];
-                if (box_gap2(ilo, ihi, jlo, jhi) >= 1.0f) continue;  // the same for the warp
-                const bool diag = own && s == warp;
-                bool dense = full && 32 * s + 32 <= cnt && box_near(ilo, ihi, jlo, jhi);
+            for (int s = max(-rel, 0); 32 * s < cnt; ++s) {
+                const float3 alo = sm.ilo[warp], ahi = sm.ihi[warp], jlo = sm.blo[s], jhi = sm.bhi[s];
+                if (box_gap2(alo, ahi, jlo, jhi) >= 1.0f) continue;  // the same for the warp
+                const bool diag = rel + s == 0;  // the warp's own bodies: each pair once
+                bool dense = full && 32 * s + 32 <= cnt && box_near(alo, ahi, jlo, jhi);
                 unsigned int m = 0u;
                 if (!dense) {
                     for (int k = 0; k < 32 && 32 * s + k < cnt; k += 8) {
@@ -846,11 +876,11 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
                 if (dense) {
                     const int cls = sm.bcls[s];
                     if (cls == 2)
-                        tile_block<true>(acc, sm, s, diag, lane, pi, vi, ife, cls, delta, sw,
-                                         tab.sep_test, inv_unit);
+                        tile_block<true>(acc, sm, s, diag, lane, pi, cls, delta, sw, tab.sep_test,
+                                         inv_unit);
                     else
-                        tile_block<false>(acc, sm, s, diag, lane, pi, vi, ife, cls, delta, sw,
-                                          tab.sep_test, inv_unit);
+                        tile_block<false>(acc, sm, s, diag, lane, pi, cls, delta, sw, tab.sep_test,
+                                          inv_unit);
                     continue;
                 }
                 // Queue the hits, one of each lane at a time and from staggered
@@ -888,11 +918,12 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
         __syncthreads();  // the last tile's j-side sums are complete; sm.w is read
         flush_slot(sm.js, t, __float_as_int(sm.sp[t].w), delta);
         if (t == 0) sm.w = nw;
-        __syncthreads();  // the next item's index is visible
+        __syncthreads();  // the next unit's index is visible
         fix_fold(acc);
         const long long ax = acc.x, ay = acc.y, az = acc.z;
         if (valid && (ax | ay | az)) {
-            unsigned long long *d = reinterpret_cast<unsigned long long *>(delta + 3 * (size_t)i);
+            unsigned long long *d = reinterpret_cast<unsigned long long *>(
+                delta + 3 * (size_t)__float_as_int(pi.w));
             atomicAdd(d + 0, (unsigned long long)ax);
             atomicAdd(d + 1, (unsigned long long)ay);
             atomicAdd(d + 2, (unsigned long long)az);
