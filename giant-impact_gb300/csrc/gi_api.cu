@@ -257,6 +257,14 @@ struct StreamScratch {
     double *fsum = nullptr;  // far-field sums, 3 per body: FP64 (one-sided GI_EPI_SUM launches)
                              // or int64 fixed point (paired far field); behind them the
                              // contact pass's counters (kCtrWords), cleared with them
+    // Leading bytes of fsum that are zero once the stream's work is done.  The
+    // paired epilogue leaves the sums and counters it has read at zero, so a
+    // call that finds enough of them clean needs no clear (4 us of a small
+    // run's step); 0 from before a call's first launch until its last.  A call
+    // under capture clears always, whatever comes before its replays, and so
+    // does every call once a one-sided call was captured (replayed unseen).
+    size_t clean = 0;
+    bool always_clear = false;
     // The contact pass runs on `aux`, beside the far field on the caller's
     // stream: forked after the previous step, joined before the epilogue.
     cudaStream_t aux = nullptr;
@@ -817,6 +825,7 @@ static int ensure_scratch(gi_ctx *c, const Plan &plan, cudaStream_t s, StreamScr
         x.delta = nullptr;
         x.fsum = nullptr;
         x.delta_cap = 0;
+        x.clean = 0;
         GI_CUDA(cudaMalloc(&x.delta, (size_t)plan.max_end * 3 * sizeof(long long)), "cudaMalloc delta");
         GI_CUDA(cudaMalloc(&x.fsum, (size_t)plan.max_end * 3 * sizeof(double) +
                                         gi::kCtrWords * sizeof(unsigned int)),
@@ -874,10 +883,11 @@ constexpr int kSideBySideCtas = 8;
 // The epilogue then runs on the caller's stream with the fused epilogue's
 // arithmetic.  Larger tables run the contact pass first.  Either way the
 // results are the same bits.
-static int run_force_plan(gi_ctx *c, const StreamScratch *x, const Plan &plan, int epi,
+static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi,
                           const float4 *pos, const float4 *vel, float4 *force,
                           float4 *pos_out, float4 *vel_out, cudaStream_t s)
 {
+    const bool capturing = stream_capturing(s);
     for (size_t t = 0; t < plan.tables.size(); ++t) {
         const LaunchTable &tab = plan.tables[t];
         ForceArgs a;
@@ -904,12 +914,16 @@ static int run_force_plan(gi_ctx *c, const StreamScratch *x, const Plan &plan, i
         const GridWork gw(x->grid_work, plan.bodies[t], plan.max_end);
         if (plan.paired) {
             // The far-field sums and the contact pass's counters start at
-            // zero; captured with the launches when the stream is capturing.
+            // zero; a clear is captured with the launches when the stream is
+            // capturing.
             a.fsum_fx = reinterpret_cast<long long *>(x->fsum);
             a.fsum_plane = (size_t)plan.max_end;
-            GI_CUDA(cudaMemsetAsync(a.fsum_fx, 0, (size_t)plan.max_end * 3 * sizeof(long long) +
-                                                      gi::kCtrWords * sizeof(unsigned int), s),
-                    "cudaMemsetAsync far-field sums");
+            const size_t bytes = (size_t)plan.max_end * 3 * sizeof(long long) +
+                                 gi::kCtrWords * sizeof(unsigned int);
+            const size_t clean = std::max(x->clean, bytes);
+            if (capturing || x->always_clear || x->clean < bytes)
+                GI_CUDA(cudaMemsetAsync(a.fsum_fx, 0, bytes, s), "cudaMemsetAsync far-field sums");
+            if (!capturing) x->clean = 0;
             const bool beside = pairs >= kBesideMinPairs && pairs < kOverlapMaxPairs;
             const cudaStream_t q = beside ? x->aux : s;
             if (beside) {
@@ -928,8 +942,11 @@ static int run_force_plan(gi_ctx *c, const StreamScratch *x, const Plan &plan, i
                 GI_CUDA(cudaStreamWaitEvent(s, x->ev_join, 0), "cudaStreamWaitEvent");
             }
             GI_CUDA(gi_launch_pair_finish(epi, a, tab, maxn, c->sm_count, s), "epilogue launch");
+            if (!capturing) x->clean = clean;
             continue;
         }
+        x->clean = 0;  // one-sided: FP64 sums there
+        x->always_clear |= capturing;
         const int p = plan.ipt[t];
         const int occ = c->occ[c->opt.accum][p];
         // The queue and this table's tickets start at zero (the kernel also

@@ -628,7 +628,9 @@ potential_sum_kernel(const __grid_constant__ LaunchTable tab, const double *__re
 
 // The epilogue: F = fixed-point far field + contact correction, rounded once
 // to float, stored (GI_EPI_FORCE) or applied as the kick-drift (GI_EPI_STEP)
-// by finish_body, the one-sided kernel's own epilogue arithmetic.
+// by finish_body, the one-sided kernel's own epilogue arithmetic.  The sums
+// and, behind them, the contact pass's counters are left at zero for the next
+// call.
 template <int EPI>
 __global__ void __launch_bounds__(256) pair_finish_kernel(const ForceArgs a,
                                                           const __grid_constant__ LaunchTable tab)
@@ -636,12 +638,15 @@ __global__ void __launch_bounds__(256) pair_finish_kernel(const ForceArgs a,
     const RunDev &R = tab.runs[blockIdx.y];
     const double unit = tab.params[R.param].fx_unit;
     const double far_unit = R.far_unit;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kCtrWords)
+        reinterpret_cast<unsigned int *>(a.fsum_fx + 3 * a.fsum_plane)[threadIdx.x] = 0u;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < R.n; k += gridDim.x * blockDim.x) {
         const int i = R.offset + k;
-        const long long *q = a.fsum_fx + i;
+        long long *q = a.fsum_fx + i;
         const double fd[3] = {(double)__ldcg(q) * far_unit,
                               (double)__ldcg(q + a.fsum_plane) * far_unit,
                               (double)__ldcg(q + 2 * a.fsum_plane) * far_unit};
+        q[0] = q[a.fsum_plane] = q[2 * a.fsum_plane] = 0;
         finish_body<EPI>(a, R, unit, i, fd);
     }
 }

@@ -124,3 +124,51 @@ def test_crowded_cell_sizes(gi, torch_cuda, m, spread):
         out.append(f)
         ctx.close()
     assert torch.equal(out[0], out[1])
+
+
+def test_calls_after_one_another(gi, torch_cuda):
+    """The far-field sums are left clean for the next call on the stream: a
+    run's forces are a fresh context's, after larger and smaller runs, runs
+    with bodies between them, one-sided calls and graphs of either kind."""
+    import gi_workloads as wl
+    torch = torch_cuda
+    p = wl.params(gi)
+    sizes = [(20000, 0), (700, 0), (5000, 300), (33000, 7), (1, 0), (9000, 20000)]
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        s = st.cuda_stream
+        pos, vel = _aliased(3, 42000)
+        dp, dv = _dev(torch, pos), _dev(torch, vel)
+        state = [t.clone() for t in (dp, dv, dp, dv)]
+        ctx = gi.Context(0)
+
+        def force(c, n, off):
+            f = torch.zeros_like(dp)
+            c.forces(dp.data_ptr(), dv.data_ptr(), f.data_ptr(), [wl.run_desc(gi, off, n, n // 5)], p, s)
+            st.synchronize()
+            return f
+
+        def graph(n):
+            q = [t.data_ptr() for t in state]
+            return ctx.graph(*q, [wl.run_desc(gi, 0, n, n // 5)], p, 3, s)
+
+        want = []
+        for n, off in sizes:
+            c = gi.Context(0)
+            want.append(force(c, n, off))
+            c.close()
+        force(ctx, 42000, 0)  # a graph keeps the scratch it was captured with: no call may outgrow it
+        graphs = [graph(30000)]
+        for rep in range(3):
+            for (n, off), w in zip(sizes, want):
+                assert torch.equal(force(ctx, n, off), w)
+                for g in graphs:
+                    g.launch(s)
+            if rep == 0:
+                ctx.set_options(accum=gi.GI_ACCUM_FP64)
+                force(ctx, 25000, 0)
+                graphs.append(graph(12000))
+                ctx.set_options()
+        for g in graphs:
+            g.close()
+        ctx.close()
