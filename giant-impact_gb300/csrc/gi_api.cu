@@ -261,14 +261,15 @@ struct StreamScratch {
     // paired epilogue leaves the sums and counters it has read at zero, so a
     // call that finds enough of them clean needs no clear (4 us of a small
     // run's step); 0 from before a call's first launch until its last.  A call
-    // under capture clears always, whatever comes before its replays, and so
-    // does every call once a one-sided call was captured (replayed unseen).
+    // under capture clears first, whatever comes before its replays, and so does
+    // every call once a one-sided call was captured (replayed unseen).
     size_t clean = 0;
     bool always_clear = false;
-    // The contact pass runs on `aux`, beside the far field on the caller's
-    // stream: forked after the previous step, joined before the epilogue.
-    cudaStream_t aux = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // The contact pass runs on `aux` (paired: its row contacts on aux_rows),
+    // beside the far field on the caller's stream: see run_force_plan.
+    cudaStream_t aux = nullptr, aux_rows = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_grid = nullptr, ev_rows = nullptr,
+                ev_far = nullptr;
 };
 
 struct gi_ctx {
@@ -333,9 +334,10 @@ static void ctx_free(gi_ctx *c)
         cudaFree(x.grid_work);
         cudaFree(x.delta);
         cudaFree(x.fsum);
-        if (x.ev_fork) cudaEventDestroy(x.ev_fork);
-        if (x.ev_join) cudaEventDestroy(x.ev_join);
+        for (cudaEvent_t e : {x.ev_fork, x.ev_join, x.ev_grid, x.ev_rows, x.ev_far})
+            if (e) cudaEventDestroy(e);
         if (x.aux) cudaStreamDestroy(x.aux);
+        if (x.aux_rows) cudaStreamDestroy(x.aux_rows);
     }
     c->scratch.clear();
     cudaFree(c->mirror_pos);
@@ -785,13 +787,16 @@ static int ensure_scratch(gi_ctx *c, const Plan &plan, cudaStream_t s, StreamScr
         return fail(GI_ERR_INVALID_ARG,
                     "scratch must grow (run once outside stream capture before capturing)");
     GI_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
-    if (!x.aux) {
+    if (!x.aux) {  // created last: the others are there when it is
         int lo = 0, hi = 0;  // hi: the greatest priority (numerically lowest)
         GI_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi), "cudaDeviceGetStreamPriorityRange");
+        for (cudaEvent_t *e : {&x.ev_fork, &x.ev_join, &x.ev_grid, &x.ev_rows, &x.ev_far})
+            if (!*e) GI_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
+        if (!x.aux_rows)
+            GI_CUDA(cudaStreamCreateWithPriority(&x.aux_rows, cudaStreamNonBlocking, lo),
+                    "cudaStreamCreateWithPriority");
         GI_CUDA(cudaStreamCreateWithPriority(&x.aux, cudaStreamNonBlocking, hi),
                 "cudaStreamCreateWithPriority");
-        GI_CUDA(cudaEventCreateWithFlags(&x.ev_fork, cudaEventDisableTiming), "cudaEventCreate");
-        GI_CUDA(cudaEventCreateWithFlags(&x.ev_join, cudaEventDisableTiming), "cudaEventCreate");
     }
     if (grow_t || !x.counters) {
         cudaFree(x.counters);
@@ -855,12 +860,13 @@ static int convert_params(const gi_pair_params *params, int nparams, std::vector
 // uniform balls (default tuning): the side-by-side pass takes 33 % off at
 // n = 8,192, 5 % at 49,152, 2 % at 98,304, and adds 5 % at 131,072.
 constexpr long long kOverlapMaxPairs = 1LL << 34;
-// Paired far field: tables of fewer pairs (n = 7,000) run everything on the
+// Paired far field: tables of fewer pairs (n = 4,500) run everything on the
 // caller's stream, their far field being shorter than what the events between
-// streams and the waiting for room cost.  Measured, us a step (settled bodies,
-// side by side / one stream): n = 4,500 49 / 48, 6,000 53 / 52, 8,000 61 / 63,
-// 11,000 66 / 82, 20,000 141 / 165, 66,000 1,062 / 1,098.
-constexpr long long kBesideMinPairs = 50000000LL;
+// streams cost.  Measured, us a step (side by side / one stream): settled
+// bodies n = 4,200 49 / 47, 5,000 51 / 54, 6,000 49 / 56, 8,000 57 / 68,
+// 20,000 145 / 171, 66,000 1,047 / 1,098, 140,000 (six steps) 26.6 / 27.1 ms;
+// a remnant of 4,500 88 / 105.
+constexpr long long kBesideMinPairs = 20000000LL;
 // Far-field CTAs per SM while the contact pass runs beside it.  Measured on
 // the 66,000-body impact (ms per fused step, settled / collision phase):
 // 3 CTAs 1.72 / 2.60, 4: 1.68 / 2.57, 6: 1.68 / 2.59, 8: 1.67 / 2.54; the
@@ -869,25 +875,41 @@ constexpr long long kBesideMinPairs = 50000000LL;
 constexpr int kSideBySideCtas = 8;
 
 // One force evaluation (or fused step) per table.  The contact pass and the
-// far field are independent until the epilogue, so for tables of fewer than
-// kOverlapMaxPairs pairs they run side by side, forked from the caller's
-// stream with events and joined before the epilogue:
-//   - paired far field (the default): the far field on the caller's stream,
-//     the grid and the contacts on one of the highest priority, the row
-//     contacts of large tables on another (their one-warp blocks fit in the
-//     registers the far field's CTAs leave free);
-//   - one-sided modes: the contact pass on the aux stream, the far field on
-//     the caller's stream with kSideBySideCtas resident CTAs per SM (at that
-//     size it runs as fast as at full occupancy and leaves room on every SM
-//     for the contact kernels).
-// The epilogue then runs on the caller's stream with the fused epilogue's
-// arithmetic.  Larger tables run the contact pass first.  Either way the
-// results are the same bits.
+// far field are independent until the epilogue:
+//   - paired far field (the default), tables of at least kBesideMinPairs pairs:
+//     the far field on the caller's stream, the grid, the tiled contacts and
+//     the epilogue on one of the highest priority (the steps of a call follow
+//     one another there: StepCall), the row contacts on one of the lowest.
+//     The far field's one-warp CTAs fill whatever the grid leaves of the GPU,
+//     so a grid that waits for an event of the caller's stream first finds no
+//     room (six steps of 8,000 settled bodies 340 us with the epilogue on the
+//     caller's stream, 279 this way; 66,000 bodies 6.34 and 6.20 ms).  Row
+//     contacts ahead of the far field slow it more than they gain (66,000
+//     bodies 1,063 us a step at the highest priority, 1,047 at the lowest) and
+//     keep the tiled contacts waiting (20,000 remnant bodies 304 and 290 us).
+//     Streams may share a hardware queue, which runs its work in the order it
+//     was handed over: whatever waits for an event goes after what does not.
+//     Smaller tables run everything on the caller's stream;
+//   - one-sided modes: below kOverlapMaxPairs pairs the contact pass on the aux
+//     stream, the far field on the caller's with kSideBySideCtas resident CTAs
+//     per SM (at that size it runs as fast as at full occupancy and leaves room
+//     on every SM for the contact kernels), joined before the epilogue; larger
+//     tables run the contact pass first.
+// Either way the results are the same bits.
+struct StepCall {
+    bool capturing;
+    bool chained = false;  // the previous step's epilogue is the aux stream's last work
+    size_t clean;          // StreamScratch::clean as far as this call knows
+    StepCall(const StreamScratch *x, cudaStream_t s)
+        : capturing(stream_capturing(s)), clean(capturing || x->always_clear ? 0 : x->clean)
+    {
+    }
+};
+
 static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi,
                           const float4 *pos, const float4 *vel, float4 *force,
-                          float4 *pos_out, float4 *vel_out, cudaStream_t s)
+                          float4 *pos_out, float4 *vel_out, StepCall *call, cudaStream_t s)
 {
-    const bool capturing = stream_capturing(s);
     for (size_t t = 0; t < plan.tables.size(); ++t) {
         const LaunchTable &tab = plan.tables[t];
         ForceArgs a;
@@ -913,20 +935,20 @@ static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi
             reinterpret_cast<unsigned int *>(x->fsum + 3 * (size_t)plan.max_end);
         const GridWork gw(x->grid_work, plan.bodies[t], plan.max_end);
         if (plan.paired) {
-            // The far-field sums and the contact pass's counters start at
-            // zero; a clear is captured with the launches when the stream is
-            // capturing.
+            // The far-field sums and the contact pass's counters start at zero.
             a.fsum_fx = reinterpret_cast<long long *>(x->fsum);
             a.fsum_plane = (size_t)plan.max_end;
             const size_t bytes = (size_t)plan.max_end * 3 * sizeof(long long) +
                                  gi::kCtrWords * sizeof(unsigned int);
-            const size_t clean = std::max(x->clean, bytes);
-            if (capturing || x->always_clear || x->clean < bytes)
+            if (call->clean < bytes) {
                 GI_CUDA(cudaMemsetAsync(a.fsum_fx, 0, bytes, s), "cudaMemsetAsync far-field sums");
-            if (!capturing) x->clean = 0;
-            const bool beside = pairs >= kBesideMinPairs && pairs < kOverlapMaxPairs;
+                call->clean = bytes;
+                call->chained = false;  // the contact pass waits for it
+            }
+            if (!call->capturing) x->clean = 0;
+            const bool beside = tab.gridn > 0 && pairs >= kBesideMinPairs;
             const cudaStream_t q = beside ? x->aux : s;
-            if (beside) {
+            if (beside && !call->chained) {
                 GI_CUDA(cudaEventRecord(x->ev_fork, s), "cudaEventRecord");
                 GI_CUDA(cudaStreamWaitEvent(x->aux, x->ev_fork, 0), "cudaStreamWaitEvent");
             }
@@ -936,17 +958,26 @@ static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi
                 GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, s), "tiled contacts");
             GI_CUDA(gi_launch_pair_force(a, tab, gw, x->delta, ctr, !beside, s), "paired force kernel launch");
             if (beside) {
-                GI_CUDA(gi_launch_rows(pos, vel, tab, gw, x->delta, ctr, q), "row contacts");
+                GI_CUDA(cudaEventRecord(x->ev_grid, q), "cudaEventRecord");
                 GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, q), "tiled contacts");
-                GI_CUDA(cudaEventRecord(x->ev_join, x->aux), "cudaEventRecord");
+                GI_CUDA(cudaStreamWaitEvent(x->aux_rows, x->ev_grid, 0), "cudaStreamWaitEvent");
+                GI_CUDA(gi_launch_rows(pos, vel, tab, gw, x->delta, ctr, x->aux_rows), "row contacts");
+                GI_CUDA(cudaEventRecord(x->ev_rows, x->aux_rows), "cudaEventRecord");
+                GI_CUDA(cudaEventRecord(x->ev_far, s), "cudaEventRecord");
+                GI_CUDA(cudaStreamWaitEvent(q, x->ev_rows, 0), "cudaStreamWaitEvent");
+                GI_CUDA(cudaStreamWaitEvent(q, x->ev_far, 0), "cudaStreamWaitEvent");
+            }
+            GI_CUDA(gi_launch_pair_finish(epi, a, tab, maxn, c->sm_count, q), "epilogue launch");
+            if (beside) {
+                GI_CUDA(cudaEventRecord(x->ev_join, q), "cudaEventRecord");
                 GI_CUDA(cudaStreamWaitEvent(s, x->ev_join, 0), "cudaStreamWaitEvent");
             }
-            GI_CUDA(gi_launch_pair_finish(epi, a, tab, maxn, c->sm_count, s), "epilogue launch");
-            if (!capturing) x->clean = clean;
+            call->chained = beside;
+            if (!call->capturing) x->clean = call->clean;
             continue;
         }
         x->clean = 0;  // one-sided: FP64 sums there
-        x->always_clear |= capturing;
+        x->always_clear |= call->capturing;
         const int p = plan.ipt[t];
         const int occ = c->occ[c->opt.accum][p];
         // The queue and this table's tickets start at zero (the kernel also
@@ -1003,8 +1034,9 @@ extern "C" int gi_forces(gi_ctx *c, const float *pos, const float *vel, float *f
     cudaStream_t s = (cudaStream_t)stream;
     StreamScratch *x = nullptr;
     if ((st = ensure_scratch(c, plan, s, &x))) return st;
+    StepCall call(x, s);
     return run_force_plan(c, x, plan, GI_EPI_FORCE, (const float4 *)pos, (const float4 *)vel,
-                          (float4 *)force, nullptr, nullptr, s);
+                          (float4 *)force, nullptr, nullptr, &call, s);
 }
 
 static int move_tables(const gi_run *runs, int nruns, std::vector<LaunchTable> &out)
@@ -1093,8 +1125,10 @@ extern "C" int gi_step(gi_ctx *c, float *pos, float *vel, const gi_run *runs, in
     if ((st = ensure_scratch(c, plan, s, &x))) return st;
     if ((st = ensure_pingpong(x, (size_t)plan.max_end, s))) return st;
     float4 *ip = (float4 *)pos, *iv = (float4 *)vel, *op = x->pp_pos, *ov = x->pp_vel;
+    StepCall call(x, s);
     for (int k = 0; k < nsteps; ++k) {
-        if ((st = run_force_plan(c, x, plan, GI_EPI_STEP, ip, iv, nullptr, op, ov, s))) return st;
+        if ((st = run_force_plan(c, x, plan, GI_EPI_STEP, ip, iv, nullptr, op, ov, &call, s)))
+            return st;
         std::swap(ip, op);
         std::swap(iv, ov);
     }
@@ -1136,8 +1170,10 @@ extern "C" int gi_step_pingpong(gi_ctx *c, float *pos_a, float *vel_a, float *po
     if ((st = ensure_scratch(c, plan, s, &x))) return st;
     float4 *ip = (float4 *)pos_a, *iv = (float4 *)vel_a, *op = (float4 *)pos_b,
            *ov = (float4 *)vel_b;
+    StepCall call(x, s);
     for (int k = 0; k < nsteps; ++k) {
-        if ((st = run_force_plan(c, x, plan, GI_EPI_STEP, ip, iv, nullptr, op, ov, s))) return st;
+        if ((st = run_force_plan(c, x, plan, GI_EPI_STEP, ip, iv, nullptr, op, ov, &call, s)))
+            return st;
         std::swap(ip, op);
         std::swap(iv, ov);
     }

@@ -646,8 +646,8 @@ __global__ void __launch_bounds__(256) pair_finish_kernel(const ForceArgs a,
         const double fd[3] = {(double)__ldcg(q) * far_unit,
                               (double)__ldcg(q + a.fsum_plane) * far_unit,
                               (double)__ldcg(q + 2 * a.fsum_plane) * far_unit};
-        q[0] = q[a.fsum_plane] = q[2 * a.fsum_plane] = 0;
         finish_body<EPI>(a, R, unit, i, fd);
+        q[0] = q[a.fsum_plane] = q[2 * a.fsum_plane] = 0;
     }
 }
 
