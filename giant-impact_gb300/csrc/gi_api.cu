@@ -860,13 +860,13 @@ static int convert_params(const gi_pair_params *params, int nparams, std::vector
 // uniform balls (default tuning): the side-by-side pass takes 33 % off at
 // n = 8,192, 5 % at 49,152, 2 % at 98,304, and adds 5 % at 131,072.
 constexpr long long kOverlapMaxPairs = 1LL << 34;
-// Paired far field: tables of fewer pairs (n = 4,500) run everything on the
+// Paired far field: tables of fewer pairs (n = 5,500) run everything on the
 // caller's stream, their far field being shorter than what the events between
 // streams cost.  Measured, us a step (side by side / one stream): settled
-// bodies n = 4,200 49 / 47, 5,000 51 / 54, 6,000 49 / 56, 8,000 57 / 68,
-// 20,000 145 / 171, 66,000 1,047 / 1,098, 140,000 (six steps) 26.6 / 27.1 ms;
-// a remnant of 4,500 88 / 105.
-constexpr long long kBesideMinPairs = 20000000LL;
+// bodies n = 4,600 49 / 46, 5,500 48 / 49, 6,500 50 / 57, 8,000 57 / 63, 10,000
+// 67 / 74, 66,000 1,047 / 1,098, 140,000 (six steps) 26.6 / 27.1 ms; a remnant
+// of 4,600 91 / 100, 8,000 129 / 150.
+constexpr long long kBesideMinPairs = 30000000LL;
 // Far-field CTAs per SM while the contact pass runs beside it.  Measured on
 // the 66,000-body impact (ms per fused step, settled / collision phase):
 // 3 CTAs 1.72 / 2.60, 4: 1.68 / 2.57, 6: 1.68 / 2.59, 8: 1.67 / 2.54; the
@@ -955,11 +955,11 @@ static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi
             // the grid goes first, while the GPU has room for its clusters
             GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count, true, q), "cell grid");
             if (!beside)
-                GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, s), "tiled contacts");
-            GI_CUDA(gi_launch_pair_force(a, tab, gw, x->delta, ctr, !beside, s), "paired force kernel launch");
+                GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, true, s), "tiled contacts");
+            GI_CUDA(gi_launch_pair_force(a, tab, gw, x->delta, ctr, !beside, !beside, s), "paired force kernel launch");
             if (beside) {
                 GI_CUDA(cudaEventRecord(x->ev_grid, q), "cudaEventRecord");
-                GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, q), "tiled contacts");
+                GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, false, q), "tiled contacts");
                 GI_CUDA(cudaStreamWaitEvent(x->aux_rows, x->ev_grid, 0), "cudaStreamWaitEvent");
                 GI_CUDA(gi_launch_rows(pos, vel, tab, gw, x->delta, ctr, x->aux_rows), "row contacts");
                 GI_CUDA(cudaEventRecord(x->ev_rows, x->aux_rows), "cudaEventRecord");
@@ -967,7 +967,7 @@ static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi
                 GI_CUDA(cudaStreamWaitEvent(q, x->ev_rows, 0), "cudaStreamWaitEvent");
                 GI_CUDA(cudaStreamWaitEvent(q, x->ev_far, 0), "cudaStreamWaitEvent");
             }
-            GI_CUDA(gi_launch_pair_finish(epi, a, tab, maxn, c->sm_count, q), "epilogue launch");
+            GI_CUDA(gi_launch_pair_finish(epi, a, tab, maxn, c->sm_count, !beside, q), "epilogue launch");
             if (beside) {
                 GI_CUDA(cudaEventRecord(x->ev_join, q), "cudaEventRecord");
                 GI_CUDA(cudaStreamWaitEvent(s, x->ev_join, 0), "cudaStreamWaitEvent");
@@ -997,7 +997,7 @@ static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi
         // cluster's CTAs would keep the far field's off their SMs for good.
         GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count, !beside, q), "cell grid");
         GI_CUDA(gi_launch_rows(pos, vel, tab, gw, x->delta, ctr, q), "row contacts");
-        GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, q), "tiled contacts");
+        GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, false, q), "tiled contacts");
         if (!beside) {
             GI_CUDA(gi_launch_force(p, c->opt.accum, epi, a, tab, c->sm_count * occ, s),
                     "force kernel launch");

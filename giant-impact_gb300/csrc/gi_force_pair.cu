@@ -350,6 +350,7 @@ pair_force_kernel(const ForceArgs a, const GridView g, long long *__restrict__ d
         RowSmem row;
         __device__ Smem() {}
     } sm;
+    launch_wait();
     if ((int)blockIdx.x < rows)
         contact_rows(sm.row, a.pos, a.vel, g, delta, tab, blockIdx.x);
     else
@@ -638,6 +639,7 @@ __global__ void __launch_bounds__(256) pair_finish_kernel(const ForceArgs a,
     const RunDev &R = tab.runs[blockIdx.y];
     const double unit = tab.params[R.param].fx_unit;
     const double far_unit = R.far_unit;
+    launch_wait();
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kCtrWords)
         reinterpret_cast<unsigned int *>(a.fsum_fx + 3 * a.fsum_plane)[threadIdx.x] = 0u;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < R.n; k += gridDim.x * blockDim.x) {
@@ -657,27 +659,26 @@ using namespace gi;
 
 cudaError_t gi_launch_pair_force(const ForceArgs &a, const LaunchTable &tab, const GridWork &g,
                                  long long *delta, const unsigned int *ctr, bool with_rows,
-                                 cudaStream_t s)
+                                 bool early, cudaStream_t s)
 {
     if (tab.nitems <= 0) return cudaSuccess;
     static std::atomic<int> known[64];
     cudaError_t e = gi_full_carveout(reinterpret_cast<const void *>(pair_force_kernel), known);
     if (e != cudaSuccess) return e;
     const int rows = with_rows ? tab.rows : 0;
-    pair_force_kernel<<<rows + tab.nitems, 32, 0, s>>>(a, g.view(ctr), delta, rows, tab);
-    return cudaGetLastError();
+    return gi_launch(pair_force_kernel, dim3(rows + tab.nitems), 32, early, s, a, g.view(ctr), delta,
+                     rows, tab);
 }
 
 cudaError_t gi_launch_pair_finish(int epi, const ForceArgs &a, const LaunchTable &tab, int maxn,
-                                  int nsm, cudaStream_t s)
+                                  int nsm, bool early, cudaStream_t s)
 {
     if (tab.nruns <= 0 || maxn <= 0) return cudaSuccess;
     const int bx = std::max(1, std::min((maxn + 255) / 256, 4 * nsm));
-    dim3 grid(bx, tab.nruns);
-    if (epi == GI_EPI_FORCE) pair_finish_kernel<GI_EPI_FORCE><<<grid, 256, 0, s>>>(a, tab);
-    else if (epi == GI_EPI_STEP) pair_finish_kernel<GI_EPI_STEP><<<grid, 256, 0, s>>>(a, tab);
-    else return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    const dim3 grid(bx, tab.nruns);
+    if (epi == GI_EPI_FORCE) return gi_launch(pair_finish_kernel<GI_EPI_FORCE>, grid, 256, early, s, a, tab);
+    if (epi == GI_EPI_STEP) return gi_launch(pair_finish_kernel<GI_EPI_STEP>, grid, 256, early, s, a, tab);
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t gi_launch_potential(const float4 *pos, const LaunchTable &tab, double *per_cta,

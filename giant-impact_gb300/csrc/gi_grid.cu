@@ -762,6 +762,7 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
     unsigned short *const queue = sm.queue[warp];
 #pragma unroll
     for (int d = 0; d < 6; ++d) sm.js[d][t] = sm.is[d][t] = 0u;
+    launch_wait();
     // Thread 0 takes the next unit from the queue when the current one
     // reaches its last tile: the atomic's latency hides behind that tile,
     // and the CTA still takes items close to the queue's longest-first order.
@@ -1044,14 +1045,13 @@ cudaError_t gi_launch_rows(const float4 *pos, const float4 *vel, const LaunchTab
 }
 
 cudaError_t gi_launch_tiles(const LaunchTable &tab, const GridWork &g, long long *delta,
-                            unsigned int *ctr, int nsm, cudaStream_t s)
+                            unsigned int *ctr, int nsm, bool early, cudaStream_t s)
 {
     if (tab.gridn == 0) return cudaSuccess;  // no grid, no crowded cells
     static std::atomic<int> known[64];
     const cudaError_t e = gi_full_carveout(reinterpret_cast<const void *>(gi::contact_tile_kernel), known);
     if (e != cudaSuccess) return e;
     const int gt = (int)std::min<size_t>(g.icap, 7 * (size_t)nsm);
-    gi::contact_tile_kernel<<<gt, 128, 0, s>>>(g.spos, g.svel, g.dpos, g.dvel, delta, tab, g.items,
-                                               ctr);
-    return cudaGetLastError();
+    return gi_launch(gi::contact_tile_kernel, dim3(gt), 128, early, s, g.spos, g.svel, g.dpos, g.dvel,
+                     delta, tab, g.items, ctr);
 }

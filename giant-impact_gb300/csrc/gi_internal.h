@@ -133,13 +133,13 @@ static_assert(kPairMaxCpi <= kPairBlockChunks && kPairBlockChunks % kPairMaxCpi 
 struct GridWork;
 cudaError_t gi_launch_pair_force(const ForceArgs &a, const LaunchTable &tab, const GridWork &g,
                                  long long *delta, const unsigned int *ctr, bool with_rows,
-                                 cudaStream_t s);
+                                 bool early, cudaStream_t s);
 // Pair potentials of the table's runs (planned as for gi_launch_pair_force):
 // one double per CTA in per_cta, one per run in out, in table order.
 cudaError_t gi_launch_potential(const float4 *pos, const LaunchTable &tab, double *per_cta,
                                 double *out, cudaStream_t s);
 cudaError_t gi_launch_pair_finish(int epi, const ForceArgs &a, const LaunchTable &tab, int maxn,
-                                  int nsm, cudaStream_t s);
+                                  int nsm, bool early, cudaStream_t s);
 
 // gi_grid.cu: contact corrections of every body of the table's runs into
 // delta (3 x int64 per body) through a cell grid.  Its scratch layout
@@ -244,7 +244,30 @@ cudaError_t gi_launch_rows(const float4 *pos, const float4 *vel, const LaunchTab
                            const GridWork &g, long long *delta, const unsigned int *ctr,
                            cudaStream_t s);
 cudaError_t gi_launch_tiles(const LaunchTable &tab, const GridWork &g, long long *delta,
-                            unsigned int *ctr, int nsm, cudaStream_t s);
+                            unsigned int *ctr, int nsm, bool early, cudaStream_t s);
+
+// Launches a kernel whose blocks begin with launch_wait().  early: its blocks
+// may be put on the GPU when the last of the stream's previous kernel have
+// left it, before its writes are all in place (what launch_wait waits for).  A
+// kernel that depends on the one before it starts 2 us sooner: forces of 1,500
+// bodies, two kernels, 14.5 -> 10.9 us; a step of 4,200 settled ones, four,
+// 47.8 -> 40.4.  Not for work that shares the GPU with another stream's:
+// blocks that wait hold their registers.
+template <class... P, class... A>
+inline cudaError_t gi_launch(void (*kernel)(P...), dim3 grid, int threads, bool early, cudaStream_t s,
+                             const A &...args)
+{
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 // Asks once per device (known: its flags) for the largest shared-memory
 // carveout of a kernel.  Kernels that are to share an SM need the same one: an

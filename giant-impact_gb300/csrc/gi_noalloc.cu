@@ -191,7 +191,7 @@ extern "C" int gi_forces_collision_noalloc(const float *pos, const float *vel, f
     const float4 *p4 = reinterpret_cast<const float4 *>(pos), *v4 = reinterpret_cast<const float4 *>(vel);
     const GridWork g(grid, n, n);
     if (gi_launch_grid(p4, v4, tab, g, delta, ctr, nsm, true, s) != cudaSuccess ||
-        gi_launch_tiles(tab, g, delta, ctr, nsm, s) != cudaSuccess)
+        gi_launch_tiles(tab, g, delta, ctr, nsm, true, s) != cudaSuccess)
         return gi_internal_fail(GI_ERR_CUDA, "contact pass launch failed");
     ForceArgs a;
     std::memset(&a, 0, sizeof a);
@@ -201,9 +201,9 @@ extern "C" int gi_forces_collision_noalloc(const float *pos, const float *vel, f
     a.delta = delta;
     a.fsum_fx = sums;
     a.fsum_plane = (size_t)n;
-    if (gi_launch_pair_force(a, tab, g, delta, ctr, true, s) != cudaSuccess)
+    if (gi_launch_pair_force(a, tab, g, delta, ctr, true, true, s) != cudaSuccess)
         return gi_internal_fail(GI_ERR_CUDA, "force kernel launch failed");
-    if (gi_launch_pair_finish(GI_EPI_FORCE, a, tab, n, nsm, s) != cudaSuccess)
+    if (gi_launch_pair_finish(GI_EPI_FORCE, a, tab, n, nsm, true, s) != cudaSuccess)
         return gi_internal_fail(GI_ERR_CUDA, "epilogue launch failed");
     return GI_OK;
 }
