@@ -1360,7 +1360,14 @@ extern "C" int gi_diag_fp64(gi_ctx *c, const float *pos, const float *vel,
     cudaStream_t s = (cudaStream_t)stream;
     const size_t nb = (size_t)c->diag_blocks;
     if (!c->diag_work) {
-        GI_CUDA(cudaMalloc(&c->diag_work, (nb + 1) * 16 * sizeof(double)), "cudaMalloc diag");
+        double *work = nullptr;
+        GI_CUDA(cudaMalloc(&work, (nb + 1) * 16 * sizeof(double)), "cudaMalloc diag");
+        const cudaError_t e = cudaMemset(work + nb * 16, 0, sizeof(int));  // the ticket
+        if (e != cudaSuccess) {
+            cudaFree(work);
+            return cuda_fail(e, "cudaMemset diag");
+        }
+        c->diag_work = work;
     }
     if (!c->diag_host) {
         GI_CUDA(cudaMallocHost(&c->diag_host, 16 * sizeof(double)), "cudaMallocHost diag");

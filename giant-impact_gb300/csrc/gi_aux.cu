@@ -247,23 +247,30 @@ diag_kernel(const float4 *__restrict__ pos, const float4 *__restrict__ vel,
         if (lane == 0) sum[c] = x;
     }
     __syncthreads();
-    if (threadIdx.x != 0) return;
+    if (warp != 0) return;
+    if (lane == 0) *ticket = 0;  // for the next call
     const double count = sum[kDiagSums], cfe = sum[kDiagParts];
     const double M = mfe * cfe + msi * (count - cfe);
-    double rc[3], wc[3];
-    out[0] = M;
-    for (int d = 0; d < 3; ++d) {
-        out[1 + d] = M > 0.0 ? sum[d] / M : 0.0;
-        out[4 + d] = M > 0.0 ? sum[3 + d] / M : 0.0;
-        out[11 + d] = sum[3 + d];
-        rc[d] = M > 0.0 ? out[1 + d] - (double)x0[d] : 0.0;
-        wc[d] = M > 0.0 ? out[4 + d] - (double)x0[3 + d] : 0.0;
+    // lane c < 6: the centre's position and velocity, one FP64 division each
+    const int c = min(lane, 5);
+    float from = x0[0];
+#pragma unroll
+    for (int k = 1; k < 6; ++k) from = c == k ? x0[k] : from;
+    const double mean = M > 0.0 ? sum[c] / M : 0.0, rel = M > 0.0 ? mean - (double)from : 0.0;
+    // lane d < 3: component d of the angular momentum
+    const int d = lane % 3, p = (d + 1) % 3, q = (d + 2) % 3;
+    const double rp = __shfl_sync(0xffffffffu, rel, p), rq = __shfl_sync(0xffffffffu, rel, q),
+                 wp = __shfl_sync(0xffffffffu, rel, 3 + p), wq = __shfl_sync(0xffffffffu, rel, 3 + q);
+    if (lane < 6) out[1 + lane] = mean;
+    if (lane < 3) {
+        out[7 + lane] = sum[7 + lane] - M * (rp * wq - rq * wp);
+        out[11 + lane] = sum[3 + lane];
     }
-    out[7] = sum[7] - M * (rc[1] * wc[2] - rc[2] * wc[1]);
-    out[8] = sum[8] - M * (rc[2] * wc[0] - rc[0] * wc[2]);
-    out[9] = sum[9] - M * (rc[0] * wc[1] - rc[1] * wc[0]);
-    out[10] = 0.5 * sum[6];
-    out[14] = count;
+    if (lane == 0) {
+        out[0] = M;
+        out[10] = 0.5 * sum[6];
+        out[14] = count;
+    }
 }
 
 // ------------------------------------------------------------ FFMA peak --
@@ -323,8 +330,6 @@ cudaError_t gi_launch_diag(const float4 *pos, const float4 *vel,
     int nbfe = run.n > 0 ? (int)((long long)nblocks * run.nfe / run.n) : 0;
     if (run.nfe > 0 && nbfe < 1) nbfe = 1;
     if (nbfe > nblocks - 1) nbfe = nblocks - 1;
-    cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof(int), s);
-    if (e != cudaSuccess) return e;
     gi::diag_kernel<<<nblocks, 256, 0, s>>>(pos, vel, label, scope, run.offset, run.n, run.nfe, nbfe,
                                             mass_fe, mass_si, work, ticket, out);
     return cudaGetLastError();

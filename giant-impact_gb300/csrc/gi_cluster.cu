@@ -129,6 +129,7 @@ cluster_insert(const float4 *__restrict__ pos, int n, double inv_cell, unsigned 
 __global__ void __launch_bounds__(256)
 cluster_ranges(CellTable tab, CellInfo *__restrict__ info, ClusterCounters *ctr)
 {
+    launch_wait();
     const int lane = threadIdx.x & 31;
     const unsigned int cells = ctr->cells;
     const unsigned int stride = gridDim.x * blockDim.x;
@@ -164,6 +165,7 @@ cluster_scatter(const float4 *__restrict__ pos, int n, CellTable tab,
                 const int *__restrict__ slot_of, float4 *__restrict__ list,
                 int *__restrict__ parent)
 {
+    launch_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int s = slot_of[i];
         parent[i] = s < 0 ? i : (int)tab.leader[s];
@@ -287,6 +289,7 @@ cluster_link(const float4 *__restrict__ list, CellTable tab, const CellInfo *__r
              unsigned int mask, float touch, int tries, int *parent,
              const ClusterCounters *__restrict__ ctr, int *__restrict__ err)
 {
+    launch_wait();
     const int lane = threadIdx.x & 31;
     const unsigned int cells = ctr->cells, nwarps = (gridDim.x * blockDim.x) >> 5;
     for (unsigned int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < cells; k += nwarps) {
@@ -345,6 +348,7 @@ cluster_link_loose(const float4 *__restrict__ pos, int n, const int *__restrict_
                    float touch, int tries, int *parent, const ClusterCounters *__restrict__ ctr,
                    int *__restrict__ err)
 {
+    launch_wait();
     const int lane = threadIdx.x & 31;
     const unsigned int total = ctr->loose, nwarps = (gridDim.x * blockDim.x) >> 5;
     for (unsigned int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < total; w += nwarps) {
@@ -360,6 +364,7 @@ cluster_link_loose(const float4 *__restrict__ pos, int n, const int *__restrict_
 __global__ void __launch_bounds__(256)
 cluster_flatten(int *parent, int n, int *__restrict__ size, int *__restrict__ ngroups)
 {
+    launch_wait();
     const int lane = threadIdx.x & 31;
     int roots = 0;
     for (int i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; i0 < n; i0 += gridDim.x * blockDim.x) {
@@ -392,6 +397,7 @@ __global__ void __launch_bounds__(256)
 cluster_pick(const int *__restrict__ group, const int *__restrict__ size, int n,
              const unsigned long long *exclude_key, unsigned long long *best)
 {
+    launch_wait();
     const int skip = exclude_key ? key_name(*exclude_key) : -1;
     unsigned long long k = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -406,6 +412,7 @@ cluster_tag(const int *__restrict__ group, int n, const unsigned long long *__re
             int b0, int b1, int b2, int *__restrict__ group_out,
             unsigned char *__restrict__ scope_out, int *__restrict__ counts)
 {
+    launch_wait();
     __shared__ int sc[8];
     if (threadIdx.x < 8) sc[threadIdx.x] = 0;
     __syncthreads();
@@ -508,20 +515,25 @@ extern "C" int gi_find_earth_moon(gi_ctx *ctx, const float *pos, int n, float to
         if ((e = cudaMemsetAsync(tab.rep, 0xff, 4 * (3 * M + N), s)) != cudaSuccess) break;
         gi::cluster_insert<<<gridded, 256, 0, s>>>(P, n, inv_cell, m - 1, tab, info, slot_of, loose,
                                                    &res->ctr);
-        gi::cluster_ranges<<<gridded, 256, 0, s>>>(tab, info, &res->ctr);
-        gi::cluster_scatter<<<gridded, 256, 0, s>>>(P, n, tab, slot_of, list, parent);
-        gi::cluster_link<false><<<warps, 128, 0, s>>>(list, tab, info, m - 1, touch, tries, parent,
-                                                      &res->ctr, &res->err);
-        gi::cluster_link<true><<<warps, 128, 0, s>>>(list, tab, info, m - 1, touch, tries, parent,
-                                                     &res->ctr, &res->err);
-        gi::cluster_link_loose<<<std::min(warps, 1024), 128, 0, s>>>(P, n, loose, touch, tries, parent,
-                                                                     &res->ctr, &res->err);
-        gi::cluster_flatten<<<gridded, 256, 0, s>>>(parent, n, size, &res->ngroups);
-        gi::cluster_pick<<<gridded, 256, 0, s>>>(parent, size, n, nullptr, &res->keys[0]);
-        gi::cluster_pick<<<gridded, 256, 0, s>>>(parent, size, n, &res->keys[0], &res->keys[1]);
-        gi::cluster_tag<<<gridded, 256, 0, s>>>(parent, n, res->keys, bounds[0], bounds[1],
-                                                bounds[2], group, scope, res->counts);
-        if ((e = cudaGetLastError()) != cudaSuccess) break;
+        // each launch follows the one before it early
+        const auto next = [&](auto kernel, int grid, int threads, auto &&...args) {
+            if (e == cudaSuccess) e = gi_launch(kernel, dim3(grid), threads, true, s, args...);
+        };
+        e = cudaGetLastError();
+        next(gi::cluster_ranges, gridded, 256, tab, info, &res->ctr);
+        next(gi::cluster_scatter, gridded, 256, P, n, tab, slot_of, list, parent);
+        next(gi::cluster_link<false>, warps, 128, list, tab, info, m - 1, touch, tries, parent, &res->ctr,
+             &res->err);
+        next(gi::cluster_link<true>, warps, 128, list, tab, info, m - 1, touch, tries, parent, &res->ctr,
+             &res->err);
+        next(gi::cluster_link_loose, std::min(warps, 1024), 128, P, n, loose, touch, tries, parent,
+             &res->ctr, &res->err);
+        next(gi::cluster_flatten, gridded, 256, parent, n, size, &res->ngroups);
+        next(gi::cluster_pick, gridded, 256, parent, size, n, nullptr, &res->keys[0]);
+        next(gi::cluster_pick, gridded, 256, parent, size, n, &res->keys[0], &res->keys[1]);
+        next(gi::cluster_tag, gridded, 256, parent, n, res->keys, bounds[0], bounds[1], bounds[2], group,
+             scope, res->counts);
+        if (e != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(&host, res, sizeof host, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
             break;
     } while (false);
@@ -571,6 +583,7 @@ disk_kernel(const float4 *__restrict__ pos, const float4 *__restrict__ vel,
             double ux, double uy, double uz, double gm, const unsigned long long *__restrict__ rmax,
             int *__restrict__ counts)
 {
+    launch_wait();
     __shared__ int sc[3];
     if (threadIdx.x < 3) sc[threadIdx.x] = 0;
     __syncthreads();
@@ -642,11 +655,11 @@ extern "C" int gi_find_disk(gi_ctx *ctx, const float *pos, const float *vel, con
         if ((e = cudaMemsetAsync(res, 0, sizeof(Res), s)) != cudaSuccess) break;
         gi::earth_radius_kernel<<<blocks, 256, 0, s>>>(P, scope, run->offset, run->n, earth[1], earth[2],
                                                        earth[3], &res->rmax);
-        gi::disk_kernel<<<blocks, 256, 0, s>>>(P, reinterpret_cast<const float4 *>(vel), scope,
-                                               run->offset, run->n, earth[1], earth[2], earth[3],
-                                               earth[4], earth[5], earth[6], G * earth[0], &res->rmax,
-                                               res->counts);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
+        e = gi_launch(gi::disk_kernel, dim3(blocks), 256, true, s, P, reinterpret_cast<const float4 *>(vel),
+                      scope, run->offset, run->n, earth[1], earth[2], earth[3], earth[4], earth[5],
+                      earth[6], G * earth[0], &res->rmax, res->counts);
+        if (e != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(&host, res, sizeof host, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
             break;
     } while (false);

@@ -7,9 +7,6 @@
 
 namespace gi {
 
-// Waits for the kernels this one was launched to follow (see gi_launch).
-__device__ __forceinline__ void launch_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 __device__ __forceinline__ int cell_of(float x)
 {
     float f = floorf(x);

@@ -246,6 +246,9 @@ cudaError_t gi_launch_rows(const float4 *pos, const float4 *vel, const LaunchTab
 cudaError_t gi_launch_tiles(const LaunchTable &tab, const GridWork &g, long long *delta,
                             unsigned int *ctr, int nsm, bool early, cudaStream_t s);
 
+// Waits for the kernels this one was launched to follow (see gi_launch).
+__device__ __forceinline__ void launch_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Launches a kernel whose blocks begin with launch_wait().  early: its blocks
 // may be put on the GPU when the last of the stream's previous kernel have
 // left it, before its writes are all in place (what launch_wait waits for).  A
@@ -255,7 +258,7 @@ cudaError_t gi_launch_tiles(const LaunchTable &tab, const GridWork &g, long long
 // blocks that wait hold their registers.
 template <class... P, class... A>
 inline cudaError_t gi_launch(void (*kernel)(P...), dim3 grid, int threads, bool early, cudaStream_t s,
-                             const A &...args)
+                             A &&...args)
 {
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -289,7 +292,7 @@ cudaError_t gi_launch_move(float4 *pos, float4 *vel, const float4 *force,
 // The FP64 diagnostics' resident blocks on sm_count SMs.
 int gi_diag_blocks(int sm_count);
 // work holds 16 doubles per block, out 15 doubles (device, or pinned host
-// memory), ticket an int (cleared here).
+// memory), ticket an int that is zero between launches.
 cudaError_t gi_launch_diag(const float4 *pos, const float4 *vel,
                            const unsigned char *label, int scope,
                            const RunDev &run, float mass_fe, float mass_si, double *work,
