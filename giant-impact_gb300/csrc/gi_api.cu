@@ -1425,8 +1425,14 @@ extern "C" int gi_potential_fp64(gi_ctx *c, const float *pos, const gi_run *runs
                 ctas += d.pitems;
                 continue;
             }
-            // the far field's items, all rows eight to a lane
-            ctas += gi_internal_pair_run(d, d.n, gi_internal_pair_default_pcl(d.n), pd[d.param], ctas, 3);
+            // the far field's items, all rows eight to a lane, and fewer chunks
+            // each: without per-body sums a short item costs no atomics, and
+            // the last ones leave less of the GPU idle.  us an energy log
+            // (diagnostics and potential) at the far field's chunks, half and a
+            // quarter of them: 20,000 bodies 259, 241, 225; 33,000 446, 438,
+            // 397; 66,000 1,211, 1,139, 1,151; 130,000 3,825, 3,817, 3,933.
+            const int pcl = gi_internal_pair_default_pcl(d.n) - (d.n < 65536 ? 2 : 1);
+            ctas += gi_internal_pair_run(d, d.n, pcl, pd[d.param], ctas, 3);
         }
         if (!t.nruns) continue;
         if (ctas > 0x7fffffffLL) return fail(GI_ERR_BAD_SIZE, "too many work items");
