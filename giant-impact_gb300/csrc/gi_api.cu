@@ -432,6 +432,13 @@ static void tuning_for(const gi_ctx *c, int n, int *ipt, int *jchunk)
     const int T = (n + GI_NT - 1) / GI_NT;
     const int nib = (n + GI_NT * p - 1) / (GI_NT * p);
     long long ct = std::max(1LL, (long long)T * nib / (4LL * slots));
+    // Below about 30,000 bodies that is a tile or two, and an item's own costs
+    // (the i-bodies, the partial sums, a place in the queue) outweigh an even
+    // finish: at least a 16th of the run then, up to 8 tiles.  us a force pass
+    // (Kahan) before / after: n = 5,000 86 / 80, 12,000 154 / 126, 20,001
+    // 252 / 225.  Not where a chunk is summed in plain FP32, whose error grows
+    // with it.
+    if (c->opt.accum != GI_ACC_FP32) ct = std::max(ct, std::min(8LL, T / 16LL));
     const int shift = c->bucket_shift[b];
     ct = shift >= 0 ? (ct << shift) : std::max(1LL, ct >> (-shift));
     int lg = 0;
