@@ -819,7 +819,7 @@ def study_drift(a):
         m["sd_fe"], m["sd_si"])
     run = wl.run_desc(gi, 0, n, nfe)
     out = {"study": "drift", "workload": "plain two-body impact, 66,000 bodies, dt 1e-3",
-           "steps": steps, "every": every, "dense_min": a.dense_min or 256,
+           "steps": steps, "every": every, "dense_min": a.dense_min or 128,
            "material": "KR = K (conservative control)" if kr is not None else "config 2"}
     # this library: fused step, config units
     dp, dv = torch.from_numpy(pos).cuda(), torch.from_numpy(vel).cuda()

@@ -75,11 +75,10 @@ __device__ __forceinline__ bool has_crowds(const unsigned int *ctr, unsigned int
 }
 
 // The bodies of a bucket that share its majority cell take the tiled path when
-// they are at least tab.dense_min (256 unless set), or at least a quarter of
+// they are at least tab.dense_min (kDenseMin unless set), or at least a quarter of
 // that next to a bucket of that many: near a crowded remnant its bodies have
-// enough contacts to pay the tiled path's fixed costs per item, while the
-// cores of settled bodies (cells of tens to a few hundred bodies, ~20
-// contacts a body) stay on the row path.  Either bound is at least
+// enough contacts to pay the tiled path's fixed costs per item, while cells
+// of ordinary settled bodies stay on the row path.  Either bound is at least
 // kDenseFloor, which bounds the item count.  Buckets of at least dense_lo
 // bodies are listed as candidates while they are counted.
 // (kDenseFloor itself lives in gi_internal.h: it sizes the scratch.)

@@ -25,7 +25,7 @@
 //
 // Two passes share the bodies.  contact_row_kernel takes a few consecutive
 // slots per warp, an ordinary body's path.  Crowded buckets
-// (gi_options.dense_min bodies, 256 by default, or a quarter of that next to
+// (gi_options.dense_min bodies, 128 by default, or a quarter of that next to
 // such a cell; e.g. an interpenetrating collision remnant with thousands of
 // contacts per body) whose bodies all share one cell are sorted by sub-cell
 // and go through contact_tile_kernel: a work item is (bucket, neighbour

@@ -149,6 +149,12 @@ namespace gi {
 // A bucket goes through the tiled path only when it holds at least this many
 // bodies; that bounds the number of tiled buckets and work items.
 constexpr unsigned int kDenseFloor = 32;
+// Bodies of a cell from which it goes that way unless gi_options.dense_min says
+// otherwise.  A row-path warp with the cells of a body's dense core around it
+// (no more than 180 bodies each there) runs 100 us longer than the others; ms a
+// step at 64, 128, 192 and 256: the 66,000-body impact settled 1.052, 1.050,
+// 1.090, 1.131, after 6,000 steps 1.620, 1.619, 1.630, 1.763.  (48: 1.092.)
+constexpr int kDenseMin = 128;
 // Cost classes of the tiled path's work items (128-body tiles staged - 1).
 constexpr unsigned int kItemClasses = 16;
 // Tiled-path counters: items, tiled buckets, queue head, candidate buckets,

@@ -163,7 +163,7 @@ extern "C" int gi_forces_collision_noalloc(const float *pos, const float *vel, f
     tab.nitems = (int)items;
     gi_grid_runs(tab);
     tab.sep_test = GI_SEP_REF_INT;
-    tab.dense_min = 256;
+    tab.dense_min = gi::kDenseMin;
 
     // Carve the static array (the largest run is checked to fit at compile
     // time; this guards the arithmetic at run time as well).

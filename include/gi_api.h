@@ -165,7 +165,7 @@ typedef struct gi_options {
     int accum;             /* GI_ACCUM_*, 0 = GI_ACCUM_PAIRED */
     int dense_min;         /* contact pass: cells of at least this many bodies,
                               or of a quarter of it next to such a cell, take
-                              the shared-memory tiled path; 0 = 256.
+                              the shared-memory tiled path; 0 = 128.
                               Results do not depend on it. */
     int cluster_tries;     /* gi_find_earth_moon: attempts one union-find
                               link may make (each failed attempt moves to a
