@@ -636,7 +636,7 @@ def hbm_section(gi, torch, wl, ctx, pos, vel, nfe, p, copies=128, reps=7):
       move: gi_move = one move_kernel launch, the unfused kick-drift
             (impactAddTime.cu:379-394): 80 B/body (read pos, vel, force;
             write pos, vel).
-      diag: gi_diag_fp64, scope all = a ticket clear + one diag_kernel (FP64
+      diag: gi_diag_fp64, scope all = one diag_kernel (FP64
             mass, centre of mass, momentum, kinetic energy, angular momentum
             about the centre of mass; finalised by its last block, which
             writes the result to pinned host memory): 32 B/body (pos + vel
@@ -676,7 +676,7 @@ def hbm_section(gi, torch, wl, ctx, pos, vel, nfe, p, copies=128, reps=7):
            "l2": "flushed before every timed call (256 MB write, outside the events)"}
     for name, ms, mm, per_body, what in (
             ("move", move_ms, move_mm, 80, "move_kernel (unfused kick-drift), one launch"),
-            ("diag", diag_ms, diag_mm, 32, "gi_diag_fp64 scope all: ticket clear + one diag_kernel, "
+            ("diag", diag_ms, diag_mm, 32, "gi_diag_fp64 scope all: one diag_kernel, "
                                            "finalised by its last block into pinned memory")):
         gbs = per_body * n / (ms * 1e-3) / 1e9
         out[name] = {"ms": ms, "ms_min_max": mm, "algorithmic_bytes": per_body * n,
@@ -1090,7 +1090,7 @@ def run_ours(a):
                                "back-to-back runs; MEASURED_PEAKS.json has no FP32 figure",
                 "nominal_peak": info["sm_count"] * 128 * 2 * 2.07e9 / 1e12,
                 "kernel": "gi::pair_force_kernel (far field, each unordered pair once; the "
-                          "contact pass runs beside it on a second stream, then "
+                          "contact pass runs beside it on two other streams, then "
                           "gi::pair_finish_kernel adds the corrections and the kick-drift), one "
                           "step per gi_step_pingpong call",
                 "work": "FMA-pipe lane operations of the paired far field, 2 flops each "

@@ -14,9 +14,10 @@
 // For them, gi_forces_collision_noalloc computes the same forces, bit for bit
 // (the same kernels with the same default decomposition), with all of its
 // scratch in one statically allocated device array, g_noalloc_scratch, of
-// GI_NOALLOC_BYTES (8 MiB; the largest run takes 5.6 MiB of it).  Every GPU that loads the library holds that
-// array until the process exits.  The array limits a call to
-// GI_NOALLOC_MAX_BODIES (32,768) bodies; larger calls are refused.
+// GI_NOALLOC_BYTES (8 MiB; the largest run takes 5.6 MiB of it).  Every GPU
+// that loads the library holds that array until the process exits.  The array
+// limits a call to GI_NOALLOC_MAX_BODIES (32,768) bodies; larger calls are
+// refused.
 //
 // Every call shares the one array and leaves its contents behind: the
 // far-field sums and the grid's counters, which must start at zero, are

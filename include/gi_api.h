@@ -656,7 +656,7 @@ typedef struct gi_earth_moon {
     int moon_counts[4];
 } gi_earth_moon;
 
-/* Groups on the GPU (hashed cell grid of cell size > touch, lock-free
+/* Groups on the GPU (cells whose bodies all touch, linked by a lock-free
  * union-find); synchronous.  pos: device, n float4.  bounds = NFe1,
  * NFe1 + NFe2, NFe1 + NFe2 + NSi1 for the origin counts.  group (device,
  * n ints, may be NULL) receives each body's group name; scope (device, n
