@@ -585,7 +585,7 @@ static void pair_far_unit(int n, const PairDev &p, RunDev &d)
     d.far_inv = (float)std::ldexp(1.0, -E);
 }
 
-constexpr int kPairSplitN = 32768;  // runs below it cut an item's chunks between warps
+constexpr int kPairSplitN = 65536;  // runs below it cut an item's chunks between warps
 
 // Stride of a run's item permutation: coprime with the item count, about
 // the items of one i-block, so that consecutive CTAs hold different i-blocks.
@@ -611,6 +611,8 @@ static int pair_stride(long long items, int nblocks)
 //   n = 8,192: 4/1 26.7, 8/1 26.6, 8/2 28.7, 8/4 32.2
 //   n = 16,000: 4/2 79.9, 8/1 76.8, 8/2 77.1, 8/4 87.5
 //   n = 24,000: 4/4 165, 8/1 159, 8/2 156.6, 8/4 164
+// and a step of settled bodies, 8 rows a lane: 40,000 8/8 428 us, 8/4 411;
+// 50,000 629, 615; 66,000 the same.
 // A short warp pays the staging and the i-side atomics for fewer pairs, which
 // costs a batch of such runs 2 to 8 %, so the cut is no finer than a lone run
 // needs.
