@@ -147,19 +147,46 @@ __device__ __forceinline__ void ff_add_cross(FF &a, FF u, FF v, FF w, FF z)
 }
 
 // The sums of a block's bodies, all of one material class.
-constexpr int kDiagSums = 10;    // x, v (3 each), v.v, r x w (3)
-constexpr int kDiagParts = 11;   // the same times the class mass, then the count
+constexpr int kDiagSums = 10;    // r, w (3 each), v.v, r x w (3)
+constexpr int kDiagParts = 12;   // the same times the class mass, r.r's, then the count
+constexpr int kDiagLook = 32;    // bodies a thread looks at for the reference
+
+// The body that the sums are taken about: the run's first, or where that one is
+// not in scope the first of its first 8,192 that is, if any.  By the whole block.
+__device__ __forceinline__ int diag_reference(const unsigned char *__restrict__ label, int scope, int n)
+{
+    if (label == nullptr || scope == 0 || label_in_scope(label[0], scope)) return 0;
+    __shared__ int first;
+    if (threadIdx.x == 0) first = n;
+    __syncthreads();
+    int mine = n;
+#pragma unroll 16
+    for (int v = kDiagLook - 1; v >= 0; --v) {
+        const int k = 256 * v + (int)threadIdx.x;
+        if (k < n && label_in_scope(label[k], scope)) mine = k;
+    }
+    if (mine < n) atomicMin(&first, mine);
+    __syncthreads();
+    return first < n ? first : 0;
+}
 
 // The whole diagnostic in one pass over the state (32 B per body): with r = x
-// - x0 and w = v - v0 taken from one body of the run (exact as float-float
-// pairs), the sums of m, m x, m v, m v.v and m r x w give the mass, the centre
-// of mass, the momenta, and the angular momentum about the centre of mass
-// relative to its velocity, L = sum m r x w - M rc x wc (impactBasicFunctions.h:
-// 507-652 in double; rc, wc the centre's r and w).  Taking x0 from the run
-// keeps that difference harmless wherever the system is and however it moves.
-// The call, read-back included, takes 108 us on 8.4M bodies and 25 us on 66,000;
-// a first pass for the centre, then a second over the same 32 B, took 144 and
-// 65.  What bounds it is the FP32 pipe beside HBM: 225 operations a body.
+// - x0 and w = v - v0 about a reference body of the scope (exact as float-float
+// pairs), the sums of m, m r, m w, m v.v and m r x w give the mass, the centre of
+// mass, the momenta, and the angular momentum about the centre of mass relative
+// to its velocity, L = sum m r x w - M rc x wc (impactBasicFunctions.h:507-652 in
+// double; rc, wc the centre's r and w).  That is as good as sums about the centre
+// wherever the scope is and however it moves, while the reference is about as
+// near to the centre as the scope's bodies are.  Where it is not (a body that
+// escaped or ran away) L would lose digits to the difference, or overflow:
+// gi_diag_fp64 sees that from rc, wc and the sum of m r.r, and repeats the pass
+// about the centre it found.
+// The call, read-back included, takes 110 us on 8.4M bodies and 23 us on 66,000
+// (24 where it looks for the reference).  Two passes, the first for the centre,
+// took 144 and 65; one about the run's first body whatever the scope 108 and 22,
+// but L of a Moon with that body in the Earth was off by 8e-13 of sqrt(sum m r.r
+// sum m w.w), with it 1e6 D away by 2e-9 (now 6e-16 and 1e-15).  What bounds the
+// pass is the FP32 pipe beside HBM: 219 operations a body.
 //
 // Each block takes one material class, so the class mass multiplies the
 // block's sums once, in FP64: blocks [0, nbfe) the run's Fe bodies [0, nfe),
@@ -168,42 +195,68 @@ constexpr int kDiagParts = 11;   // the same times the class mass, then the coun
 // last ticket sums them in a fixed order (a warp per value: lane l takes
 // blocks l, l + 32, ..., then a fixed shuffle tree), so the result is
 // deterministic for a given grid.
-// out = [mass, com3, vcom3, L3, ke, p3, count].
-__global__ void __launch_bounds__(256)
+// out = [mass, com3, vcom3, L3, ke, p3, count, sum of m r.r (FP32 sums), rc3, wc3].
+// Four blocks an SM (64 registers, two words spilled outside the loop); three of
+// 75 registers took 135 us.
+__global__ void __launch_bounds__(256, 4)
 diag_kernel(const float4 *__restrict__ pos, const float4 *__restrict__ vel,
             const unsigned char *__restrict__ label, int scope, int off, int n, int nfe, int nbfe,
-            double mfe, double msi, double *__restrict__ work, int *__restrict__ ticket,
-            double *__restrict__ out)
+            double mfe, double msi, const DiagOrigin origin, double *__restrict__ work,
+            int *__restrict__ ticket, double *__restrict__ out)
 {
     const bool fe = (int)blockIdx.x < nbfe;
     const int k0 = fe ? 0 : nfe, k1 = fe ? nfe : n;
     const int b = fe ? (int)blockIdx.x : (int)blockIdx.x - nbfe;
     const int nb = fe ? nbfe : (int)gridDim.x - nbfe;
     const double m = fe ? mfe : msi;
-    // the run's first body; a component that is not finite counts as 0
-    float x0[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-    if (n > 0) {
-        const float4 p = pos[off], u = vel[off];
-        const float c[6] = {p.x, p.y, p.z, u.x, u.y, u.z};
+    __shared__ float ref[6];  // the reference; a component that is not finite counts as 0
+    {
+        float x[6];
 #pragma unroll
-        for (int d = 0; d < 6; ++d) x0[d] = fabsf(c[d]) <= 3.0e38f ? c[d] : 0.0f;
+        for (int d = 0; d < 6; ++d) x[d] = origin.x[d];
+        if (!origin.given && n > 0) {
+            float4 p = pos[off], u = vel[off];
+            if (const int k = diag_reference(label ? label + off : nullptr, scope, n)) {
+                p = pos[off + k];
+                u = vel[off + k];
+            }
+            x[0] = p.x; x[1] = p.y; x[2] = p.z;
+            x[3] = u.x; x[4] = u.y; x[5] = u.z;
+        }
+#pragma unroll
+        for (int d = 0; d < 6; ++d)
+            if ((int)threadIdx.x == d) ref[d] = fabsf(x[d]) <= 3.0e38f ? x[d] : 0.0f;
     }
+    __syncthreads();
+    float x0[6];
+#pragma unroll
+    for (int d = 0; d < 6; ++d) x0[d] = ref[d];
     FF v[kDiagSums];
 #pragma unroll
     for (int c = 0; c < kDiagSums; ++c) v[c] = FF{0.0f, 0.0f};
     int cnt = 0;
+    float rr = 0.0f;
     stream_bodies(pos, vel, label, scope, off, k0 + b * blockDim.x + threadIdx.x, k1,
                   nb * blockDim.x, [&](float4 p, float4 u) {
                       const FF r[3] = {ff_diff(p.x, x0[0]), ff_diff(p.y, x0[1]), ff_diff(p.z, x0[2])};
                       const FF w[3] = {ff_diff(u.x, x0[3]), ff_diff(u.y, x0[4]), ff_diff(u.z, x0[5])};
-                      const float pp[3] = {p.x, p.y, p.z}, uu[3] = {u.x, u.y, u.z};
+                      const float uu[3] = {u.x, u.y, u.z};
 #pragma unroll
                       for (int d = 0; d < 3; ++d) {
-                          ff_add(v[d], pp[d], 0.0f);
-                          ff_add(v[3 + d], uu[d], 0.0f);
-                          const float q = __fmul_rn(uu[d], uu[d]);
-                          ff_add(v[6], q, __fmaf_rn(uu[d], uu[d], -q));
+                          ff_add(v[d], r[d].hi, r[d].lo);
+                          ff_add(v[3 + d], w[d].hi, w[d].lo);
+                          rr = __fmaf_rn(r[d].hi, r[d].hi, rr);
                       }
+                      float q = __fmul_rn(uu[0], uu[0]), e = __fmaf_rn(uu[0], uu[0], -q);
+#pragma unroll
+                      for (int d = 1; d < 3; ++d) {
+                          const float y = __fmul_rn(uu[d], uu[d]);
+                          float t;
+                          e = __fadd_rn(e, __fmaf_rn(uu[d], uu[d], -y));
+                          two_sum(q, y, q, t);
+                          e = __fadd_rn(e, t);
+                      }
+                      ff_add(v[6], q, e);
                       ff_add_cross(v[7], r[1], w[2], r[2], w[1]);
                       ff_add_cross(v[8], r[2], w[0], r[0], w[2]);
                       ff_add_cross(v[9], r[0], w[1], r[1], w[0]);
@@ -223,13 +276,18 @@ diag_kernel(const float4 *__restrict__ pos, const float4 *__restrict__ vel,
         }
         if (lane == 0) part[c][warp] = (double)v[c].hi + (double)v[c].lo;
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) rr += __shfl_down_sync(0xffffffffu, rr, o);
     cnt = __reduce_add_sync(0xffffffffu, cnt);
-    if (lane == 0) part[kDiagSums][warp] = (double)cnt;
+    if (lane == 0) {
+        part[kDiagSums][warp] = (double)rr;
+        part[kDiagSums + 1][warp] = (double)cnt;
+    }
     __syncthreads();
     if (threadIdx.x < kDiagParts) {
         double x = 0.0;
         for (int w = 0; w < 8; ++w) x += part[threadIdx.x][w];
-        work[16 * blockIdx.x + threadIdx.x] = threadIdx.x < kDiagSums ? m * x : x;
+        work[16 * blockIdx.x + threadIdx.x] = threadIdx.x <= kDiagSums ? m * x : x;
     }
     __threadfence();
     __syncthreads();
@@ -241,7 +299,7 @@ diag_kernel(const float4 *__restrict__ pos, const float4 *__restrict__ vel,
     for (int c = warp; c < kDiagParts + 1; c += 8) {
         const int end = c == kDiagParts ? nbfe : (int)gridDim.x;
         double x = 0.0;
-        for (int q = lane; q < end; q += 32) x += __ldcg(work + 16 * q + min(c, kDiagSums));
+        for (int q = lane; q < end; q += 32) x += __ldcg(work + 16 * q + min(c, kDiagSums + 1));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
         if (lane == 0) sum[c] = x;
@@ -249,27 +307,26 @@ diag_kernel(const float4 *__restrict__ pos, const float4 *__restrict__ vel,
     __syncthreads();
     if (warp != 0) return;
     if (lane == 0) *ticket = 0;  // for the next call
-    const double count = sum[kDiagSums], cfe = sum[kDiagParts];
+    const double count = sum[kDiagSums + 1], cfe = sum[kDiagParts];
     const double M = mfe * cfe + msi * (count - cfe);
     // lane c < 6: the centre's position and velocity, one FP64 division each
     const int c = min(lane, 5);
-    float from = x0[0];
-#pragma unroll
-    for (int k = 1; k < 6; ++k) from = c == k ? x0[k] : from;
-    const double mean = M > 0.0 ? sum[c] / M : 0.0, rel = M > 0.0 ? mean - (double)from : 0.0;
+    const double rel = M > 0.0 ? sum[c] / M : 0.0, mean = M > 0.0 ? (double)ref[c] + rel : 0.0;
     // lane d < 3: component d of the angular momentum
     const int d = lane % 3, p = (d + 1) % 3, q = (d + 2) % 3;
     const double rp = __shfl_sync(0xffffffffu, rel, p), rq = __shfl_sync(0xffffffffu, rel, q),
                  wp = __shfl_sync(0xffffffffu, rel, 3 + p), wq = __shfl_sync(0xffffffffu, rel, 3 + q);
-    if (lane < 6) out[1 + lane] = mean;
-    if (lane < 3) {
-        out[7 + lane] = sum[7 + lane] - M * (rp * wq - rq * wp);
-        out[11 + lane] = sum[3 + lane];
+    if (lane < 6) {
+        out[1 + lane] = mean;
+        out[16 + lane] = rel;
+        if (lane >= 3) out[8 + lane] = M * (double)ref[c] + sum[lane];
     }
+    if (lane < 3) out[7 + lane] = sum[7 + lane] - M * (rp * wq - rq * wp);
     if (lane == 0) {
         out[0] = M;
         out[10] = 0.5 * sum[6];
         out[14] = count;
+        out[15] = sum[kDiagSums];
     }
 }
 
@@ -318,7 +375,8 @@ int gi_diag_blocks(int sm_count)
 cudaError_t gi_launch_diag(const float4 *pos, const float4 *vel,
                            const unsigned char *label, int scope,
                            const RunDev &run, float mass_fe, float mass_si, double *work,
-                           int max_blocks, double *out, int *ticket, cudaStream_t s)
+                           const DiagOrigin &origin, int max_blocks, double *out, int *ticket,
+                           cudaStream_t s)
 {
     if (max_blocks < 2) return cudaErrorInvalidValue;
     // One resident wave (the grid-stride loops give every block the same
@@ -331,7 +389,7 @@ cudaError_t gi_launch_diag(const float4 *pos, const float4 *vel,
     if (run.nfe > 0 && nbfe < 1) nbfe = 1;
     if (nbfe > nblocks - 1) nbfe = nblocks - 1;
     gi::diag_kernel<<<nblocks, 256, 0, s>>>(pos, vel, label, scope, run.offset, run.n, run.nfe, nbfe,
-                                            mass_fe, mass_si, work, ticket, out);
+                                            mass_fe, mass_si, origin, work, ticket, out);
     return cudaGetLastError();
 }
 

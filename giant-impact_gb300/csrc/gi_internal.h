@@ -297,12 +297,20 @@ cudaError_t gi_launch_move(float4 *pos, float4 *vel, const float4 *force,
                            const LaunchTable &tab, cudaStream_t s);
 // The FP64 diagnostics' resident blocks on sm_count SMs.
 int gi_diag_blocks(int sm_count);
-// work holds 16 doubles per block, out 15 doubles (device, or pinned host
-// memory), ticket an int that is zero between launches.
+// The point that the angular momentum's terms are taken about (position, then
+// velocity); not given: a body of the scope.
+struct DiagOrigin {
+    float x[6];
+    bool given;
+};
+// work holds 16 doubles per block, out kDiagOut doubles (device, or pinned
+// host memory), ticket an int that is zero between launches.
+constexpr int kDiagOut = 22;
 cudaError_t gi_launch_diag(const float4 *pos, const float4 *vel,
                            const unsigned char *label, int scope,
                            const RunDev &run, float mass_fe, float mass_si, double *work,
-                           int max_blocks, double *out, int *ticket, cudaStream_t s);
+                           const DiagOrigin &origin, int max_blocks, double *out, int *ticket,
+                           cudaStream_t s);
 cudaError_t gi_launch_ffma_peak(float *sink, int blocks, int iters, cudaStream_t s);
 
 // gi_api.cu helpers for the library's other translation units: record an
