@@ -552,7 +552,9 @@ potential_kernel(const float4 *__restrict__ pos, const __grid_constant__ LaunchT
             // in every other group of four chunks the pairs' roots are weighted
             // with i's mass, and j's is applied at the fold
             const int g0 = jc0 & ~255;  // the group's first body
-            const bool swap = (jc0 & 256) && !(g0 < nfe && nfe < g0 + 256) && jc0 >= wi0 + 32 * IPL;
+            // (not in the last, which may have places past the run: their mass is 0)
+            const bool swap = (jc0 & 256) && g0 + 256 <= n && !(g0 < nfe && nfe < g0 + 256) &&
+                              jc0 >= wi0 + 32 * IPL;
             float near = 0.0f;
                 if (jc0 < wi0 + 32 * IPL) {  // diagonal: each pair by itself
 #pragma unroll 1
