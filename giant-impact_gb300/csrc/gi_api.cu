@@ -1426,10 +1426,10 @@ extern "C" int gi_diag_fp64(gi_ctx *c, const float *pos, const float *vel,
     return GI_OK;
 }
 
-// Runs up to this size take every ordered pair (potential_tile): their sums of
+// Runs up to this size take every ordered pair (potential_tile_kernel): their sums of
 // 128 are too few for the rounding of other ones to average out to 1e-9 (7e-10
-// at 10,000 bodies, 2e-10 from 13,000 on), and a call takes 110 us at 8,000
-// either way (before: 550).
+// at 10,000 bodies, 2e-10 from 13,000 on), and a call takes 92 us at 9,000
+// (paired 93 at 12,289).
 constexpr int kPotentialOneSided = 12288;
 
 extern "C" int gi_potential_fp64(gi_ctx *c, const float *pos, const gi_run *runs, int nruns,
@@ -1449,37 +1449,43 @@ extern "C" int gi_potential_fp64(gi_ctx *c, const float *pos, const gi_run *runs
         LaunchTable t;
         std::memset(&t, 0, sizeof t);
         int idx[GI_MAX_RUNS];
-        long long ctas = 0;
-        for (int r = r0; r < std::min(nruns, r0 + GI_MAX_RUNS); ++r) {
-            if (runs[r].n <= 0) continue;
-            idx[t.nruns] = r;
-            RunDev &d = t.runs[t.nruns++];
-            d.offset = runs[r].offset;
-            d.n = runs[r].n;
-            d.nfe = runs[r].nfe;
-            d.param = runs[r].params;
-            if (d.n <= kPotentialOneSided) {
-                d.item_start = (int)std::min(ctas, 0x7fffffffLL);
-                d.pitems = ((d.n + 31) / 32) * ((d.n + 127) / 128);
-                ctas += d.pitems;
-                continue;
+        long long partials = 0, blocks = 0;
+        for (const bool longer : {true, false}) {
+            for (int r = r0; r < std::min(nruns, r0 + GI_MAX_RUNS); ++r) {
+                if (runs[r].n <= 0 || (runs[r].n > kPotentialOneSided) != longer) continue;
+                idx[t.nruns] = r;
+                RunDev &d = t.runs[t.nruns++];
+                d.offset = runs[r].offset;
+                d.n = runs[r].n;
+                d.nfe = runs[r].nfe;
+                d.param = runs[r].params;
+                if (!longer) {
+                    const int tiles = (d.n + 127) / 128;
+                    d.item_start = (int)std::min(partials, 0x7fffffffLL);
+                    d.pitems = ((d.n + 31) / 32) * tiles;
+                    d.row_start = (int)blocks;
+                    partials += d.pitems;
+                    blocks += tiles * tiles;
+                    continue;
+                }
+                // the far field's items, all rows eight to a lane, and fewer chunks
+                // each: without per-body sums a short item costs no atomics, and
+                // the last ones leave less of the GPU idle.  us an energy log
+                // (diagnostics and potential) at the far field's chunks, half and a
+                // quarter of them: 20,000 bodies 259, 241, 225; 33,000 446, 438,
+                // 397; 66,000 1,211, 1,139, 1,151; 130,000 3,825, 3,817, 3,933.
+                const int pcl = gi_internal_pair_default_pcl(d.n) - (d.n < 65536 ? 2 : 1);
+                partials += gi_internal_pair_run(d, d.n, pcl, pd[d.param], partials, 3);
             }
-            // the far field's items, all rows eight to a lane, and fewer chunks
-            // each: without per-body sums a short item costs no atomics, and
-            // the last ones leave less of the GPU idle.  us an energy log
-            // (diagnostics and potential) at the far field's chunks, half and a
-            // quarter of them: 20,000 bodies 259, 241, 225; 33,000 446, 438,
-            // 397; 66,000 1,211, 1,139, 1,151; 130,000 3,825, 3,817, 3,933.
-            const int pcl = gi_internal_pair_default_pcl(d.n) - (d.n < 65536 ? 2 : 1);
-            ctas += gi_internal_pair_run(d, d.n, pcl, pd[d.param], ctas, 3);
+            if (longer) t.nitems = (int)std::min(partials, 0x7fffffffLL);
         }
         if (!t.nruns) continue;
-        if (ctas > 0x7fffffffLL) return fail(GI_ERR_BAD_SIZE, "too many work items");
-        t.nitems = (int)ctas;
+        if (partials > 0x7fffffffLL) return fail(GI_ERR_BAD_SIZE, "too many work items");
+        t.rows = (int)blocks;
         for (size_t m = 0; m < pd.size(); ++m) t.params[m] = pd[m];
         void *work = nullptr, *pinned = nullptr;
         const size_t head = GI_MAX_RUNS * sizeof(double);
-        if ((st = gi_internal_ctx_workspace(c, head + (size_t)ctas * sizeof(double), &work, &pinned)))
+        if ((st = gi_internal_ctx_workspace(c, head + (size_t)partials * sizeof(double), &work, &pinned)))
             return st;
         double *res = static_cast<double *>(work), *host = static_cast<double *>(pinned);
         cudaError_t e = gi_launch_potential((const float4 *)pos, t, res + GI_MAX_RUNS, res, s);
