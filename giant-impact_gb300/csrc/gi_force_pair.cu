@@ -407,18 +407,19 @@ __device__ __forceinline__ float contact_potential(float G, float K, float r2)
 }
 
 // A chunk wholly after the rows: far[k] gathers row k's pairs, weighted with
-// j's mass, or with i's (SWAP); returns the contact potentials.  jfe: Fe
-// bodies of the chunk (its first ones); i0: the lane's first row.
+// j's mass, or with i's (SWAP); the contact potentials go to acc, an FP32 sum for
+// each step's 16 pairs (over the lane's 512 pairs, equal terms, as of bodies in one
+// point, were off by up to 4e-6).  jfe: Fe bodies of the chunk (its first ones);
+// i0: the lane's first row.
 template <bool SWAP>
-__device__ __forceinline__ float potential_chunk(const float4 *__restrict__ cxy,
-                                                 const float4 *__restrict__ czg, const PairDev &P,
-                                                 int jfe, int i0, int nfe,
-                                                 const float (&nx)[kPairIpl],
-                                                 const float (&ny)[kPairIpl],
-                                                 const float (&nz)[kPairIpl],
-                                                 float2 (&far)[kPairIpl])
+__device__ __forceinline__ void potential_chunk(const float4 *__restrict__ cxy,
+                                                const float4 *__restrict__ czg, const PairDev &P,
+                                                int jfe, int i0, int nfe,
+                                                const float (&nx)[kPairIpl],
+                                                const float (&ny)[kPairIpl],
+                                                const float (&nz)[kPairIpl],
+                                                float2 (&far)[kPairIpl], double &acc)
 {
-    float near = 0.0f;
 #pragma unroll 1
     for (int s = 0; s < 32; ++s) {
         const float4 q = cxy[s], g = czg[s];
@@ -443,6 +444,7 @@ __device__ __forceinline__ float potential_chunk(const float4 *__restrict__ cxy,
             far[k] = __ffma2_rn(gm, __fmul2_rn(ri, t), far[k]);
         }
         if (close) {
+            float sum = 0.0f;
 #pragma unroll
             for (int k = 0; k < kPairIpl; ++k) {
                 const float2 dx = __fadd2_rn(X, make_float2(nx[k], nx[k]));
@@ -453,13 +455,13 @@ __device__ __forceinline__ float potential_chunk(const float4 *__restrict__ cxy,
                 r2 = __ffma2_rn(dz, dz, r2);
                 const int ic = i0 + k * 32 < nfe;
                 if (r2.x < 1.0f)
-                    near += contact_potential(P.G[ic + (s < jfe)], P.K[ic + (s < jfe)], r2.x);
+                    sum += contact_potential(P.G[ic + (s < jfe)], P.K[ic + (s < jfe)], r2.x);
                 if (r2.y < 1.0f)
-                    near += contact_potential(P.G[ic + (s + 32 < jfe)], P.K[ic + (s + 32 < jfe)], r2.y);
+                    sum += contact_potential(P.G[ic + (s + 32 < jfe)], P.K[ic + (s + 32 < jfe)], r2.y);
             }
+            acc += (double)sum;
         }
     }
-    return near;
 }
 
 // Short runs (pipl 0): every ordered pair, a lane's body against a tile of 128;
@@ -563,8 +565,8 @@ potential_kernel(const float4 *__restrict__ pos, const __grid_constant__ LaunchT
             // (not in the last, which may have places past the run: their mass is 0)
             const bool swap = (jc0 & 256) && g0 + 256 <= n && !(g0 < nfe && nfe < g0 + 256) &&
                               jc0 >= wi0 + 32 * IPL;
-            float near = 0.0f;
-                if (jc0 < wi0 + 32 * IPL) {  // diagonal: each pair by itself
+            const bool diag = jc0 < wi0 + 32 * IPL;
+            if (diag) {  // each pair by itself
 #pragma unroll 1
                 for (int s = 0; s < kPairChunk; ++s) {
                     const int j = jc0 + s;
@@ -572,6 +574,7 @@ potential_kernel(const float4 *__restrict__ pos, const __grid_constant__ LaunchT
                     const float4 q = cxy[s & 31], g = czg[s & 31];
                     const float X = s < 32 ? q.x : q.y, Y = s < 32 ? q.z : q.w,
                                 Z = s < 32 ? g.x : g.y, gmj = s < 32 ? g.z : g.w;
+                    float sum = 0.0f;
 #pragma unroll
                     for (int k = 0; k < IPL; ++k) {
                         const int i = wi0 + k * 32 + lane;
@@ -579,17 +582,16 @@ potential_kernel(const float4 *__restrict__ pos, const __grid_constant__ LaunchT
                         const float dx = X + nx[k], dy = Y + ny[k], dz = Z + nz[k];
                         const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
                         const int cls = (i < nfe) + (j < nfe);
-                        if (r2 < 1.0f) near += contact_potential(P.G[cls], P.K[cls], r2);
+                        if (r2 < 1.0f) sum += contact_potential(P.G[cls], P.K[cls], r2);
                         else far[k].x = __fmaf_rn(gmj, rsqrt_refined(r2), far[k].x);
                     }
+                    if (sum != 0.0f) acc += (double)sum;
                 }
             } else if (swap) {
-                near = potential_chunk<true>(cxy, czg, P, nfe - jc0, wi0 + lane, nfe, nx, ny, nz, far);
+                potential_chunk<true>(cxy, czg, P, nfe - jc0, wi0 + lane, nfe, nx, ny, nz, far, acc);
             } else {
-                near = potential_chunk<false>(cxy, czg, P, nfe - jc0, wi0 + lane, nfe, nx, ny, nz, far);
+                potential_chunk<false>(cxy, czg, P, nfe - jc0, wi0 + lane, nfe, nx, ny, nz, far, acc);
             }
-            acc += (double)near;
-            const bool diag = jc0 < wi0 + 32 * IPL;
             if (((c - c0) & (diag ? 1 : 3)) == (diag ? 1 : 3) || c + 1 == c1) {
                 // 128 bodies a sum: the rows' sums without rounding (hi + lo);
                 // each with its own mass where that differs

@@ -1,5 +1,5 @@
-"""gi_potential_fp64 above 12,288 bodies: states so wide that a place past the run's
-end would count."""
+"""gi_potential_fp64 above 12,288 bodies: crowded states, whose contacts carry the
+sum, and states so wide that a place past the run's end would count."""
 from __future__ import annotations
 
 import numpy as np
@@ -10,6 +10,46 @@ pytestmark = pytest.mark.gpu
 
 def _dev(torch, a):
     return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+@pytest.mark.parametrize("n,nfe", [(12289, 0), (12545, 12545), (13000, 4000)])
+def test_coincident_bodies(gi, torch_cuda, n, nfe):
+    """All bodies in one point: every pair of a class has the same potential, so
+    that sums in FP32 would be off by the same rounding each time (2e-6 of a sum
+    of 128 equal terms, 4e-6 of 512).  The pair's own FP32 arithmetic has four
+    roundings of at most 2^-24 of 2 G + 2 K / 3."""
+    import gi_workloads as wl
+    torch = torch_cuda
+    p = wl.params(gi)
+    pos = np.zeros((n, 4), np.float32)
+    pos[:, :3] = [0.25, -3.5, 7.0]
+    ctx = gi.Context(0)
+    got = ctx.potential(_dev(torch, pos).data_ptr(), [wl.run_desc(gi, 0, n, nfe)], p)[0]
+    ctx.close()
+    m = wl.MATERIAL
+    nsi = n - nfe
+    classes = [(nsi * (nsi - 1) // 2, m["mass_si"] ** 2, 2 * m["k_si"]),
+               (nsi * nfe, m["mass_fe"] * m["mass_si"], m["k_fe"] + m["k_si"]),
+               (nfe * (nfe - 1) // 2, m["mass_fe"] ** 2, 2 * m["k_fe"])]
+    want = sum(c * (-2.0 * g + 2.0 * k / 3.0) for c, g, k in classes)
+    tol = sum(c * 4 * 2.0 ** -24 * (2.0 * g + 2.0 * k / 3.0) for c, g, k in classes)
+    assert abs(got - want) <= tol
+
+
+@pytest.mark.parametrize("n,nfe", [(12801, 700), (20011, 20011)])
+def test_crowded_ball(gi, orc, torch_cuda, n, nfe):
+    """A remnant's density (600 bodies in a cell): each pair to about 1e-7, as in
+    ordinary states."""
+    import gi_workloads as wl
+    torch = torch_cuda
+    p = wl.params(gi)
+    pos, _, _ = gi.ic_uniform_ball(n, n, (n / 2500.0) ** (1 / 3))
+    run = wl.run_desc(gi, 0, n, nfe)
+    ctx = gi.Context(0)
+    got = ctx.potential(_dev(torch, pos).data_ptr(), [run], p)[0]
+    ctx.close()
+    want = orc.potential_fp64(pos, [run], p).sum() / 2.0
+    assert abs(got - want) <= 2e-7 * abs(want)
 
 
 @pytest.mark.parametrize("n", [12545, 12608, 12799])
