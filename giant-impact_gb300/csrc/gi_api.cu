@@ -1449,7 +1449,7 @@ extern "C" int gi_potential_fp64(gi_ctx *c, const float *pos, const gi_run *runs
         LaunchTable t;
         std::memset(&t, 0, sizeof t);
         int idx[GI_MAX_RUNS];
-        long long partials = 0, blocks = 0;
+        int partials = 0, blocks = 0;
         for (const bool longer : {true, false}) {
             for (int r = r0; r < std::min(nruns, r0 + GI_MAX_RUNS); ++r) {
                 if (runs[r].n <= 0 || (runs[r].n > kPotentialOneSided) != longer) continue;
@@ -1461,10 +1461,10 @@ extern "C" int gi_potential_fp64(gi_ctx *c, const float *pos, const gi_run *runs
                 d.param = runs[r].params;
                 if (!longer) {
                     const int tiles = (d.n + 127) / 128;
-                    d.item_start = (int)std::min(partials, 0x7fffffffLL);
-                    d.pitems = ((d.n + 31) / 32) * tiles;
-                    d.row_start = (int)blocks;
-                    partials += d.pitems;
+                    d.item_start = partials;
+                    d.nsplit = ((d.n + 31) / 32) * tiles;
+                    d.row_start = blocks;
+                    partials += d.nsplit;
                     blocks += tiles * tiles;
                     continue;
                 }
@@ -1475,13 +1475,16 @@ extern "C" int gi_potential_fp64(gi_ctx *c, const float *pos, const gi_run *runs
                 // quarter of them: 20,000 bodies 259, 241, 225; 33,000 446, 438,
                 // 397; 66,000 1,211, 1,139, 1,151; 130,000 3,825, 3,817, 3,933.
                 const int pcl = gi_internal_pair_default_pcl(d.n) - (d.n < 65536 ? 2 : 1);
-                partials += gi_internal_pair_run(d, d.n, pcl, pd[d.param], partials, 3);
+                // From 262,000 bodies on a warp takes several tasks: one partial each
+                // would come to 41 MB at 1.15M bodies and grow with n^2.
+                const long long tasks = gi_internal_pair_run(d, d.n, pcl, pd[d.param], partials, 3);
+                d.nsplit = (int)std::min(tasks, (long long)kPotentialPartials);
+                partials += d.nsplit;
             }
-            if (longer) t.nitems = (int)std::min(partials, 0x7fffffffLL);
+            if (longer) t.nitems = partials;
         }
         if (!t.nruns) continue;
-        if (partials > 0x7fffffffLL) return fail(GI_ERR_BAD_SIZE, "too many work items");
-        t.rows = (int)blocks;
+        t.rows = blocks;
         for (size_t m = 0; m < pd.size(); ++m) t.params[m] = pd[m];
         void *work = nullptr, *pinned = nullptr;
         const size_t head = GI_MAX_RUNS * sizeof(double);

@@ -295,15 +295,13 @@ __device__ __forceinline__ void pair_task(PairSmem &sm, const ForceArgs &a, cons
     }
 }
 
-// CTA `cta` of run R: its first row wi0 and its chunks [c0, c1) (none when
-// they are all before the rows, or there are no rows).
-__device__ __forceinline__ void pair_decode(const RunDev &R, int cta, int &wi0, int &c0, int &c1)
+// Warp `part` of item t of run R: its first row wi0 and its chunks [c0, c1) (none
+// when they are all before the rows, or there are no rows).
+__device__ __forceinline__ void pair_place(const RunDev &R, long long t, int part, int &wi0, int &c0,
+                                           int &c1)
 {
-    // item slot, rows and chunks of the item; then (i-block, item of the block)
-    const int local = cta - R.item_start;
-    const int slot = local >> R.ptpi, part = local & ((1 << R.ptpi) - 1);
+    // (i-block, item of the block), then rows and chunks of the item
     const int rlog = kPairRowsLog2 - 5 - R.pipl;  // log2 of the row groups of an i-block
-    const long long t = ((long long)slot * R.pstride) % R.pitems;
     const long long k0 = R.pk0, q = kPairBlockChunks >> R.pcl;
     int lo = 0, hi = R.pnb - 1;
     while (lo < hi) {
@@ -317,6 +315,14 @@ __device__ __forceinline__ void pair_decode(const RunDev &R, int cta, int &wi0, 
                    (part >> rlog) * cpt;
     c0 = max(cb, wi0 / kPairChunk);
     c1 = min(cb + cpt, R.pnc);
+}
+
+// CTA `cta` of run R, likewise.
+__device__ __forceinline__ void pair_decode(const RunDev &R, int cta, int &wi0, int &c0, int &c1)
+{
+    const int local = cta - R.item_start;
+    const int slot = local >> R.ptpi, part = local & ((1 << R.ptpi) - 1);
+    pair_place(R, ((long long)slot * R.pstride) % R.pitems, part, wi0, c0, c1);
 }
 
 __device__ __forceinline__ void pair_item(PairSmem &sm, const ForceArgs &a, const LaunchTable &tab,
@@ -519,20 +525,13 @@ potential_tile_kernel(const float4 *__restrict__ pos, const __grid_constant__ La
     if ((t & 31) == 0) partials[R.item_start + (i >> 5) * tiles + jt / 128] = u;
 }
 
-// One potential per CTA into per_cta (0 for an empty one).
-__global__ void __launch_bounds__(32)
-potential_kernel(const float4 *__restrict__ pos, const __grid_constant__ LaunchTable tab,
-                 double *__restrict__ per_cta)
+// What one warp of the far field's decomposition adds to the potential: rows from
+// wi0 on, chunks [c0, c1).
+__device__ __forceinline__ void potential_task(PairSmem &sm, const float4 *__restrict__ run,
+                                               const RunDev &R, const PairDev &P, int wi0, int c0,
+                                               int c1, int lane, double &acc)
 {
-    __shared__ PairSmem sm;
     constexpr int IPL = kPairIpl;
-    const int lane = threadIdx.x;
-    const RunDev &R = tab.runs[find_run(tab, blockIdx.x)];
-    const PairDev &P = tab.params[R.param];
-    const float4 *const run = pos + R.offset;
-    int wi0, c0, c1;
-    pair_decode(R, blockIdx.x, wi0, c0, c1);
-    double acc = 0.0;
     const int n = R.n, nfe = R.nfe;
     const bool imix = wi0 < nfe && nfe < wi0 + 32 * IPL;
     float nx[IPL], ny[IPL], nz[IPL];
@@ -612,9 +611,37 @@ potential_kernel(const float4 *__restrict__ pos, const __grid_constant__ LaunchT
             }
         }
     }
+}
+
+// A run's tasks, a CTA and a partial for each; MANY: for tables with a run of more
+// than kPotentialPartials, whose nsplit CTAs take several in turn (the loop and its
+// 64-bit item numbers cost runs of short items 1 to 7 %).
+template <bool MANY>
+__global__ void __launch_bounds__(32)
+potential_kernel(const float4 *__restrict__ pos, const __grid_constant__ LaunchTable tab,
+                 double *__restrict__ partials)
+{
+    __shared__ PairSmem sm;
+    const int lane = threadIdx.x;
+    const RunDev &R = tab.runs[find_run(tab, blockIdx.x)];
+    const PairDev &P = tab.params[R.param];
+    const float4 *const run = pos + R.offset;
+    int wi0, c0, c1;
+    double acc = 0.0;
+    if (MANY) {
+        const unsigned long long items = pair_items_before(R.pnb, R.pk0, kPairBlockChunks >> R.pcl);
+        for (unsigned long long k = blockIdx.x - R.item_start; k < items << R.ptpi; k += R.nsplit) {
+            pair_place(R, (long long)(((k >> R.ptpi) * R.pstride) % items), (int)k & ((1 << R.ptpi) - 1),
+                       wi0, c0, c1);
+            potential_task(sm, run, R, P, wi0, c0, c1, lane, acc);
+        }
+    } else {
+        pair_decode(R, blockIdx.x, wi0, c0, c1);
+        potential_task(sm, run, R, P, wi0, c0, c1, lane, acc);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (lane == 0) per_cta[blockIdx.x] = acc;
+    if (lane == 0) partials[blockIdx.x] = acc;
 }
 
 // Each run's partials summed in a fixed order: thread t takes t, t + 1024, ...,
@@ -625,7 +652,7 @@ potential_sum_kernel(const __grid_constant__ LaunchTable tab, const double *__re
 {
     __shared__ double sh[32];
     const RunDev &R = tab.runs[blockIdx.x];
-    const int end = R.item_start + (R.pitems << R.ptpi);
+    const int end = R.item_start + R.nsplit;
     double v = 0.0;
     for (int k = R.item_start + threadIdx.x; k < end; k += 1024) v += partials[k];
 #pragma unroll
@@ -697,7 +724,10 @@ cudaError_t gi_launch_potential(const float4 *pos, const LaunchTable &tab, doubl
                                 double *out, cudaStream_t s)
 {
     if (tab.nruns <= 0) return cudaSuccess;
-    if (tab.nitems > 0) potential_kernel<<<tab.nitems, 32, 0, s>>>(pos, tab, partials);
+    bool many = false;
+    for (int r = 0; r < tab.nruns; ++r) many |= tab.runs[r].nsplit == kPotentialPartials;
+    if (tab.nitems > 0 && many) potential_kernel<true><<<tab.nitems, 32, 0, s>>>(pos, tab, partials);
+    else if (tab.nitems > 0) potential_kernel<false><<<tab.nitems, 32, 0, s>>>(pos, tab, partials);
     if (tab.rows > 0) potential_tile_kernel<<<tab.rows, 128, 0, s>>>(pos, tab, partials);
     potential_sum_kernel<<<tab.nruns, 1024, 0, s>>>(tab, partials, out);
     return cudaGetLastError();

@@ -135,9 +135,10 @@ cudaError_t gi_launch_pair_force(const ForceArgs &a, const LaunchTable &tab, con
                                  long long *delta, const unsigned int *ctr, bool with_rows,
                                  bool early, cudaStream_t s);
 // Pair potentials of the table's runs, one double per run in out, in table order.
-// First the runs planned as for gi_launch_pair_force (tab.nitems CTAs, a partial
-// each), then the short ones (pipl 0; tab.rows blocks from row_start on, partials
-// from item_start on, pitems of them).
+// First the runs planned as for gi_launch_pair_force (tab.nitems CTAs), then the
+// short ones (pipl 0; tab.rows blocks from row_start on); each run has nsplit
+// partials from item_start on (the former a CTA for each).
+constexpr int kPotentialPartials = 262144;  // of a run, at most (2 MB)
 cudaError_t gi_launch_potential(const float4 *pos, const LaunchTable &tab, double *partials,
                                 double *out, cudaStream_t s);
 cudaError_t gi_launch_pair_finish(int epi, const ForceArgs &a, const LaunchTable &tab, int maxn,
