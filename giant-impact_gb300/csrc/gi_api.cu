@@ -295,6 +295,7 @@ struct gi_ctx {
     void *work = nullptr;     // workspace of the synchronous calls (gi_internal_ctx_workspace)
     void *work_pinned = nullptr;
     size_t work_cap = 0;
+    int cluster_ctas = 0;     // largest cluster of the grid build (gi_grid_cluster_ctas)
     int occ[4][9];  // resident one-sided force CTAs per SM: [accum][i-bodies per thread]
 };
 
@@ -311,6 +312,9 @@ static int ctx_init(gi_ctx *c, int device)
                     device, prop.major, prop.minor);
     c->sm_count = prop.multiProcessorCount;
     DeviceGuard g(device);
+    c->cluster_ctas = gi_grid_cluster_ctas();
+    GI_CUDA(gi_pair_setup(), "cudaFuncSetAttribute");
+    GI_CUDA(gi_contact_setup(), "cudaFuncSetAttribute");
     c->diag_blocks = gi_diag_blocks(c->sm_count);  // shared by the two material classes
     for (int acc : {GI_ACC_KAHAN, GI_ACC_FP32, GI_ACC_FP64})
         for (int p : {1, 2, 4, 8}) {
@@ -962,7 +966,7 @@ static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi
                 GI_CUDA(cudaStreamWaitEvent(x->aux, x->ev_fork, 0), "cudaStreamWaitEvent");
             }
             // the grid goes first, while the GPU has room for its clusters
-            GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count, true, q), "cell grid");
+            GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count, c->cluster_ctas, q), "cell grid");
             if (!beside)
                 GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, true, s), "tiled contacts");
             GI_CUDA(gi_launch_pair_force(a, tab, gw, x->delta, ctr, !beside, !beside, s), "paired force kernel launch");
@@ -1004,7 +1008,8 @@ static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi
         }
         // Beside the persistent far field the grid is built by small blocks: a
         // cluster's CTAs would keep the far field's off their SMs for good.
-        GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count, !beside, q), "cell grid");
+        GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count,
+                               beside ? 0 : c->cluster_ctas, q), "cell grid");
         GI_CUDA(gi_launch_rows(pos, vel, tab, gw, x->delta, ctr, q), "row contacts");
         GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, false, q), "tiled contacts");
         if (!beside) {

@@ -360,11 +360,6 @@ cudaError_t launch_force_ipt(int acc, int epi, const ForceArgs &a, const LaunchT
     dim3 g(grid), block(GI_NT);
 #define GI_CASE(A, E)                                                    \
     if (acc == A && epi == E) {                                          \
-        /* the contact kernels share its SMs (GI_EPI_SUM) */             \
-        static std::atomic<int> known[64];                               \
-        const cudaError_t e = gi_full_carveout(                          \
-            reinterpret_cast<const void *>(force_kernel<IPT, A, E>), known); \
-        if (e != cudaSuccess) return e;                                  \
         force_kernel<IPT, A, E><<<g, block, 0, s>>>(a, tab);             \
         return cudaGetLastError();                                       \
     }
@@ -381,14 +376,19 @@ cudaError_t launch_force_ipt(int acc, int epi, const ForceArgs &a, const LaunchT
     return cudaErrorInvalidValue;
 }
 
+// Also sets the kernel up in the current CUDA context: the contact kernels share
+// its SMs (GI_EPI_SUM).
 template <int IPT>
 int occupancy_ipt(int acc, int epi)
 {
     int nb = 0;
     cudaError_t e = cudaErrorInvalidValue;
 #define GI_OCC(A, E)                                                              \
-    if (acc == A && epi == E)                                                     \
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, force_kernel<IPT, A, E>, GI_NT, 0);
+    if (acc == A && epi == E) {                                                   \
+        e = gi_full_carveout(reinterpret_cast<const void *>(force_kernel<IPT, A, E>)); \
+        if (e == cudaSuccess)                                                     \
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, force_kernel<IPT, A, E>, GI_NT, 0); \
+    }
     GI_OCC(GI_ACC_KAHAN, GI_EPI_FORCE)
     GI_OCC(GI_ACC_KAHAN, GI_EPI_STEP)
     GI_OCC(GI_ACC_FP32, GI_EPI_FORCE)

@@ -78,7 +78,6 @@
 // stores the force or steps the bodies with the arithmetic of the one-sided
 // kernel's epilogue.
 #include <algorithm>
-#include <atomic>
 
 #include "gi_contact.cuh"
 
@@ -696,14 +695,13 @@ __global__ void __launch_bounds__(256) pair_finish_kernel(const ForceArgs a,
 
 using namespace gi;
 
+cudaError_t gi_pair_setup() { return gi_full_carveout(reinterpret_cast<const void *>(pair_force_kernel)); }
+
 cudaError_t gi_launch_pair_force(const ForceArgs &a, const LaunchTable &tab, const GridWork &g,
                                  long long *delta, const unsigned int *ctr, bool with_rows,
                                  bool early, cudaStream_t s)
 {
     if (tab.nitems <= 0) return cudaSuccess;
-    static std::atomic<int> known[64];
-    cudaError_t e = gi_full_carveout(reinterpret_cast<const void *>(pair_force_kernel), known);
-    if (e != cudaSuccess) return e;
     const int rows = with_rows ? tab.rows : 0;
     return gi_launch(pair_force_kernel, dim3(rows + tab.nitems), 32, early, s, a, g.view(ctr), delta,
                      rows, tab);

@@ -41,7 +41,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
-#include <atomic>
+#include <climits>
 
 #include "gi_contact.cuh"
 
@@ -958,35 +958,36 @@ void gi_grid_runs(LaunchTable &tab)
     tab.gridn = maxn;
 }
 
-// Clusters of 16 CTAs need leave once per device; false: not available here.
-static bool large_clusters()
+cudaError_t gi_contact_setup()
 {
-    static std::atomic<int> known[64];  // 0 unknown, 1 yes, 2 no
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    if (!known[dev].load()) {
-        bool ok = cudaFuncSetAttribute(gi::grid_cluster_kernel,
-                                       cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(gi::kClusterLarge);
-        cfg.blockDim = dim3(1024);
-        cfg.dynamicSmemBytes = (size_t)(gi::kClusterMax / gi::kClusterLarge) * sizeof(unsigned int);
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim = {(unsigned int)gi::kClusterLarge, 1, 1};
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        ok = ok && cudaOccupancyMaxActiveClusters(&clusters, gi::grid_cluster_kernel, &cfg) == cudaSuccess &&
-             clusters > 0;
-        known[dev].store(ok ? 1 : 2);
-    }
-    return known[dev].load() == 1;
+    const cudaError_t e = gi_full_carveout(reinterpret_cast<const void *>(gi::contact_row_kernel));
+    return e != cudaSuccess ? e : gi_full_carveout(reinterpret_cast<const void *>(gi::contact_tile_kernel));
+}
+
+int gi_grid_cluster_ctas()
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(gi::kClusterLarge);
+    cfg.blockDim = dim3(1024);
+    cfg.dynamicSmemBytes = (size_t)(gi::kClusterMax / gi::kClusterLarge) * sizeof(unsigned int);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {(unsigned int)gi::kClusterLarge, 1, 1};
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(gi::grid_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+            cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, gi::grid_cluster_kernel, &cfg) == cudaSuccess &&
+        clusters > 0)
+        return gi::kClusterLarge;
+    cudaGetLastError();  // not an error of the calls that follow
+    return gi::kClusterSmall;
 }
 
 cudaError_t gi_launch_grid(const float4 *pos, const float4 *vel, const LaunchTable &tab,
                            const GridWork &g, long long *delta, unsigned int *ctr, int nsm,
-                           bool clusters, cudaStream_t s)
+                           int clusters, cudaStream_t s)
 {
     if (tab.gridn == 0) return cudaSuccess;
     if (g.buckets > 1024u * 8192u) return cudaErrorInvalidValue;
@@ -999,9 +1000,10 @@ cudaError_t gi_launch_grid(const float4 *pos, const float4 *vel, const LaunchTab
         m = (unsigned int)d.gbase + (1u << d.glog);
     }
     if (m > g.buckets) return cudaErrorInvalidValue;
-    const bool small = tab.gridn < gi::kClusterSmallMax;
-    if (clusters && (small || (tab.gridn < gi::kClusterMax && large_clusters()))) {
-        const int ctas = small ? gi::kClusterSmall : gi::kClusterLarge;
+    const int ctas = tab.gridn < gi::kClusterSmallMax ? gi::kClusterSmall
+                     : tab.gridn < gi::kClusterMax    ? gi::kClusterLarge
+                                                      : INT_MAX;
+    if (clusters >= ctas) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(ctas, tab.nruns);
         cfg.blockDim = dim3(1024);
@@ -1037,9 +1039,6 @@ cudaError_t gi_launch_rows(const float4 *pos, const float4 *vel, const LaunchTab
                            cudaStream_t s)
 {
     if (tab.rows == 0) return cudaSuccess;
-    static std::atomic<int> known[64];
-    const cudaError_t e = gi_full_carveout(reinterpret_cast<const void *>(gi::contact_row_kernel), known);
-    if (e != cudaSuccess) return e;
     gi::contact_row_kernel<<<tab.rows, 32, 0, s>>>(pos, vel, g.view(ctr), delta, tab);
     return cudaGetLastError();
 }
@@ -1048,9 +1047,6 @@ cudaError_t gi_launch_tiles(const LaunchTable &tab, const GridWork &g, long long
                             unsigned int *ctr, int nsm, bool early, cudaStream_t s)
 {
     if (tab.gridn == 0) return cudaSuccess;  // no grid, no crowded cells
-    static std::atomic<int> known[64];
-    const cudaError_t e = gi_full_carveout(reinterpret_cast<const void *>(gi::contact_tile_kernel), known);
-    if (e != cudaSuccess) return e;
     const int gt = (int)std::min<size_t>(g.icap, 7 * (size_t)nsm);
     return gi_launch(gi::contact_tile_kernel, dim3(gt), 128, early, s, g.spos, g.svel, g.dpos, g.dvel,
                      delta, tab, g.items, ctr);

@@ -5,8 +5,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <atomic>
-
 #include "../../include/gi_api.h"
 
 // Threads per CTA of the one-sided force kernel (gi_force_impl.cuh); also
@@ -244,11 +242,15 @@ void gi_grid_runs(LaunchTable &tab);
 // The contact pass, in this order: the grid (with the tiled path's work
 // items); the row path, here or in gi_launch_pair_force, and the tiled path.
 // delta receives every body's correction.  ctr: gi::kCtrWords words, zero on
-// entry of the first.  clusters: build the grids of runs below 131,072 bodies
-// with one thread-block cluster each (see grid_cluster_kernel).
+// entry of the first.  clusters: CTAs of the largest thread-block cluster that may
+// build a run's grid (see grid_cluster_kernel): 8 for runs below 65,536 bodies, 16
+// below 131,072 (gi_grid_cluster_ctas), 0 for none.
 cudaError_t gi_launch_grid(const float4 *pos, const float4 *vel, const LaunchTable &tab,
                            const GridWork &g, long long *delta, unsigned int *ctr, int nsm,
-                           bool clusters, cudaStream_t s);
+                           int clusters, cudaStream_t s);
+// Asks leave for clusters of 16 CTAs in the current CUDA context, which is where
+// that is kept (gone with cudaDeviceReset): 16, or 8 where they are not available.
+int gi_grid_cluster_ctas();
 cudaError_t gi_launch_rows(const float4 *pos, const float4 *vel, const LaunchTable &tab,
                            const GridWork &g, long long *delta, const unsigned int *ctr,
                            cudaStream_t s);
@@ -281,19 +283,18 @@ inline cudaError_t gi_launch(void (*kernel)(P...), dim3 grid, int threads, bool 
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// Asks once per device (known: its flags) for the largest shared-memory
-// carveout of a kernel.  Kernels that are to share an SM need the same one: an
-// SM changes its carveout only when it is empty.
-inline cudaError_t gi_full_carveout(const void *kernel, std::atomic<int> (&known)[64])
+// The largest shared-memory carveout for a kernel, in the current CUDA context.
+// Kernels that are to share an SM need the same one: an SM changes its carveout
+// only when it is empty.
+inline cudaError_t gi_full_carveout(const void *kernel)
 {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess || (dev >= 0 && dev < 64 && known[dev].load())) return e;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess && dev >= 0 && dev < 64) known[dev].store(1);
-    return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                cudaSharedmemCarveoutMaxShared);
 }
+// That for the paired far field's kernel and for the contact kernels; a gi_ctx
+// does it when it is created (it is gone with cudaDeviceReset).
+cudaError_t gi_pair_setup();
+cudaError_t gi_contact_setup();
 
 // gi_aux.cu
 cudaError_t gi_launch_move(float4 *pos, float4 *vel, const float4 *force,

@@ -54,6 +54,9 @@ static_assert(gi::kCtrWords * sizeof(unsigned int) <= kCtrRoom, "the counters mu
 constexpr size_t kDeltaOff = kSumOff + kTriple * kMaxBodies + kCtrRoom;  // contact corrections
 constexpr size_t kGridOff = kDeltaOff + kTriple * kMaxBodies;  // the cell grid
 
+// The portable cluster size, which needs no leave: enough for kMaxBodies.
+constexpr int kClusterCtas = 8;
+
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // The carve of the static array: far-field sums and contact corrections
@@ -191,7 +194,7 @@ extern "C" int gi_forces_collision_noalloc(const float *pos, const float *vel, f
         return gi_internal_fail(GI_ERR_CUDA, "clearing the static scratch sums failed");
     const float4 *p4 = reinterpret_cast<const float4 *>(pos), *v4 = reinterpret_cast<const float4 *>(vel);
     const GridWork g(grid, n, n);
-    if (gi_launch_grid(p4, v4, tab, g, delta, ctr, nsm, true, s) != cudaSuccess ||
+    if (gi_launch_grid(p4, v4, tab, g, delta, ctr, nsm, kClusterCtas, s) != cudaSuccess ||
         gi_launch_tiles(tab, g, delta, ctr, nsm, true, s) != cudaSuccess)
         return gi_internal_fail(GI_ERR_CUDA, "contact pass launch failed");
     ForceArgs a;
