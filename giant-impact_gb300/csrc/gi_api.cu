@@ -665,6 +665,19 @@ extern "C" int gi_debug_pair_plan(gi_ctx *c, int n, int pcl_in, long long out[6]
     return GI_OK;
 }
 
+extern "C" int gi_debug_contact_plan(const int *n, int nruns, int *buckets)
+{
+    if (!n || !buckets) return fail(GI_ERR_INVALID_ARG, "NULL argument");
+    if (nruns < 0 || nruns > GI_MAX_RUNS) return fail(GI_ERR_BAD_SIZE, "nruns = %d", nruns);
+    LaunchTable t;
+    std::memset(&t, 0, sizeof t);
+    t.nruns = nruns;
+    for (int r = 0; r < nruns; ++r) t.runs[r].n = n[r];
+    gi_grid_runs(t);
+    for (int r = 0; r < nruns; ++r) buckets[r] = t.runs[r].glog ? 1 << t.runs[r].glog : 0;
+    return GI_OK;
+}
+
 static int make_pair_plan(const gi_ctx *c, const gi_run *runs, int nruns,
                           const std::vector<PairDev> &pd, Plan &plan)
 {
@@ -767,7 +780,7 @@ static int make_plan(const gi_ctx *c, const gi_run *runs, int nruns,
         if (items > 0x7fffffffLL) return fail(GI_ERR_BAD_SIZE, "too many work items");
         t.nitems = (int)items;
         for (size_t m = 0; m < pd.size(); ++m) t.params[m] = pd[m];
-        gi_grid_runs(t);
+        gi_grid_runs(t, gi::kDirectCandidatesOneSided);
         plan.tables.push_back(t);
         plan.ipt.push_back(p);
         plan.bodies.push_back(nb);
@@ -966,7 +979,8 @@ static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi
                 GI_CUDA(cudaStreamWaitEvent(x->aux, x->ev_fork, 0), "cudaStreamWaitEvent");
             }
             // the grid goes first, while the GPU has room for its clusters
-            GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count, c->cluster_ctas, q), "cell grid");
+            GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count,
+                                   c->cluster_ctas, q), "cell grid");
             if (!beside)
                 GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, true, s), "tiled contacts");
             GI_CUDA(gi_launch_pair_force(a, tab, gw, x->delta, ctr, !beside, !beside, s), "paired force kernel launch");

@@ -19,8 +19,9 @@ __device__ __forceinline__ int3 cell_of(float4 p)
     return make_int3(cell_of(p.x), cell_of(p.y), cell_of(p.z));
 }
 
-// The torus of a run's buckets: glog bits, x >= y >= z of them (4 at least:
-// the 3 x 3 x 3 neighbours of a cell are distinct buckets).
+// The torus of a run's buckets: glog bits, x >= y >= z of them (z at least 3 for a
+// run of more than kDirectAlways bodies: the 3 x 3 x 3 neighbours of a cell are
+// distinct buckets, and cells that share one are too far apart to touch).
 struct Torus {
     unsigned int base;
     int xb, yb;      // bits of x and y
@@ -275,7 +276,7 @@ __device__ __forceinline__ void fix_add3(FixSum3 &a, float c, float dx, float dy
 // The bodies of bucket b (of the torus T) that take the tiled path (see
 // dense_hi), by one warp: their number and their cell c, 0 for none.  They are
 // the bucket's majority cell; bodies of another cell that share the bucket
-// (the torus is at least 16 cells wide, so they are far away) stay on the row
+// (the torus is at least 8 cells wide, so they are far away) stay on the row
 // path.
 __device__ __forceinline__ unsigned int bucket_tiled(const Torus &T, const unsigned int *start,
                                                      const float4 *spos, unsigned int b,

@@ -24,20 +24,20 @@
 // The all-pairs epilogue adds the correction before its single rounding.
 //
 // Two passes share the bodies.  contact_row_kernel takes a few consecutive
-// slots per warp, an ordinary body's path.  Crowded buckets
-// (gi_options.dense_min bodies, 128 by default, or a quarter of that next to
-// such a cell; e.g. an interpenetrating collision remnant with thousands of
-// contacts per body) whose bodies all share one cell are sorted by sub-cell
-// and go through contact_tile_kernel: a work item is (bucket, neighbour
-// bucket, chunk of 128 of its bodies); its CTA stages the neighbour bucket in
-// shared memory 128 bodies at a time, evaluates the law on the hits only, or on
-// whole blocks of pairs that are mostly hits, and a pair of two dense cells
-// is evaluated once for both bodies.  The candidate sets, the pair law and
-// the fixed-point terms are the same on both paths and integer addition is
-// exact, so the corrections are bit-identical whichever path a body takes.
+// slots per warp, an ordinary body's path.  The bodies of a crowded bucket's
+// majority cell (gi_options.dense_min of them, 128 by default, or a quarter of
+// that next to such a cell; e.g. an interpenetrating collision remnant with
+// thousands of contacts per body) are sorted by sub-cell and go through
+// contact_tile_kernel: a work item is (bucket, neighbour bucket, chunk of 128 of
+// its bodies); its CTA stages the neighbour bucket in shared memory 128 bodies at
+// a time, evaluates the law on the hits only, or on whole blocks of pairs that are
+// mostly hits, and a pair of two dense cells is evaluated once for both bodies.
+// The candidate sets, the pair law and the fixed-point terms are the same on both
+// paths and integer addition is exact, so the corrections are bit-identical
+// whichever path a body takes.
 //
-// Runs of at most kDirectMax bodies need no grid: every body of the run is a
-// candidate.
+// Short runs (kDirectMax) need no grid where a table has few: every body of the run
+// is a candidate.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -936,19 +936,22 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
 
 // gi_grid_buckets and gi_grid_words (the scratch layout) are in gi_internal.h.
 
-void gi_grid_runs(LaunchTable &tab)
+void gi_grid_runs(LaunchTable &tab, long long candidates)
 {
     int slots = 0, buckets = 0, rows = 0;
     int maxn = 0;
+    for (int r = 0; r < tab.nruns; ++r)
+        if (tab.runs[r].n <= gi::kDirectMax) candidates -= (long long)tab.runs[r].n * tab.runs[r].n;
+    const int direct = candidates >= 0 ? gi::kDirectMax : gi::kDirectAlways;
     for (int r = 0; r < tab.nruns; ++r) {
         RunDev &d = tab.runs[r];
         d.gslot = slots;
         d.gbase = buckets;
         d.glog = 0;
         d.row_start = rows;
-        const int per = d.n > gi::kDirectMax ? gi::kRowBodies : gi::kDirectBodies;
+        const int per = d.n > direct ? gi::kRowBodies : gi::kDirectBodies;
         rows += (d.n + per - 1) / per;
-        if (d.n <= gi::kDirectMax) continue;
+        if (d.n <= direct) continue;
         while ((2LL << d.glog) <= 2LL * d.n) ++d.glog;  // the largest power of two <= 2 n
         slots += d.n;
         buckets += 1 << d.glog;

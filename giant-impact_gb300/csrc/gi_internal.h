@@ -161,8 +161,18 @@ constexpr unsigned int kItemClasses = 16;
 // Tiled-path counters: items, tiled buckets, queue head, candidate buckets,
 // then a count and a fill cursor per cost class, then a bit per run.
 constexpr int kCtrWords = 4 + 2 * (int)kItemClasses + GI_MAX_RUNS / 32;
-// Runs of at most this many bodies take no grid.
-constexpr int kDirectMax = 4096;
+// Runs of at most kDirectMax bodies take no grid (every body of the run is a
+// candidate) where all such runs of a table together have at most kDirectCandidates
+// candidates (one run of 3,500); in fuller tables those of at most kDirectAlways.
+// The candidates of a full GPU cost more than a grid build, whose launches are what
+// a lone short run spends its step on.  us a step of settled bodies, without a grid /
+// with one: one run of 2,000 13 / 33, 3,000 26 / 30, 4,000 40 / 31; two of 3,000 41 /
+// 32; eight of 1,000 28 / 30, 2,000 72 / 52; 24 of 500 27 / 39, 1,000 65 / 56, 2,000
+// 200 / 102; 64 of 500 60 / 79, 1,000 160 / 95, 4,000 1,757 / 480.  Beside the
+// one-sided far field, where the grid-wide kernels build the grid: one of 4,000 41 /
+// 66, 24 of 1,000 60 / 78, eight of 2,000 72 / 86, 24 of 2,000 182 / 128.
+constexpr int kDirectMax = 4096, kDirectAlways = 512;
+constexpr long long kDirectCandidates = 3500 * 3500, kDirectCandidatesOneSided = 40000000;
 // Bodies of a row-path CTA (one warp), of a run with a grid and without.
 constexpr int kRowBodies = 8, kDirectBodies = 2;
 }  // namespace gi
@@ -237,8 +247,9 @@ struct GridWork {
         return GridView{spos, svel, dpos, start, state, ctr};
     }
 };
-// Sets the grid and row fields of the table and its runs.
-void gi_grid_runs(LaunchTable &tab);
+// Sets the grid and row fields of the table and its runs; candidates: what its runs
+// without a grid may have.
+void gi_grid_runs(LaunchTable &tab, long long candidates = gi::kDirectCandidates);
 // The contact pass, in this order: the grid (with the tiled path's work
 // items); the row path, here or in gi_launch_pair_force, and the tiled path.
 // delta receives every body's correction.  ctr: gi::kCtrWords words, zero on

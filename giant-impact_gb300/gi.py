@@ -217,6 +217,7 @@ _SIGS = {
     "gi_measure_ffma_peak": ([C.c_int, C.POINTER(C.c_double)], C.c_int),
     "gi_debug_fill_counters": ([_P, _P, C.c_uint], C.c_int),
     "gi_debug_pair_plan": ([_P, C.c_int, C.c_int, C.POINTER(C.c_longlong)], C.c_int),
+    "gi_debug_contact_plan": ([C.POINTER(C.c_int), C.c_int, C.POINTER(C.c_int)], C.c_int),
     "gi_server_create": ([C.c_int, C.POINTER(ServerConfig), C.POINTER(PairParams), C.c_int,
                           C.POINTER(_P)], C.c_int),
     "gi_server_destroy": ([_P], C.c_int),
@@ -333,6 +334,15 @@ def pair_plan(n: int, pcl: int = -1, ctx=None) -> dict:
     check(lib().gi_debug_pair_plan(ctx.h if ctx is not None else None, n, pcl, out))
     return {"pcl": out[0], "chunks": out[1], "iblocks": out[2], "items": out[3],
             "stride": out[4], "items_block0": out[5]}
+
+
+def contact_plan(sizes) -> list[int]:
+    """Buckets of the contact pass's cell grid for runs of these sizes in one call
+    (0: every body of the run is a candidate); usable without a GPU."""
+    n = (C.c_int * len(sizes))(*sizes)
+    out = (C.c_int * len(sizes))()
+    check(lib().gi_debug_contact_plan(n, len(sizes), out))
+    return list(out)
 
 
 def params_from_material(G=1.0, diameter=1.0, mass_fe=1.0, mass_si=0.4, k_fe=5.0, k_si=1.5,

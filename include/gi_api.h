@@ -364,6 +364,11 @@ int gi_debug_fill_counters(gi_ctx *ctx, void *stream, unsigned int value);
  * permutation, items of i-block 0}. */
 int gi_debug_pair_plan(gi_ctx *ctx, int n, int pcl, long long out[6]);
 
+/* Test hook: buckets of the contact pass's cell grid for each of up to 64 runs
+ * of n[k] bodies in one call (0: every body of the run is a candidate); host
+ * arithmetic only. */
+int gi_debug_contact_plan(const int *n, int nruns, int *buckets);
+
 /* ------------------------------------------------------------------------ */
 /* Serving loop (continuous batching of impact runs)                        */
 /* ------------------------------------------------------------------------ */
