@@ -893,6 +893,14 @@ constexpr long long kOverlapMaxPairs = 1LL << 34;
 // 67 / 74, 66,000 1,047 / 1,098, 140,000 (six steps) 26.6 / 27.1 ms; a remnant
 // of 4,600 91 / 100, 8,000 129 / 150.
 constexpr long long kBesideMinPairs = 30000000LL;
+// Beside the far field a table's grids are built by the grid-wide kernels, whose
+// small blocks find room among its CTAs, where their chain (45 us) hides behind it:
+// several runs and at least this many pairs, or more clusters than fit at one CTA an
+// SM.  A cluster of eight 1,024-thread CTAs waits for the far field's to leave.  us
+// a step of settled bodies, clusters / grid-wide: 2 x 9,000 bodies 69 / 82, 3 x 96 /
+// 95, 4 x 122 / 116, 8 x 220 / 215; 12 x 2,500 76 / 79, 24 x 2,000 112 / 102, 64 x
+// 112 / 95 (1,000), 255 / 228 (2,000); one run of 66,000 1,026 / 1,029.
+constexpr long long kWideGridMinPairs = 240000000LL;
 // Far-field CTAs per SM while the contact pass runs beside it.  Measured on
 // the 66,000-body impact (ms per fused step, settled / collision phase):
 // 3 CTAs 1.72 / 2.60, 4: 1.68 / 2.57, 6: 1.68 / 2.59, 8: 1.67 / 2.54; the
@@ -974,13 +982,15 @@ static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi
             if (!call->capturing) x->clean = 0;
             const bool beside = tab.gridn > 0 && pairs >= kBesideMinPairs;
             const cudaStream_t q = beside ? x->aux : s;
+            const bool wide = beside && ((tab.gridruns > 1 && pairs >= kWideGridMinPairs) ||
+                                         8 * tab.gridruns > c->sm_count);
             if (beside && !call->chained) {
                 GI_CUDA(cudaEventRecord(x->ev_fork, s), "cudaEventRecord");
                 GI_CUDA(cudaStreamWaitEvent(x->aux, x->ev_fork, 0), "cudaStreamWaitEvent");
             }
             // the grid goes first, while the GPU has room for its clusters
             GI_CUDA(gi_launch_grid(pos, vel, tab, gw, x->delta, ctr, c->sm_count,
-                                   c->cluster_ctas, q), "cell grid");
+                                   wide ? 0 : c->cluster_ctas, q), "cell grid");
             if (!beside)
                 GI_CUDA(gi_launch_tiles(tab, gw, x->delta, ctr, c->sm_count, true, s), "tiled contacts");
             GI_CUDA(gi_launch_pair_force(a, tab, gw, x->delta, ctr, !beside, !beside, s), "paired force kernel launch");

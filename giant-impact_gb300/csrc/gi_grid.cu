@@ -938,7 +938,7 @@ contact_tile_kernel(const float4 *__restrict__ spos, const float4 *__restrict__ 
 
 void gi_grid_runs(LaunchTable &tab, long long candidates)
 {
-    int slots = 0, buckets = 0, rows = 0;
+    int slots = 0, buckets = 0, rows = 0, grids = 0;
     int maxn = 0;
     for (int r = 0; r < tab.nruns; ++r)
         if (tab.runs[r].n <= gi::kDirectMax) candidates -= (long long)tab.runs[r].n * tab.runs[r].n;
@@ -956,9 +956,11 @@ void gi_grid_runs(LaunchTable &tab, long long candidates)
         slots += d.n;
         buckets += 1 << d.glog;
         maxn = std::max(maxn, d.n);
+        ++grids;
     }
     tab.rows = rows;
     tab.gridn = maxn;
+    tab.gridruns = grids;
 }
 
 cudaError_t gi_contact_setup()

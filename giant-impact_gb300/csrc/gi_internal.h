@@ -78,6 +78,7 @@ struct LaunchTable {
     int dense_min;  // contact pass: bucket size from which the tiled kernel takes it
     int rows;       // row-path CTAs of all runs
     int gridn;      // bodies of the largest run with a grid (0: none)
+    int gridruns;   // runs with a grid
     RunDev runs[GI_MAX_RUNS];
     PairDev params[GI_MAX_PARAMS];
 };
