@@ -507,6 +507,58 @@ __device__ __forceinline__ void row_group(RowSmem &sm, const float4 *__restrict_
     }
 }
 
+// A lone body with at most 32 candidates, one to a lane, straight from memory: no
+// staging, no list.  [beg, beg + cnt): the lane's range, excl the candidates before it.
+__device__ __forceinline__ void row_few(const GridView &g, long long *__restrict__ delta,
+                                        const LaunchTable &tab, const RunDev &R, const PairDev &P,
+                                        unsigned int self, unsigned int beg, unsigned int cnt,
+                                        unsigned int total, bool add, int lane)
+{
+    unsigned int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const unsigned int excl = incl - cnt;
+    int src = 0;  // the lane whose range holds candidate `lane`: the last one with excl <= it
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) {
+        const unsigned int e = __shfl_sync(0xffffffffu, excl, (src + step) & 31);
+        if (src + step < 32 && e <= (unsigned int)lane) src += step;
+    }
+    const unsigned int slot = __shfl_sync(0xffffffffu, beg - excl, src) + (unsigned int)lane;
+    const float4 pi = __ldg(&g.spos[self]);
+    float4 p = make_float4(__int_as_float(0x7fffffff), 0.f, 0.f, 0.f);
+    if ((unsigned int)lane < total) p = __ldg(&g.spos[slot]);
+    const float dx = p.x - pi.x, dy = p.y - pi.y, dz = p.z - pi.z;
+    const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+    const bool hit = r2 < 1.0f && slot != self;
+    FixSum3 acc;
+    fix_zero(acc);
+    if (hit) {
+        const int sw = R.offset + R.nfe;
+        const PairRow row = pair_row(P, __float_as_int(pi.w) < sw, __float_as_int(p.w) < sw);
+        const float c = contact_coef(row, tab.sep_test, dx, dy, dz, r2, __ldg(&g.svel[self]),
+                                     __ldg(&g.svel[slot])) * P.inv_unit;
+        fix_add3<false>(acc, c, dx, dy, dz, r2);
+        fix_fold(acc);
+    }
+    long long a[3] = {0, 0, 0};
+    for (unsigned int m = __ballot_sync(0xffffffffu, hit); m; m &= m - 1u) {
+        const int l = __ffs(m) - 1;
+        a[0] += __shfl_sync(0xffffffffu, acc.x, l);
+        a[1] += __shfl_sync(0xffffffffu, acc.y, l);
+        a[2] += __shfl_sync(0xffffffffu, acc.z, l);
+    }
+    if (lane < 3) {
+        long long *const d = &delta[3 * (size_t)__float_as_int(pi.w) + lane];
+        const long long v = lane == 0 ? a[0] : lane == 1 ? a[1] : a[2];
+        if (!add) *d = v;
+        else if (v) atomicAdd(reinterpret_cast<unsigned long long *>(d), (unsigned long long)v);
+    }
+}
+
 // Runs without a grid: kDirectBodies bodies from `first` on, every body of the
 // run a candidate.
 __device__ __forceinline__ void row_direct(RowSmem &sm, const float4 *__restrict__ pos,
@@ -590,6 +642,14 @@ __device__ __forceinline__ void row_slots(RowSmem &sm, const GridView &g,
             }
         }
         rest &= ~(((1u << n) - 1u) << src);
+        if (n == 1) {
+            const unsigned int total = __reduce_add_sync(0xffffffffu, end - beg);
+            if (total <= 32u) {
+                row_few(g, delta, tab, R, P, (unsigned int)(R.gslot + first + src), beg, end - beg, total,
+                        crowds, lane);
+                continue;
+            }
+        }
         // the lanes among the group's bodies
         const int wlog = n > 4 ? 2 : n > 2 ? 3 : n > 1 ? 4 : 5;
         const int k = lane >> wlog;
