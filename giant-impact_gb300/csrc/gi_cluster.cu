@@ -17,7 +17,8 @@
 //      those already in its tree and tests body pairs (the reference's FP32
 //      test, evaluated with the same roundings) until one touches, which
 //      links the two trees.  The 13 forward adjacent cells come first, the 49
-//      further ones in a second launch, when most are in the same tree.  Links
+//      further ones in a second launch, when most are in the same tree (small
+//      cells among many bodies: all 62 at once, cluster_link_sparse).  Links
 //      always hang the root with the larger index under the one with the
 //      smaller index (one atomicCAS on a root), so a tree's root is its
 //      smallest member: the reference's group number;
@@ -59,15 +60,14 @@ __device__ __forceinline__ bool cluster_cell(float4 p, double inv_cell, int3 &c)
     return true;
 }
 
-__device__ __forceinline__ unsigned int cluster_hash(int cx, int cy, int cz, unsigned int mask)
+__device__ __forceinline__ unsigned int cluster_hash(int cx, int cy, int cz)
 {
     unsigned int h = (unsigned int)cx * 2246822519u;
     h ^= (unsigned int)cy * 3266489917u;
     h ^= (unsigned int)cz * 668265263u;
     h ^= h >> 13;
     h *= 2654435761u;
-    h ^= h >> 16;
-    return h & mask;
+    return h ^ h >> 16;
 }
 
 // One slot of the cell table.  All words start at ~0.
@@ -76,7 +76,14 @@ struct CellTable {
     unsigned int *leader;  // the cell's smallest body index
     unsigned int *count;   // bodies - 1; then the next place of its list
     int4 *cell;            // coordinates and cell number
+    unsigned int *absent;  // NULL, or a bit per eighth of a slot: no cell of this hash
 };
+
+// A hash's bit of the filter `absent` (see cluster_link_sparse).
+__device__ __forceinline__ unsigned int filter_bit(unsigned int h, unsigned int mask)
+{
+    return (h ^ h >> 15) * 2654435769u >> 3 & (8u * mask + 7u);
+}
 
 // Occupied cell k: first place in the list, bodies, slot, smallest body.
 struct CellInfo {
@@ -103,7 +110,8 @@ cluster_insert(const float4 *__restrict__ pos, int n, double inv_cell, unsigned 
             loose[atomicAdd(&ctr->loose, 1u)] = i;
             continue;
         }
-        unsigned int s = cluster_hash(c.x, c.y, c.z, mask);
+        const unsigned int h = cluster_hash(c.x, c.y, c.z);
+        unsigned int s = h & mask;
         for (unsigned int t = 0; t <= mask; ++t, s = (s + 1u) & mask) {
             int cur = __ldcg(&tab.rep[s]);
             if (cur < 0) {
@@ -112,6 +120,10 @@ cluster_insert(const float4 *__restrict__ pos, int n, double inv_cell, unsigned 
                     const unsigned int k = atomicAdd(&ctr->cells, 1u);
                     tab.cell[s] = make_int4(c.x, c.y, c.z, (int)k);
                     info[k].slot = (int)s;
+                    if (tab.absent) {
+                        const unsigned int f = filter_bit(h, mask);
+                        atomicAnd(&tab.absent[f >> 5], ~(1u << (f & 31u)));
+                    }
                     break;
                 }
             }
@@ -280,6 +292,39 @@ __device__ __forceinline__ bool cells_touch_warp(const float4 *__restrict__ list
 // Pair tests a lane makes by itself; larger cell pairs go to the whole warp.
 constexpr unsigned int kLanePairs = 64;
 
+// Links cell a (the warp's) with each lane's cell b (cnt 0: none) where bodies of
+// theirs touch.  Trees that are already one are not tested; of a lane's pairs of at
+// most `few` bodies that is not looked at first.
+__device__ __forceinline__ void link_cells(const float4 *__restrict__ list, const CellInfo &a,
+                                           const CellInfo &b, float touch, unsigned int few, int tries,
+                                           int *parent, int *err, int lane)
+{
+    const unsigned long long pairs = (unsigned long long)a.cnt * b.cnt;
+    bool open = pairs > 0u &&
+                (pairs <= few || find_root(parent, a.leader) != find_root(parent, b.leader));
+    bool hit = false;
+    if (open && pairs <= kLanePairs) {
+        for (unsigned int u = 0; u < a.cnt && !hit; ++u) {
+            const float4 p = list[a.beg + u];
+            for (unsigned int v = 0; v < b.cnt && !hit; ++v)
+                hit = touching(p, list[b.beg + v], touch);
+        }
+        open = false;
+    }
+    for (unsigned int todo = __ballot_sync(0xffffffffu, open); todo; todo &= todo - 1u) {
+        const int src = __ffs(todo) - 1;
+        CellInfo q;
+        q.beg = __shfl_sync(0xffffffffu, b.beg, src);
+        q.cnt = __shfl_sync(0xffffffffu, b.cnt, src);
+        const bool swap = a.cnt < q.cnt;  // the larger cell's bodies on the lanes
+        const bool any = cells_touch_warp(list, swap ? q : a, swap ? a : q, touch, lane);
+        if (lane == src) hit = any;
+    }
+    // the lanes link together: their attempts on one root collide and
+    // are tried again on the root that won
+    if (hit && !link(parent, a.leader, b.leader, tries)) atomicExch(err, 1);
+}
+
 // One warp per occupied cell.  FAR = false: its 13 forward neighbours that
 // share a face, edge or corner; FAR = true: the 49 forward cells beyond them,
 // two a lane.
@@ -305,7 +350,7 @@ cluster_link(const float4 *__restrict__ list, CellTable tab, const CellInfo *__r
             if (FAR) look = look && (abs(ox) == 2 || abs(oy) == 2 || abs(oz) == 2);
             CellInfo b{0u, 0u, 0, 0};
             if (look) {
-                unsigned int s = cluster_hash(c.x + ox, c.y + oy, c.z + oz, mask);
+                unsigned int s = cluster_hash(c.x + ox, c.y + oy, c.z + oz) & mask;
                 for (unsigned int t = 0; t <= mask; ++t, s = (s + 1u) & mask) {
                     if (__ldg(&tab.rep[s]) < 0) break;
                     const int4 d = __ldg(&tab.cell[s]);
@@ -315,29 +360,72 @@ cluster_link(const float4 *__restrict__ list, CellTable tab, const CellInfo *__r
                     }
                 }
             }
-            bool open = b.cnt > 0u && find_root(parent, a.leader) != find_root(parent, b.leader);
-            bool hit = false;
-            if (open && (unsigned long long)a.cnt * b.cnt <= kLanePairs) {
-                for (unsigned int u = 0; u < a.cnt && !hit; ++u) {
-                    const float4 p = list[a.beg + u];
-                    for (unsigned int v = 0; v < b.cnt && !hit; ++v)
-                        hit = touching(p, list[b.beg + v], touch);
-                }
-                open = false;
-            }
-            for (unsigned int todo = __ballot_sync(0xffffffffu, open); todo; todo &= todo - 1u) {
-                const int src = __ffs(todo) - 1;
-                CellInfo q;
-                q.beg = __shfl_sync(0xffffffffu, b.beg, src);
-                q.cnt = __shfl_sync(0xffffffffu, b.cnt, src);
-                const bool swap = a.cnt < q.cnt;  // the larger cell's bodies on the lanes
-                const bool any = cells_touch_warp(list, swap ? q : a, swap ? a : q, touch, lane);
-                if (lane == src) hit = any;
-            }
-            // the lanes link together: their attempts on one root collide and
-            // are tried again on the root that won
-            if (hit && !link(parent, a.leader, b.leader, tries)) atomicExch(err, 1);
+            link_cells(list, a, b, touch, 0u, tries, parent, err, lane);
         }
+    }
+}
+
+// The same for many bodies, whose table is larger than L2: there a cell costs its
+// chain of dependent loads from memory, and most of a sparse state's cells hold one
+// body among empty neighbours.  So the chain is made short and taken once: the
+// filter, a sixteenth of the table, says from L2 which neighbours are empty; all 62
+// are looked up before any is linked, two to a lane, their first probes together;
+// one or two pairs are tested sooner than two trees are climbed; and a cell of at
+// most kFew bodies takes its near and far neighbours in the first launch.  Grouping
+// a raw ball of 4M bodies took 14.0 ms with the two launches above (9.1 with one
+// thread per body and its 27 cells), now 8.5; of 1M 2.6 (2.2) and 1.6; 200,000 0.50
+// and 0.33; 4M settled bodies 5.2 both ways.  Below kSparseMin bodies more lanes
+// linking at once collide on the roots: 20,000 settled ones 0.14 and 0.19.
+constexpr unsigned int kFew = 2u;
+constexpr int kSparseMin = 150000;
+template <bool FAR>
+__global__ void __launch_bounds__(128)
+cluster_link_sparse(const float4 *__restrict__ list, CellTable tab, const CellInfo *__restrict__ info,
+                    unsigned int mask, float touch, int tries, int *parent,
+                    const ClusterCounters *__restrict__ ctr, int *__restrict__ err)
+{
+    launch_wait();
+    const int lane = threadIdx.x & 31;
+    const unsigned int cells = ctr->cells, nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (unsigned int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < cells; k += nwarps) {
+        const CellInfo a = info[k];
+        const bool few = a.cnt <= kFew;
+        if (FAR && few) continue;
+        const int4 c = tab.cell[a.slot];
+        int3 at[2];
+        unsigned int s[2];
+        bool look[2];
+        int rep[2];
+        int4 d[2];
+        CellInfo b[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int o = 63 + r * 32 + lane;  // of the 5^3 block
+            const int ox = o % 5 - 2, oy = o / 5 % 5 - 2, oz = o / 25 - 2;
+            const bool near = abs(ox) < 2 && abs(oy) < 2 && oz < 2;
+            at[r] = make_int3(c.x + ox, c.y + oy, c.z + oz);
+            const unsigned int h = cluster_hash(at[r].x, at[r].y, at[r].z), f = filter_bit(h, mask);
+            s[r] = h & mask;
+            look[r] = o < 125 && (few || near != FAR) && !(__ldg(&tab.absent[f >> 5]) >> (f & 31u) & 1u);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            rep[r] = look[r] ? __ldg(&tab.rep[s[r]]) : -1;
+            d[r] = look[r] ? __ldg(&tab.cell[s[r]]) : c;
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            for (unsigned int t = 0; t <= mask && rep[r] >= 0; ++t) {
+                if (d[r].x == at[r].x && d[r].y == at[r].y && d[r].z == at[r].z) break;
+                s[r] = (s[r] + 1u) & mask;
+                rep[r] = __ldg(&tab.rep[s[r]]);
+                d[r] = __ldg(&tab.cell[s[r]]);
+            }
+            b[r] = CellInfo{0u, 0u, 0, 0};
+            if (rep[r] >= 0) b[r] = info[d[r].w];
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) link_cells(list, a, b[r], touch, kFew, tries, parent, err, lane);
     }
 }
 
@@ -483,10 +571,12 @@ extern "C" int gi_find_earth_moon(gi_ctx *ctx, const float *pos, int n, float to
     if (m > 1024u * 8192u) return gi_internal_fail(GI_ERR_BAD_SIZE, "gi_find_earth_moon: n too large");
     // One block of the context's workspace: the result, the cell
     // coordinates, the body list and the cell list (16-byte words), then the
-    // words that start at ~0 (rep, leader, count, size), then the rest.
+    // words that start at ~0 (rep, leader, count, absent, size), then the rest.
     const size_t M = m, N = (size_t)n;
     const size_t head = (sizeof(ClusterResult) + 15) & ~(size_t)15;
-    const size_t bytes = head + 16 * (M + 2 * N) + 4 * (3 * M + N) + 4 * 3 * N;
+    const bool sparse = n >= gi::kSparseMin;
+    const size_t F = sparse ? M / 4 : 0;
+    const size_t bytes = head + 16 * (M + 2 * N) + 4 * (3 * M + F + N) + 4 * 3 * N;
     void *work = nullptr, *pinned = nullptr;
     if (int st = gi_internal_ctx_workspace(ctx, bytes, &work, &pinned)) return st;
     unsigned char *buf = static_cast<unsigned char *>(work);
@@ -498,7 +588,8 @@ extern "C" int gi_find_earth_moon(gi_ctx *ctx, const float *pos, int n, float to
     tab.rep = reinterpret_cast<int *>(info + N);
     tab.leader = reinterpret_cast<unsigned int *>(tab.rep + M);
     tab.count = tab.leader + M;
-    int *size = reinterpret_cast<int *>(tab.count + M);
+    tab.absent = sparse ? tab.count + M : nullptr;
+    int *size = reinterpret_cast<int *>(tab.count + M + F);
     int *parent = size + N, *slot_of = parent + N, *loose = slot_of + N;
     ClusterResult &host = *static_cast<ClusterResult *>(pinned);
     // Where the squares of the touch test leave FP32's normal range, cells
@@ -512,7 +603,7 @@ extern "C" int gi_find_earth_moon(gi_ctx *ctx, const float *pos, int n, float to
     cudaError_t e;
     do {
         if ((e = cudaMemsetAsync(res, 0, sizeof(ClusterResult), s)) != cudaSuccess) break;
-        if ((e = cudaMemsetAsync(tab.rep, 0xff, 4 * (3 * M + N), s)) != cudaSuccess) break;
+        if ((e = cudaMemsetAsync(tab.rep, 0xff, 4 * (3 * M + F + N), s)) != cudaSuccess) break;
         gi::cluster_insert<<<gridded, 256, 0, s>>>(P, n, inv_cell, m - 1, tab, info, slot_of, loose,
                                                    &res->ctr);
         // each launch follows the one before it early
@@ -522,10 +613,10 @@ extern "C" int gi_find_earth_moon(gi_ctx *ctx, const float *pos, int n, float to
         e = cudaGetLastError();
         next(gi::cluster_ranges, gridded, 256, tab, info, &res->ctr);
         next(gi::cluster_scatter, gridded, 256, P, n, tab, slot_of, list, parent);
-        next(gi::cluster_link<false>, warps, 128, list, tab, info, m - 1, touch, tries, parent, &res->ctr,
-             &res->err);
-        next(gi::cluster_link<true>, warps, 128, list, tab, info, m - 1, touch, tries, parent, &res->ctr,
-             &res->err);
+        next(sparse ? gi::cluster_link_sparse<false> : gi::cluster_link<false>, warps, 128, list, tab, info,
+             m - 1, touch, tries, parent, &res->ctr, &res->err);
+        next(sparse ? gi::cluster_link_sparse<true> : gi::cluster_link<true>, warps, 128, list, tab, info,
+             m - 1, touch, tries, parent, &res->ctr, &res->err);
         next(gi::cluster_link_loose, std::min(warps, 1024), 128, P, n, loose, touch, tries, parent,
              &res->ctr, &res->err);
         next(gi::cluster_flatten, gridded, 256, parent, n, size, &res->ngroups);
