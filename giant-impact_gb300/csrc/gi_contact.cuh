@@ -582,7 +582,8 @@ __device__ __forceinline__ void row_direct(RowSmem &sm, const float4 *__restrict
 // Runs with a grid: kRowBodies (8) consecutive slots.  Slots run along x, so
 // the bodies of one cell row (same y and z cell) a few cells apart share their
 // candidates: nine rows' slots over the bodies' x range and one cell to either
-// side, each one contiguous range (two where the torus wraps).
+// side, each one contiguous range (two where the torus wraps).  FEW: with row_few.
+template <bool FEW>
 __device__ __forceinline__ void row_slots(RowSmem &sm, const GridView &g,
                                           long long *__restrict__ delta, const LaunchTable &tab,
                                           const RunDev &R, unsigned int run, int first, int lane)
@@ -642,7 +643,7 @@ __device__ __forceinline__ void row_slots(RowSmem &sm, const GridView &g,
             }
         }
         rest &= ~(((1u << n) - 1u) << src);
-        if (n == 1) {
+        if (FEW && n == 1) {
             const unsigned int total = __reduce_add_sync(0xffffffffu, end - beg);
             if (total <= 32u) {
                 row_few(g, delta, tab, R, P, (unsigned int)(R.gslot + first + src), beg, end - beg, total,
@@ -664,6 +665,7 @@ __device__ __forceinline__ void row_slots(RowSmem &sm, const GridView &g,
 }
 
 // Row-path CTA (one warp) w of the table: bodies of one run.
+template <bool FEW>
 __device__ __forceinline__ void contact_rows(RowSmem &sm, const float4 *__restrict__ pos,
                                              const float4 *__restrict__ vel, const GridView &g,
                                              long long *__restrict__ delta, const LaunchTable &tab,
@@ -677,7 +679,7 @@ __device__ __forceinline__ void contact_rows(RowSmem &sm, const float4 *__restri
     }
     const RunDev &R = tab.runs[lo];
     const int first = (w - R.row_start) * (R.glog ? kRowBodies : kDirectBodies);
-    if (R.glog) row_slots(sm, g, delta, tab, R, lo, first, threadIdx.x);
+    if (R.glog) row_slots<FEW>(sm, g, delta, tab, R, lo, first, threadIdx.x);
     else row_direct(sm, pos, vel, delta, tab, R, first, threadIdx.x);
 }
 

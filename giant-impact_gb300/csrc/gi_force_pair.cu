@@ -345,7 +345,10 @@ __device__ __forceinline__ void pair_item(PairSmem &sm, const ForceArgs &a, cons
 // 5 us, a step of a few thousand bodies 20 to 50.
 // 162 registers (no spills): 12 CTAs per SM.  ptxas's allocation moves the
 // loop by 5 %: held to 160 it takes 1.073 ms at N = 66,000 (262,144: 16.8),
-// at 162 1.012 (15.25), at 168 1.037, with the sums in another order 1.032.
+// at 162 1.012 (15.25), at 168 1.037, with the sums in another order 1.032.  (The
+// cap is 168; ptxas takes 162 of its own.)  Code beside the loop moves it too: with
+// the row path's row_few in this kernel every run from 66,000 bodies on took 0.3 %
+// more, so it is left to contact_row_kernel.
 __global__ void __maxnreg__(168)
 pair_force_kernel(const ForceArgs a, const GridView g, long long *__restrict__ delta, int rows,
                   const __grid_constant__ LaunchTable tab)
@@ -357,7 +360,7 @@ pair_force_kernel(const ForceArgs a, const GridView g, long long *__restrict__ d
     } sm;
     launch_wait();
     if ((int)blockIdx.x < rows)
-        contact_rows(sm.row, a.pos, a.vel, g, delta, tab, blockIdx.x);
+        contact_rows<false>(sm.row, a.pos, a.vel, g, delta, tab, blockIdx.x);
     else
         pair_item(sm.pair, a, tab, blockIdx.x - rows, threadIdx.x);
 }

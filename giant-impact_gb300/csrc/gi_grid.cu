@@ -138,7 +138,7 @@ contact_row_kernel(const float4 *__restrict__ pos, const float4 *__restrict__ ve
                    long long *__restrict__ delta, const __grid_constant__ LaunchTable tab)
 {
     __shared__ RowSmem sm;
-    contact_rows(sm, pos, vel, g, delta, tab, blockIdx.x);
+    contact_rows<true>(sm, pos, vel, g, delta, tab, blockIdx.x);
 }
 // Work item of the tiled path, self-contained so that the tile kernel reads
 // it in one load, with no hop through the bucket bounds:
