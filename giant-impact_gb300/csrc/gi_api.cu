@@ -521,6 +521,13 @@ static int pair_pcl_for(const gi_ctx *c, int n)
 
 int gi_internal_pair_default_pcl(int n) { return 2 + (n >= 32768) + (n >= 131072); }
 
+// The far field's items, all rows eight to a lane, and fewer chunks each: without
+// per-body sums a short item costs no atomics, and the last ones leave less of the
+// GPU idle.  us an energy log (diagnostics and potential) at the far field's chunks,
+// half and a quarter of them: 20,000 bodies 259, 241, 225; 33,000 446, 438, 397;
+// 66,000 1,211, 1,139, 1,151; 130,000 3,825, 3,817, 3,933.
+int gi_internal_potential_pcl(int n) { return gi_internal_pair_default_pcl(n) - (n < 65536 ? 2 : 1); }
+
 extern "C" int gi_ctx_get_tuning(gi_ctx *c, int n, gi_tuning *out)
 {
     if (!c || !out) return fail(GI_ERR_INVALID_ARG, "NULL argument");
@@ -631,16 +638,17 @@ long long gi_internal_pair_run(RunDev &d, int n, int pcl, const PairDev &p, long
                                int ipl)
 {
     d.ipt = gi::kPairIpl;
-    d.pcl = pcl;
     d.pnc = (n + gi::kPairChunk - 1) / gi::kPairChunk;
-    d.pnb = (n + gi::kPairRows - 1) / gi::kPairRows;
-    d.pk0 = (d.pnc + (1 << pcl) - 1) >> pcl;
+    d.pblk = gi::kPairRowsLog2 - gi::kPairChunkLog2;
+    d.pcl = pcl;
+    pair_shape(n, pcl, ipl, &d.pipl, &d.ptpi);
+    d.pnb = (d.pnc + (1 << d.pblk) - 1) >> d.pblk;
+    d.pk0 = (d.pnc + (1 << d.pcl) - 1) >> d.pcl;
     pair_far_unit(n, p, d);
     d.item_start = (int)std::min(item_start, 0x7fffffffLL);
-    const long long ri = pair_items(n, pcl);
+    const long long b = d.pnb, ri = b * d.pk0 - (b * (b - 1) / 2 << (d.pblk - d.pcl));
     d.pitems = (int)std::min(ri, 0x7fffffffLL);
     d.pstride = pair_stride(ri, d.pnb);
-    pair_shape(n, pcl, ipl, &d.pipl, &d.ptpi);
     return ri << d.ptpi;
 }
 
@@ -655,13 +663,36 @@ extern "C" int gi_debug_pair_plan(gi_ctx *c, int n, int pcl_in, long long out[6]
     std::memset(&p, 0, sizeof p);
     p.gm_fe = p.gm_si = 1.0f;
     const int pcl = pcl_in >= 0 ? pcl_in : (c ? pair_pcl_for(c, n) : gi_internal_pair_default_pcl(n));
-    const long long items = gi_internal_pair_run(d, n, pcl, p, 0);
-    out[0] = d.pcl;
+    gi_internal_pair_run(d, n, pcl, p, 0);
+    // in i-blocks of kPairRows and items of 2^pcl chunks, whose warps the run's are
+    out[0] = pcl;
     out[1] = d.pnc;
-    out[2] = d.pnb;
-    out[3] = items >> d.ptpi;
-    out[4] = d.pstride;
-    out[5] = d.pk0;
+    out[2] = (n + gi::kPairRows - 1) / gi::kPairRows;
+    out[3] = pair_items(n, pcl);
+    out[4] = pair_stride(out[3], (int)out[2]);
+    out[5] = (d.pnc + (1 << pcl) - 1) >> pcl;
+    return GI_OK;
+}
+
+extern "C" int gi_debug_pair_task(int n, int pcl, int potential, long long task, long long out[5])
+{
+    if (!out) return fail(GI_ERR_INVALID_ARG, "out is NULL");
+    if (n <= 0 || task < 0) return fail(GI_ERR_BAD_SIZE, "n = %d, task = %lld", n, task);
+    if (pcl > log2_floor(gi::kPairMaxCpi)) return fail(GI_ERR_INVALID_ARG, "pcl = %d", pcl);
+    RunDev d;
+    std::memset(&d, 0, sizeof d);
+    PairDev p;
+    std::memset(&p, 0, sizeof p);
+    p.gm_fe = p.gm_si = 1.0f;
+    if (pcl < 0) pcl = potential ? gi_internal_potential_pcl(n) : gi_internal_pair_default_pcl(n);
+    gi_internal_pair_run(d, n, pcl, p, 0, potential ? 3 : 0);
+    int row = 0, c0 = 0, c1 = 0;
+    out[0] = gi_pair_task(d, task, &row, &c0, &c1);
+    if (task >= out[0]) return fail(GI_ERR_BAD_SIZE, "task %lld of %lld", task, out[0]);
+    out[1] = row;
+    out[2] = 32 << d.pipl;
+    out[3] = c0;
+    out[4] = c1;
     return GI_OK;
 }
 
@@ -1497,16 +1528,10 @@ extern "C" int gi_potential_fp64(gi_ctx *c, const float *pos, const gi_run *runs
                     blocks += tiles * tiles;
                     continue;
                 }
-                // the far field's items, all rows eight to a lane, and fewer chunks
-                // each: without per-body sums a short item costs no atomics, and
-                // the last ones leave less of the GPU idle.  us an energy log
-                // (diagnostics and potential) at the far field's chunks, half and a
-                // quarter of them: 20,000 bodies 259, 241, 225; 33,000 446, 438,
-                // 397; 66,000 1,211, 1,139, 1,151; 130,000 3,825, 3,817, 3,933.
-                const int pcl = gi_internal_pair_default_pcl(d.n) - (d.n < 65536 ? 2 : 1);
                 // From 262,000 bodies on a warp takes several tasks: one partial each
                 // would come to 41 MB at 1.15M bodies and grow with n^2.
-                const long long tasks = gi_internal_pair_run(d, d.n, pcl, pd[d.param], partials, 3);
+                const long long tasks =
+                    gi_internal_pair_run(d, d.n, gi_internal_potential_pcl(d.n), pd[d.param], partials, 3);
                 d.nsplit = (int)std::min(tasks, (long long)kPotentialPartials);
                 partials += d.nsplit;
             }

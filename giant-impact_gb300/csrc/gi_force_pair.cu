@@ -83,7 +83,7 @@
 
 namespace gi {
 
-__device__ __forceinline__ long long pair_items_before(long long a, long long k0, long long q)
+__host__ __device__ __forceinline__ long long pair_items_before(long long a, long long k0, long long q)
 {
     return a * k0 - q * ((a * (a - 1)) / 2);
 }
@@ -296,24 +296,38 @@ __device__ __forceinline__ void pair_task(PairSmem &sm, const ForceArgs &a, cons
 
 // Warp `part` of item t of run R: its first row wi0 and its chunks [c0, c1) (none
 // when they are all before the rows, or there are no rows).
-__device__ __forceinline__ void pair_place(const RunDev &R, long long t, int part, int &wi0, int &c0,
-                                           int &c1)
+__host__ __device__ __forceinline__ void pair_place(const RunDev &R, long long t, int part, int &wi0,
+                                                    int &c0, int &c1)
 {
     // (i-block, item of the block), then rows and chunks of the item
-    const int rlog = kPairRowsLog2 - 5 - R.pipl;  // log2 of the row groups of an i-block
-    const long long k0 = R.pk0, q = kPairBlockChunks >> R.pcl;
+    const int rlog = R.pblk + 1 - R.pipl;  // log2 of the row groups of an i-block
+    const long long k0 = R.pk0, q = 1 << (R.pblk - R.pcl);
     int lo = 0, hi = R.pnb - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (pair_items_before(mid, k0, q) <= t) lo = mid;
         else hi = mid - 1;
     }
-    wi0 = lo * kPairRows + ((part & ((1 << rlog) - 1)) << (5 + R.pipl));
+    wi0 = (lo << R.pblk) * kPairChunk + ((part & ((1 << rlog) - 1)) << (5 + R.pipl));
     const int cpt = 1 << (R.pcl - (R.ptpi - rlog));  // chunks of this warp
-    const int cb = lo * kPairBlockChunks + ((int)(t - pair_items_before(lo, k0, q)) << R.pcl) +
+    const int cb = (lo << R.pblk) + ((int)(t - pair_items_before(lo, k0, q)) << R.pcl) +
                    (part >> rlog) * cpt;
     c0 = max(cb, wi0 / kPairChunk);
     c1 = min(cb + cpt, R.pnc);
+}
+
+// Task k of the run's items << ptpi, in 64 bits.
+__host__ __device__ __forceinline__ unsigned long long pair_items_of(const RunDev &R)
+{
+    return pair_items_before(R.pnb, R.pk0, 1 << (R.pblk - R.pcl));
+}
+
+__host__ __device__ __forceinline__ void pair_task_place(const RunDev &R, unsigned long long k,
+                                                         unsigned long long items, int &wi0, int &c0,
+                                                         int &c1)
+{
+    pair_place(R, (long long)(((k >> R.ptpi) * R.pstride) % items), (int)k & ((1 << R.ptpi) - 1), wi0, c0,
+               c1);
 }
 
 // CTA `cta` of run R, likewise.
@@ -631,10 +645,9 @@ potential_kernel(const float4 *__restrict__ pos, const __grid_constant__ LaunchT
     int wi0, c0, c1;
     double acc = 0.0;
     if (MANY) {
-        const unsigned long long items = pair_items_before(R.pnb, R.pk0, kPairBlockChunks >> R.pcl);
+        const unsigned long long items = pair_items_of(R);
         for (unsigned long long k = blockIdx.x - R.item_start; k < items << R.ptpi; k += R.nsplit) {
-            pair_place(R, (long long)(((k >> R.ptpi) * R.pstride) % items), (int)k & ((1 << R.ptpi) - 1),
-                       wi0, c0, c1);
+            pair_task_place(R, k, items, wi0, c0, c1);
             potential_task(sm, run, R, P, wi0, c0, c1, lane, acc);
         }
     } else {
@@ -697,6 +710,13 @@ __global__ void __launch_bounds__(256) pair_finish_kernel(const ForceArgs a,
 }  // namespace gi
 
 using namespace gi;
+
+long long gi_pair_task(const RunDev &R, long long task, int *row, int *c0, int *c1)
+{
+    const unsigned long long items = pair_items_of(R);
+    pair_task_place(R, (unsigned long long)task, items, *row, *c0, *c1);
+    return (long long)(items << R.ptpi);
+}
 
 cudaError_t gi_pair_setup() { return gi_full_carveout(reinterpret_cast<const void *>(pair_force_kernel)); }
 

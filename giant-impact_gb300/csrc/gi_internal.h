@@ -55,9 +55,10 @@ struct RunDev {
     float dt, dtm_fe, dtm_si, damp;
     int ipt;          // i-bodies per thread this run was planned for
     // GI_ACC_PAIRED decomposition (gi_force_pair.cu)
+    int pblk;         // log2 of the chunks (of rows) in an i-block
     int pcl;          // log2 of the j-chunks per work item
     int pnc;          // j-chunks of the run, ceil(n / kPairChunk)
-    int pnb;          // i-blocks of the run, ceil(n / kPairRows)
+    int pnb;          // i-blocks of the run, ceil(pnc / 2^pblk)
     int pk0;          // work items of i-block 0, ceil(pnc / 2^pcl)
     int pitems;       // work items of the run
     int pstride;      // item slot t of the run is item (t * pstride) mod pitems (coprime)
@@ -119,7 +120,8 @@ constexpr int kPairIpl = 8;                               // i-bodies per lane, 
 constexpr int kPairWarpRows = 32 * kPairIpl;              // 256 rows per warp, at most
 constexpr int kPairRowsLog2 = 10;
 constexpr int kPairRows = 1 << kPairRowsLog2;             // 1024: the i-block
-constexpr int kPairChunk = 64;                            // j-chunk: two bodies per lane
+constexpr int kPairChunkLog2 = 6;
+constexpr int kPairChunk = 1 << kPairChunkLog2;           // 64, the j-chunk: two bodies per lane
 constexpr int kPairBlockChunks = kPairRows / kPairChunk;  // 16
 constexpr int kPairMaxCpi = 16;                           // j-chunks per work item, at most
 constexpr int kPairStage = 8;                             // chunks staged at a time (8 KB)
@@ -140,6 +142,9 @@ cudaError_t gi_launch_pair_force(const ForceArgs &a, const LaunchTable &tab, con
 constexpr int kPotentialPartials = 262144;  // of a run, at most (2 MB)
 cudaError_t gi_launch_potential(const float4 *pos, const LaunchTable &tab, double *partials,
                                 double *out, cudaStream_t s);
+// The kernels' own decode of a task (CTA) of a run planned by gi_internal_pair_run: its
+// first row and chunks [c0, c1); returns the run's tasks.
+long long gi_pair_task(const RunDev &R, long long task, int *row, int *c0, int *c1);
 cudaError_t gi_launch_pair_finish(int epi, const ForceArgs &a, const LaunchTable &tab, int maxn,
                                   int nsm, bool early, cudaStream_t s);
 
@@ -344,6 +349,8 @@ long long gi_internal_pair_run(RunDev &d, int n, int pcl, const PairDev &p, long
                                int ipl = 0);
 // log2 of the j-chunks per item of a run of n bodies without a tuning table.
 int gi_internal_pair_default_pcl(int n);
+// The same of the potential (gi_potential_fp64), all rows eight to a lane.
+int gi_internal_potential_pcl(int n);
 // Device ordinal of a context (-1 for NULL).
 int gi_internal_ctx_device(gi_ctx *ctx);
 // The context's workspace of at least `bytes` device bytes (16-byte aligned)

@@ -217,6 +217,7 @@ _SIGS = {
     "gi_measure_ffma_peak": ([C.c_int, C.POINTER(C.c_double)], C.c_int),
     "gi_debug_fill_counters": ([_P, _P, C.c_uint], C.c_int),
     "gi_debug_pair_plan": ([_P, C.c_int, C.c_int, C.POINTER(C.c_longlong)], C.c_int),
+    "gi_debug_pair_task": ([C.c_int, C.c_int, C.c_int, C.c_longlong, C.POINTER(C.c_longlong)], C.c_int),
     "gi_debug_contact_plan": ([C.POINTER(C.c_int), C.c_int, C.POINTER(C.c_int)], C.c_int),
     "gi_server_create": ([C.c_int, C.POINTER(ServerConfig), C.POINTER(PairParams), C.c_int,
                           C.POINTER(_P)], C.c_int),
@@ -334,6 +335,25 @@ def pair_plan(n: int, pcl: int = -1, ctx=None) -> dict:
     check(lib().gi_debug_pair_plan(ctx.h if ctx is not None else None, n, pcl, out))
     return {"pcl": out[0], "chunks": out[1], "iblocks": out[2], "items": out[3],
             "stride": out[4], "items_block0": out[5]}
+
+
+def pair_task_count(n: int, pcl: int = -1, potential: bool = False) -> int:
+    """Warps (CTAs) of the far field's, or the potential's, decomposition of a run."""
+    out = (C.c_longlong * 5)()
+    check(lib().gi_debug_pair_task(n, pcl, int(potential), 0, out))
+    return out[0]
+
+
+def pair_task(n: int, pcl: int, potential: bool, task: int) -> tuple[int, int, int, int]:
+    """(first row, rows, first j-chunk, end of the j-chunks) of one of them, as the
+    kernel decodes it; usable without a GPU."""
+    out = (C.c_longlong * 5)()
+    check(lib().gi_debug_pair_task(n, pcl, int(potential), task, out))
+    return tuple(out[1:])
+
+
+def pair_tasks(n: int, pcl: int = -1, potential: bool = False) -> list[tuple[int, int, int, int]]:
+    return [pair_task(n, pcl, potential, k) for k in range(pair_task_count(n, pcl, potential))]
 
 
 def contact_plan(sizes) -> list[int]:

@@ -364,6 +364,12 @@ int gi_debug_fill_counters(gi_ctx *ctx, void *stream, unsigned int value);
  * permutation, items of i-block 0}. */
 int gi_debug_pair_plan(gi_ctx *ctx, int n, int pcl, long long out[6]);
 
+/* Test hook: one warp's task of that decomposition as the kernel decodes it, of
+ * the far field or of the potential's warps (pcl < 0: the default); host
+ * arithmetic only.  out[5] = {tasks of the run, first row, rows, first j-chunk,
+ * end of the j-chunks (not after the first: none)}. */
+int gi_debug_pair_task(int n, int pcl, int potential, long long task, long long out[5]);
+
 /* Test hook: buckets of the contact pass's cell grid for each of up to 64 runs
  * of n[k] bodies in one call (0: every body of the run is a candidate); host
  * arithmetic only. */
