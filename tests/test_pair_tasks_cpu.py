@@ -1,6 +1,7 @@
 """The far field's CTAs as the kernel decodes them, on the host (no GPU):
 gi_debug_pair_task runs the kernel's own decode of one CTA of a run.  Every
-unordered pair must be some warp's exactly once."""
+unordered pair must be some warp's exactly once, and no warp of the far field's
+finer split may be without pairs."""
 from __future__ import annotations
 
 import numpy as np
@@ -13,22 +14,26 @@ def _cover(gi, n, pcl, potential):
     """How often each pair i < j is evaluated: a warp has rows r0 .. r0 + rows and the
     chunks [c0, c1); it keeps i < j, and no chunk that ends before its rows."""
     count = np.zeros((n, n), np.uint8)
-    for r0, rows, c0, c1 in gi.pair_tasks(n, pcl, potential):
+    tasks, empty = gi.pair_tasks(n, pcl, potential), 0
+    for r0, rows, c0, c1 in tasks:
         assert r0 % rows == 0
+        empty += c0 >= c1
         i, j = np.arange(r0, min(r0 + rows, n)), np.arange(c0 * CHUNK, min(c1 * CHUNK, n))
         if len(i) and len(j):
             assert c0 * CHUNK >= r0  # the kernel's diagonal rule covers the rest
             count[np.ix_(i, j)] += (i[:, None] < j[None, :]).astype(np.uint8)
-    return count
+    return count, tasks, empty
 
 
 @pytest.mark.parametrize("potential", [False, True])
 @pytest.mark.parametrize("pcl", [-1, 0, 2, 4])
 @pytest.mark.parametrize("n", [1, 64, 65, 129, 1000, 1025, 2049, 3072, 3073, 4000, 6145])
 def test_every_pair_once(gi, n, pcl, potential):
-    count = _cover(gi, n, pcl, potential)
+    count, tasks, empty = _cover(gi, n, pcl, potential)
     upper = np.triu(np.ones((n, n), bool), 1)
     assert (count[upper] == 1).all() and (count[~upper] == 0).all()
+    if pcl < 0 and not potential:
+        assert empty == 0
 
 
 @pytest.mark.parametrize("n", [12287, 12288, 20011, 32767, 32768, 65535, 65536, 131072])
