@@ -17,6 +17,10 @@ int gi_force_occupancy_ipt1(int acc, int epi);
 int gi_force_occupancy_ipt2(int acc, int epi);
 int gi_force_occupancy_ipt4(int acc, int epi);
 int gi_force_occupancy_ipt8(int acc, int epi);
+cudaError_t gi_force_carveout_ipt1(int acc);
+cudaError_t gi_force_carveout_ipt2(int acc);
+cudaError_t gi_force_carveout_ipt4(int acc);
+cudaError_t gi_force_carveout_ipt8(int acc);
 
 // ------------------------------------------------------------------ errors --
 
@@ -104,6 +108,17 @@ int gi_force_occupancy(int ipt, int acc, int epi)
     case 4: return gi_force_occupancy_ipt4(acc, epi);
     case 8: return gi_force_occupancy_ipt8(acc, epi);
     default: return 0;
+    }
+}
+
+cudaError_t gi_force_carveout(int ipt, int acc)
+{
+    switch (ipt) {
+    case 1: return gi_force_carveout_ipt1(acc);
+    case 2: return gi_force_carveout_ipt2(acc);
+    case 4: return gi_force_carveout_ipt4(acc);
+    case 8: return gi_force_carveout_ipt8(acc);
+    default: return cudaErrorInvalidValue;
     }
 }
 
@@ -295,7 +310,9 @@ struct gi_ctx {
     void *work = nullptr;     // workspace of the synchronous calls (gi_internal_ctx_workspace)
     void *work_pinned = nullptr;
     size_t work_cap = 0;
-    int cluster_ctas = 0;     // largest cluster of the grid build (gi_grid_cluster_ctas)
+    int cluster_ctas = 8;     // largest cluster of the grid build (gi_grid_cluster_ctas)
+    bool cluster_asked = false;
+    bool carved[4][9] = {};   // gi_force_carveout done: [accum][i-bodies per thread]
     int occ[4][9];  // resident one-sided force CTAs per SM: [accum][i-bodies per thread]
 };
 
@@ -312,7 +329,6 @@ static int ctx_init(gi_ctx *c, int device)
                     device, prop.major, prop.minor);
     c->sm_count = prop.multiProcessorCount;
     DeviceGuard g(device);
-    c->cluster_ctas = gi_grid_cluster_ctas();
     GI_CUDA(gi_pair_setup(), "cudaFuncSetAttribute");
     GI_CUDA(gi_contact_setup(), "cudaFuncSetAttribute");
     c->diag_blocks = gi_diag_blocks(c->sm_count);  // shared by the two material classes
@@ -1014,6 +1030,10 @@ static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi
         unsigned int *const ctr =
             reinterpret_cast<unsigned int *>(x->fsum + 3 * (size_t)plan.max_end);
         const GridWork gw(x->grid_work, plan.bodies[t], plan.max_end);
+        if (tab.gridn >= gi::kClusterSmallMax && !c->cluster_asked) {
+            c->cluster_ctas = gi_grid_cluster_ctas();
+            c->cluster_asked = true;
+        }
         if (plan.paired) {
             // The far-field sums and the contact pass's counters start at zero.
             a.fsum_fx = reinterpret_cast<long long *>(x->fsum);
@@ -1063,6 +1083,10 @@ static int run_force_plan(gi_ctx *c, StreamScratch *x, const Plan &plan, int epi
         x->always_clear |= call->capturing;
         const int p = plan.ipt[t];
         const int occ = c->occ[c->opt.accum][p];
+        if (!c->carved[c->opt.accum][p]) {
+            GI_CUDA(gi_force_carveout(p, c->opt.accum), "cudaFuncSetAttribute");
+            c->carved[c->opt.accum][p] = true;
+        }
         // The queue and this table's tickets start at zero (the kernel also
         // re-arms them on the way out; this covers a launch that never got
         // there).  Captured with the launch when the stream is capturing.

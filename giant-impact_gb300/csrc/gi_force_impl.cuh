@@ -376,19 +376,32 @@ cudaError_t launch_force_ipt(int acc, int epi, const ForceArgs &a, const LaunchT
     return cudaErrorInvalidValue;
 }
 
-// Also sets the kernel up in the current CUDA context: the contact kernels share
-// its SMs (GI_EPI_SUM).
+// gi_full_carveout of the three kernels of an accumulation mode: the contact kernels
+// share their SMs (GI_EPI_SUM).
+template <int IPT>
+cudaError_t carveout_ipt(int acc)
+{
+    cudaError_t e = cudaErrorInvalidValue;
+#define GI_CARVE(A, E)                                                                    \
+    if (acc == A && (e == cudaSuccess || E == GI_EPI_FORCE))                              \
+        e = gi_full_carveout(reinterpret_cast<const void *>(force_kernel<IPT, A, E>));
+#define GI_CARVE3(A) GI_CARVE(A, GI_EPI_FORCE) GI_CARVE(A, GI_EPI_STEP) GI_CARVE(A, GI_EPI_SUM)
+    GI_CARVE3(GI_ACC_KAHAN)
+    GI_CARVE3(GI_ACC_FP32)
+    GI_CARVE3(GI_ACC_FP64)
+#undef GI_CARVE3
+#undef GI_CARVE
+    return e;
+}
+
 template <int IPT>
 int occupancy_ipt(int acc, int epi)
 {
     int nb = 0;
     cudaError_t e = cudaErrorInvalidValue;
 #define GI_OCC(A, E)                                                              \
-    if (acc == A && epi == E) {                                                   \
-        e = gi_full_carveout(reinterpret_cast<const void *>(force_kernel<IPT, A, E>)); \
-        if (e == cudaSuccess)                                                     \
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, force_kernel<IPT, A, E>, GI_NT, 0); \
-    }
+    if (acc == A && epi == E)                                                     \
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, force_kernel<IPT, A, E>, GI_NT, 0);
     GI_OCC(GI_ACC_KAHAN, GI_EPI_FORCE)
     GI_OCC(GI_ACC_KAHAN, GI_EPI_STEP)
     GI_OCC(GI_ACC_FP32, GI_EPI_FORCE)

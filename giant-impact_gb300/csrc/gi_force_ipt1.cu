@@ -11,6 +11,7 @@ cudaError_t gi_launch_force_ipt1(int acc, int epi, const ForceArgs &a,
 }
 
 int gi_force_occupancy_ipt1(int acc, int epi) { return gi::occupancy_ipt<1>(acc, epi); }
+cudaError_t gi_force_carveout_ipt1(int acc) { return gi::carveout_ipt<1>(acc); }
 
 cudaError_t gi_launch_finish(int epi, const ForceArgs &a, const LaunchTable &tab, int maxn,
                              int nsm, cudaStream_t s)

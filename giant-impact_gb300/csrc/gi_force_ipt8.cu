@@ -8,3 +8,4 @@ cudaError_t gi_launch_force_ipt8(int acc, int epi, const ForceArgs &a,
 }
 
 int gi_force_occupancy_ipt8(int acc, int epi) { return gi::occupancy_ipt<8>(acc, epi); }
+cudaError_t gi_force_carveout_ipt8(int acc) { return gi::carveout_ipt<8>(acc); }

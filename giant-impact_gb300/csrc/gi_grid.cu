@@ -297,7 +297,7 @@ __device__ __forceinline__ void dense_items(const Torus &T, const GridWork &g, u
 // buckets.)
 constexpr int kClusterItems = 8;  // bodies per thread, at most
 constexpr int kClusterSmall = 8, kClusterLarge = 16;
-constexpr int kClusterSmallMax = kClusterSmall * 1024 * kClusterItems;  // 65,536
+static_assert(kClusterSmallMax == kClusterSmall * 1024 * kClusterItems, "runs of the small cluster");
 constexpr int kClusterMax = kClusterLarge * 1024 * kClusterItems;       // 131,072
 
 // Counters of a run's crowded buckets, in the cluster's first CTA.

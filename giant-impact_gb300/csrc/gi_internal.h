@@ -108,6 +108,7 @@ cudaError_t gi_launch_force_ipt4(int acc, int epi, const ForceArgs &a, const Lau
 cudaError_t gi_launch_force_ipt8(int acc, int epi, const ForceArgs &a, const LaunchTable &tab, int grid, cudaStream_t s);
 // Resident CTAs per SM of a force kernel instance (for the planner).
 int gi_force_occupancy(int ipt, int acc, int epi);
+cudaError_t gi_force_carveout(int ipt, int acc);
 // The epilogue of a GI_EPI_SUM launch (epi = GI_EPI_FORCE or GI_EPI_STEP):
 // adds the contact corrections and stores or steps, one thread per body.
 cudaError_t gi_launch_finish(int epi, const ForceArgs &a, const LaunchTable &tab, int maxn,
@@ -179,6 +180,8 @@ constexpr int kCtrWords = 4 + 2 * (int)kItemClasses + GI_MAX_RUNS / 32;
 // 66, 24 of 1,000 60 / 78, eight of 2,000 72 / 86, 24 of 2,000 182 / 128.
 constexpr int kDirectMax = 4096, kDirectAlways = 512;
 constexpr long long kDirectCandidates = 3500 * 3500, kDirectCandidatesOneSided = 40000000;
+// Runs below it have their grid built by a cluster of 8 CTAs, larger ones by 16.
+constexpr int kClusterSmallMax = 65536;
 // Bodies of a row-path CTA (one warp), of a run with a grid and without.
 constexpr int kRowBodies = 8, kDirectBodies = 2;
 }  // namespace gi
@@ -308,8 +311,9 @@ inline cudaError_t gi_full_carveout(const void *kernel)
     return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 cudaSharedmemCarveoutMaxShared);
 }
-// That for the paired far field's kernel and for the contact kernels; a gi_ctx
-// does it when it is created (it is gone with cudaDeviceReset).
+// That for the paired far field's kernel and for the contact kernels; a gi_ctx does
+// it when it is created, and gi_force_carveout and gi_grid_cluster_ctas when a call
+// first needs them (it is gone with cudaDeviceReset).
 cudaError_t gi_pair_setup();
 cudaError_t gi_contact_setup();
 
