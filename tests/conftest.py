@@ -54,6 +54,17 @@ def orc(built):
     return oracle
 
 
+# Tests that run the reference's own kernels to the end, and so have nothing to
+# compare with where those could not be built.
+NEEDS_REFERENCE_KERNELS = {"test_config1_trajectory_against_fp64_and_reference"}
+
+
+@pytest.hookimpl(tryfirst=True)
+def pytest_runtest_call(item):
+    if item.originalname in NEEDS_REFERENCE_KERNELS and item.funcargs["orc"].ref_lib() is None:
+        pytest.skip("reference kernels not built (oracle/_ref absent)")
+
+
 @pytest.fixture(scope="session")
 def torch_cuda():
     import torch
