@@ -1518,8 +1518,12 @@ extern "C" int gi_diag_fp64(gi_ctx *c, const float *pos, const float *vel,
                 "diag launch");
         GI_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
         if (diag_exact(c->diag_host)) break;
-        origin.given = true;
-        for (int d = 0; d < 6; ++d) origin.x[d] = (float)c->diag_host[1 + d];
+        DiagOrigin centre{};
+        centre.given = true;
+        for (int d = 0; d < 6; ++d)  // one that is not finite counts as 0
+            centre.x[d] = std::isfinite((float)c->diag_host[1 + d]) ? (float)c->diag_host[1 + d] : 0.0f;
+        if (origin.given && std::equal(centre.x, centre.x + 6, origin.x)) break;  // nothing left to gain
+        origin = centre;
     }
     std::memcpy(out, c->diag_host, 15 * sizeof(double));
     return GI_OK;
