@@ -170,16 +170,17 @@ constexpr unsigned int kItemClasses = 16;
 constexpr int kCtrWords = 4 + 2 * (int)kItemClasses + GI_MAX_RUNS / 32;
 // Runs of at most kDirectMax bodies take no grid (every body of the run is a
 // candidate) where all such runs of a table together have at most kDirectCandidates
-// candidates (one run of 3,500); in fuller tables those of at most kDirectAlways.
-// The candidates of a full GPU cost more than a grid build, whose launches are what
-// a lone short run spends its step on.  us a step of settled bodies, without a grid /
-// with one: one run of 2,000 13 / 33, 3,000 26 / 30, 4,000 40 / 31; two of 3,000 41 /
-// 32; eight of 1,000 28 / 30, 2,000 72 / 52; 24 of 500 27 / 39, 1,000 65 / 56, 2,000
-// 200 / 102; 64 of 500 60 / 79, 1,000 160 / 95, 4,000 1,757 / 480.  Beside the
-// one-sided far field, where the grid-wide kernels build the grid: one of 4,000 41 /
-// 66, 24 of 1,000 60 / 78, eight of 2,000 72 / 86, 24 of 2,000 182 / 128.
+// candidates, one run of 3,648, whose row CTAs are what the GPU holds at once; in
+// fuller tables those of at most kDirectAlways.  The candidates of a full GPU cost
+// more than a grid build, whose launches are what a lone short run spends its step
+// on.  us a step of settled bodies, without a grid / with one: one run of 2,000 13 /
+// 33, 3,000 26 / 30, 3,600 35 / 30 (a remnant 64 / 75), 4,000 40 / 30 (101 / 81); two
+// of 3,000 41 / 32; eight of 1,000 28 / 30, 2,000 72 / 52; 24 of 500 27 / 39, 1,000 65
+// / 56, 2,000 200 / 102; 64 of 500 60 / 79, 1,000 160 / 95, 4,000 1,757 / 480.  Beside
+// the one-sided far field, where the grid-wide kernels build the grid: one of 4,000
+// 41 / 66, 24 of 1,000 60 / 78, eight of 2,000 72 / 86, 24 of 2,000 182 / 128.
 constexpr int kDirectMax = 4096, kDirectAlways = 512;
-constexpr long long kDirectCandidates = 3500 * 3500, kDirectCandidatesOneSided = 40000000;
+constexpr long long kDirectCandidates = 3648 * 3648, kDirectCandidatesOneSided = 40000000;
 // Runs below it have their grid built by a cluster of 8 CTAs, larger ones by 16.
 constexpr int kClusterSmallMax = 65536;
 // Bodies of a row-path CTA (one warp), of a run with a grid and without.

@@ -11,7 +11,7 @@ from test_gpu_contact_paths import _dev
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("sizes", [[3501], [4097], [5477], [3400, 3400], [700] * 20, [1500, 5000],
+@pytest.mark.parametrize("sizes", [[3649], [4097], [5477], [3400, 3400], [700] * 20, [1500, 5000],
                                    [2000] * 64 + [300] * 6, [300] * 64 + [9000] * 3])
 def test_graph_matches_eager_steps(gi, torch_cuda, sizes):
     """Eight steps by two launches of a four-step graph, an eager call between them,
