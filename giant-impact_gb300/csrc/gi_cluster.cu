@@ -368,7 +368,7 @@ cluster_link(const float4 *__restrict__ list, CellTable tab, const CellInfo *__r
 // The same for many bodies, whose table is larger than L2: there a cell costs its
 // chain of dependent loads from memory, and most of a sparse state's cells hold one
 // body among empty neighbours.  So the chain is made short and taken once: the
-// filter, a sixteenth of the table, says from L2 which neighbours are empty; all 62
+// filter, a byte for each slot's 28, says from L2 which neighbours are empty; all 62
 // are looked up before any is linked, two to a lane, their first probes together;
 // one or two pairs are tested sooner than two trees are climbed; and a cell of at
 // most kFew bodies takes its near and far neighbours in the first launch.  Grouping

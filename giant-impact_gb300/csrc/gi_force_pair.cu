@@ -34,7 +34,9 @@
 // slot t of a run is item (t * stride) mod items, the stride coprime with the
 // item count and about one i-block's items long: warps resident together then
 // hold different i-blocks, so their i-side atomics do not queue on the same
-// addresses.
+// addresses.  Where cpt chunks are no more than a warp's rows (runs below 65,536
+// bodies at the default) the i-block is the row group and the item its cpt chunks:
+// the same warps, without those that would skip all their chunks.
 //
 // Inner loop (per warp and chunk): the chunk is staged in shared memory as
 // (x_a, x_b, y_a, y_b) and (z_a, z_b, gm_a, gm_b) of slots a = l, b = l + 32,

@@ -14,7 +14,7 @@
 // For them, gi_forces_collision_noalloc computes the same forces, bit for bit
 // (the same kernels with the same default decomposition), with all of its
 // scratch in one statically allocated device array, g_noalloc_scratch, of
-// GI_NOALLOC_BYTES (8 MiB; the largest run takes 5.6 MiB of it).  Every GPU
+// GI_NOALLOC_BYTES (8 MiB; the largest run takes 5.4 MiB of it).  Every GPU
 // that loads the library holds that array until the process exits.  The array
 // limits a call to GI_NOALLOC_MAX_BODIES (32,768) bodies; larger calls are
 // refused.
